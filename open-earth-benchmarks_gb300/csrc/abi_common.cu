@@ -13,6 +13,7 @@
 
 #include "oeb_common.cuh"
 #include "launch.cuh"
+#include "march.cuh"
 #include "stage.cuh"
 
 namespace oeb {
@@ -102,7 +103,8 @@ constexpr int kMaxDevices = 64;
 std::atomic<int> g_sms[kMaxDevices];
 }  // namespace
 
-int staged_kb(int tiles, int nz, int ctas_per_sm) {
+namespace {
+int device_sms() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
   int sms = dev < kMaxDevices ? g_sms[dev].load(std::memory_order_relaxed) : 0;
@@ -110,6 +112,12 @@ int staged_kb(int tiles, int nz, int ctas_per_sm) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
     if (dev < kMaxDevices) g_sms[dev].store(sms, std::memory_order_relaxed);
   }
+  return sms;
+}
+}  // namespace
+
+int staged_kb(int tiles, int nz, int ctas_per_sm) {
+  const int sms = device_sms();
   // the most k-chunks per tile that still fit every CTA into one wave, then levels per chunk
   const long slots = (long)sms * (ctas_per_sm > 0 ? ctas_per_sm : 1);
   long chunks = tiles > 0 ? slots / tiles : 1;
@@ -117,6 +125,34 @@ int staged_kb(int tiles, int nz, int ctas_per_sm) {
   if (chunks > nz) chunks = nz;
   const long kb = (nz + chunks - 1) / (chunks > 0 ? chunks : 1);
   return (int)(kb < 1 ? 1 : kb);
+}
+
+// A chunk of R rows marches R + apron, and about three rows' time passes before its first row's
+// loads have landed; a launch takes at least one wave of CTAs' time.  The split with the least
+// product of the two wins: fvtp2d (apron 5, three CTAs an SM) measured best with 32 rows at
+// 256 x 256 x 80 (89.7 us; 16 rows 93.9, 12 rows 101.7, 8 rows 102.7, 64 rows 113) and with 16 at
+// 128 x 128 x 80 (28.1 us; 8 rows 32.5, 22 rows 31.1, 32 rows 36.6), as the product says, which is
+// taken over at most 32 rows.
+MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm) {
+  const double slots = (double)device_sms() * ctas_per_sm;
+  const int strips = (nx + cols - 1) / cols, levels = (nz + kb - 1) / kb;
+  MarchShape best{};
+  double least = 0.0;
+  for (int wl = 0; wl <= 3; ++wl) {
+    const int wx = 1 << wl, wy = kTY >> wl;
+    for (int rows = 4; rows <= 32; ++rows) {
+      const int chunks = (ny + rows - 1) / rows;
+      const dim3 grid((unsigned)((strips + wx - 1) / wx), (unsigned)((chunks + wy - 1) / wy), (unsigned)levels);
+      const double waves = (double)grid.x * grid.y * grid.z / slots;
+      const double cost = (waves > 1.0 ? waves : 1.0) * (rows + apron + 3);
+      if (best.rows == 0 || cost < least) {
+        least = cost;
+        best = MarchShape{rows, wl, grid};
+      }
+      if (rows >= ny) break;
+    }
+  }
+  return best;
 }
 
 Recorder* recorder() { return t_recorder; }

@@ -10,8 +10,8 @@
 //                   transport fluxes fx1 = (fx1+fx2)/2 * xfx, fy1 = (fy1+fy2)/2 * yfx (:160-176).
 // q_i, q_j, fx2 and fy2 are outputs of the reference signature; launch 2 reads them back
 // from global memory (the FP64 pipe, not HBM, bounds this kernel, so storing them costs
-// less than recomputing their aprons).  FP32, bound by memory instead, runs one launch that
-// recomputes the aprons (fvtp2d_fused_kernel).
+// less than recomputing their aprons).  FP32 runs one launch that reads nothing back
+// (fvtp2d_march_f32).
 //
 // Compiled with --fmad=false (see k_pointwise.cu).  In FP32 the monotonicity flag smt5 is decided
 // on the exact product (precision.cuh).
@@ -19,7 +19,7 @@
 
 #include "oeb_reach.cuh"
 #include "precision.cuh"
-#include "stage.cuh"
+#include "march.cuh"
 #include "stencil_util.cuh"
 #include "tangent.cuh"
 
@@ -336,211 +336,162 @@ inline dim3 flux_grid(const Dims& d, int kb) {
   return g;
 }
 
-// ------------------------------ FP32: one launch -------------------------------------
-// The FP32 call is bound by memory, and the two launches above move 2.1x its algorithmic
-// bytes: launch 2 reads back q_i, q_j, fx2 and fy2, which launch 1 has just written.  Here one
-// CTA per interior 32 x 32 tile and k-level does both sweeps of q over a 3-cell apron, in
-// shared memory, and then the sweeps of q_i and q_j: nothing it writes is read back.
-//   y pass of q on the columns [i0-3, i0+34): fy2 on rows [j0, j0+33), q_i on [j0, j0+32);
-//   x pass of q on the rows [j0-3, j0+34): fx2 on columns [i0, i0+33), q_j on [i0, i0+32);
-//   x-PPM of q_i and y-PPM of q_j on the tile: fx1 and fy1.
-// The apron costs about 16 % more PPM arithmetic than the two launches.  Each value of q_i,
-// q_j, fx2 and fy2 is written by the one tile that owns it: its own columns (rows), plus the
-// three before the first tile and the extra ones after the last (those arrays' boxes reach
-// 3 cells before the interior and 1 or 2 after it).  The arithmetic is launch 1's and launch
-// 2's, operation for operation, so the results are the same bits.
-// Shared layout (per k-level), tile origin (i0, j0), 37 = the apron width:
-//   q    : 39 x 39, (i0-3+a, j0-3+b)
-//   y pass (columns i0-3+a, a < 37): ya = al on rows j0-1+b (35), then fyy on rows j0+b (33);
-//          ym, yr, ys = almq, br, smt5 on rows j0-1+b (34); qi on rows j0+b (32)
-//   x pass (rows j0-3+b, b < 37): xa = al on columns i0-1+a (35), then fxx on i0+a (33);
-//          xm, xr, xs on columns i0-1+a (34); qj on columns i0+a (32)
-//   fx2c, fy2c: fx2 and fy2 on the tile (32 x 32)
-//   second stage, over the dead aux arrays: x-PPM of qi (al on i0-1+a, 34; aux 33) and
-//   y-PPM of qj (al on j0-1+b, 34; aux 33)
-template <class T>
-struct FvFusedSmem {
-  T q[39][39];
-  T ya[35][37];
-  T ym[34][37], yr[34][37];
-  unsigned char ys[34][37];
-  T qi[32][37];
-  T xa[37][35];
-  T xm[37][34], xr[37][34];
-  unsigned char xs[37][34];
-  T qj[37][32];
-  T fx2c[32][32], fy2c[32][32];
-};
+// ------------------------------ FP32: one marching launch ----------------------------
+// FP32 runs both sweeps of q and the sweeps of q_i and q_j in one launch of marching warps
+// (march.cuh): lane = column i0 - 3 + lane, 26 columns a strip (the x sweeps' shuffles consume an
+// apron of three lanes below and three above), rows from ja - 3 to jb + 2 of a chunk [ja, jb).
+// At iteration s a warp holds q on rows s .. s+3 and computes
+//   the y sweep's edge value at s+2, aux values and flux fy2 at s+1, and from it q_i at s;
+//   the x sweep of row s: fx2, and q_j at s;
+//   the x sweep of q_i's row s: fx1;    the y sweep of q_j: fy1 at row s - 2.
+// Every input is read once a warp, and q_i, q_j, fx2 and fy2 are never read back.  Each value is
+// written by the one warp that owns it: its own 26 columns and rows, plus the columns (rows)
+// before the first strip (chunk) and after the last.  The arithmetic is launch 1's and launch
+// 2's on the same operands in the same order: the same bits.
+//
+// What bounds it: instruction issue and the latency of its dependent chains (about 300
+// instructions a row of 26 columns, 110 of them the arithmetic; DRAM traffic 1.3x the outputs and
+// inputs once).  80 registers, three CTAs an SM: at 256 x 256 x 80 two CTAs (113 registers)
+// measured 106 us, four (64, spilling) 110, three 90; two rows unrolled 91.  Two levels a warp in
+// packed FP32 instructions (f32x2) took a quarter fewer instructions but 128 registers: 98 us.
+// The form before it, a 32 x 32 shared-memory tile in nine phases, took 180 us (56 against 28 us
+// at 128 x 128 x 80).
 
-// Asks L2 for the lines of field f (level offset kofs) that hold the cells [ilo, ihi) x
-// [jlo, jhi) (empty ranges ask nothing), spread over the CTA's threads; the ranges lie in the
-// field's reach.
-template <class T>
-__device__ __forceinline__ void prefetch_box(const T* f, int64_t kofs, int ilo, int ihi, int jlo, int jhi, int sj) {
-  if (ihi <= ilo || jhi <= jlo) return;
-  const uintptr_t first = reinterpret_cast<uintptr_t>(f + kofs + ilo) / 128;
-  const int lines = (int)((reinterpret_cast<uintptr_t>(f + kofs + ihi - 1) / 128) - first) + 1;
-  const int tid = threadIdx.y * kTX + threadIdx.x;
-  for (int e = tid; e < lines * (jhi - jlo); e += kThreads) {
-    const int r = e / lines, l = e - r * lines;
-    const T* row = f + kofs + (int64_t)(jlo + r) * sj;
-    const uintptr_t a = (reinterpret_cast<uintptr_t>(row + ilo) / 128 + l) * 128;
-    // the line's first cell of the range (clamped into it), so the address lies in the field
-    const uintptr_t lo = reinterpret_cast<uintptr_t>(row + ilo), hi = reinterpret_cast<uintptr_t>(row + ihi - 1);
-    prefetch_l2(reinterpret_cast<const void*>(a < lo ? lo : (a > hi ? hi : a)));
-  }
+// The aux values of one cell of a PPM sweep (fvtp2d.h:20-23).  a b < 0 is decided on the exact
+// product: with both factors scaled by 2^100 a nonzero product cannot underflow, one that overflows
+// keeps its sign, and 0 times an overflow is a NaN, which compares false as 0 does.
+struct PpmCell {
+  float m, r, b0;  // almq, br, b0
+  bool smt;
+};
+__device__ __forceinline__ PpmCell ppm_cell(float al0, float al1, float q0) {
+  constexpr float s = 1.2676506002282294e30f;
+  PpmCell c;
+  c.m = al0 - q0;
+  c.r = al1 - q0;
+  c.b0 = c.m + c.r;
+  c.smt = (c.m * s) * (c.r * s) < 0.f;
+  return c;
+}
+// The flux at a face (fvtp2d.h:28-34) from its upwind cell's values: ql, rl, bl of the cell below
+// the face, qh, mh, bh of the cell above it.  (1 - c) and (1 + c) are both 1 - |c|, and the
+// products with c both -(|c| b0), on the side that takes them.
+__device__ __forceinline__ float ppm_face(float c, float ql, float rl, float bl, float qh, float mh, float bh,
+                                          bool flag) {
+  const bool pos = c > 0.f;
+  const float n = neg_abs(c);
+  const float v = (pos ? rl : mh) + n * (pos ? bl : bh);
+  return fmaf((1.f + n) * v, flag ? 1.f : 0.f, pos ? ql : qh);
 }
 
-template <class T>
-struct fvtp2d_fused_kernel {
-  static constexpr int kStepOp = step_op<T>(kOpFvFused);  // the step kernel's id
-  static constexpr int kCtasPerSm = 4;
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ q_i, T* __restrict__ q_j,
-                                             T* __restrict__ fx1, T* __restrict__ fx2, T* __restrict__ fy1,
-                                             T* __restrict__ fy2, const T* __restrict__ q, const T* __restrict__ crx,
-                                             const T* __restrict__ cry, const T* __restrict__ ra_x,
-                                             const T* __restrict__ ra_y, const T* __restrict__ xfx,
-                                             const T* __restrict__ yfx, const T* __restrict__ area, T p1, T p2, Dims d,
-                                             int kb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    FvFusedSmem<T>& s = *reinterpret_cast<FvFusedSmem<T>*>(smem_raw);
-    // second-stage arrays over the dead aux arrays of the first
-    T(*xa2)[34] = reinterpret_cast<T(*)[34]>(&s.ym[0][0]);  // x-PPM of qi: al, 32 rows x 34
-    T(*xm2)[33] = reinterpret_cast<T(*)[33]>(&s.yr[0][0]);  // almq, 32 x 33
-    T(*xr2)[33] = reinterpret_cast<T(*)[33]>(&s.ya[0][0]);  // br, 32 x 33
-    unsigned char(*xs2)[33] = reinterpret_cast<unsigned char(*)[33]>(&s.ys[0][0]);
-    T(*ya3)[32] = reinterpret_cast<T(*)[32]>(&s.xm[0][0]);  // y-PPM of qj: al, 34 rows x 32
-    T(*ym3)[32] = reinterpret_cast<T(*)[32]>(&s.xr[0][0]);  // almq, 33 x 32
-    T(*yr3)[32] = reinterpret_cast<T(*)[32]>(&s.xa[0][0]);  // br, 33 x 32
-    unsigned char(*ys3)[32] = reinterpret_cast<unsigned char(*)[32]>(&s.xs[0][0]);
-    const int i0 = (int)blk.x * kT, j0 = (int)blk.y * kT;
-    const int sj = (int)d.sj;
+// The x sweep of one row: f the lane's value, c the Courant number of its low face; the flux there.
+// Valid from lane 3 to lane 29 (the edge value at i reads i-2 .. i+1, the flux the aux values at
+// i-1 and i).
+__device__ __forceinline__ float ppm_row(float p1, float p2, float f, float c) {
+  const float fm1 = lane_below<1>(f), fm2 = lane_below<2>(f), fp1 = lane_above<1>(f);
+  const float al = ppm_al(p1, p2, fm2, fm1, f, fp1);
+  const PpmCell x = ppm_cell(al, lane_above<1>(al), f);
+  return ppm_face(c, fm1, lane_below<1>(x.r), lane_below<1>(x.b0), f, x.m, x.b0, here_or_below(x.smt));
+}
+
+struct fvtp2d_march_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpFvMarch);  // the step kernel's id
+  static constexpr int kCols = 26, kApron = 5, kMinCtas = 3;
+  // The inputs of iteration s: q on row s + 3, cry and yfx on row s + 1, the rest on s.
+  struct Row {
+    float q, cry, yfx, crx, xfx, area, rax, ray;
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ q_i, float* __restrict__ q_j,
+                                             float* __restrict__ fx1, float* __restrict__ fx2, float* __restrict__ fy1,
+                                             float* __restrict__ fy2, const float* __restrict__ q,
+                                             const float* __restrict__ crx, const float* __restrict__ cry,
+                                             const float* __restrict__ ra_x, const float* __restrict__ ra_y,
+                                             const float* __restrict__ xfx, const float* __restrict__ yfx,
+                                             const float* __restrict__ area, float p1, float p2, Dims d, int rows,
+                                             int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
     const int nx = d.nx, ny = d.ny;
-    const int k0 = (int)blk.z * kb, k1 = min(k0 + kb, d.nz);
-    // cells this tile owns in the extended boxes of fy2 / q_i (columns) and fx2 / q_j (rows)
-    const int ci0 = i0 == 0 ? -3 : i0, ci1 = i0 + kT >= nx ? nx + 2 : i0 + kT;
-    const int rj0 = j0 == 0 ? -3 : j0, rj1 = j0 + kT >= ny ? ny + 2 : j0 + kT;
-    const int fyr1 = j0 + kT >= ny ? ny + 1 : j0 + kT;  // rows of fy2 owned
-    const int fxc1 = i0 + kT >= nx ? nx + 1 : i0 + kT;  // columns of fx2 owned
-    auto qok = [&](int i, int j) { return i >= -3 && i < nx + 3 && j >= -3 && j < ny + 3; };
-    // L2 prefetches: at each level, the inputs its later phases read, and the next level's q
-    // (the loads of the late phases and of the next q tile then find their lines in L2)
-    auto late_prefetch = [&](int64_t kofs) {
-      prefetch_box(cry, kofs, max(i0 - 3, -3), min(i0 + 34, nx + 2), max(j0, 0), min(j0 + 33, ny + 1), sj);
-      prefetch_box(yfx, kofs, max(i0 - 3, -3), min(i0 + 34, nx + 2), max(j0, 0), min(j0 + 33, ny + 1), sj);
-      prefetch_box(crx, kofs, max(i0, 0), min(i0 + 33, nx + 1), max(j0 - 3, -3), min(j0 + 34, ny + 2), sj);
-      prefetch_box(xfx, kofs, max(i0, 0), min(i0 + 33, nx + 1), max(j0 - 3, -3), min(j0 + 34, ny + 2), sj);
-      prefetch_box(area, kofs, max(i0 - 3, -3), min(i0 + 34, nx + 2), max(j0 - 3, -3), min(j0 + 34, ny + 2), sj);
-      prefetch_box(ra_y, kofs, max(i0 - 3, -3), min(i0 + 34, nx + 2), max(j0, 0), min(j0 + 32, ny), sj);
-      prefetch_box(ra_x, kofs, max(i0, 0), min(i0 + 32, nx), max(j0 - 3, -3), min(j0 + 34, ny + 2), sj);
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = i0 - 3 + lane;
+    const bool first_i = i0 == 0, last_i = i0 + kCols >= nx, first_j = ja == 0, last_j = jb == ny;
+    const bool own = lane >= 3 && lane < 3 + kCols;
+    // columns this lane writes: fy2 and q_i; fx2; q_j, fx1 and fy1 -- and reads
+    const bool st_y = i < nx + 2 && (own || (first_i && lane < 3) || (last_i && lane >= 3));
+    const bool st_x = i >= 0 && i < nx + 1 && (own || (last_i && lane >= 3));
+    const bool st = own && i < nx;
+    const bool in_q = i < nx + 3, in_y = i < nx + 2, in_x = i >= 0 && i < nx + 1, in_r = i >= 0 && i < nx;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)(ja - 3) * d.sj + i) * 4;  // (i, s)
+    Row nxt{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f};  // off a field's reach nothing is read: 0 (divisors 1)
+    // the inputs of iteration s, (i, s) at offset c; ALL: every row of them is this chunk's
+    auto fetch = [&](auto all, int s, int64_t c) {
+      constexpr bool ALL = decltype(all)::value;
+      if (in_q && (ALL || s + 3 <= jb + 2)) nxt.q = get(q, c + 3 * sjb);
+      if (in_y && (ALL || (s + 1 >= ja && s < jb))) nxt.cry = get(cry, c + sjb), nxt.yfx = get(yfx, c + sjb);  // fy2's
+      if (in_x && (ALL || s <= jb + 1)) nxt.crx = get(crx, c), nxt.xfx = get(xfx, c);                          // fx2's
+      if (in_y && (ALL || s <= jb + 1)) nxt.area = get(area, c);
+      if (in_r && (ALL || s <= jb + 1)) nxt.rax = get(ra_x, c);
+      if (in_y && (ALL || (s >= ja && s < jb))) nxt.ray = get(ra_y, c);  // q_i's
     };
+    float q0 = 0.f, q1 = 0.f, q2 = 0.f;  // q on rows s, s+1, s+2
+    if (in_q) q0 = get(q, o), q1 = get(q, o + sjb), q2 = get(q, o + 2 * sjb);
+    float al_lo = 0.f;                        // the y sweep's edge value at s+1
+    PpmCell yc = ppm_cell(0.f, 0.f, 0.f);     // its aux values at s
+    float fyy0 = 0.f;                         // yfx fy2 at s
+    float j1 = 0.f, j2 = 0.f, j3 = 0.f;       // q_j on rows s-1, s-2, s-3
+    float jal = 0.f;                          // the edge value of q_j's y sweep at s-2
+    PpmCell jc = ppm_cell(0.f, 0.f, 0.f);     // its aux values at s-3
+    float cy0 = 0.f, cy1 = 0.f, cy2 = 0.f;    // cry on rows s, s-1, s-2
+    float yf0 = 0.f, yf1 = 0.f, yf2 = 0.f;    // yfx
+    float fy0 = 0.f, fyA = 0.f, fyB = 0.f;    // fy2 on rows s, s-1, s-2
+    // one iteration; ALL: rows s-2 .. s+1 all lie in the chunk
+    auto step_row = [&](auto all, int s) {
+      constexpr bool ALL = decltype(all)::value;
+      const Row w = nxt;
+      fetch(all, s + 1, o + sjb);
+      // y sweep of q: fy2 at s+1
+      const float al_hi = ppm_al(p1, p2, q0, q1, q2, w.q);  // at s+2
+      const PpmCell yn = ppm_cell(al_lo, al_hi, q1);        // at s+1
+      const float fyn = ppm_face(w.cry, q0, yc.r, yc.b0, q1, yn.m, yn.b0, yc.smt || yn.smt);
+      const float fyy1 = w.yfx * fyn;
+      if (st_y && (ALL || (s + 1 >= ja && (s + 1 < jb || (last_j && s + 1 == ny))))) put(fy2, o + sjb, fyn);
+      // x sweep of q's row s: fx2, and q_j
+      const float fxn = ppm_row(p1, p2, q0, w.crx);
+      const float fxx = w.xfx * fxn;
+      const float qa = q0 * w.area;
+      const float jn = ((qa + fxx) - lane_above<1>(fxx)) / w.rax;
+      const bool row_own = ALL || ((s >= ja || first_j) && (s < jb || last_j));
+      if (st_x && row_own) put(fx2, o, fxn);
+      if (st && row_own) put(q_j, o, jn);
+      if (ALL || (s >= ja && s < jb)) {
+        // q_i, and its x sweep
+        const float qi = ((qa + fyy0) - fyy1) / w.ray;
+        if (st_y) put(q_i, o, qi);
+        const float f = ppm_row(p1, p2, qi, w.crx);
+        if (st) put(fx1, o, (0.5f * (f + fxn)) * w.xfx);
+      }
+      // y sweep of q_j: fy1 at s-2
+      const float jah = ppm_al(p1, p2, j3, j2, j1, jn);  // the edge value at s-1
+      const PpmCell jd = ppm_cell(jal, jah, j2);         // aux at s-2
+      const float f1 = ppm_face(cy2, j3, jc.r, jc.b0, j2, jd.m, jd.b0, jc.smt || jd.smt);
+      if (st && (ALL || s - 2 >= ja)) put(fy1, o - 2 * sjb, (0.5f * (f1 + fyB)) * yf2);
+      q0 = q1, q1 = q2, q2 = w.q;
+      al_lo = al_hi, yc = yn, fyy0 = fyy1;
+      j3 = j2, j2 = j1, j1 = jn, jal = jah, jc = jd;
+      cy2 = cy1, cy1 = cy0, cy0 = w.cry;
+      yf2 = yf1, yf1 = yf0, yf0 = w.yfx;
+      fyB = fyA, fyA = fy0, fy0 = fyn;
+      o += sjb;
+    };
+    fetch(std::false_type{}, ja - 3, o);
+    int s = ja - 3;
   #pragma unroll 1
-    for (int k = k0; k < k1; ++k) {
-      const int64_t kofs = (int64_t)k * d.sk;
-      late_prefetch(kofs);
-      for_region<39, 39>([&](int a, int b) {
-        const int i = i0 - 3 + a, j = j0 - 3 + b;
-        s.q[b][a] = qok(i, j) ? ld(q + kofs + i + j * sj) : T(0);
-      });
-      if (k + 1 < k1)
-        prefetch_box(q, kofs + d.sk, max(i0 - 3, -3), min(i0 + 36, nx + 3), max(j0 - 3, -3), min(j0 + 36, ny + 3), sj);
-      __syncthreads();
-      // edge values (fvtp2d.h:12, :57, :88, :133)
-      for_region<37, 35>([&](int a, int b) {
-        s.ya[b][a] = ppm_al(p1, p2, s.q[b][a], s.q[b + 1][a], s.q[b + 2][a], s.q[b + 3][a]);
-      });
-      for_region<35, 37>([&](int a, int b) {
-        s.xa[b][a] = ppm_al(p1, p2, s.q[b][a], s.q[b][a + 1], s.q[b][a + 2], s.q[b][a + 3]);
-      });
-      __syncthreads();
-      for_region<37, 34>([&](int a, int b) {
-        ppm_aux(s.ya[b][a], s.ya[b + 1][a], s.q[b + 2][a], &s.ym[b][a], &s.yr[b][a], &s.ys[b][a]);
-      });
-      for_region<34, 37>([&](int a, int b) {
-        ppm_aux(s.xa[b][a], s.xa[b][a + 1], s.q[b][a + 2], &s.xm[b][a], &s.xr[b][a], &s.xs[b][a]);
-      });
-      __syncthreads();
-      // fy2 (fvtp2d.h:26-34) on (i0-3+a, j0+b) and fyy = yfx fy2 (:43), over the dead al
-      for_region<37, 33>([&](int a, int b) {
-        const int i = i0 - 3 + a, j = j0 + b;
-        T fyy = T(0);
-        if (i >= -3 && i < nx + 2 && j >= 0 && j < ny + 1) {
-          const int64_t o = kofs + i + j * sj;
-          const T f = ppm_flux(ld(cry + o), s.q[b + 2][a], s.q[b + 3][a], s.ym[b][a], s.yr[b][a], s.ym[b + 1][a],
-                               s.yr[b + 1][a], s.ys[b][a], s.ys[b + 1][a]);
-          if (i >= ci0 && i < ci1 && j < fyr1) fy2[o] = f;
-          if (a >= 3 && a < 3 + kT && b < kT) s.fy2c[b][a - 3] = f;
-          fyy = ld(yfx + o) * f;
-        }
-        s.ya[b][a] = fyy;
-      });
-      // fx2 (fvtp2d.h:102-110) on (i0+a, j0-3+b) and fxx = xfx fx2 (:119)
-      for_region<33, 37>([&](int a, int b) {
-        const int i = i0 + a, j = j0 - 3 + b;
-        T fxx = T(0);
-        if (i >= 0 && i < nx + 1 && j >= -3 && j < ny + 2) {
-          const int64_t o = kofs + i + j * sj;
-          const T f = ppm_flux(ld(crx + o), s.q[b][a + 2], s.q[b][a + 3], s.xm[b][a], s.xr[b][a], s.xm[b][a + 1],
-                               s.xr[b][a + 1], s.xs[b][a], s.xs[b][a + 1]);
-          if (j >= rj0 && j < rj1 && i < fxc1) fx2[o] = f;
-          if (b >= 3 && b < 3 + kT && a < kT) s.fx2c[b - 3][a] = f;
-          fxx = ld(xfx + o) * f;
-        }
-        s.xa[b][a] = fxx;
-      });
-      __syncthreads();
-      // q_i (fvtp2d.h:48) on (i0-3+a, j0+b) and q_j (:124) on (i0+a, j0-3+b)
-      for_region<37, 32>([&](int a, int b) {
-        const int i = i0 - 3 + a, j = j0 + b;
-        T v = T(0);
-        if (i >= -3 && i < nx + 2 && j >= 0 && j < ny) {
-          const int64_t o = kofs + i + j * sj;
-          v = (((s.q[b + 3][a] * ld(area + o)) + s.ya[b][a]) - s.ya[b + 1][a]) / ld(ra_y + o);
-          if (i >= ci0 && i < ci1) q_i[o] = v;
-        }
-        s.qi[b][a] = v;
-      });
-      for_region<32, 37>([&](int a, int b) {
-        const int i = i0 + a, j = j0 - 3 + b;
-        T v = T(0);
-        if (i >= 0 && i < nx && j >= -3 && j < ny + 2) {
-          const int64_t o = kofs + i + j * sj;
-          v = (((s.q[b][a + 3] * ld(area + o)) + s.xa[b][a]) - s.xa[b][a + 1]) / ld(ra_x + o);
-          if (j >= rj0 && j < rj1) q_j[o] = v;
-        }
-        s.qj[b][a] = v;
-      });
-      __syncthreads();
-      // x-PPM of q_i (fvtp2d.h:53-82) and y-PPM of q_j (:129-158): edge values
-      for_region<34, 32>([&](int a, int b) {
-        xa2[b][a] = ppm_al(p1, p2, s.qi[b][a], s.qi[b][a + 1], s.qi[b][a + 2], s.qi[b][a + 3]);
-      });
-      for_region<32, 34>([&](int a, int b) {
-        ya3[b][a] = ppm_al(p1, p2, s.qj[b][a], s.qj[b + 1][a], s.qj[b + 2][a], s.qj[b + 3][a]);
-      });
-      __syncthreads();
-      for_region<33, 32>([&](int a, int b) {
-        ppm_aux(xa2[b][a], xa2[b][a + 1], s.qi[b][a + 2], &xm2[b][a], &xr2[b][a], &xs2[b][a]);
-      });
-      for_region<32, 33>([&](int a, int b) {
-        ppm_aux(ya3[b][a], ya3[b + 1][a], s.qj[b + 2][a], &ym3[b][a], &yr3[b][a], &ys3[b][a]);
-      });
-      __syncthreads();
-      // fx1, fy1 (fvtp2d.h:164, :173)
-      for_region<32, 32>([&](int a, int b) {
-        const int i = i0 + a, j = j0 + b;
-        if (i < nx && j < ny) {
-          const int64_t o = kofs + i + j * sj;
-          const T fx = ppm_flux(ld(crx + o), s.qi[b][a + 2], s.qi[b][a + 3], xm2[b][a], xr2[b][a], xm2[b][a + 1],
-                                xr2[b][a + 1], xs2[b][a], xs2[b][a + 1]);
-          fx1[o] = (scale2<-1>(fx + s.fx2c[b][a]) * ld(xfx + o));
-          const T fy = ppm_flux(ld(cry + o), s.qj[b + 2][a], s.qj[b + 3][a], ym3[b][a], yr3[b][a], ym3[b + 1][a],
-                                yr3[b + 1][a], ys3[b][a], ys3[b + 1][a]);
-          fy1[o] = (scale2<-1>(fy + s.fy2c[b][a]) * ld(yfx + o));
-        }
-      });
-      __syncthreads();
-    }
+    for (; s < min(ja + 2, jb + 2); ++s) step_row(std::false_type{}, s);
+  #pragma unroll 1
+    for (; s < jb - 1; ++s) step_row(std::true_type{}, s);
+  #pragma unroll 1
+    for (; s < jb + 2; ++s) step_row(std::false_type{}, s);
   }
 };
 
@@ -579,13 +530,11 @@ oeb_status fvtp2d_entry(const M3* q_i, const M3* q_j, const M3* fx1, const M3* f
   cudaStream_t st = (cudaStream_t)stream;
   const int kb = tuned_kb(kKB);
   if constexpr (std::is_same<T, float>::value) {
-    // FP32 is bound by memory: one launch, nothing read back
-    const int tiles = ((d.nx + kT - 1) / kT) * ((d.ny + kT - 1) / kT);
-    const int kbf = tuned_kb(staged_kb(tiles, d.nz, fvtp2d_fused_kernel<T>::kCtasPerSm));
-    return launch<fvtp2d_fused_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kbf), sizeof(FvFusedSmem<T>), st,
-                                          gqi.origin, gqj.origin, gfx1.origin, gfx2.origin, gfy1.origin, gfy2.origin,
-                                          gq.origin, gcx.origin, gcy.origin, grx.origin, gry.origin, gxf.origin,
-                                          gyf.origin, gar.origin, p1, p2, d, kbf);
+    using B = fvtp2d_march_f32;
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, st, gqi.origin, gqj.origin, gfx1.origin, gfx2.origin, gfy1.origin, gfy2.origin,
+                     gq.origin, gcx.origin, gcy.origin, grx.origin, gry.origin, gxf.origin, gyf.origin, gar.origin, p1,
+                     p2, d, m.rows, m.wx_log);
   }
   OEB_TRY(launch<fvtp2d_q_kernel<T>>(q_grid(d, kb), sizeof(FvQSmem<T>), st,
                                      gqi.origin, gqj.origin, gfx2.origin, gfy2.origin, gq.origin, gcx.origin,

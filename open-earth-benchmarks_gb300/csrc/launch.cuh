@@ -125,7 +125,7 @@ enum StepOpBase : int {
   kOpSmagAdjFused,
   kOpFvQ,
   kOpFvFlux,
-  kOpFvFused,
+  kOpFvMarch,       // fvtp2d_march_f32: the FP32 fvtp2d in one launch
   kOpFvAdjQij,
   kOpFvAdjF2,
   kOpFvAdjQ,

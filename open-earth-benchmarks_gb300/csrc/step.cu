@@ -80,7 +80,7 @@ using StepBodies = OpList<
     step_hd::hdiffsmag_adj_gather_kernel<float>, step_pw::hadv_adj_f32<5>,
     step_fws::fastwavesuv_adj_terms_kernel<float>, step_fws::fastwavesuv_adj_kernel<float, 0>,
     step_fv::fvtp2d_q_kernel<F64i>, step_fv::fvtp2d_q_kernel<float>, step_fv::fvtp2d_flux_kernel<F64i>,
-    step_fv::fvtp2d_fused_kernel<float>, step_fv::fvtp2d_adj_qij_kernel<F64i>,
+    step_fv::fvtp2d_march_f32, step_fv::fvtp2d_adj_qij_kernel<F64i>,
     step_fv::fvtp2d_adj_qij_kernel<float>, step_fv::fvtp2d_adj_f2_kernel<F64i>,
     step_fv::fvtp2d_adj_f2_kernel<float>, step_fv::fvtp2d_adj_q_kernel<F64i>,
     step_fv::fvtp2d_adj_q_kernel<float>>;

@@ -1,0 +1,46 @@
+"""The marching FP32 kernels (csrc/march.cuh) at the sizes where a strip or a chunk can go wrong:
+one column or row, a strip's width and one beside it, a chunk's rows and one beside them, padded
+and larger halos.  Every output cell is the oracle's, compiled for float, bit for bit (the same
+operations in the same order; the limiter and monotonicity signs are decided on exact products, which
+agree with the float products wherever those do not underflow), and nothing outside the written
+boxes changes.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (nx, ny, nz, halo, columns of row padding)
+SIZES = [(1, 1, 1, 3, 0), (5, 3, 2, 3, 0), (26, 4, 3, 3, 0), (27, 5, 2, 4, 1), (30, 33, 2, 3, 0), (31, 9, 2, 3, 2),
+         (32, 8, 1, 4, 0), (33, 31, 2, 3, 3), (52, 65, 2, 3, 0), (53, 12, 5, 4, 0), (61, 129, 1, 3, 0),
+         (127, 70, 3, 3, 0), (209, 17, 2, 3, 1)]
+NAMES = ("fvtp2d",)
+
+
+@pytest.mark.parametrize("size", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
+@pytest.mark.parametrize("name", NAMES)
+def test_marching_kernel_is_the_float_oracle(pkg, fields, orc, cuda, name, size):
+    import torch
+    nx, ny, nz, h, pad = size
+    spec = pkg.KERNELS[name]
+    inputs = fields.make_inputs(name, nx, ny, nz, seed=23, workload="fronts", halo=h)
+    sc = fields.make_scalars(name, seed=23)
+    sc32 = {s.name: (sc[s.name] if s.always_double else float(np.float32(sc[s.name]))) for s in spec.scalars}
+    outs = fields.make_outputs(name, nx, ny, nz, halo=h)
+    want = {k: v.astype(np.float32) for k, v in {**inputs, **outs}.items()}
+    dev = {}
+    for k, v in want.items():
+        a = np.full(v.shape[:-1] + (v.shape[-1] + pad,), np.float32(fields.SENTINEL)) if v.ndim == 3 else v.copy()
+        if v.ndim == 3:
+            a[..., :v.shape[-1]] = v
+        dev[k] = pkg.Storage(torch.from_numpy(a).to(cuda), h, nx=nx if v.ndim == 3 else None)
+    orc.run_oracle(spec, want, sc32, nx, ny, nz, h)
+    pkg.call(name, dev, sc32, domain=(nx, ny, nz))
+    torch.cuda.synchronize()
+    for a in spec.by_role("out3"):
+        got = dev[a.name].numpy()
+        np.testing.assert_array_equal(got[..., :nx + 2 * h].copy().view(np.uint32), want[a.name].view(np.uint32),
+                                      err_msg="%s.%s %s vs the float oracle" % (name, a.name, size))
+        assert (got[..., nx + 2 * h:] == np.float32(fields.SENTINEL)).all(), "%s.%s wrote its row padding" % (name, a.name)
