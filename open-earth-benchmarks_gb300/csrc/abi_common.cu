@@ -140,11 +140,12 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
   double least = 0.0;
   for (int wl = 0; wl <= 3; ++wl) {
     const int wx = 1 << wl, wy = kTY >> wl;
-    for (int rows = 4; rows <= 32; ++rows) {
+    for (int rows = 4; rows <= 64; ++rows) {
       const int chunks = (ny + rows - 1) / rows;
       const dim3 grid((unsigned)((strips + wx - 1) / wx), (unsigned)((chunks + wy - 1) / wy), (unsigned)levels);
       const double waves = (double)grid.x * grid.y * grid.z / slots;
-      const double cost = (waves > 1.0 ? waves : 1.0) * (rows + apron + 3);
+      const double full = (double)(int64_t)waves, rest = waves - full;
+      const double cost = (full < 1.0 ? 1.0 : full + (rest == 0.0 || rest > 0.5 ? rest : 0.5)) * (rows + apron + 3);
       if (best.rows == 0 || cost < least) {
         least = cost;
         best = MarchShape{rows, wl, grid};

@@ -19,6 +19,7 @@
 // computes 4 rows.  Neighbour reads go through L1.
 #include <type_traits>
 
+#include "march.cuh"
 #include "precision.cuh"
 #include "stage.cuh"
 #include "stencil_util.cuh"
@@ -324,6 +325,111 @@ struct hadv_kernel {
       const T vt = vres - (ld(tgrlatda1 + jo) * u_atvpos) * u_atvpos;
       vout[o] = update ? alpha * vt + v0 : vt;
     });
+  }
+};
+
+// ---- FP32 hadvuv / hadvuv5th, marching -------------------------------------------------
+// A warp marches rows (march.cuh): the seven (five) rows of u and v that its y axes read stay in
+// registers, each read from memory once a chunk; the x neighbours come from L1 at constant offsets
+// from one address a field, those that the winds wait on a row ahead.  hadv_kernel's operations on
+// the same operands in the same order: the same bits.
+//
+// What bounds it: instruction issue (about 190 instructions a row, 119 of them the arithmetic and
+// its upwind selects; 65-70 % of the issue slots taken) and what its loads leave unhidden.  64
+// registers, four CTAs an SM, two rows unrolled: hadvuv5th 41.0 us at 256 x 256 x 80 (three CTAs
+// 46.1, one row unrolled 42.7), 98.9 us at 320 x 304 x 137; hadvuv 34.4 us.  hadv_kernel<float>, a
+// point at a time with every neighbour read through L1 (4 of them at selected addresses an axis),
+// took 49.8, 118.6 and 42.9 us.  Warps that branch where all lanes agree on the wind, instead of
+// the selects, measured slower (43.4 us; the arithmetic of a row is then cut into blocks).
+template <int ORDER>
+struct hadv_march_f32 {
+  static constexpr int kStepOp = step_op<float>(ORDER == 5 ? kOpHadv5Fwd : -1);  // the step kernel's id
+  static constexpr int H = ORDER == 5 ? 3 : 2, W = 2 * H + 1;
+  static constexpr int kCols = 32, kApron = W - 1, kMinCtas = 4;
+  // the upwind sum along one axis: f[0 .. 2H] from offset -H to H
+  static __device__ __forceinline__ float axis(const float (&f)[W], float a) {
+    const bool pos = a > 0.f;
+    float sum;
+    if constexpr (ORDER == 3) {
+      constexpr float c6 = -1.f / 6.f, c3 = -1.f / 3.f;
+      const float ph = -(0.5f * f[2]);
+      const float p0 = (pos ? c6 : c3) * (pos ? f[0] : f[1]), p3 = (pos ? c3 : c6) * (pos ? f[3] : f[4]);
+      sum = ((p0 + (pos ? f[1] : ph)) + (pos ? ph : f[3])) + p3;
+    } else {
+      constexpr float c30 = 1.f / 30.f, c3 = -1.f / 3.f, c20 = 1.f / 20.f;
+      const float p0 = (pos ? c30 : c20) * (pos ? f[0] : f[1]), p1 = (pos ? -0.25f : -0.5f) * (pos ? f[1] : f[2]),
+                  pm = c3 * f[3], p4 = (pos ? -0.5f : -0.25f) * (pos ? f[4] : f[5]),
+                  p5 = (pos ? c20 : c30) * (pos ? f[5] : f[6]);
+      sum = ((((p0 + p1) + (pos ? f[2] : pm)) + (pos ? pm : f[4])) + p4) + p5;
+    }
+    return (pos ? a : -a) * sum;
+  }
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uout, float* __restrict__ vout,
+                                             const float* __restrict__ uin, const float* __restrict__ vin,
+                                             const float* __restrict__ acrlat0, const float* __restrict__ acrlat1,
+                                             const float* __restrict__ tgrlatda0, const float* __restrict__ tgrlatda1,
+                                             int64_t s1d, float eddlat, float eddlon, Dims d, int rows, int wx_log,
+                                             float alpha, int update) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = min(i0 + lane, nx - 1);  // lanes past the domain repeat its last column
+    const bool st = i0 + lane < nx;
+    constexpr float third = 1.f / 3.f, rr = earth_radius_recip<float>();
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, j)
+    // the metric terms of 32 rows, one a lane, handed round by shuffles
+    float la0, la1, lt0, lt1;
+    auto metric = [&](int j) {
+      const int64_t jo = (int64_t)min(j + lane, ny - 1) * s1d;
+      la0 = ld(acrlat0 + jo), la1 = ld(acrlat1 + jo), lt0 = ld(tgrlatda0 + jo), lt1 = ld(tgrlatda1 + jo);
+    };
+    metric(ja);
+    float u[W], v[W];  // rows j-H .. j+H
+#pragma unroll
+    for (int q = 0; q < W - 1; ++q) u[q] = get(uin, o + (q - H) * sjb), v[q] = get(vin, o + (q - H) * sjb);
+    float un = get(uin, o + H * sjb), vn = get(vin, o + H * sjb);
+    // u(i-1), u(i+1) and v(i+1) on row j, loaded a row ahead (the winds wait on them), v(i+1) on j-1
+    float um1 = get(uin, o - 4), up1 = get(uin, o + 4), vp1 = get(vin, o + 4), vp0 = get(vin, o - sjb + 4);
+#pragma unroll 2
+    for (int j = ja; j < jb; ++j) {
+      float ux[W], vx[W];
+      const float* pu = reinterpret_cast<const float*>(reinterpret_cast<const char*>(uin) + o);
+      const float* pv = reinterpret_cast<const float*>(reinterpret_cast<const char*>(vin) + o);
+#pragma unroll
+      for (int q = 0; q < W; ++q) {
+        if (q < H - 1 || q > H + 1) ux[q] = ld(pu + (q - H));
+        if (q < H || q > H + 1) vx[q] = ld(pv + (q - H));
+      }
+      const float ump = get(uin, o + sjb - 4), upp = get(uin, o + sjb + 4), vpp = get(vin, o + sjb + 4);
+      u[W - 1] = un, v[W - 1] = vn;
+      if (j + 1 < jb) un = get(uin, o + (H + 1) * sjb), vn = get(vin, o + (H + 1) * sjb);
+      const float u0 = u[H], v0 = v[H];
+      ux[H] = u0, ux[H - 1] = um1, ux[H + 1] = up1, vx[H] = v0, vx[H + 1] = vp1;
+      const int src = (j - ja) & 31;
+      if (src == 0 && j > ja) metric(j);
+      const float a0 = __shfl_sync(kWarpMask, la0, src), a1 = __shfl_sync(kWarpMask, la1, src),
+                  t0 = __shfl_sync(kWarpMask, lt0, src), t1 = __shfl_sync(kWarpMask, lt1, src);
+      const float um = um1 + u0;
+      const float u_atupos = third * (um + up1);
+      const float v_atupos = 0.25f * (((vp1 + vp0) + v0) + v[H - 1]);
+      const float u_atvpos = 0.25f * ((um + u[H + 1]) + ump);
+      const float v_atvpos = third * ((v[H - 1] + v0) + v[H + 1]);
+      const float uy = axis(u, rr * v_atupos), vy = axis(v, rr * v_atvpos);
+      const float ures = eddlat * axis(ux, a0 * u_atupos) + eddlon * uy;
+      const float ut = ures + (t0 * u0) * v_atupos;
+      const float vres = eddlat * axis(vx, a1 * u_atvpos) + eddlon * vy;
+      const float vt = vres - (t1 * u_atvpos) * u_atvpos;
+      if (st) {
+        put(uout, o, update ? alpha * ut + u0 : ut);
+        put(vout, o, update ? alpha * vt + v0 : vt);
+      }
+      um1 = ump, up1 = upp, vp0 = vp1, vp1 = vpp;
+#pragma unroll
+      for (int q = 0; q < W - 1; ++q) u[q] = u[q + 1], v[q] = v[q + 1];
+      o += sjb;
+    }
   }
 };
 
@@ -815,19 +921,26 @@ oeb_status hadv_entry(const M3* uout, const M3* vout, const M3* uin, const M3* v
   OEB_TRY(check_no_alias({gu.lo, gu.hi, gv.lo, gv.hi}, {gui.lo, gui.hi, gvi.lo, gvi.hi, a0.lo, a0.hi, a1.lo, a1.hi,
                                                         t0.lo, t0.hi, t1.lo, t1.hi}));
   OEB_RETURN_IF_VALIDATING();
-  const int kb = tuned_kb(kKB);
-  auto go = [&](auto body, int shape) {
-    using B = decltype(body);
-    constexpr int S = B::kShape;
-    (void)shape;
-    return launch<B>(tile_grid((int)dom->nx, (int)dom->ny, (int)dom->nz, TileOf<S>::I, TileOf<S>::J, kb), 0,
-                     (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin, a1.origin,
-                     t0.origin, t1.origin, a0.s, eddlat, eddlon, make_dims(*dom, gu), kb, alpha, update);
-  };
-  switch (tuned_shape()) {
-    case 1: return go(hadv_kernel<T, ORDER, 1>{}, 1);
-    case 2: return go(hadv_kernel<T, ORDER, 2>{}, 2);
-    default: return go(hadv_kernel<T, ORDER, 0>{}, 0);
+  if constexpr (std::is_same<T, float>::value) {
+    using B = hadv_march_f32<ORDER>;
+    const Dims d = make_dims(*dom, gu);
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin,
+                     a1.origin, t0.origin, t1.origin, a0.s, eddlat, eddlon, d, m.rows, m.wx_log, alpha, update);
+  } else {
+    const int kb = tuned_kb(kKB);
+    auto go = [&](auto body) {
+      using B = decltype(body);
+      constexpr int S = B::kShape;
+      return launch<B>(tile_grid((int)dom->nx, (int)dom->ny, (int)dom->nz, TileOf<S>::I, TileOf<S>::J, kb), 0,
+                       (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin, a1.origin,
+                       t0.origin, t1.origin, a0.s, eddlat, eddlon, make_dims(*dom, gu), kb, alpha, update);
+    };
+    switch (tuned_shape()) {
+      case 1: return go(hadv_kernel<T, ORDER, 1>{});
+      case 2: return go(hadv_kernel<T, ORDER, 2>{});
+      default: return go(hadv_kernel<T, ORDER, 0>{});
+    }
   }
 }
 

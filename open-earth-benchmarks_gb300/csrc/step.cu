@@ -68,7 +68,7 @@ using StepBodies = OpList<
     step_fws::fastwavesuv_adj_terms_kernel<F64i>, step_fws::fastwavesuv_adj_kernel<F64i, 0>,
     step_fws::fastwavesuv_adj_kernel<float, 1>,
     step_pw::hadv_kernel<F64i, 5, 0>, step_pw::hadv_kernel<F64i, 5, 1>, step_pw::hadv_kernel<F64i, 5, 2>,
-    step_pw::hadv_kernel<float, 5, 0>, step_pw::hadv_kernel<float, 5, 1>, step_pw::hadv_kernel<float, 5, 2>,
+    step_pw::hadv_march_f32<5>,
     step_pw::hadv_adj_terms_kernel<F64i, 5, 0>, step_pw::hadv_adj_terms_kernel<F64i, 5, 1>,
     step_pw::hadv_adj_terms_kernel<F64i, 5, 2>, step_pw::hadv_adj_terms_kernel<float, 5, 0>,
     step_pw::hadv_adj_terms_kernel<float, 5, 1>, step_pw::hadv_adj_terms_kernel<float, 5, 2>,
