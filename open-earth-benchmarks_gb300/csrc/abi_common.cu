@@ -128,11 +128,11 @@ int staged_kb(int tiles, int nz, int ctas_per_sm) {
 }
 
 // A chunk of R rows marches R + apron, and about three rows' time passes before its first row's
-// loads have landed; a launch takes at least one wave of CTAs' time.  The split with the least
-// product of the two wins: fvtp2d (apron 5, three CTAs an SM) measured best with 32 rows at
-// 256 x 256 x 80 (89.7 us; 16 rows 93.9, 12 rows 101.7, 8 rows 102.7, 64 rows 113) and with 16 at
-// 128 x 128 x 80 (28.1 us; 8 rows 32.5, 22 rows 31.1, 32 rows 36.6), as the product says, which is
-// taken over at most 32 rows.
+// loads have landed; a launch takes at least one wave of CTAs' time, and a part of a wave after
+// the first at least half of one.  The split with the least product of the two wins.  Measured for
+// fvtp2d (apron 5, three CTAs an SM): best with 32 rows at 256 x 256 x 80 (89.7 us; 16 rows 93.9,
+// 12 rows 101.7, 8 rows 102.7, 64 rows 113) and with 16 at 128 x 128 x 80 (28.1 us; 8 rows 32.5,
+// 22 rows 31.1, 32 rows 36.6), as the product says.
 MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm) {
   const double slots = (double)device_sms() * ctas_per_sm;
   const int strips = (nx + cols - 1) / cols, levels = (nz + kb - 1) / kb;

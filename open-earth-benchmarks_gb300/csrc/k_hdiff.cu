@@ -19,7 +19,7 @@
 #include <vector>
 
 #include "precision.cuh"
-#include "stage.cuh"
+#include "march.cuh"
 #include "stencil_util.cuh"
 #include "tangent.cuh"
 
@@ -114,91 +114,79 @@ struct hdiffsa_kernel {
   }
 };
 
-// FP32 hdiffsa.  In FP32 the kernel above is bound by instruction issue, not by HBM (ncu at
-// 256 x 256 x 80: 72 % issue active, "not selected" the top stall, 13 % of DRAM throughput):
-// five shared-memory phases a level, each with its own index arithmetic.  Here a level takes
-// two: the laplacian on its 34 x 34 box straight from the `in` tile (the differences
-// in(j+1) - in and in(j-1) - in formed where they are used; the kernel above stores
-// in(j+1) - in once and negates it, which gives the same bits), then each output forms the
-// four limited fluxes it reads (each flux is formed by the two outputs beside it, with the
-// same operations on the same operands).  The k-levels are marched: the `in` tile of level
-// k+1 is copied by cp.async into a second buffer while level k is computed.  Results are
-// hdiffsa_kernel<float>'s, bit for bit.  kb from staged_kb: about one wave of CTAs.
-// Measured alone (back-to-back launches): 256 x 256 x 80 41.3 -> 38.6 us, 128 x 128 x 80
-// 14.5 -> 12.7 us; 20 % fewer warp instructions (35.7 M -> 28.7 M a launch), still 67 % issue
-// active.  The marching alone, with the five phases, measured 41.2 us: the kernel waits on
-// its instructions, not on its loads.
-struct hdiffsa_f32 {
-  static constexpr int kCtasPerSm = 6;  // by registers (40)
-  struct Smem {
-    float in[2][36][36];  // (i0-2+a, j0-2+b)
-    float lap[34][34];    // (i0-1+a, j0-1+b)
-    float crlato[34], crlatu[34];  // j0-1+b
-  };
+// FP32 hdiffsa, marching rows (march.cuh): lane = column i0 - 1 + lane, 30 columns a strip.  At row j
+// a lane holds `in` on rows j .. j+2 (its x neighbours, loaded with each row, on j and j+1) and forms
+// the laplacian at j+1 and from it fly at j; flx at j takes the laplacian of the lane above, the
+// output the flx of the lane below.  Each laplacian and flux is formed once.  hdiffsa_kernel<float>'s
+// operations on the same operands (the limiter tests on the exact product, its factors scaled by
+// 2^100, so that a nonzero product neither underflows nor loses its sign): the same bits.
+//
+// What bounds it: instruction issue (about 108 instructions a row of 30 columns, 66 % of the issue
+// slots taken) and the ends of a short launch.  48 registers, five CTAs an SM, two rows unrolled:
+// 23.4 us at 256 x 256 x 80 and 50.3 at 320 x 304 x 137 (four CTAs 24.1 / 50.6, six 28.1 / 61.7,
+// one row unrolled 26.5 / 58.9; two rows of loads in flight instead of one 26.4 / 59.0); the form
+// before it, a 32 x 32 shared-memory tile marched over the levels, took 37.4 and 94.7 us.
+struct hdiffsa_march_f32 {
+  static constexpr int kCols = 30, kApron = 3, kMinCtas = 5;
+  static __device__ __forceinline__ float limited(float f, float d) {
+    constexpr float s = 1.2676506002282294e30f;
+    return (f * s) * (d * s) > 0.f ? 0.f : f;
+  }
   static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ out, const float* __restrict__ in,
                                              const float* __restrict__ mask, const float* __restrict__ crlato,
-                                             const float* __restrict__ crlatu, int64_t s1d, Dims d, int kb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-    const int i0 = blk.x * kT, j0 = blk.y * kT;
-    const int sj = (int)d.sj;
-    const int tid = threadIdx.y * kTX + threadIdx.x;
-    if (tid < 34) {
-      const int j = j0 - 1 + tid;
-      const bool ok = j >= -1 && j < d.ny + 1;
-      s.crlato[tid] = ok ? ld(crlato + (int64_t)j * s1d) : 0.f;
-      s.crlatu[tid] = ok ? ld(crlatu + (int64_t)j * s1d) : 0.f;
-    }
-    const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
-    const int vx = max(0, min(kT, d.nx - i0)), vy = max(0, min(kT, d.ny - j0));
-    auto issue = [&](int k, float (*t)[36]) {
-      if (k < k1) {
-        const float* pin = in + (int64_t)k * d.sk;
-        for_region_lim<36, 36>(vx + 4, vy + 4, [&](int a, int b) {
-          const int i = i0 - 2 + a, j = j0 - 2 + b;
-          const bool ok = i >= -2 && i < d.nx + 2 && j >= -2 && j < d.ny + 2;
-          cp_async4(&t[b][a], ok ? pin + i + j * sj : pin, ok);
-        });
-      }
-      cp_async_commit();
+                                             const float* __restrict__ crlatu, int64_t s1d, Dims d, int rows,
+                                             int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = min(i0 - 1 + lane, nx);  // lanes past the reach repeat its last column
+    const bool st = lane >= 1 && lane <= kCols && i0 - 1 + lane < nx;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, j)
+    const int64_t om = (int64_t)(max(0, min(i, nx - 1)) - i) * 4;      // to the mask's column
+    // the metric terms of rows ja - 1 + lane
+    float lo, lu;
+    auto metric = [&](int j) {
+      const int64_t jo = (int64_t)min(j + lane, ny) * s1d;
+      lo = ld(crlato + jo), lu = ld(crlatu + jo);
     };
-    issue(k0, s.in[0]);
-  #pragma unroll 1
-    for (int k = k0; k < k1; ++k) {
-      const int cur = (k - k0) & 1;
-      issue(k + 1, s.in[cur ^ 1]);  // the buffer level k-1 left
-      const int64_t kofs = (int64_t)k * d.sk;
-      cp_async_wait<1>();  // level k has landed
-      __syncthreads();
-      const float(*t)[36] = s.in[cur];
-      // hdiffsa.h:101: in(i-1)+in(i+1) - 2 in + crlato (in(j+1)-in) + crlatu (in(j-1)-in)
-      for_region_lim<34, 34>(vx + 2, vy + 2, [&](int a, int b) {
-        const float c = t[b + 1][a + 1];
-        s.lap[b][a] = (((t[b + 1][a] + t[b + 1][a + 2]) - 2.f * c) + s.crlato[b] * (t[b + 2][a + 1] - c)) +
-                      s.crlatu[b] * (t[b][a + 1] - c);
-      });
-      __syncthreads();
-      // hdiffsa.h:106-113 (limited fluxes) and :118-119 (the update)
-      const int a = threadIdx.x;
-#pragma unroll
-      for (int r = 0; r < kT / kTY; ++r) {
-        const int b = threadIdx.y + kTY * r;
-        if (a < vx && b < vy) {
-          const float lc = s.lap[b + 1][a + 1];
-          const float ic = t[b + 2][a + 2];
-          float fxw = lc - s.lap[b + 1][a];
-          if (Prec<float>::prod_gt0(fxw, ic - t[b + 2][a + 1])) fxw = 0.f;
-          float fxe = s.lap[b + 1][a + 2] - lc;
-          if (Prec<float>::prod_gt0(fxe, t[b + 2][a + 3] - ic)) fxe = 0.f;
-          float fys = s.crlato[b] * (lc - s.lap[b][a + 1]);
-          if (Prec<float>::prod_gt0(fys, ic - t[b + 1][a + 2])) fys = 0.f;
-          float fyn = s.crlato[b + 1] * (s.lap[b + 2][a + 1] - lc);
-          if (Prec<float>::prod_gt0(fyn, t[b + 3][a + 2] - ic)) fyn = 0.f;
-          const int64_t o = kofs + (i0 + a) + (int64_t)(j0 + b) * sj;
-          out[o] = ic + (((fxw - fxe) + fys) - fyn) * ld(mask + o);
-        }
+    metric(ja - 1);
+    auto lapl = [](float m, float c, float p, float co, float dyp, float cu, float dym) {
+      return (((m + p) - 2.f * c) + co * dyp) + cu * (-dym);
+    };
+    // rows ja - 2 .. ja + 1: the laplacian at ja - 1 and ja, and fly at ja - 1
+    const float a0 = get(in, o - 2 * sjb), a1 = get(in, o - sjb);
+    float c0 = get(in, o), c1 = get(in, o + sjb);
+    const float a1m = get(in, o - sjb - 4), a1p = get(in, o - sjb + 4), c0m = get(in, o - 4), c0p = get(in, o + 4);
+    float c1m = get(in, o + sjb - 4), c1p = get(in, o + sjb + 4);
+    // `in` on row j + 2 and the mask on j, loaded a row ahead
+    float n = get(in, o + 2 * sjb), nm = get(in, o + 2 * sjb - 4), np = get(in, o + 2 * sjb + 4), w = get(mask, o + om);
+    float cm = __shfl_sync(kWarpMask, lo, 0), co = __shfl_sync(kWarpMask, lo, 1);
+    const float dm = c0 - a1;
+    float dy = c1 - c0, dx = c0p - c0;
+    const float lm = lapl(a1m, a1, a1p, cm, dm, __shfl_sync(kWarpMask, lu, 0), a1 - a0);
+    float lap = lapl(c0m, c0, c0p, co, dy, __shfl_sync(kWarpMask, lu, 1), dm);
+    float fly = limited(cm * (lap - lm), dm);  // at ja - 1
+#pragma unroll 2
+    for (int j = ja; j < jb; ++j) {
+      const float x = n, xm = nm, xp = np, wj = w;
+      if (j + 1 < jb) {
+        n = get(in, o + 3 * sjb), nm = get(in, o + 3 * sjb - 4), np = get(in, o + 3 * sjb + 4);
+        w = get(mask, o + om + sjb);
       }
-      __syncthreads();
+      const int src = (j + 2 - ja) & 31;
+      if (src == 0) metric(j + 1);
+      const float cn = __shfl_sync(kWarpMask, lo, src), un = __shfl_sync(kWarpMask, lu, src);  // at j + 1
+      const float dn = x - c1;
+      const float ln = lapl(c1m, c1, c1p, cn, dn, un, dy);
+      const float fn = limited(co * (ln - lap), dy);
+      const float fx = limited(lane_above<1>(lap) - lap, dx);
+      const float r = c0 + (((lane_below<1>(fx) - fx) + fly) - fn) * wj;
+      if (st) put(out, o, r);
+      dx = c1p - c1, c0 = c1, c1 = x, c1m = xm, c1p = xp;
+      dy = dn, lap = ln, fly = fn, co = cn;
+      o += sjb;
     }
   }
 };
@@ -322,6 +310,97 @@ struct hdiffsmag_kernel {
   }
 };
 
+// FP32 hdiffsmag, marching rows (march.cuh): lane = column i0 - 1 + lane, 30 columns a strip.  At row j
+// a lane holds u and v on rows j and j+1 (their x neighbours handed over by the neighbouring lanes as
+// each row arrives) and forms T^2 at j+1 and S^2 at j, each once; T^2(i+1) and S^2(i-1) come from the
+// lanes beside it.  hdiffsmag_kernel's operations on the same operands in the same order.
+//
+// What bounds it: instruction issue (about 150 instructions a row, two square roots among them) and
+// load latency.  48 registers, five CTAs an SM: 39.1 us at 256 x 256 x 80, 89.0 at 320 x 304 x 137
+// and 19.7 at 201 x 173 x 61 (four CTAs 47.6 / 107 / 23.3, six, which spills, 43.7 / 102 / 19.5);
+// hdiffsmag_kernel<float>'s shared-memory tile took 44.2, 103.8 and 24.2 us.
+struct hdiffsmag_march_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpSmagFwd);  // the step kernel's id
+  static constexpr int kCols = 30, kApron = 2, kMinCtas = 5;
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uout, float* __restrict__ vout,
+                                             const float* __restrict__ uin, const float* __restrict__ vin,
+                                             const float* __restrict__ mask, const float* __restrict__ crlavo,
+                                             const float* __restrict__ crlavu, const float* __restrict__ crlato,
+                                             const float* __restrict__ crlatu, const float* __restrict__ acrlat0,
+                                             int64_t s1d, float eddlat, float eddlon, float tau_smag,
+                                             float weight_smag, Dims d, int rows, int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    constexpr float rr = earth_radius_recip<float>();
+    const int lane = (int)threadIdx.x, i = min(i0 - 1 + lane, nx);  // lanes past the reach repeat its last column
+    const bool st = lane >= 1 && lane <= kCols && i0 - 1 + lane < nx;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, j)
+    const int64_t om = (int64_t)(max(0, min(i, nx - 1)) - i) * 4;      // to the mask's column
+    // the metric terms of 32 rows, one a lane: acrlat0 from row ja - 1, the others from ja
+    float la, lto, ltu, lvo, lvu;
+    auto metric_a = [&](int j) { la = ld(acrlat0 + (int64_t)min(j + lane, ny) * s1d); };
+    auto metric = [&](int j) {
+      const int64_t jo = (int64_t)min(j + lane, ny - 1) * s1d;
+      lto = ld(crlato + jo), ltu = ld(crlatu + jo), lvo = ld(crlavo + jo), lvu = ld(crlavu + jo);
+    };
+    metric_a(ja - 1);
+    metric(ja);
+    // T from dyv(j-1) and dxu(j), S from dyu(j) and dxv(j)
+    auto tsq_of = [&](float dyv, float dxu, float ac) {
+      const float t = ((-dyv) * eddlat) * rr - ((-dxu) * ac) * eddlon;
+      return t * t;
+    };
+    auto ssq_of = [&](float dyu, float dxv, float ac) {
+      const float q = (dyu * eddlat) * rr + (dxv * ac) * eddlon;
+      return q * q;
+    };
+    const float ua = get(uin, o - sjb), va = get(vin, o - sjb);
+    float u0 = get(uin, o), v0 = get(vin, o);
+    // u and v on row j + 1 and the mask on j, loaded a row ahead
+    float un = get(uin, o + sjb), vn = get(vin, o + sjb), w = get(mask, o + om);
+    const float am = __shfl_sync(kWarpMask, la, 0);
+    float ac = __shfl_sync(kWarpMask, la, 1);
+    float dyu = u0 - ua, dyv = v0 - va;                                    // at j - 1
+    float um = lane_below<1>(u0), up = lane_above<1>(u0), vm = lane_below<1>(v0), vp = lane_above<1>(v0);  // on row j
+    float tsq = tsq_of(dyv, u0 - um, ac);                                  // at j
+    float ssq = ssq_of(dyu, lane_above<1>(va) - va, am);                   // at j - 1
+#pragma unroll 1
+    for (int j = ja; j < jb; ++j) {
+      const float u1 = un, v1 = vn, wj = w;
+      if (j + 1 < jb) un = get(uin, o + 2 * sjb), vn = get(vin, o + 2 * sjb), w = get(mask, o + om + sjb);
+      const int src = (j - ja) & 31, sra = (j + 2 - ja) & 31;
+      if (src == 0 && j > ja) metric(j);
+      if (sra == 0) metric_a(j + 1);
+      const float an = __shfl_sync(kWarpMask, la, sra);
+      const float cto = __shfl_sync(kWarpMask, lto, src), ctu = __shfl_sync(kWarpMask, ltu, src),
+                  cvo = __shfl_sync(kWarpMask, lvo, src), cvu = __shfl_sync(kWarpMask, lvu, src);
+      const float um1 = lane_below<1>(u1), up1 = lane_above<1>(u1), vm1 = lane_below<1>(v1), vp1 = lane_above<1>(v1);
+      const float dyu1 = u1 - u0, dyv1 = v1 - v0;
+      const float tsq1 = tsq_of(dyv1, u1 - um1, an);
+      const float ssq1 = ssq_of(dyu1, vp - v0, ac);
+      const float hdweight = weight_smag * wj;
+      // hdiffsmag.h:233-244
+      const float su = clamp_smag(
+          tau_smag * sqrtf(0.5f * (lane_above<1>(tsq) + tsq) + 0.5f * (ssq + ssq1)) - hdweight);
+      const float lu = (((up + um) + -(2.f * u0)) + cto * dyu1) + ctu * (-dyu);
+      // hdiffsmag.h:248-259
+      const float sv = clamp_smag(
+          tau_smag * sqrtf(0.5f * (tsq1 + tsq) + 0.5f * (lane_below<1>(ssq1) + ssq1)) - hdweight);
+      const float lv = (((vp + vm) + -(2.f * v0)) + cvo * dyv1) + cvu * (-dyv);
+      if (st) {
+        put(uout, o, u0 + su * lu);
+        put(vout, o, v0 + sv * lv);
+      }
+      u0 = u1, v0 = v1, um = um1, up = up1, vm = vm1, vp = vp1;
+      dyu = dyu1, dyv = dyv1, tsq = tsq1, ssq = ssq1, ac = an;
+      o += sjb;
+    }
+  }
+};
+
 constexpr int kKB = 1;  // k-levels per CTA by default (the most CTAs hide latency best)
 
 template <class T, class M3, class M1>
@@ -341,10 +420,10 @@ oeb_status hdiffsa_entry(const M3* out, const M3* in, const M3* mask, const M1* 
   OEB_RETURN_IF_VALIDATING();
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gin.sj, gin.sk};
   if constexpr (std::is_same<T, float>::value) if (!fields_in_host_memory()) {
-    const int tiles = ((d.nx + kT - 1) / kT) * ((d.ny + kT - 1) / kT);
-    const int kb = tuned_kb(staged_kb(tiles, d.nz, hdiffsa_f32::kCtasPerSm));
-    return launch<hdiffsa_f32>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(hdiffsa_f32::Smem), (cudaStream_t)stream,
-                               gout.origin, gin.origin, gmask.origin, lo.origin, lu.origin, lo.s, d, kb);
+    using B = hdiffsa_march_f32;
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, (cudaStream_t)stream, gout.origin, gin.origin, gmask.origin, lo.origin, lu.origin, lo.s,
+                     d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
   return launch<hdiffsa_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsaSmem<T>), (cudaStream_t)stream,
@@ -375,11 +454,19 @@ oeb_status hdiffsmag_entry(const M3* uout, const M3* vout, const M3* uin, const 
                           lto.hi, ltu.lo, ltu.hi, la0.lo, la0.hi}));
   OEB_RETURN_IF_VALIDATING();
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gui.sj, gui.sk};
-  const int kb = tuned_kb(kKB);
-  return launch<hdiffsmag_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsmagSmem<T>),
+  if constexpr (std::is_same<T, float>::value) {
+    using B = hdiffsmag_march_f32;
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, gm.origin, lvo.origin,
+                     lvu.origin, lto.origin, ltu.origin, la0.origin, lvo.s, eddlat, eddlon, tau_smag, weight_smag, d,
+                     m.rows, m.wx_log);
+  } else {
+    const int kb = tuned_kb(kKB);
+    return launch<hdiffsmag_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsmagSmem<T>),
                                      (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, gm.origin,
                                      lvo.origin, lvu.origin, lto.origin, ltu.origin, la0.origin, lvo.s, eddlat, eddlon,
                                      tau_smag, weight_smag, d, kb);
+  }
 }
 
 // Tangent-linear hdiffsmag: d(uout, vout) = J(uin, vin) d(uin, vin), the kernel on Dual<T>.
