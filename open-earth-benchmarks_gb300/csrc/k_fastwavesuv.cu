@@ -1,4 +1,5 @@
-// k_fastwavesuv.cu -- fastwavesuv (kernels/fastwavesuv.h:154-191) in FP64 and FP32.
+// k_fastwavesuv.cu -- fastwavesuv (kernels/fastwavesuv.h:154-191) in FP64 and FP32 (the latter by
+// fastwavesuv_march_f32 below).
 //
 // The OpenMP variant evaluates ppgk = wgtfac*ppuv + (1-wgtfac)*ppuv(k-1) six times per point
 // ((i,j),(i+1,j),(i,j+1) at k and k+1).  Here each CTA marches upward through kb k-levels
@@ -10,6 +11,7 @@
 // Compiled with --fmad=false (see k_pointwise.cu).
 #include <type_traits>
 
+#include "march.cuh"
 #include "precision.cuh"
 #include "stencil_util.cuh"
 #include "tangent.cuh"
@@ -125,6 +127,84 @@ struct fastwavesuv_kernel {
   }
 };
 
+// FP32 fastwavesuv, marching rows (march.cuh) of one level: lane = column i0 + lane, 31 columns a strip.
+// Each row's ppgc, hhl sum and difference, ppuv and rho are formed once; uout at that row takes the
+// lane above's, vout at the row before takes the row's own.  ppgk at k and k+1 are both formed (the
+// level's neighbours are read again from L2, where the CTAs of the levels beside it have just read
+// them).  fastwavesuv_kernel's operations on the same operands in the same order: the same bits.
+//
+// What bounds it: instruction issue (about 190 instructions a row, its four IEEE divisions a quarter of
+// them) and DRAM latency; DRAM moves the inputs and outputs once.  64 registers, four CTAs an SM:
+// 49.8 us at 256 x 256 x 80 (0.62 of the HBM copy rate), 17.3 at 128 x 128 x 80, 113.9 at
+// 320 x 304 x 137 (five CTAs 48.3 / 17.3 / 114.0, slower on small domains; six, which spills, 75.2);
+// fastwavesuv_kernel<float>'s shared-memory tile took 95.7, 33.5 and 228.8 us.
+struct fastwavesuv_march_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpFwsFwd);  // the step kernel's id
+  static constexpr int kCols = 31, kApron = 1, kMinCtas = 4;
+  struct Row {
+    float w0, w1, pm, p0, p1, h0, h1, r;  // row j: wgtfac, ppuv, hhl at k (and beside it), rho
+    float u, ut, v, vt;                   // uin, utens on row j; vin, vtens on row j - 1
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uout, float* __restrict__ vout,
+                                             const float* __restrict__ uin, const float* __restrict__ vin,
+                                             const float* __restrict__ utens, const float* __restrict__ vtens,
+                                             const float* __restrict__ wgtfac, const float* __restrict__ ppuv,
+                                             const float* __restrict__ hhl, const float* __restrict__ rho,
+                                             const float* __restrict__ fx, int64_t s1d, float ed2, float dt, Dims d,
+                                             int rows, int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = min(i0 + lane, nx);  // lanes past the reach repeat its last column
+    const bool st = lane < kCols && i0 + lane < nx;
+    const int64_t sjb = d.sj * 4, skb = d.sk * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, j)
+    const int64_t oi = (int64_t)(min(i, nx - 1) - i) * 4;              // to an interior column
+    float lf;
+    auto metric = [&](int j) { lf = 2.f * ld(fx + (int64_t)min(j + lane, ny - 1) * s1d); };
+    metric(ja);
+    Row n;
+    auto fetch = [&](int j, int64_t q) {
+      n.w0 = get(wgtfac, q), n.w1 = get(wgtfac, q + skb);
+      n.pm = get(ppuv, q - skb), n.p0 = get(ppuv, q), n.p1 = get(ppuv, q + skb);
+      n.h0 = get(hhl, q), n.h1 = get(hhl, q + skb), n.r = get(rho, q);
+      if (j < jb) n.u = get(uin, q + oi), n.ut = get(utens, q + oi);
+      if (j > ja) n.v = get(vin, q + oi - sjb), n.vt = get(vtens, q + oi - sjb);
+    };
+    fetch(ja, o);
+    float pc = 0.f, hs = 0.f, hd = 0.f, p = 0.f, r = 0.f;  // of row j - 1
+#pragma unroll 1
+    for (int j = ja; j <= jb; ++j) {
+      const Row c = n;
+      if (j < jb) fetch(j + 1, o + sjb);
+      const float cur = c.w0 * c.p0 + (1.f - c.w0) * c.pm;   // ppgk at k (fastwavesuv.h:162)
+      const float next = c.w1 * c.p1 + (1.f - c.w1) * c.p0;  // and at k + 1
+      const float pcj = next - cur, hsj = c.h1 + c.h0, hdj = c.h1 - c.h0;
+      if (j < jb) {
+        const int src = (j - ja) & 31;
+        if (src == 0 && j > ja) metric(j);
+        const float fx2 = __shfl_sync(kWarpMask, lf, src);
+        // fastwavesuv.h:172-175, :182-183
+        // (a lane that writes nothing has itself or a copy above it: 1 in place of its zero numerator,
+        // which would send the warp through the division's slow path)
+        const float num = (0.5f * (lane_above<1>(pcj) + pcj)) * (hsj - lane_above<1>(hsj));
+        const float ppgu = (lane_above<1>(c.p0) - c.p0) + (st ? num : 1.f) / (hdj + lane_above<1>(hdj));
+        const float uo = c.u + dt * (c.ut - ppgu * (fx2 / (lane_above<1>(c.r) + c.r)));
+        if (st) put(uout, o, uo);
+      }
+      if (j > ja) {
+        // fastwavesuv.h:177-180, :185-186, at row j - 1
+        const float ppgv = (c.p0 - p) + ((0.5f * (pcj + pc)) * (hs - hsj)) / (hd + hdj);
+        const float vo = c.v + dt * (c.vt - ppgv * (ed2 / (c.r + r)));
+        if (st) put(vout, o - sjb, vo);
+      }
+      pc = pcj, hs = hsj, hd = hdj, p = c.p0, r = c.r;
+      o += sjb;
+    }
+  }
+};
+
 constexpr int kKB = 1;     // k-levels per CTA by default (the most CTAs hide latency best)
 // the adjoint march's k-levels per CTA (measured at 128 x 128 x 80: FP64 best at 3, FP32 at
 // 2; a block of kb levels reads the coefficients of kb + 2)
@@ -161,11 +241,19 @@ oeb_status fastwavesuv_entry(const M3* uout, const M3* vout, const M3* uin, cons
   OEB_RETURN_IF_VALIDATING();
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gu.sj, gu.sk};
   const T ed2 = T(2.0) * edadlat;  // ElementType(2.0) * edadlat, fastwavesuv.h:186
-  const int kb = tuned_kb(kKB);
-  return launch<fastwavesuv_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(FastwavesSmem<T>),
+  if constexpr (std::is_same<T, float>::value) {
+    using B = fastwavesuv_march_f32;
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, gut.origin,
+                     gvt.origin, gw.origin, gp.origin, gh.origin, gr.origin, lfx.origin, lfx.s, ed2, dt, d, m.rows,
+                     m.wx_log);
+  } else {
+    const int kb = tuned_kb(kKB);
+    return launch<fastwavesuv_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(FastwavesSmem<T>),
                                        (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, gut.origin,
                                        gvt.origin, gw.origin, gp.origin, gh.origin, gr.origin, lfx.origin, lfx.s, ed2,
                                        dt, d, kb);
+  }
 }
 
 // Tangent-linear fastwavesuv with respect to (uin, vin, utens, vtens, ppuv); wgtfac, hhl,

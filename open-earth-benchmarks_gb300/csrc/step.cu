@@ -64,7 +64,7 @@ struct OpList {};
 // adjoints in either form (oeb_set_adjoint_tiles).
 using StepBodies = OpList<
     step_ch::combine_kernel<F64i>, step_ch::combine_kernel<float>,
-    step_fws::fastwavesuv_kernel<F64i>, step_fws::fastwavesuv_kernel<float>,
+    step_fws::fastwavesuv_kernel<F64i>, step_fws::fastwavesuv_march_f32,
     step_fws::fastwavesuv_adj_terms_kernel<F64i>, step_fws::fastwavesuv_adj_kernel<F64i, 0>,
     step_fws::fastwavesuv_adj_kernel<float, 1>,
     step_pw::hadv_kernel<F64i, 5, 0>, step_pw::hadv_kernel<F64i, 5, 1>, step_pw::hadv_kernel<F64i, 5, 2>,

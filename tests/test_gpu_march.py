@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 SIZES = [(1, 1, 1, 3, 0), (5, 3, 2, 3, 0), (26, 4, 3, 3, 0), (27, 5, 2, 4, 1), (30, 33, 2, 3, 0), (31, 9, 2, 3, 2),
          (32, 8, 1, 4, 0), (33, 31, 2, 3, 3), (52, 65, 2, 3, 0), (53, 12, 5, 4, 0), (61, 129, 1, 3, 0),
          (127, 70, 3, 3, 0), (209, 17, 2, 3, 1)]
-NAMES = ("fvtp2d", "hadvuv", "hadvuv5th", "hdiffsa", "hdiffsmag")
+NAMES = ("fvtp2d", "hadvuv", "hadvuv5th", "hdiffsa", "hdiffsmag", "fastwavesuv")
 
 
 @pytest.mark.parametrize("size", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
