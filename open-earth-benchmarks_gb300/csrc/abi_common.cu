@@ -14,7 +14,6 @@
 #include "oeb_common.cuh"
 #include "launch.cuh"
 #include "march.cuh"
-#include "stage.cuh"
 
 namespace oeb {
 
@@ -115,17 +114,6 @@ int device_sms() {
   return sms;
 }
 }  // namespace
-
-int staged_kb(int tiles, int nz, int ctas_per_sm) {
-  const int sms = device_sms();
-  // the most k-chunks per tile that still fit every CTA into one wave, then levels per chunk
-  const long slots = (long)sms * (ctas_per_sm > 0 ? ctas_per_sm : 1);
-  long chunks = tiles > 0 ? slots / tiles : 1;
-  if (chunks < 1) chunks = 1;
-  if (chunks > nz) chunks = nz;
-  const long kb = (nz + chunks - 1) / (chunks > 0 ? chunks : 1);
-  return (int)(kb < 1 ? 1 : kb);
-}
 
 // A chunk of R rows marches R + apron, and about three rows' time passes before its first row's
 // loads have landed; a launch takes at least one wave of CTAs' time, and a part of a wave after

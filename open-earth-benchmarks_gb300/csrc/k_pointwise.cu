@@ -21,7 +21,6 @@
 
 #include "march.cuh"
 #include "precision.cuh"
-#include "stage.cuh"
 #include "stencil_util.cuh"
 #include "tangent.cuh"
 #include "fused.cuh"
@@ -435,204 +434,154 @@ struct hadv_march_f32 {
 
 constexpr int kKB = 1;  // k-levels per CTA (one: the most CTAs, which hides FP64 and load latency best)
 
-// ---- FP32 forms staged through shared memory (stage.cuh) -----------------------------
-// laplace and nh_p_grad: a CTA owns a 32 x 32 tile and the k-levels [k0, k0+kb); the input
-// boxes read at neighbouring points are copied level by level into a ring of NB shared-memory
-// buffers by cp.async, ahead of the level being computed.  nh_p_grad reads level k+1 as well,
-// so it computes level k once levels k and k+1 are resident, with one more level in flight;
-// laplace keeps two levels in flight.  Measured at 256 x 256 x 80 (each stencil alone, average
-// over back-to-back launches): laplace 0.38 -> 0.49 of the HBM copy rate, nh_p_grad 0.32 ->
-// 0.42.  uvbke and p_grad_c measured faster as the plain kernels above (0.69 and 0.60 against
-// 0.62 and 0.48 staged) and keep them: their loads are all independent, and eight CTAs an SM
-// of plain loads keep more bytes in flight than the two or four CTAs their staged rings allowed.
-
-// Marches the levels of a staged CTA: issue(k) copies level k (or commits an empty group),
-// compute(k) reads the resident levels k .. k+LEAD; NB - 1 - LEAD levels are in flight while
-// level k is computed.
-template <int NB, int LEAD, class Issue, class Compute>
-__device__ __forceinline__ void staged_march(int k0, int k1, Issue&& issue, Compute&& compute) {
-  static_assert(NB >= LEAD + 2, "at least one level in flight beyond those a level reads");
-#pragma unroll 1
-  for (int t = 0; t < NB - 1; ++t) issue(k0 + t);
-#pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    issue(k + NB - 1);  // into the buffer level k-1 left
-    cp_async_wait<NB - 1 - LEAD>();  // every level up to k + LEAD has landed
-    __syncthreads();
-    compute(k);
-    __syncthreads();  // the buffer of level k is refilled next
-  }
-}
-
-// laplace.h:39, FP32: one 34 x 34 box of `in` a level, summed in the difference form of
-// laplace_kernel above.
-struct laplace_staged_f32 {
-  static constexpr int NB = 3;
-  static constexpr int kCtasPerSm = 8;
-  using B = RowBox<34, 34>;
-  struct Smem {
-    float in[NB][B::N];
-  };
+// ---- FP32 laplace and pressure gradients ---------------------------------------------------
+// The pressure gradients march rows of one level (march.cuh), each row's values read once.
+// p_grad_c's neighbour is the lane below for u and the row before for v, its two directions one
+// packed evaluation (F2: u in .x, v in .y); nh_p_grad's is the lane above for u and, for v at the
+// row before, the row itself, the paired products of pk3 and pp packed.  The fields read at k and
+// k+1 are read again by the CTAs of the level above, from L2.  The plain kernels' operations on the
+// same operands: the same bits.  Fields in host memory keep the plain kernels.
+//
+// laplace.h:39 has too little arithmetic to hide a row's loads behind the row before: a thread
+// loads its four rows (six with the neighbours', and both x neighbours of the four) at once instead
+// of marching.  31 registers, eight CTAs an SM: 11.0 us at 256 x 256 x 80, 23.5 at 320 x 304 x 137,
+// 3.1 at 128 x 128 x 80 (eight rows 10.9 / 23.1 / 3.2, marching 13.5 / 32.1 / 3.7; boxes staged by
+// cp.async, the form before, 12.3 / 30.2 / 4.4).
+struct laplace_rows_f32 {
+  static constexpr int kRowsPer = 4;
   static __device__ __forceinline__ void run(const uint3& blk, const float* __restrict__ in, float* __restrict__ out,
-                                             Dims d, int kb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-    const int i0 = blk.x * kTI, j0 = blk.y * kTJ;
-    const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
-    const int ie = min(i0 + kTI, d.nx), je = min(j0 + kTJ, d.ny);
-    auto issue = [&](int k) {
-      if (k < k1)
-        stage_rows<34, 34>(s.in[k % NB], in, (int64_t)k * d.sk, i0 - 1, j0 - 1, d.sj, i0 - 1, ie + 1, j0 - 1, je + 1);
-      cp_async_commit();
-    };
-    staged_march<NB, 0>(k0, k1, issue, [&](int k) {
-      const int64_t kofs = (int64_t)k * d.sk;
-      const RowMis mis = row_mis(in, kofs, i0 - 1, j0 - 1, d.sj);
-      const float* t = s.in[k % NB];
-      const int a = threadIdx.x, i = i0 + a;
-      if (i >= ie) return;
+                                             Dims d) {
+    constexpr int R = kRowsPer;
+    const int i = blk.x * 32 + (int)threadIdx.x, ja = (blk.y * kTY + (int)threadIdx.y) * R;
+    if (i >= d.nx || ja >= d.ny) return;
+    const int64_t sjb = d.sj * 4;
+    const int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, ja)
+    const int last = d.ny - ja;  // row ny is the reach's last
+    float c[R + 2], m[R], p[R];
 #pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        const int b = threadIdx.y + kTY * r, j = j0 + b;
-        if (j < je) {
-          const float* up = t + b * B::SW + mis(b) + a;  // row j-1 from cell i-1
-          const float* mid = t + (b + 1) * B::SW + mis(b + 1) + a;
-          const float* dn = t + (b + 2) * B::SW + mis(b + 2) + a;
-          const float c = mid[1];
-          out[kofs + i + (int64_t)j * d.sj] = ((mid[0] - c) + (mid[2] - c)) + ((dn[1] - c) + (up[1] - c));
-        }
-      }
-    });
+    for (int r = -1; r <= R; ++r) {
+      const int64_t q = o + (r <= last ? r : last) * sjb;
+      c[r + 1] = get(in, q);
+      if (r >= 0 && r < R) m[r] = get(in, q - 4), p[r] = get(in, q + 4);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (r < last) put(out, o + r * sjb, ((m[r] - c[r + 1]) + (p[r] - c[r + 1])) + ((c[r + 2] - c[r + 1]) + (c[r] - c[r + 1])));
   }
 };
 
-// The four fields a staged nh_p_grad thread reads at its own points only, loaded into registers
-// one level ahead of the level it computes (the loads of level k+1 are in flight while level k
-// is computed).
-struct PointRegs {
-  float v[4][kRows];
-  __device__ __forceinline__ void fetch(const float* __restrict__ f0, const float* __restrict__ f1,
-                                        const float* __restrict__ f2, const float* __restrict__ f3, int64_t kofs,
-                                        int i, int j0, int je, int64_t sj) {
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      const int j = j0 + (int)threadIdx.y + kTY * r;
-      const bool ok = j < je;
-      const int64_t o = kofs + i + (int64_t)(ok ? j : j0) * sj;
-      v[0][r] = ok ? ld(f0 + o) : 0.f;
-      v[1][r] = ok ? ld(f1 + o) : 0.f;
-      v[2][r] = ok ? ld(f2 + o) : 0.f;
-      v[3][r] = ok ? ld(f3 + o) : 0.f;
+// p_grad_c.h:80-101.  Bound by DRAM and instruction issue about alike: 38.1 us at 256 x 256 x 80 (0.73
+// of the HBM copy rate), 89.3 at 320 x 304 x 137, 13.2 at 128 x 128 x 80 with 48 registers, five CTAs
+// an SM (four 45.6 / 104.8 / 15.8, six, which spills, 39.9 / 92.7 / 14.1); p_grad_c_kernel<float>, a
+// point at a time, took 44.5, 106.5 and 15.2 us.
+struct p_grad_c_march_f32 {
+  static constexpr int kCols = 31, kApron = 1, kMinCtas = 5;
+  struct Row {
+    float g0, g1, p0, p1, w, u, v, rx, ry;
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uout, float* __restrict__ vout,
+                                             const float* __restrict__ uin, const float* __restrict__ vin,
+                                             const float* __restrict__ rdxc, const float* __restrict__ rdyc,
+                                             const float* __restrict__ delpc, const float* __restrict__ gz,
+                                             const float* __restrict__ pkc, float dt2, Dims d, int rows, int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = min(i0 - 1 + lane, nx - 1);  // lanes past the domain repeat its last column
+    const bool st = lane >= 1 && i0 - 1 + lane < nx;
+    const int64_t sjb = d.sj * 4, skb = d.sk * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, j)
+    const int64_t oi = (int64_t)(max(i, 0) - i) * 4;                   // to an interior column
+    auto fetch = [&](int64_t q) {
+      return Row{get(gz, q), get(gz, q + skb), get(pkc, q), get(pkc, q + skb), get(delpc, q),
+                 get(uin, q + oi), get(vin, q + oi), get(rdxc, q + oi), get(rdyc, q + oi)};
+    };
+    // of row j - 1
+    float g0 = get(gz, o - sjb), g1 = get(gz, o - sjb + skb), p0 = get(pkc, o - sjb), p1 = get(pkc, o - sjb + skb),
+          w = get(delpc, o - sjb);
+    Row n = fetch(o);
+#pragma unroll 1
+    for (int j = ja; j < jb; ++j) {
+      const Row c = n;
+      if (j + 1 < jb) n = fetch(o + sjb);
+      const F2 g0n{lane_below<1>(c.g0), g0}, g1n{lane_below<1>(c.g1), g1}, p0n{lane_below<1>(c.p0), p0},
+          p1n{lane_below<1>(c.p1), p1};
+      const F2 gc0{c.g0, c.g0}, gc1{c.g1, c.g1}, pc0{c.p0, c.p0}, pc1{c.p1, c.p1};
+      const F2 f = dot_diff2(diff2(g1n, gc0), diff2(pc1, p0n), diff2(g0n, gc1), diff2(p1n, pc0));
+      const float uo = c.u + ((dt2 * c.rx) / (lane_below<1>(c.w) + c.w)) * f.x;
+      const float vo = c.v + ((dt2 * c.ry) / (w + c.w)) * f.y;
+      if (st) put(uout, o, uo), put(vout, o, vo);
+      g0 = c.g0, g1 = c.g1, p0 = c.p0, p1 = c.p1, w = c.w;
+      o += sjb;
     }
   }
 };
 
-// nh_p_grad.h:121-141, FP32: gz, pp, pk3 staged on 33 x 33 from (i0, j0) at k and k+1, wk1 at
-// k; uin, vin, rdx, rdy in registers a level ahead.
-struct nh_p_grad_staged_f32 {
-  static constexpr int NB = 3;
-  static constexpr int kCtasPerSm = 3;
-  static constexpr int kMinCtas = 3;  // registers for three CTAs an SM
-  using Q = RowBox<33, 33>;
-  struct Level {
-    float gz[Q::N], pp[Q::N], pk[Q::N], w1[Q::N];
-  };
-  struct Smem {
-    Level l[NB];
+// nh_p_grad.h:121-141.  Bound by instruction issue (about 250 a row: 52 packed for the two paired
+// products, four IEEE divisions).  64 registers, four CTAs an SM, two rows unrolled: 52.5 us at
+// 256 x 256 x 80, 120 at 320 x 304 x 137, 18.5 at 128 x 128 x 80 (three CTAs 61.3 / 137.9 / 17.7, five,
+// which spills, 69 / 172 / 25; the two directions instead of the two products in the halves, which
+// takes twenty more register moves a row, 55.8 / 125 / 19.7); the form before it, boxes staged by
+// cp.async and marched over the levels, took 69.7, 194.4 and 21.0 us.
+struct nh_p_grad_march_f32 {
+  static constexpr int kCols = 31, kApron = 1, kMinCtas = 4;
+  struct Row {
+    float g0, g1, p0, p1, q0, q1, w;  // row j: gz, pk3, pp at k and k + 1, wk1
+    float u, rx, v, ry;               // uin, rdx on row j; vin, rdy on row j - 1
   };
   static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uout, float* __restrict__ vout,
                                              const float* __restrict__ uin, const float* __restrict__ vin,
                                              const float* __restrict__ rdx, const float* __restrict__ rdy,
                                              const float* __restrict__ gz, const float* __restrict__ pp,
                                              const float* __restrict__ pk3, const float* __restrict__ wk1, float dt,
-                                             Dims d, int kb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-    const int i0 = blk.x * kTI, j0 = blk.y * kTJ;
-    const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
-    const int ie = min(i0 + kTI, d.nx), je = min(j0 + kTJ, d.ny);
-    const int a = threadIdx.x, i = i0 + a;
-    const int ic = i < ie ? i : i0;  // a column of the tile for the register loads
-    auto issue = [&](int k) {
-      if (k <= k1) {  // level k1 only for the fields read at k+1
-        const int64_t ko = (int64_t)k * d.sk;
-        Level& L = s.l[k % NB];
-        if (k < k1) stage_rows<33, 33>(L.w1, wk1, ko, i0, j0, d.sj, i0, ie + 1, j0, je + 1);
-        stage_rows<33, 33>(L.gz, gz, ko, i0, j0, d.sj, i0, ie + 1, j0, je + 1);
-        stage_rows<33, 33>(L.pp, pp, ko, i0, j0, d.sj, i0, ie + 1, j0, je + 1);
-        stage_rows<33, 33>(L.pk, pk3, ko, i0, j0, d.sj, i0, ie + 1, j0, je + 1);
-      }
-      cp_async_commit();
+                                             Dims d, int rows, int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (i0 >= nx || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = min(i0 + lane, nx);  // lanes past the reach repeat its last column
+    const bool st = lane < kCols && i0 + lane < nx;
+    const int64_t sjb = d.sj * 4, skb = d.sk * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)ja * d.sj + i) * 4;  // (i, j)
+    const int64_t oi = (int64_t)(min(i, nx - 1) - i) * 4;              // to an interior column
+    Row n;
+    auto fetch = [&](int j, int64_t q) {
+      n.g0 = get(gz, q), n.g1 = get(gz, q + skb), n.p0 = get(pk3, q), n.p1 = get(pk3, q + skb);
+      n.q0 = get(pp, q), n.q1 = get(pp, q + skb), n.w = get(wk1, q);
+      if (j < jb) n.u = get(uin, q + oi), n.rx = get(rdx, q + oi);
+      if (j > ja) n.v = get(vin, q + oi - sjb), n.ry = get(rdy, q + oi - sjb);
     };
-    PointRegs cur;
-    cur.fetch(uin, vin, rdx, rdy, (int64_t)k0 * d.sk, ic, j0, je, d.sj);
-    staged_march<NB, 1>(k0, k1, issue, [&](int k) {
-      PointRegs nxt;
-      if (k + 1 < k1) nxt.fetch(uin, vin, rdx, rdy, (int64_t)(k + 1) * d.sk, ic, j0, je, d.sj);
-      const int64_t kofs = (int64_t)k * d.sk, kofs1 = kofs + d.sk;
-      const Level& C = s.l[k % NB];
-      const Level& N = s.l[(k + 1) % NB];
-      const RowMis mw = row_mis(wk1, kofs, i0, j0, d.sj);
-      const RowMis mg0 = row_mis(gz, kofs, i0, j0, d.sj), mg1 = row_mis(gz, kofs1, i0, j0, d.sj);
-      const RowMis mq0 = row_mis(pp, kofs, i0, j0, d.sj), mq1 = row_mis(pp, kofs1, i0, j0, d.sj);
-      const RowMis mp0 = row_mis(pk3, kofs, i0, j0, d.sj), mp1 = row_mis(pk3, kofs1, i0, j0, d.sj);
-      if (i < ie) {
-#pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-          const int b = threadIdx.y + kTY * r, j = j0 + b;
-          if (j < je) {
-            // rows j (box row b) and j+1 (box row b+1); cell i is a in them
-            const float* wc = C.w1 + b * Q::SW + mw(b) + a;
-            const float* wn = C.w1 + (b + 1) * Q::SW + mw(b + 1) + a;
-            const float* g0c = C.gz + b * Q::SW + mg0(b) + a;
-            const float* g0n = C.gz + (b + 1) * Q::SW + mg0(b + 1) + a;
-            const float* g1c = N.gz + b * Q::SW + mg1(b) + a;
-            const float* g1n = N.gz + (b + 1) * Q::SW + mg1(b + 1) + a;
-            const float* q0c = C.pp + b * Q::SW + mq0(b) + a;
-            const float* q0n = C.pp + (b + 1) * Q::SW + mq0(b + 1) + a;
-            const float* q1c = N.pp + b * Q::SW + mq1(b) + a;
-            const float* q1n = N.pp + (b + 1) * Q::SW + mq1(b + 1) + a;
-            const float* p0c = C.pk + b * Q::SW + mp0(b) + a;
-            const float* p0n = C.pk + (b + 1) * Q::SW + mp0(b + 1) + a;
-            const float* p1c = N.pk + b * Q::SW + mp1(b) + a;
-            const float* p1n = N.pk + (b + 1) * Q::SW + mp1(b + 1) + a;
-            const float pk0 = p0c[0], pk1 = p1c[0], gz0 = g0c[0], gz1 = g1c[0], pp0 = q0c[0], pp1 = q1c[0];
-            const float w1 = wc[0];
-            const float wk = pk1 - pk0;
-            const int64_t o = kofs + i + (int64_t)j * d.sj;
-            {  // u: neighbour i+1
-              const float pkx0 = p0c[1], pkx1 = p1c[1];
-              const float wkx = pkx1 - pkx0;
-              const float gx0 = g0c[1], gx1 = g1c[1];
-              const float fk = diff_dot(gz1, gx0, pkx1, pk0, gz0, gx1, pk1, pkx0);
-              const float fp = diff_dot(gz1, gx0, q1c[1], pp0, gz0, gx1, pp1, q0c[1]);
-              const float du = ((dt / (wk + wkx)) * fk);
-              uout[o] = (((cur.v[0][r] + du) + ((dt / (w1 + wc[1])) * fp)) * cur.v[2][r]);
-            }
-            {  // v: neighbour j+1
-              const float pky0 = p0n[0], pky1 = p1n[0];
-              const float wky = pky1 - pky0;
-              const float gy0 = g0n[0], gy1 = g1n[0];
-              const float fk = diff_dot(gz1, gy0, pky1, pk0, gz0, gy1, pk1, pky0);
-              const float fp = diff_dot(gz1, gy0, q1n[0], pp0, gz0, gy1, pp1, q0n[0]);
-              const float dv = ((dt / (wk + wky)) * fk);
-              vout[o] = (((cur.v[1][r] + dv) + ((dt / (w1 + wn[0])) * fp)) * cur.v[3][r]);
-            }
-          }
-        }
-      }
-      cur = nxt;
-    });
+    n.u = n.rx = n.v = n.ry = 0.f;
+    fetch(ja, o);
+    Row b = n;  // of row j - 1 (at ja: nothing it gives is written)
+    float wb = n.p1 - n.p0;
+#pragma unroll 2
+    for (int j = ja; j <= jb; ++j) {
+      const Row c = n;
+      if (j < jb) fetch(j + 1, o + sjb);
+      // one direction: of a cell a and its neighbour e, (fk, fp) in the halves
+      auto pair = [](const Row& a, const Row& e) {
+        const Diff2 g = diff2(F2{a.g1, a.g0}, F2{e.g0, e.g1});
+        const Diff2 y = diff2(F2{e.p1, e.q1}, F2{a.p0, a.q0}), t = diff2(F2{a.p1, a.q1}, F2{e.p0, e.q0});
+        return dot_diff2(Diff2{F2{g.s.x, g.s.x}, F2{g.e.x, g.e.x}}, y, Diff2{F2{g.s.y, g.s.y}, F2{g.e.y, g.e.y}}, t);
+      };
+      Row e;  // the lane above
+      e.g0 = lane_above<1>(c.g0), e.g1 = lane_above<1>(c.g1), e.p0 = lane_above<1>(c.p0), e.p1 = lane_above<1>(c.p1);
+      e.q0 = lane_above<1>(c.q0), e.q1 = lane_above<1>(c.q1), e.w = lane_above<1>(c.w);
+      // u at row j against the lane above, v at row j - 1 against row j
+      const F2 fu = pair(c, e), fv = pair(b, c);
+      const float wc = c.p1 - c.p0;
+      const float uo = ((c.u + (dt / (wc + (e.p1 - e.p0))) * fu.x) + (dt / (c.w + e.w)) * fu.y) * c.rx;
+      const float vo = ((c.v + (dt / (wb + wc)) * fv.x) + (dt / (b.w + c.w)) * fv.y) * c.ry;
+      wb = wc;
+      if (st && j < jb) put(uout, o, uo);
+      if (st && j > ja) put(vout, o - sjb, vo);
+      b = c;
+      o += sjb;
+    }
   }
 };
-
-// Grid and k-levels a CTA of a staged body: about one wave of CTAs (stage.cuh).
-template <class S>
-void staged_launch_shape(const oeb_domain& dom, dim3* grid, int* kb) {
-  const int tiles = (int)(((dom.nx + kTI - 1) / kTI) * ((dom.ny + kTJ - 1) / kTJ));
-  *kb = tuned_kb(staged_kb(tiles, (int)dom.nz, S::kCtasPerSm));
-  *grid = tile_grid((int)dom.nx, (int)dom.ny, (int)dom.nz, kTI, kTJ, *kb);
-}
 
 template <class T>
 Dims make_dims(const oeb_domain& dom, const Grid<T>& g) {
@@ -653,11 +602,10 @@ oeb_status laplace_entry(const M3* in, const M3* out, const oeb_domain* dom, voi
   OEB_TRY(check_no_alias({gout.lo, gout.hi}, {gin.lo, gin.hi}));
   OEB_RETURN_IF_VALIDATING();
   if constexpr (std::is_same<T, float>::value) if (!fields_in_host_memory()) {
-    dim3 grid;
-    int kb;
-    staged_launch_shape<laplace_staged_f32>(*dom, &grid, &kb);
-    return launch<laplace_staged_f32>(grid, sizeof(laplace_staged_f32::Smem), (cudaStream_t)stream, gin.origin,
-                                      gout.origin, make_dims(*dom, gin), kb);
+    using B = laplace_rows_f32;
+    const Dims d = make_dims(*dom, gin);
+    return launch<B>(tile_grid(d.nx, d.ny, d.nz, 32, kTY * B::kRowsPer, 1), 0, (cudaStream_t)stream, gin.origin,
+                     gout.origin, d);
   }
   const int kb = tuned_kb(kKB);
   return launch<laplace_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, gin.origin, gout.origin,
@@ -708,6 +656,13 @@ oeb_status p_grad_c_entry(const M3* uout, const M3* vout, const M3* uin, const M
   Grid<T> g[9];
   OEB_TRY(p_grad_c_check<T>(uout, vout, uin, vin, rdxc, rdyc, delpc, gz, pkc, dom, g));
   OEB_RETURN_IF_VALIDATING();
+  if constexpr (std::is_same<T, float>::value) if (!fields_in_host_memory()) {
+    using B = p_grad_c_march_f32;
+    const Dims d = make_dims(*dom, g[0]);
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, (cudaStream_t)stream, g[0].origin, g[1].origin, g[2].origin, g[3].origin, g[4].origin,
+                     g[5].origin, g[6].origin, g[7].origin, g[8].origin, dt2, d, m.rows, m.wx_log);
+  }
   const int kb = tuned_kb(kKB);
   return launch<p_grad_c_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
                                     g[2].origin, g[3].origin, g[4].origin, g[5].origin, g[6].origin, g[7].origin,
@@ -739,12 +694,11 @@ oeb_status nh_p_grad_entry(const M3* uout, const M3* vout, const M3* uin, const 
   OEB_TRY(nh_p_grad_check<T>(uout, vout, uin, vin, rdx, rdy, gz, pp, pk3, wk1, dom, g));
   OEB_RETURN_IF_VALIDATING();
   if constexpr (std::is_same<T, float>::value) if (!fields_in_host_memory()) {
-    dim3 grid;
-    int kb;
-    staged_launch_shape<nh_p_grad_staged_f32>(*dom, &grid, &kb);
-    return launch<nh_p_grad_staged_f32>(grid, sizeof(nh_p_grad_staged_f32::Smem), (cudaStream_t)stream, g[0].origin,
-                                        g[1].origin, g[2].origin, g[3].origin, g[4].origin, g[5].origin, g[6].origin,
-                                        g[7].origin, g[8].origin, g[9].origin, dt, make_dims(*dom, g[0]), kb);
+    using B = nh_p_grad_march_f32;
+    const Dims d = make_dims(*dom, g[0]);
+    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    return launch<B>(m.grid, 0, (cudaStream_t)stream, g[0].origin, g[1].origin, g[2].origin, g[3].origin, g[4].origin,
+                     g[5].origin, g[6].origin, g[7].origin, g[8].origin, g[9].origin, dt, d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
   return launch<nh_p_grad_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,

@@ -44,8 +44,8 @@ struct ValidateOnly {
   } while (0)
 
 // While a HostInPlace guard is alive on this thread, the fields the entry points receive are
-// host memory the device reads in place (the host entry points' direct mode); the kernels that
-// stage their tiles with cp.async then keep to ordinary loads, which are what that mode was
+// host memory the device reads in place (the host entry points' direct mode); the FP32 laplace,
+// hdiffsa, p_grad_c and nh_p_grad then keep their plain kernels, which are what that mode was
 // measured and tested with.
 bool fields_in_host_memory();
 struct HostInPlace {

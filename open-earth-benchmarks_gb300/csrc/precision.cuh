@@ -548,6 +548,57 @@ __device__ __forceinline__ T diff_dot(T a, T b, T c, T d, T e, T f, T g, T h) {
   }
 }
 
+// Two FP32 values computed by the packed FP32 instructions (PTX add/mul/fma.rn.f32x2): one issue slot
+// for both, each half rounded as the scalar operation rounds it.  a - b is fma(b, -1, a).  ptxas
+// (CUDA 13.0) was seen to contract a mul.rn.f32x2 and the add.rn.f32x2 of its result into one fma,
+// which rounds once instead of twice: no product may be an operand of + or - here.
+struct F2 {
+  float x, y;
+};
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+      " fma.rn.f32x2 a, a, b, c;\n mov.b64 {%0, %1}, a;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("{\n .reg .b64 a, b;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 a, a, b;\n"
+      " mov.b64 {%0, %1}, a;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("{\n .reg .b64 a, b;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mul.rn.f32x2 a, a, b;\n"
+      " mov.b64 {%0, %1}, a;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, F2{-1.f, -1.f}, a); }
+__device__ __forceinline__ F2 neg2(F2 a) { return F2{-a.x, -a.y}; }
+
+// A difference a - b as the TwoSum pair s + e.
+struct Diff2 {
+  F2 s, e;
+};
+__device__ __forceinline__ Diff2 diff2(F2 a, F2 b) {
+  const F2 s = sub2(a, b), bb = sub2(s, a);
+  return Diff2{s, add2(sub2(a, sub2(s, bb)), sub2(neg2(b), bb))};
+}
+// diff_dot's evaluation of x y + z w for differences x, y, z, w already formed, in both halves.
+__device__ __forceinline__ F2 dot_diff2(const Diff2& x, const Diff2& y, const Diff2& z, const Diff2& w) {
+  const F2 q = mul2(z.s, w.s);
+  const F2 qe = fma2(z.s, w.s, neg2(q));
+  const F2 m = fma2(x.s, y.s, q);
+  const F2 low = fma2(x.s, y.e, fma2(x.e, y.s, fma2(z.s, w.e, fma2(z.e, w.s, qe))));
+  return add2(m, low);
+}
+
 // The same paired products for fields stored as an FP64 per-level base profile plus FP32
 // perturbations: each difference is a base difference between two levels, D (FP32, formed once
 // a level from the FP64 profile), plus the difference of the perturbations, a - b.  a - b is a

@@ -44,3 +44,26 @@ def test_marching_kernel_is_the_float_oracle(pkg, fields, orc, cuda, name, size)
         np.testing.assert_array_equal(got[..., :nx + 2 * h].copy().view(np.uint32), want[a.name].view(np.uint32),
                                       err_msg="%s.%s %s vs the float oracle" % (name, a.name, size))
         assert (got[..., nx + 2 * h:] == np.float32(fields.SENTINEL)).all(), "%s.%s wrote its row padding" % (name, a.name)
+
+
+@pytest.mark.parametrize("size", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
+@pytest.mark.parametrize("name", ("laplace", "p_grad_c", "nh_p_grad"))
+def test_row_kernels_match_the_plain_kernels(pkg, fields, cuda, name, size):
+    """The FP32 stencils whose arithmetic is not the reference's float sequence: the plain kernels,
+    which run where the fields lie in host memory, give the same bits."""
+    import torch
+    nx, ny, nz, h, pad = size
+    spec = pkg.KERNELS[name]
+    inputs = fields.make_inputs(name, nx, ny, nz, seed=29, workload="fronts", halo=h)
+    sc = {k: float(np.float32(v)) for k, v in fields.make_scalars(name, seed=29).items()}
+    arrays = {k: np.pad(v.astype(np.float32), ((0, 0), (0, 0), (0, pad)), constant_values=fields.SENTINEL)
+              for k, v in {**inputs, **fields.make_outputs(name, nx, ny, nz, halo=h)}.items()}
+    assert pkg.load_library().oeb_set_host_direct(1) == 0
+    host = {k: pkg.Storage(torch.from_numpy(v.copy()).pin_memory(), h, nx=nx) for k, v in arrays.items()}
+    dev = {k: pkg.Storage(torch.from_numpy(v.copy()).to(cuda), h, nx=nx) for k, v in arrays.items()}
+    pkg.call(name, host, sc, domain=(nx, ny, nz))
+    pkg.call(name, dev, sc, domain=(nx, ny, nz))
+    torch.cuda.synchronize()
+    for a in spec.by_role("out3"):
+        np.testing.assert_array_equal(dev[a.name].numpy().view(np.uint32), host[a.name].numpy().view(np.uint32),
+                                      err_msg="%s.%s %s vs the plain kernel" % (name, a.name, size))
