@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "precision.cuh"
+#include "stencil_util.cuh"
 
 namespace oeb {
 
@@ -68,14 +69,54 @@ OEB_DUAL_CMP(<=)
 OEB_DUAL_CMP(>=)
 #undef OEB_DUAL_CMP
 
+// A field of dual numbers as a kernel reads it: the values and the derivatives where they lie, in two
+// fields of one layout (d null: a parameter, whose derivative is zero).
 template <class T>
-__device__ __forceinline__ Dual<T> ld(const Dual<T>* p) {
-  const T* q = reinterpret_cast<const T*>(p);
+struct DualIn {
+  const T *v, *d;
+};
+template <class T>
+__device__ __forceinline__ DualIn<T> operator+(DualIn<T> p, int64_t o) {
+  return DualIn<T>{p.v + o, p.d ? p.d + o : p.d};
+}
+template <class T>
+__device__ __forceinline__ DualIn<T> operator-(DualIn<T> p, int64_t o) {
+  return p + -o;
+}
+template <class T>
+__device__ __forceinline__ Dual<T> ld(DualIn<T> p) {
 #ifdef OEB_COHERENT_LOADS  // the step kernel: see ld() in stencil_util.cuh
-  return Dual<T>(__ldca(q), __ldca(q + 1));
+  return Dual<T>(__ldca(p.v), p.d ? __ldca(p.d) : T(0));
 #else
-  return Dual<T>(__ldg(q), __ldg(q + 1));
+  return Dual<T>(__ldg(p.v), p.d ? __ldg(p.d) : T(0));
 #endif
+}
+// The same as a kernel writes it (v null: the values are not wanted).
+template <class T>
+struct DualOut {
+  T *v, *d;
+  struct Ref {
+    T *v, *d;
+    __device__ __forceinline__ void operator=(Dual<T> x) const {
+      if (v) *v = x.v;
+      *d = x.d;
+    }
+  };
+  __device__ __forceinline__ Ref operator[](int64_t o) const { return Ref{v ? v + o : v, d + o}; }
+};
+template <class T>
+struct PtrOf<Dual<T>> {
+  using in = DualIn<T>;
+  using out = DualOut<T>;
+};
+template <class T>
+struct StoredSize<Dual<T>> {
+  static constexpr int value = (int)sizeof(T);
+};
+template <class T>
+__device__ __forceinline__ void prefetch_l2(DualIn<T> p) {
+  prefetch_l2(p.v);
+  if (p.d) prefetch_l2(p.d);
 }
 
 template <class T>

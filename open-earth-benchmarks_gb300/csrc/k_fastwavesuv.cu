@@ -39,12 +39,12 @@ struct FastwavesSmem {
 template <class T>
 struct fastwavesuv_kernel {
   static constexpr int kStepOp = step_op<T>(kOpFwsFwd);  // the step kernel's id
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uout, T* __restrict__ vout,
-                                             const T* __restrict__ uin, const T* __restrict__ vin,
-                                             const T* __restrict__ utens, const T* __restrict__ vtens,
-                                             const T* __restrict__ wgtfac, const T* __restrict__ ppuv,
-                                             const T* __restrict__ hhl, const T* __restrict__ rho,
-                                             const T* __restrict__ fx, int64_t s1d, T ed2, T dt, Dims d, int kb) {
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
+                                             InPtr<T> uin, InPtr<T> vin,
+                                             InPtr<T> utens, InPtr<T> vtens,
+                                             InPtr<T> wgtfac, InPtr<T> ppuv,
+                                             InPtr<T> hhl, InPtr<T> rho,
+                                             InPtr<T> fx, int64_t s1d, T ed2, T dt, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FastwavesSmem<T>& s = *reinterpret_cast<FastwavesSmem<T>*>(smem_raw);
     const int i0 = blk.x * kT, j0 = blk.y * kT;
@@ -79,8 +79,8 @@ struct fastwavesuv_kernel {
   #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * sk;
-      const T* const late[6] = {ppuv, rho, uin, utens, vin, vtens};  // read in the last phase
-      prefetch_tile(late, kofs, i0, j0, d.nx, d.ny, sj);
+      const InPtr<T> late[6] = {ppuv, rho, uin, utens, vin, vtens};  // read in the last phase
+      prefetch_tile<T>(late, kofs, i0, j0, d.nx, d.ny, sj);
   #pragma unroll
       for (int t = 0; t < kOwned; ++t) {
         const int e = tid + t * kThreads;
@@ -273,27 +273,20 @@ oeb_status fastwavesuv_tl_entry(const M3* duout, const M3* dvout, const M3* uin,
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *u, *v, *ut, *vt, *w, *p, *h, *r, *f, *ou, *ov;
-  OEB_TRY(arr.pack(uin, duin, &u));
-  OEB_TRY(arr.pack(vin, dvin, &v));
-  OEB_TRY(arr.pack(utens, dutens, &ut));
-  OEB_TRY(arr.pack(vtens, dvtens, &vt));
-  OEB_TRY(arr.pack(wgtfac, (const M3*)nullptr, &w));
-  OEB_TRY(arr.pack(ppuv, dppuv, &p));
-  OEB_TRY(arr.pack(hhl, (const M3*)nullptr, &h));
-  OEB_TRY(arr.pack(rho, (const M3*)nullptr, &r));
-  OEB_TRY(arr.pack(fx, (const M1*)nullptr, &f));
-  OEB_TRY(arr.alloc(duout, &ou));
-  OEB_TRY(arr.alloc(dvout, &ov));
+  DualIn<T> u, v, ut, vt, p;
+  OEB_TRY((dual_in<T>(uin, duin, &u)));
+  OEB_TRY((dual_in<T>(vin, dvin, &v)));
+  OEB_TRY((dual_in<T>(utens, dutens, &ut)));
+  OEB_TRY((dual_in<T>(vtens, dvtens, &vt)));
+  OEB_TRY((dual_in<T>(ppuv, dppuv, &p)));
+  const DualIn<T> w = dual_param<T>(wgtfac), h = dual_param<T>(hhl), r = dual_param<T>(rho), f = dual_param<T>(fx);
+  const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const D ed2 = D(T(2.0) * edadlat);
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<fastwavesuv_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(FastwavesSmem<D>),
+  return launch<fastwavesuv_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(FastwavesSmem<D>),
                                         (cudaStream_t)stream, ou, ov, u, v, ut, vt, w, p, h, r, f, fx->strides[0], ed2,
-                                        D(dt), d, kb));
-  OEB_TRY(arr.unpack(duout->aligned + duout->offset, ou, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dvout->aligned + dvout->offset, ov, *dom, kInterior, d.sj, d.sk);
+                                        D(dt), d, kb);
 }
 
 // ============================== adjoint ===========================================

@@ -105,12 +105,12 @@ struct FvQSmem {
 template <class T>
 struct fvtp2d_q_kernel {
   static constexpr int kStepOp = step_op<T>(kOpFvQ);  // the step kernel's id
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ q_i, T* __restrict__ q_j,
-                                             T* __restrict__ fx2, T* __restrict__ fy2, const T* __restrict__ q,
-                                             const T* __restrict__ crx, const T* __restrict__ cry,
-                                             const T* __restrict__ ra_x, const T* __restrict__ ra_y,
-                                             const T* __restrict__ xfx, const T* __restrict__ yfx,
-                                             const T* __restrict__ area, T p1, T p2, Dims d, int kb) {
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> q_i, OutPtr<T> q_j,
+                                             OutPtr<T> fx2, OutPtr<T> fy2, InPtr<T> q,
+                                             InPtr<T> crx, InPtr<T> cry,
+                                             InPtr<T> ra_x, InPtr<T> ra_y,
+                                             InPtr<T> xfx, InPtr<T> yfx,
+                                             InPtr<T> area, T p1, T p2, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FvQSmem<T>& s = *reinterpret_cast<FvQSmem<T>*>(smem_raw);
     const int i0 = -3 + (int)blk.x * kT, j0 = -3 + (int)blk.y * kT;
@@ -130,8 +130,8 @@ struct fvtp2d_q_kernel {
         const int ax = lim(nx + 2 - i0, 32);   // columns of fy2 and q_i
         const int yfb = lim(ny + 1 - j0, 33);  // rows of fy2 / fyy
         const int qib = lim(ny - j0, 32);      // rows of q_i
-        const T* const late[4] = {cry, yfx, area, ra_y};  // read after the PPM phases
-        prefetch_tile(late, kofs, i0, j0, nx, ny, sj);
+        const InPtr<T> late[4] = {cry, yfx, area, ra_y};  // read after the PPM phases
+        prefetch_tile<T>(late, kofs, i0, j0, nx, ny, sj);
         // (one row more than the phases read, so that full tiles take the compile-time loop)
         for_region_lim<32, 39>(ax, min(39, max(yfb + 6, qib + 3)), [&](int a, int b) {
           const int i = i0 + a, j = j0 - 3 + b;
@@ -173,8 +173,8 @@ struct fvtp2d_q_kernel {
         const int xfa = lim(nx + 1 - i0, 33);  // columns of fx2 / fxx
         const int by = lim(ny + 2 - j0, 32);   // rows of fx2 and q_j
         const int qja = lim(nx - i0, 32);      // columns of q_j
-        const T* const late[4] = {crx, xfx, area, ra_x};
-        prefetch_tile(late, kofs, i0, j0, nx, ny, sj);
+        const InPtr<T> late[4] = {crx, xfx, area, ra_x};
+        prefetch_tile<T>(late, kofs, i0, j0, nx, ny, sj);
         for_region_lim<38, 32>(min(38, max(xfa + 5, qja + 3)), by, [&](int a, int b) {
           const int i = i0 - 3 + a, j = j0 + b;
           w.q[b][a] = qok(i, j) ? ld(q + kofs + i + j * sj) : T(0);
@@ -250,11 +250,11 @@ struct FvFluxSmem {
 template <class T>
 struct fvtp2d_flux_kernel {
   static constexpr int kStepOp = step_op<T>(kOpFvFlux);  // the step kernel's id
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ fx1, T* __restrict__ fy1,
-                                             const T* __restrict__ q_i, const T* __restrict__ q_j,
-                                             const T* __restrict__ fx2, const T* __restrict__ fy2,
-                                             const T* __restrict__ crx, const T* __restrict__ cry,
-                                             const T* __restrict__ xfx, const T* __restrict__ yfx, T p1, T p2, Dims d,
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> fx1, OutPtr<T> fy1,
+                                             InPtr<T> q_i, InPtr<T> q_j,
+                                             InPtr<T> fx2, InPtr<T> fy2,
+                                             InPtr<T> crx, InPtr<T> cry,
+                                             InPtr<T> xfx, InPtr<T> yfx, T p1, T p2, Dims d,
                                              int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FvFluxSmem<T>& s = *reinterpret_cast<FvFluxSmem<T>*>(smem_raw);
@@ -270,8 +270,8 @@ struct fvtp2d_flux_kernel {
       const int64_t kofs = (int64_t)k * d.sk;
       if (!ysweep) {
         // ---- x-PPM of q_i -> fx1 and the x transport flux
-        const T* const late[3] = {crx, fx2, xfx};  // read in the last phase only
-        prefetch_tile(late, kofs, i0, j0, nx, ny, sj);
+        const InPtr<T> late[3] = {crx, fx2, xfx};  // read in the last phase only
+        prefetch_tile<T>(late, kofs, i0, j0, nx, ny, sj);
         for_region_lim<37, 32>(vx + 5, vy, [&](int a, int b) {
           const int i = i0 - 3 + a, j = j0 + b;
           s.w.x.qi[b][a] = (i < nx + 2 && j < ny) ? ld(q_i + kofs + i + j * sj) : T(0);
@@ -298,8 +298,8 @@ struct fvtp2d_flux_kernel {
         __syncthreads();
       } else {
         // ---- y-PPM of q_j -> fy1 and the y transport flux
-        const T* const late[3] = {cry, fy2, yfx};
-        prefetch_tile(late, kofs, i0, j0, nx, ny, sj);
+        const InPtr<T> late[3] = {cry, fy2, yfx};
+        prefetch_tile<T>(late, kofs, i0, j0, nx, ny, sj);
         for_region_lim<32, 37>(vx, vy + 5, [&](int a, int b) {
           const int i = i0 + a, j = j0 - 3 + b;
           s.w.y.qj[b][a] = (i < nx && j < ny + 2) ? ld(q_j + kofs + i + j * sj) : T(0);
@@ -561,35 +561,41 @@ oeb_status fvtp2d_tl_entry(const M3* dq_i, const M3* dq_j, const M3* dfx1, const
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
+  DualIn<T> x;
+  OEB_TRY((dual_in<T>(q, dq, &x)));
+  const DualIn<T> cx = dual_param<T>(crx), cy = dual_param<T>(cry), rx = dual_param<T>(ra_x),
+                  ry = dual_param<T>(ra_y), xf = dual_param<T>(xfx), yf = dual_param<T>(yfx), ar = dual_param<T>(area);
   cudaStream_t st = (cudaStream_t)stream;
-  DualArrays<T> arr(st);
-  D *x, *cx, *cy, *rx, *ry, *xf, *yf, *ar, *oqi, *oqj, *ofx1, *ofx2, *ofy1, *ofy2;
-  OEB_TRY(arr.pack(q, dq, &x));
-  OEB_TRY(arr.pack(crx, (const M3*)nullptr, &cx));
-  OEB_TRY(arr.pack(cry, (const M3*)nullptr, &cy));
-  OEB_TRY(arr.pack(ra_x, (const M3*)nullptr, &rx));
-  OEB_TRY(arr.pack(ra_y, (const M3*)nullptr, &ry));
-  OEB_TRY(arr.pack(xfx, (const M3*)nullptr, &xf));
-  OEB_TRY(arr.pack(yfx, (const M3*)nullptr, &yf));
-  OEB_TRY(arr.pack(area, (const M3*)nullptr, &ar));
-  OEB_TRY(arr.alloc(dq_i, &oqi));
-  OEB_TRY(arr.alloc(dq_j, &oqj));
-  OEB_TRY(arr.alloc(dfx1, &ofx1));
-  OEB_TRY(arr.alloc(dfx2, &ofx2));
-  OEB_TRY(arr.alloc(dfy1, &ofy1));
-  OEB_TRY(arr.alloc(dfy2, &ofy2));
+  // launch 2 reads the values of q_i, q_j, fx2 and fy2 as well as their derivatives: scratch for them,
+  // each in its output's layout
+  const M3* y[4] = {dq_i, dq_j, dfx2, dfy2};
+  int64_t n[4], org[4], total = 0;
+  for (int f = 0; f < 4; ++f) {
+    const T* start = (y[f]->allocated && y[f]->allocated <= y[f]->aligned) ? y[f]->allocated : y[f]->aligned;
+    int64_t last = 0;
+    for (int r = 0; r < 3; ++r) last += (y[f]->sizes[r] - 1) * y[f]->strides[r];
+    n[f] = (int64_t)(y[f]->aligned - start) + last + 1;
+    org[f] = total + (int64_t)(y[f]->aligned - start) + y[f]->offset;
+    total += n[f];
+  }
+  void* buf = nullptr;
+  OEB_TRY(scratch_alloc(&buf, (size_t)total * sizeof(T), st));
+  T* base = static_cast<T*>(buf);
+  DualOut<T> o[4];
+  DualIn<T> v[4];
+  for (int f = 0; f < 4; ++f) {
+    o[f] = DualOut<T>{base + org[f], y[f]->aligned + y[f]->offset};
+    v[f] = DualIn<T>{o[f].v, o[f].d};
+  }
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, q->strides[1], q->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<fvtp2d_q_kernel<D>>(q_grid(d, kb), sizeof(FvQSmem<D>), st, oqi,
-                                     oqj, ofx2, ofy2, x, cx, cy, rx, ry, xf, yf, ar, D(p1), D(p2), d, kb));
-  OEB_TRY(launch<fvtp2d_flux_kernel<D>>(flux_grid(d, kb), sizeof(FvFluxSmem<D>), st, ofx1,
-                                        ofy1, oqi, oqj, ofx2, ofy2, cx, cy, xf, yf, D(p1), D(p2), d, kb));
-  OEB_TRY(arr.unpack(dq_i->aligned + dq_i->offset, oqi, *dom, kFvQi, d.sj, d.sk));
-  OEB_TRY(arr.unpack(dq_j->aligned + dq_j->offset, oqj, *dom, kFvQj, d.sj, d.sk));
-  OEB_TRY(arr.unpack(dfx1->aligned + dfx1->offset, ofx1, *dom, kInterior, d.sj, d.sk));
-  OEB_TRY(arr.unpack(dfx2->aligned + dfx2->offset, ofx2, *dom, kFvFx2, d.sj, d.sk));
-  OEB_TRY(arr.unpack(dfy1->aligned + dfy1->offset, ofy1, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dfy2->aligned + dfy2->offset, ofy2, *dom, kFvFy2, d.sj, d.sk);
+  oeb_status stt = launch<fvtp2d_q_kernel<D>>(q_grid(d, kb), sizeof(FvQSmem<D>), st, o[0], o[1], o[2], o[3], x, cx, cy,
+                                              rx, ry, xf, yf, ar, D(p1), D(p2), d, kb);
+  if (stt == OEB_OK)
+    stt = launch<fvtp2d_flux_kernel<D>>(flux_grid(d, kb), sizeof(FvFluxSmem<D>), st, dual_out<T>(dfx1),
+                                        dual_out<T>(dfy1), v[0], v[1], v[2], v[3], cx, cy, xf, yf, D(p1), D(p2), d, kb);
+  scratch_free(buf, st);
+  return stt;
 }
 
 // ============================== adjoint ===========================================

@@ -53,9 +53,9 @@ struct HdiffsaSmem {
 
 template <class T>
 struct hdiffsa_kernel {
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ out, const T* __restrict__ in,
-                                             const T* __restrict__ mask, const T* __restrict__ crlato,
-                                             const T* __restrict__ crlatu, int64_t s1d, Dims d, int kb) {
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> out, InPtr<T> in,
+                                             InPtr<T> mask, InPtr<T> crlato,
+                                             InPtr<T> crlatu, int64_t s1d, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HdiffsaSmem<T>& s = *reinterpret_cast<HdiffsaSmem<T>*>(smem_raw);
     const int i0 = blk.x * kT, j0 = blk.y * kT;
@@ -73,7 +73,7 @@ struct hdiffsa_kernel {
   #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * d.sk;
-      const T* pin = in + kofs;
+      const InPtr<T> pin = in + kofs;
       for_region_lim<36, 36>(vx + 4, vy + 4, [&](int a, int b) {
         const int i = i0 - 2 + a, j = j0 - 2 + b;
         const bool ok = i >= -2 && i < d.nx + 2 && j >= -2 && j < d.ny + 2;
@@ -216,11 +216,11 @@ struct HdiffsmagSmem {
 template <class T>
 struct hdiffsmag_kernel {
   static constexpr int kStepOp = step_op<T>(kOpSmagFwd);  // the step kernel's id
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uout, T* __restrict__ vout,
-                                             const T* __restrict__ uin, const T* __restrict__ vin,
-                                             const T* __restrict__ mask, const T* __restrict__ crlavo,
-                                             const T* __restrict__ crlavu, const T* __restrict__ crlato,
-                                             const T* __restrict__ crlatu, const T* __restrict__ acrlat0, int64_t s1d,
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
+                                             InPtr<T> uin, InPtr<T> vin,
+                                             InPtr<T> mask, InPtr<T> crlavo,
+                                             InPtr<T> crlavu, InPtr<T> crlato,
+                                             InPtr<T> crlatu, InPtr<T> acrlat0, int64_t s1d,
                                              T eddlat, T eddlon, T tau_smag, T weight_smag, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HdiffsmagSmem<T>& s = *reinterpret_cast<HdiffsmagSmem<T>*>(smem_raw);
@@ -484,25 +484,17 @@ oeb_status hdiffsmag_tl_entry(const M3* duout, const M3* dvout, const M3* uin, c
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *u, *v, *m, *l0, *l1, *l2, *l3, *l4, *ou, *ov;
-  OEB_TRY(arr.pack(uin, duin, &u));
-  OEB_TRY(arr.pack(vin, dvin, &v));
-  OEB_TRY(arr.pack(mask, (const M3*)nullptr, &m));
-  OEB_TRY(arr.pack(crlavo, (const M1*)nullptr, &l0));
-  OEB_TRY(arr.pack(crlavu, (const M1*)nullptr, &l1));
-  OEB_TRY(arr.pack(crlato, (const M1*)nullptr, &l2));
-  OEB_TRY(arr.pack(crlatu, (const M1*)nullptr, &l3));
-  OEB_TRY(arr.pack(acrlat0, (const M1*)nullptr, &l4));
-  OEB_TRY(arr.alloc(duout, &ou));
-  OEB_TRY(arr.alloc(dvout, &ov));
+  DualIn<T> u, v;
+  OEB_TRY((dual_in<T>(uin, duin, &u)));
+  OEB_TRY((dual_in<T>(vin, dvin, &v)));
+  const DualIn<T> m = dual_param<T>(mask), l0 = dual_param<T>(crlavo), l1 = dual_param<T>(crlavu),
+                  l2 = dual_param<T>(crlato), l3 = dual_param<T>(crlatu), l4 = dual_param<T>(acrlat0);
+  const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<hdiffsmag_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsmagSmem<D>),
+  return launch<hdiffsmag_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsmagSmem<D>),
                                       (cudaStream_t)stream, ou, ov, u, v, m, l0, l1, l2, l3, l4, crlavo->strides[0],
-                                      D(eddlat), D(eddlon), D(tau_smag), D(weight_smag), d, kb));
-  OEB_TRY(arr.unpack(duout->aligned + duout->offset, ou, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dvout->aligned + dvout->offset, ov, *dom, kInterior, d.sj, d.sk);
+                                      D(eddlat), D(eddlon), D(tau_smag), D(weight_smag), d, kb);
 }
 
 // ============================== hdiffsa: tangent-linear and adjoint ===============
@@ -633,18 +625,14 @@ oeb_status hdiffsa_tl_entry(const M3* dout, const M3* in, const M3* mask, const 
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *x, *m, *lo, *lu, *y;
-  OEB_TRY(arr.pack(in, din, &x));
-  OEB_TRY(arr.pack(mask, (const M3*)nullptr, &m));
-  OEB_TRY(arr.pack(crlato, (const M1*)nullptr, &lo));
-  OEB_TRY(arr.pack(crlatu, (const M1*)nullptr, &lu));
-  OEB_TRY(arr.alloc(dout, &y));
+  DualIn<T> x;
+  OEB_TRY((dual_in<T>(in, din, &x)));
+  const DualIn<T> m = dual_param<T>(mask), lo = dual_param<T>(crlato), lu = dual_param<T>(crlatu);
+  const DualOut<T> y = dual_out<T>(dout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<hdiffsa_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsaSmem<D>),
-                                    (cudaStream_t)stream, y, x, m, lo, lu, crlato->strides[0], d, kb));
-  return arr.unpack(dout->aligned + dout->offset, y, *dom, kInterior, d.sj, d.sk);
+  return launch<hdiffsa_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsaSmem<D>),
+                                    (cudaStream_t)stream, y, x, m, lo, lu, crlato->strides[0], d, kb);
 }
 
 template <class T, class M3, class M1>

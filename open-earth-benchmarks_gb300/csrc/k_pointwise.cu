@@ -92,15 +92,15 @@ __device__ __forceinline__ void for_points(const uint3& blk, const Dims& d, int 
 // (`now`) and the level above (`up`, the fields read at k+1) -- 7 % faster at 256 x 256 x 80
 // (the same made p_grad_c 7 % slower; it is not used there).  The FP64 kernels are bound by
 // arithmetic and skip it.
-template <class T, int N, int M>
-__device__ __forceinline__ void prefetch_points(const uint3& blk, const Dims& d, int kb, const T* const (&now)[N],
-                                                const T* const (&up)[M]) {
+template <class T, class P, int N, int M>
+__device__ __forceinline__ void prefetch_points(const uint3& blk, const Dims& d, int kb, const P (&now)[N],
+                                                const P (&up)[M]) {
   if constexpr (std::is_same<T, float>::value) {
     const int i0 = blk.x * kTI, j0 = blk.y * kTJ, sj = (int)d.sj;
     const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
     for (int k = k0; k < k1; ++k) {
-      prefetch_tile(now, (int64_t)k * d.sk, i0, j0, d.nx, d.ny, sj);
-      prefetch_tile(up, (int64_t)(k + 1) * d.sk, i0, j0, d.nx, d.ny, sj);
+      prefetch_tile<T>(now, (int64_t)k * d.sk, i0, j0, d.nx, d.ny, sj);
+      prefetch_tile<T>(up, (int64_t)(k + 1) * d.sk, i0, j0, d.nx, d.ny, sj);
     }
   }
 }
@@ -108,7 +108,7 @@ __device__ __forceinline__ void prefetch_points(const uint3& blk, const Dims& d,
 // ---- laplace: kernels/laplace.h:34-43 ----------------------------------------------
 template <class T>
 struct laplace_kernel {
-  static __device__ __forceinline__ void run(const uint3& blk, const T* __restrict__ in, T* __restrict__ out, Dims d,
+  static __device__ __forceinline__ void run(const uint3& blk, InPtr<T> in, OutPtr<T> out, Dims d,
                                              int kb) {
     const int64_t sj = d.sj;
     for_points<RowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) {
@@ -143,9 +143,9 @@ __device__ __forceinline__ T uvbke_scale(T t, T rs, T dt5_hi, T dt5_lo) {
 
 template <class T>
 struct uvbke_kernel {
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ ub, T* __restrict__ vb,
-                                             const T* __restrict__ uc, const T* __restrict__ vc,
-                                             const T* __restrict__ cosa, const T* __restrict__ rsina, T dt5, T dt5_lo,
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> ub, OutPtr<T> vb,
+                                             InPtr<T> uc, InPtr<T> vc,
+                                             InPtr<T> cosa, InPtr<T> rsina, T dt5, T dt5_lo,
                                              Dims d, int kb) {
     const int64_t sj = d.sj;
     for_points<RowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) {
@@ -162,11 +162,11 @@ struct uvbke_kernel {
 // ---- p_grad_c: kernels/p_grad_c.h:80-101 ---------------------------------------------
 template <class T>
 struct p_grad_c_kernel {
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uout, T* __restrict__ vout,
-                                             const T* __restrict__ uin, const T* __restrict__ vin,
-                                             const T* __restrict__ rdxc, const T* __restrict__ rdyc,
-                                             const T* __restrict__ delpc, const T* __restrict__ gz,
-                                             const T* __restrict__ pkc, T dt2, Dims d, int kb) {
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
+                                             InPtr<T> uin, InPtr<T> vin,
+                                             InPtr<T> rdxc, InPtr<T> rdyc,
+                                             InPtr<T> delpc, InPtr<T> gz,
+                                             InPtr<T> pkc, T dt2, Dims d, int kb) {
     const int64_t sj = d.sj, sk = d.sk;
     for_points<RowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) {
       const T wk = ld(delpc + o);
@@ -185,16 +185,16 @@ struct p_grad_c_kernel {
 // ---- nh_p_grad: kernels/nh_p_grad.h:116-146 --------------------------------------------
 template <class T>
 struct nh_p_grad_kernel {
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uout, T* __restrict__ vout,
-                                             const T* __restrict__ uin, const T* __restrict__ vin,
-                                             const T* __restrict__ rdx, const T* __restrict__ rdy,
-                                             const T* __restrict__ gz, const T* __restrict__ pp,
-                                             const T* __restrict__ pk3, const T* __restrict__ wk1, T dt, Dims d,
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
+                                             InPtr<T> uin, InPtr<T> vin,
+                                             InPtr<T> rdx, InPtr<T> rdy,
+                                             InPtr<T> gz, InPtr<T> pp,
+                                             InPtr<T> pk3, InPtr<T> wk1, T dt, Dims d,
                                              int kb) {
     const int64_t sj = d.sj, sk = d.sk;
-    const T* const now[8] = {pk3, gz, pp, wk1, uin, vin, rdx, rdy};
-    const T* const up[3] = {pk3, gz, pp};
-    prefetch_points(blk, d, kb, now, up);
+    const InPtr<T> now[8] = {pk3, gz, pp, wk1, uin, vin, rdx, rdy};
+    const InPtr<T> up[3] = {pk3, gz, pp};
+    prefetch_points<T>(blk, d, kb, now, up);
     for_points<HeavyRowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) {
       const T pk0 = ld(pk3 + o), pk1 = ld(pk3 + o + sk);
       const T gz0 = ld(gz + o), gz1 = ld(gz + o + sk);
@@ -246,8 +246,8 @@ struct nh_p_grad_kernel {
 // 3rd-order upwind advection along one axis (stride s): hadvuv.h:10-16 (x) and :18-24 (y).
 //   a > 0:  ((c6 f[-2] + f[-1]) + ch f[0]) + c3 f[1]
 //   else :  ((c3 f[-1] + ch f[0]) + f[1]) + c6 f[2]
-template <class T>
-__device__ __forceinline__ T adv3_axis(const T* __restrict__ f, int64_t o, int64_t s, T a) {
+template <class T, class P>
+__device__ __forceinline__ T adv3_axis(P f, int64_t o, int64_t s, T a) {
   constexpr T c6 = T(-1.0) / T(6.0), c3 = T(-1.0) / T(3.0);
   const bool pos = gt0(a);
   const T fa = ld(f + o + (pos ? -2 : -1) * s), fb = ld(f + o - s), f0 = ld(f + o), fc = ld(f + o + s),
@@ -260,8 +260,8 @@ __device__ __forceinline__ T adv3_axis(const T* __restrict__ f, int64_t o, int64
 // 5th-order upwind advection along one axis: hadvuv5th.h:10-22 (x) and :24-36 (y).
 //   a > 0:  ((((c30 f[-3] + c4 f[-2]) + f[-1]) + c3 f[0]) + c2 f[1]) + c20 f[2]
 //   else :  ((((c20 f[-2] + c2 f[-1]) + c3 f[0]) + f[1]) + c4 f[2]) + c30 f[3]
-template <class T>
-__device__ __forceinline__ T adv5_axis(const T* __restrict__ f, int64_t o, int64_t s, T a) {
+template <class T, class P>
+__device__ __forceinline__ T adv5_axis(P f, int64_t o, int64_t s, T a) {
   constexpr T c30 = T(1.0) / T(30.0), c3 = T(-1.0) / T(3.0), c20 = T(1.0) / T(20.0);
   const bool pos = gt0(a);
   const int64_t sh = pos ? 0 : s;  // the negative branch reads one cell further along the axis
@@ -280,10 +280,10 @@ template <class T, int ORDER, int SHAPE = 0>
 struct hadv_kernel {
   static constexpr int kStepOp = step_op<T>(ORDER == 5 ? kOpHadv5Fwd + SHAPE : -1);  // the step kernel's id
   static constexpr int kShape = SHAPE;
-  static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uout, T* __restrict__ vout,
-                                             const T* __restrict__ uin, const T* __restrict__ vin,
-                                             const T* __restrict__ acrlat0, const T* __restrict__ acrlat1,
-                                             const T* __restrict__ tgrlatda0, const T* __restrict__ tgrlatda1,
+  static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
+                                             InPtr<T> uin, InPtr<T> vin,
+                                             InPtr<T> acrlat0, InPtr<T> acrlat1,
+                                             InPtr<T> tgrlatda0, InPtr<T> tgrlatda1,
                                              int64_t s1d, T eddlat, T eddlon, Dims d, int kb, T alpha, int update) {
     const int64_t sj = d.sj;
     constexpr T third = T(1.0) / T(3.0);
@@ -912,22 +912,16 @@ oeb_status hadv_tl_entry(const M3* duout, const M3* dvout, const M3* uin, const 
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *u, *v, *a0, *a1, *t0, *t1, *ou, *ov;
-  OEB_TRY(arr.pack(uin, duin, &u));
-  OEB_TRY(arr.pack(vin, dvin, &v));
-  OEB_TRY(arr.pack(acrlat0, (const M1*)nullptr, &a0));
-  OEB_TRY(arr.pack(acrlat1, (const M1*)nullptr, &a1));
-  OEB_TRY(arr.pack(tgrlatda0, (const M1*)nullptr, &t0));
-  OEB_TRY(arr.pack(tgrlatda1, (const M1*)nullptr, &t1));
-  OEB_TRY(arr.alloc(duout, &ou));
-  OEB_TRY(arr.alloc(dvout, &ov));
+  DualIn<T> u, v;
+  OEB_TRY((dual_in<T>(uin, duin, &u)));
+  OEB_TRY((dual_in<T>(vin, dvin, &v)));
+  const DualIn<T> a0 = dual_param<T>(acrlat0), a1 = dual_param<T>(acrlat1), t0 = dual_param<T>(tgrlatda0),
+                  t1 = dual_param<T>(tgrlatda1);
+  const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY((launch<hadv_kernel<D, ORDER>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, a0, a1, t0, t1,
-                                         acrlat0->strides[0], D(eddlat), D(eddlon), d, kb, D(0), 0)));
-  OEB_TRY(arr.unpack(duout->aligned + duout->offset, ou, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dvout->aligned + dvout->offset, ov, *dom, kInterior, d.sj, d.sk);
+  return launch<hadv_kernel<D, ORDER>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, a0, a1, t0, t1,
+                                         acrlat0->strides[0], D(eddlat), D(eddlon), d, kb, D(0), 0);
 }
 
 // ============================== hadvuv / hadvuv5th adjoint ==========================
@@ -1344,14 +1338,12 @@ oeb_status laplace_tl_entry(const M3* dout, const M3* in, const M3* din, const o
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *x, *y;
-  OEB_TRY(arr.pack(in, din, &x));
-  OEB_TRY(arr.alloc(dout, &y));
+  DualIn<T> x;
+  OEB_TRY((dual_in<T>(in, din, &x)));
+  const DualOut<T> y = dual_out<T>(dout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<laplace_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, x, y, d, kb));
-  return arr.unpack(dout->aligned + dout->offset, y, *dom, kInterior, d.sj, d.sk);
+  return launch<laplace_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, x, y, d, kb);
 }
 
 template <class T, class M3>
@@ -1417,21 +1409,16 @@ oeb_status uvbke_tl_entry(const M3* dub, const M3* dvb, const M3* uc, const M3* 
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *u, *v, *ca, *rs, *ou, *ov;
-  OEB_TRY(arr.pack(uc, duc, &u));
-  OEB_TRY(arr.pack(vc, dvc, &v));
-  OEB_TRY(arr.pack(cosa, (const M3*)nullptr, &ca));
-  OEB_TRY(arr.pack(rsina, (const M3*)nullptr, &rs));
-  OEB_TRY(arr.alloc(dub, &ou));
-  OEB_TRY(arr.alloc(dvb, &ov));
+  DualIn<T> u, v;
+  OEB_TRY((dual_in<T>(uc, duc, &u)));
+  OEB_TRY((dual_in<T>(vc, dvc, &v)));
+  const DualIn<T> ca = dual_param<T>(cosa), rs = dual_param<T>(rsina);
+  const DualOut<T> ou = dual_out<T>(dub), ov = dual_out<T>(dvb);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uc->strides[1], uc->strides[0]};
   const T dt5_hi = T(dt5), dt5_lo = T(dt5 - (double)dt5_hi);
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<uvbke_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, ca, rs, D(dt5_hi),
-                                  D(dt5_lo), d, kb));
-  OEB_TRY(arr.unpack(dub->aligned + dub->offset, ou, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dvb->aligned + dvb->offset, ov, *dom, kInterior, d.sj, d.sk);
+  return launch<uvbke_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, ca, rs, D(dt5_hi),
+                                  D(dt5_lo), d, kb);
 }
 
 template <class T, class M3>
@@ -1687,23 +1674,18 @@ oeb_status p_grad_c_tl_entry(const M3* duout, const M3* dvout, const M3* uin, co
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *u, *v, *rx, *ry, *dp, *g, *pk, *ou, *ov;
-  OEB_TRY(arr.pack(uin, duin, &u));
-  OEB_TRY(arr.pack(vin, dvin, &v));
-  OEB_TRY(arr.pack(rdxc, (const M3*)nullptr, &rx));
-  OEB_TRY(arr.pack(rdyc, (const M3*)nullptr, &ry));
-  OEB_TRY(arr.pack(delpc, ddelpc, &dp));
-  OEB_TRY(arr.pack(gz, dgz, &g));
-  OEB_TRY(arr.pack(pkc, dpkc, &pk));
-  OEB_TRY(arr.alloc(duout, &ou));
-  OEB_TRY(arr.alloc(dvout, &ov));
+  DualIn<T> u, v, dp, g, pk;
+  OEB_TRY((dual_in<T>(uin, duin, &u)));
+  OEB_TRY((dual_in<T>(vin, dvin, &v)));
+  OEB_TRY((dual_in<T>(delpc, ddelpc, &dp)));
+  OEB_TRY((dual_in<T>(gz, dgz, &g)));
+  OEB_TRY((dual_in<T>(pkc, dpkc, &pk)));
+  const DualIn<T> rx = dual_param<T>(rdxc), ry = dual_param<T>(rdyc);
+  const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<p_grad_c_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, dp, g, pk,
-                                     D(dt2), d, kb));
-  OEB_TRY(arr.unpack(duout->aligned + duout->offset, ou, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dvout->aligned + dvout->offset, ov, *dom, kInterior, d.sj, d.sk);
+  return launch<p_grad_c_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, dp, g, pk,
+                                     D(dt2), d, kb);
 }
 
 template <class T, class M3>
@@ -2011,24 +1993,19 @@ oeb_status nh_p_grad_tl_entry(const M3* duout, const M3* dvout, const M3* uin, c
   }
   OEB_RETURN_IF_VALIDATING();
   using D = Dual<T>;
-  DualArrays<T> arr((cudaStream_t)stream);
-  D *u, *v, *rx, *ry, *g, *p, *pk, *w, *ou, *ov;
-  OEB_TRY(arr.pack(uin, duin, &u));
-  OEB_TRY(arr.pack(vin, dvin, &v));
-  OEB_TRY(arr.pack(rdx, (const M3*)nullptr, &rx));
-  OEB_TRY(arr.pack(rdy, (const M3*)nullptr, &ry));
-  OEB_TRY(arr.pack(gz, dgz, &g));
-  OEB_TRY(arr.pack(pp, dpp, &p));
-  OEB_TRY(arr.pack(pk3, dpk3, &pk));
-  OEB_TRY(arr.pack(wk1, dwk1, &w));
-  OEB_TRY(arr.alloc(duout, &ou));
-  OEB_TRY(arr.alloc(dvout, &ov));
+  DualIn<T> u, v, g, p, pk, w;
+  OEB_TRY((dual_in<T>(uin, duin, &u)));
+  OEB_TRY((dual_in<T>(vin, dvin, &v)));
+  OEB_TRY((dual_in<T>(gz, dgz, &g)));
+  OEB_TRY((dual_in<T>(pp, dpp, &p)));
+  OEB_TRY((dual_in<T>(pk3, dpk3, &pk)));
+  OEB_TRY((dual_in<T>(wk1, dwk1, &w)));
+  const DualIn<T> rx = dual_param<T>(rdx), ry = dual_param<T>(rdy);
+  const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  OEB_TRY(launch<nh_p_grad_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, g, p, pk, w,
-                                      D(dt), d, kb));
-  OEB_TRY(arr.unpack(duout->aligned + duout->offset, ou, *dom, kInterior, d.sj, d.sk));
-  return arr.unpack(dvout->aligned + dvout->offset, ov, *dom, kInterior, d.sj, d.sk);
+  return launch<nh_p_grad_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, g, p, pk, w,
+                                      D(dt), d, kb);
 }
 
 template <class T, class M3>
