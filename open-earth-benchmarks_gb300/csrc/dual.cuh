@@ -85,11 +85,7 @@ __device__ __forceinline__ DualIn<T> operator-(DualIn<T> p, int64_t o) {
 }
 template <class T>
 __device__ __forceinline__ Dual<T> ld(DualIn<T> p) {
-#ifdef OEB_COHERENT_LOADS  // the step kernel: see ld() in stencil_util.cuh
-  return Dual<T>(__ldca(p.v), p.d ? __ldca(p.d) : T(0));
-#else
-  return Dual<T>(__ldg(p.v), p.d ? __ldg(p.d) : T(0));
-#endif
+  return Dual<T>(ld(p.v), p.d ? ld(p.d) : T(0));
 }
 // The same as a kernel writes it (v null: the values are not wanted).
 template <class T>
@@ -141,6 +137,17 @@ struct Prec<Dual<T>> {
   __device__ static __forceinline__ Dual<T> add_flag(Dual<T> q, Dual<T> t, bool flag) {
     return q + t * (flag ? T(1) : T(0));
   }
+};
+
+// The FP64 kernels on dual numbers are longer code still than the FP64 kernels: rolled rows
+// (stencil_util.cuh).
+template <>
+struct RowUnroll<Dual<F64i>> {
+  static constexpr int value = 1;
+};
+template <>
+struct HeavyRowUnroll<Dual<F64i>> {
+  static constexpr int value = 1;
 };
 
 template <class T>

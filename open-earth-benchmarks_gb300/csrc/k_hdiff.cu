@@ -92,12 +92,12 @@ struct hdiffsa_kernel {
       // hdiffsa.h:106-113: limited fluxes
       for_region_lim<33, 32>(vx + 1, vy, [&](int a, int b) {
         T f = s.lap[b + 1][a + 1] - s.lap[b + 1][a];
-        if (Prec<T>::prod_gt0(f, s.in[b + 2][a + 2] - s.in[b + 2][a + 1])) f = 0;
+        if (Prec<T>::prod_gt0(f, s.in[b + 2][a + 2] - s.in[b + 2][a + 1])) f = T(0);
         s.flx[b][a] = f;
       });
       for_region_lim<32, 33>(vx, vy + 1, [&](int a, int b) {
         T f = s.crlato[b] * (s.lap[b + 1][a + 1] - s.lap[b][a + 1]);
-        if (Prec<T>::prod_gt0(f, s.dy[b + 1][a + 1])) f = 0;
+        if (Prec<T>::prod_gt0(f, s.dy[b + 1][a + 1])) f = T(0);
         s.fly[b][a] = f;
       });
       __syncthreads();

@@ -324,6 +324,21 @@ struct Rebind<K<double, N, M>> {
   static constexpr bool on = true;
 };
 
+// A kernel on dual numbers of doubles runs on dual numbers of F64i (their parts, too, are doubles:
+// DualIn, DualOut and Dual itself are reinterpreted as their F64i twins).
+template <class T>
+struct Dual;
+template <template <class> class K>
+struct Rebind<K<Dual<double>>> {
+  using type = K<Dual<F64i>>;
+  static constexpr bool on = true;
+};
+template <template <class, int, int> class K, int N, int M>
+struct Rebind<K<Dual<double>, N, M>> {
+  using type = K<Dual<F64i>, N, M>;
+  static constexpr bool on = true;
+};
+
 template <class A>
 struct ArgMap {
   using type = A;

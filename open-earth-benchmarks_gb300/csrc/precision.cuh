@@ -427,7 +427,12 @@ __host__ __device__ constexpr F64i operator-(F64i a) {
 #endif
   return F64i(-a.v);
 }
-__device__ __forceinline__ F64i operator*(F64i a, F64i b) { return F64i(fp64::mul(a.v, b.v)); }
+__host__ __device__ constexpr F64i operator*(F64i a, F64i b) {
+#if defined(__CUDA_ARCH__)
+  if (!__builtin_is_constant_evaluated()) return F64i(fp64::mul(a.v, b.v));
+#endif
+  return F64i(a.v * b.v);
+}
 __device__ __forceinline__ F64i& operator+=(F64i& a, F64i b) { return a = a + b; }
 __device__ __forceinline__ F64i& operator-=(F64i& a, F64i b) { return a = a - b; }
 __device__ __forceinline__ F64i& operator*=(F64i& a, F64i b) { return a = a * b; }
