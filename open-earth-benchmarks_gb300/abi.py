@@ -35,6 +35,8 @@ _lock = threading.Lock()
 
 def load_library() -> ctypes.CDLL:
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not LIB_PATH.exists():

@@ -108,7 +108,7 @@ class ChainPlan:
         missing = [n for n in ORDER if n not in fields]
         if missing:
             raise ValueError("chain step: missing fields %s" % missing)
-        refs = {n: fields[n].memref() for n in ORDER}
+        refs = {n: fields[n].packed()[0] for n in ORDER}
         cf = ChainFields(**{n: ctypes.pointer(refs[n]) for n in ORDER})
         self._keep = [refs, cf]  # alive until the next call; a captured graph copies them at capture
         return cf
@@ -126,8 +126,7 @@ class ChainPlan:
             raise TypeError("the plan is %s, the fields are %s" % (self.precision, prec))
         cf = self._fields(fields)
         cs = self._scalars(scalars)
-        refs = [f.memref() for f in extra]
-        args = [self._plan, ctypes.byref(cf), ctypes.byref(cs)] + [ctypes.byref(r) for r in refs]
+        args = [self._plan, ctypes.byref(cf), ctypes.byref(cs)] + [f.packed()[1] for f in extra]
         name = "oeb_chain_%s_%s" % (what, self.precision)
         check(entry(name)(*args, ctypes.c_void_p(_stream(stream))), name)
 

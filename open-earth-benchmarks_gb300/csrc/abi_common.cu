@@ -121,8 +121,9 @@ int device_sms() {
 // fvtp2d (apron 5, three CTAs an SM): best with 32 rows at 256 x 256 x 80 (89.7 us; 16 rows 93.9,
 // 12 rows 101.7, 8 rows 102.7, 64 rows 113) and with 16 at 128 x 128 x 80 (28.1 us; 8 rows 32.5,
 // 22 rows 31.1, 32 rows 36.6), as the product says.
-MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm) {
-  const double slots = (double)device_sms() * ctas_per_sm;
+namespace {
+MarchShape find_march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm, int sms) {
+  const double slots = (double)sms * ctas_per_sm;
   const int strips = (nx + cols - 1) / cols, levels = (nz + kb - 1) / kb;
   MarchShape best{};
   double least = 0.0;
@@ -142,6 +143,27 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
     }
   }
   return best;
+}
+}  // namespace
+
+// The search is a function of these sizes alone; a thread keeps the last few it made (a few hundred
+// candidates each, about a microsecond, as long as the launch itself).
+MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm) {
+  struct Kept {
+    int key[8];
+    MarchShape shape;
+  };
+  constexpr int kKept = 16;
+  static thread_local Kept kept[kKept] = {};
+  static thread_local int next = 0;
+  const int key[8] = {nx, ny, nz, kb, cols, apron, ctas_per_sm, device_sms()};
+  for (const Kept& k : kept)
+    if (memcmp(k.key, key, sizeof(key)) == 0) return k.shape;
+  Kept& k = kept[next];
+  next = (next + 1) % kKept;
+  memcpy(k.key, key, sizeof(key));
+  k.shape = find_march_shape(nx, ny, nz, kb, cols, apron, ctas_per_sm, key[7]);
+  return k.shape;
 }
 
 Recorder* recorder() { return t_recorder; }

@@ -41,15 +41,47 @@ def _domain(domain) -> Domain:
     return Domain(nx, ny, nz)
 
 
+def _current_stream() -> int:
+    """torch's current stream on the current device, as a handle."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # what current_stream() wraps in an object
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
+
+
 def _stream_handle(stream, on_device: bool) -> int:
     if stream is None:
-        if not on_device:
-            return 0
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream() if on_device else 0
     if hasattr(stream, "cuda_stream"):
         return stream.cuda_stream
     return int(stream)
+
+
+class _Signature:
+    """What a call of one kernel needs from its spec, worked out once."""
+
+    def __init__(self, spec):
+        self.spec = spec
+        self.names = tuple(a.name for a in spec.abi_args)
+        self.outs = tuple(a.name for a in spec.by_role("out3"))
+        self.ins = tuple(a.name for a in spec.args if a.role in ("in3", "in1"))
+        self.active = tuple(ACTIVE[spec.name])
+        self.seeds = tuple(spec.semantic_outputs)
+        self.scalars = {p: tuple((s.name, ctypes.c_double if (p == "f64" or s.always_double) else ctypes.c_float)
+                                 for s in spec.scalars) for p in ("f64", "f32")}
+        self.defaults = dict(DRIVER_SCALARS.get(spec.name, {}))
+
+
+_signatures: Dict[str, _Signature] = {}
+
+
+def _signature(kernel: str) -> _Signature:
+    spec = KERNELS[kernel]
+    sig = _signatures.get(kernel)
+    if sig is None or sig.spec is not spec:
+        sig = _signatures[kernel] = _Signature(spec)
+    return sig
 
 
 def set_adjoint_tiles(on: bool) -> None:
@@ -64,39 +96,38 @@ def entry_name(kernel: str, precision: str, on_device: bool) -> str:
     return "oeb_%s_%s%s" % (kernel, precision, "" if on_device else "_host")
 
 
+def _one_dtype(storages, dtype) -> bool:
+    for f in storages:
+        if f.dtype is not dtype and f.dtype != dtype:
+            return False
+    return True
+
+
 def call(kernel: str, fields: Dict[str, Storage], scalars: Optional[Dict[str, float]] = None, domain=None,
          stream=None) -> None:
     """Runs `kernel` on named fields (the reference's argument names) and scalars."""
-    spec = KERNELS[kernel]
-    abi_args = spec.abi_args
+    sig = _signature(kernel)
     st = []
-    for a in abi_args:
-        f = fields.get(a.name)
+    for name in sig.names:
+        f = fields.get(name)
         if f is None:
-            raise ValueError("%s: missing field %r" % (kernel, a.name))
+            raise ValueError("%s: missing field %r" % (kernel, name))
         if not isinstance(f, Storage):
-            raise TypeError("%s: field %r must be a Storage" % (kernel, a.name))
+            raise TypeError("%s: field %r must be a Storage" % (kernel, name))
         st.append(f)
-    dtypes = {f.dtype for f in st}
-    if len(dtypes) != 1:
-        raise TypeError("%s: all fields must share one element type, got %s" % (kernel, sorted(map(str, dtypes))))
-    precision = "f64" if st[0].dtype == np.float64 else "f32"
-    places = {f.is_cuda for f in st}
-    if len(places) != 1:
-        raise ValueError("%s: fields must be all on the device or all in host memory" % kernel)
-    on_device = places.pop()
-    vals = dict(DRIVER_SCALARS.get(kernel, {}))
-    vals.update(scalars or {})
-    cargs = [ctypes.byref(f.memref()) for f in st]
-    for s in spec.scalars:
-        if s.name not in vals:
-            raise ValueError("%s: missing scalar %r" % (kernel, s.name))
-        ctype = ctypes.c_double if (precision == "f64" or s.always_double) else ctypes.c_float
-        cargs.append(ctype(vals[s.name]))
+    dtype, on_device = st[0].dtype, st[0].is_cuda
+    if not _one_dtype(st, dtype):
+        raise TypeError("%s: all fields must share one element type, got %s"
+                        % (kernel, sorted({str(f.dtype) for f in st})))
+    for f in st:
+        if f.is_cuda != on_device:
+            raise ValueError("%s: fields must be all on the device or all in host memory" % kernel)
+    precision = "f64" if dtype == np.float64 else "f32"
+    cargs = _scalar_args(sig, scalars, precision)
+    cargs = [f.packed()[1] for f in st] + cargs
     dom = _domain(domain)
-    cargs += [ctypes.byref(dom), ctypes.c_void_p(_stream_handle(stream, on_device))]
     name = entry_name(kernel, precision, on_device)
-    check(entry(name)(*cargs), name)
+    check(entry(name)(*cargs, ctypes.byref(dom), ctypes.c_void_p(_stream_handle(stream, on_device))), name)
 
 
 # The fields of the FP32 pressure-gradient stencils that the profiled entry points take as
@@ -126,34 +157,44 @@ def call_profiled(kernel: str, fields: Dict[str, Storage], bases, scalars: Optio
             raise ValueError("%s: base profile %r must be a contiguous float64 CUDA tensor of nz + 1 = %d values"
                              % (kernel, n, dom.nz + 1))
         ptrs.append(ctypes.c_void_p(b.data_ptr()))
-    vals = dict(DRIVER_SCALARS.get(kernel, {}))
-    vals.update(scalars or {})
-    cargs = [ctypes.byref(f.memref()) for f in st] + ptrs + _scalar_args(spec, vals, "f32")
+    cargs = [f.packed()[1] for f in st] + ptrs + _scalar_args(_signature(kernel), scalars, "f32")
     cargs += [ctypes.byref(dom), ctypes.c_void_p(_stream_handle(stream, True))]
     name = "oeb_%s_f32_profiled" % kernel
     check(entry(name)(*cargs), name)
 
 
-def _scalar_args(spec, vals, precision):
+def _scalar_args(sig, scalars, precision):
     out = []
-    for s in spec.scalars:
-        if s.name not in vals:
-            raise ValueError("%s: missing scalar %r" % (spec.name, s.name))
-        ctype = ctypes.c_double if (precision == "f64" or s.always_double) else ctypes.c_float
-        out.append(ctype(vals[s.name]))
+    for name, ctype in sig.scalars[precision]:
+        if scalars is not None and name in scalars:
+            out.append(ctype(scalars[name]))
+        elif name in sig.defaults:
+            out.append(ctype(sig.defaults[name]))
+        else:
+            raise ValueError("%s: missing scalar %r" % (sig.spec.name, name))
     return out
 
 
-def _device_fields(kernel, groups):
-    flat = [f for g in groups for f in g]
-    if any(not isinstance(f, Storage) for f in flat):
-        raise TypeError("%s: every field must be a Storage" % kernel)
-    if not all(f.is_cuda for f in flat):
-        raise ValueError("%s: the tangent-linear and adjoint entry points take device fields" % kernel)
-    dtypes = {f.dtype for f in flat}
-    if len(dtypes) != 1:
+def _device_fields(kernel, flat):
+    for f in flat:
+        if not isinstance(f, Storage):
+            raise TypeError("%s: every field must be a Storage" % kernel)
+    for f in flat:
+        if not f.is_cuda:
+            raise ValueError("%s: the tangent-linear and adjoint entry points take device fields" % kernel)
+    dtype = flat[0].dtype
+    if not _one_dtype(flat, dtype):
         raise TypeError("%s: mixed element types" % kernel)
-    return "f64" if flat[0].dtype == np.float64 else "f32"
+    return "f64" if dtype == np.float64 else "f32"
+
+
+def _device_call(what, kernel, flat, scalars, domain, stream):
+    precision = _device_fields(kernel, flat)
+    cargs = _scalar_args(_signature(kernel), scalars, precision)
+    cargs = [f.packed()[1] for f in flat] + cargs
+    dom = _domain(domain)
+    name = "oeb_%s_%s_%s" % (kernel, what, precision)
+    check(entry(name)(*cargs, ctypes.byref(dom), ctypes.c_void_p(_stream_handle(stream, True))), name)
 
 
 def tangent_linear(kernel: str, state: Dict[str, Storage], dx: Dict[str, Storage], dy: Dict[str, Storage],
@@ -162,35 +203,17 @@ def tangent_linear(kernel: str, state: Dict[str, Storage], dx: Dict[str, Storage
 
     dx holds a perturbation of each active input (ACTIVE[kernel]); dy receives the
     perturbation of every output, over the output's written box."""
-    spec = KERNELS[kernel]
-    outs = [dy[a.name] for a in spec.by_role("out3")]
-    ins = [state[a.name] for a in spec.args if a.role in ("in3", "in1")]
-    dxs = [dx[n] for n in ACTIVE[kernel]]
-    precision = _device_fields(kernel, (outs, ins, dxs))
-    vals = dict(DRIVER_SCALARS.get(kernel, {}))
-    vals.update(scalars or {})
-    cargs = [ctypes.byref(f.memref()) for f in outs + ins + dxs] + _scalar_args(spec, vals, precision)
-    dom = _domain(domain)
-    cargs += [ctypes.byref(dom), ctypes.c_void_p(_stream_handle(stream, True))]
-    name = "oeb_%s_tl_%s" % (kernel, precision)
-    check(entry(name)(*cargs), name)
+    sig = _signature(kernel)
+    _device_call("tl", kernel, [dy[n] for n in sig.outs] + [state[n] for n in sig.ins] + [dx[n] for n in sig.active],
+                 scalars, domain, stream)
 
 
 def adjoint(kernel: str, state: Dict[str, Storage], ybar: Dict[str, Storage], xbar: Dict[str, Storage],
             scalars: Optional[Dict[str, float]] = None, domain=None, stream=None) -> None:
     """xbar = J(state)^T ybar for the active inputs; ybar seeds the semantic outputs."""
-    spec = KERNELS[kernel]
-    xbs = [xbar[n] for n in ACTIVE[kernel]]
-    ins = [state[a.name] for a in spec.args if a.role in ("in3", "in1")]
-    ybs = [ybar[n] for n in spec.semantic_outputs]
-    precision = _device_fields(kernel, (xbs, ins, ybs))
-    vals = dict(DRIVER_SCALARS.get(kernel, {}))
-    vals.update(scalars or {})
-    cargs = [ctypes.byref(f.memref()) for f in xbs + ins + ybs] + _scalar_args(spec, vals, precision)
-    dom = _domain(domain)
-    cargs += [ctypes.byref(dom), ctypes.c_void_p(_stream_handle(stream, True))]
-    name = "oeb_%s_adj_%s" % (kernel, precision)
-    check(entry(name)(*cargs), name)
+    sig = _signature(kernel)
+    _device_call("adj", kernel, [xbar[n] for n in sig.active] + [state[n] for n in sig.ins] + [ybar[n] for n in sig.seeds],
+                 scalars, domain, stream)
 
 
 def _make(kernel: str):

@@ -73,6 +73,7 @@ class Storage:
             self.szi = data.shape[0]
             self.pitch = data.shape[0]
         self._memref = None
+        self._packed = (None, None, None)
 
     # -- construction ------------------------------------------------------------------
     @classmethod
@@ -100,22 +101,37 @@ class Storage:
     # -- descriptor ----------------------------------------------------------------------
     @property
     def is_cuda(self) -> bool:
-        return _is_torch(self.data) and self.data.is_cuda
+        d = self.data
+        return torch is not None and isinstance(d, torch.Tensor) and d.is_cuda
 
     def data_ptr(self) -> int:
         return self.data.data_ptr() if _is_torch(self.data) else self.data.ctypes.data
 
     def memref(self):
         """The descriptor as a ctypes structure (kept alive by this object)."""
-        ptr = self.data_ptr()
+        m = self._describe(self.data_ptr())
+        self._memref = m
+        return m
+
+    def _describe(self, ptr):
         h = self.halo
         if self.rank == 3:
             szk, szj, pitch = self.data.shape
-            m = Memref3d(ptr, ptr, h * szj * pitch + h * pitch + h, (szk, szj, self.szi), (szj * pitch, pitch, 1))
-        else:
-            m = Memref1d(ptr, ptr, h, (self.data.shape[0],), (1,))
-        self._memref = m
-        return m
+            return Memref3d(ptr, ptr, h * szj * pitch + h * pitch + h, (szk, szj, self.szi), (szj * pitch, pitch, 1))
+        return Memref1d(ptr, ptr, h, (self.data.shape[0],), (1,))
+
+    def packed(self):
+        """(descriptor, byref of it) for a call that only reads it.  Kept with what it was built
+        from -- the buffer's address and shape, the halo and the row length -- and built again when
+        any of those differs."""
+        d = self.data
+        ptr = d.data_ptr() if torch is not None and isinstance(d, torch.Tensor) else d.ctypes.data
+        key = (ptr, d.shape, self.halo, self.szi)
+        kept = self._packed
+        if kept[0] != key:
+            m = self._describe(ptr)
+            self._packed = kept = (key, m, ctypes.byref(m))
+        return kept[1], kept[2]
 
     # -- views ---------------------------------------------------------------------------
     def box(self, reach=(0, 0, 0, 0, 0, 0), nx=None, ny=None, nz=None):
