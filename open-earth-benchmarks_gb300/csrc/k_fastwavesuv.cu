@@ -186,10 +186,9 @@ struct fastwavesuv_march_f32 {
         if (src == 0 && j > ja) metric(j);
         const float fx2 = __shfl_sync(kWarpMask, lf, src);
         // fastwavesuv.h:172-175, :182-183
-        // (a lane that writes nothing has itself or a copy above it: 1 in place of its zero numerator,
-        // which would send the warp through the division's slow path)
+        // a lane that writes nothing has itself or a copy above it: its numerator is zero
         const float num = (0.5f * (lane_above<1>(pcj) + pcj)) * (hsj - lane_above<1>(hsj));
-        const float ppgu = (lane_above<1>(c.p0) - c.p0) + (st ? num : 1.f) / (hdj + lane_above<1>(hdj));
+        const float ppgu = (lane_above<1>(c.p0) - c.p0) + numerator(st, num) / (hdj + lane_above<1>(hdj));
         const float uo = c.u + dt * (c.ut - ppgu * (fx2 / (lane_above<1>(c.r) + c.r)));
         if (st) put(uout, o, uo);
       }

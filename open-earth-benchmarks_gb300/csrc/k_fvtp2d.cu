@@ -352,9 +352,10 @@ inline dim3 flux_grid(const Dims& d, int kb) {
 // What bounds it: instruction issue and the latency of its dependent chains (about 300
 // instructions a row of 26 columns, 110 of them the arithmetic; DRAM traffic 1.3x the outputs and
 // inputs once).  80 registers, three CTAs an SM: at 256 x 256 x 80 two CTAs (113 registers)
-// measured 106 us, four (64, spilling) 110, three 90; two rows unrolled 91.  Two levels a warp in
+// measured 106 us, four (64, spilling) 110, three 90; two rows unrolled 91 (83 since the lanes off a
+// field divide 1 by 1, numerator() in march.cuh).  Two levels a warp in
 // packed FP32 instructions (f32x2) took a quarter fewer instructions but 128 registers: 98 us.
-// The form before it, a 32 x 32 shared-memory tile in nine phases, took 180 us (56 against 28 us
+// The form before it, a 32 x 32 shared-memory tile in nine phases, took 180 us (56 against 25 us
 // at 128 x 128 x 80).
 
 // The aux values of one cell of a PPM sweep (fvtp2d.h:20-23).  a b < 0 is decided on the exact
@@ -460,13 +461,15 @@ struct fvtp2d_march_f32 {
       const float fxn = ppm_row(p1, p2, q0, w.crx);
       const float fxx = w.xfx * fxn;
       const float qa = q0 * w.area;
-      const float jn = ((qa + fxx) - lane_above<1>(fxx)) / w.rax;
+      const float jnum = (qa + fxx) - lane_above<1>(fxx);
+      const float jn = numerator(in_r, jnum) / w.rax;
       const bool row_own = ALL || ((s >= ja || first_j) && (s < jb || last_j));
       if (st_x && row_own) put(fx2, o, fxn);
       if (st && row_own) put(q_j, o, jn);
       if (ALL || (s >= ja && s < jb)) {
         // q_i, and its x sweep
-        const float qi = ((qa + fyy0) - fyy1) / w.ray;
+        const float inum = (qa + fyy0) - fyy1;
+        const float qi = numerator(in_y, inum) / w.ray;
         if (st_y) put(q_i, o, qi);
         const float f = ppm_row(p1, p2, qi, w.crx);
         if (st) put(fx1, o, (0.5f * (f + fxn)) * w.xfx);
@@ -616,12 +619,11 @@ oeb_status fvtp2d_tl_entry(const M3* dq_i, const M3* dq_j, const M3* dfx1, const
 
 constexpr int kW = 44;  // window along the sweep axis: outputs A..A+31 need A-5 .. A+38
 
-// Lines a CTA sweeps: 16 in FP64 (23 KB a CTA: the registers, not shared memory, then bound
-// the CTAs per SM, at five or six against four with 32 lines), 32 in FP32 (eight CTAs per SM
-// either way).
+// Lines a CTA sweeps: 16 (23 KB a CTA: the registers, not shared memory, then bound the CTAs
+// per SM, at five or six against four with 32 lines).
 template <class T>
 constexpr int adj_lines() {
-  return 16;  // FP32: 16 measured faster than 32 (the FP32 adjoint 0.194 -> 0.172 ms at 128 x 128 x 80)
+  return 16;
 }
 
 // gs and als are dead once the flags smt are set; tb and al take their places
@@ -900,6 +902,319 @@ struct fvtp2d_adj_q_kernel {
   }
 };
 
+// ------------------------------ FP32: the adjoint in three marching launches ----------
+// The passes above as warps that march rows (march.cuh), with the same operations on the same
+// operands (a term that is zero is added where the passes skip it):
+//   A: q_ib.  The y sweep of q gives q_i a row at a time; its row's transposed x sweep follows at
+//      once, the neighbours handed over by the lanes.
+//   B: q_jb.  The x sweep of q gives q_j a row at a time, which feeds the transposed y sweep, its
+//      window in registers.
+//   C: qb.  fx2b and fy2b are formed where they are read, from q_jb and q_ib; a row's transposed x
+//      sweep, the transposed y sweep and the area terms meet in one store.
+// q_i, q_j, fx2b, fy2b and the partial qb are never stored: two scratch fields instead of eight.
+//
+// What bounds them: instruction issue (170, 180 and 380 instructions a row for A, B, C; 70 % of the
+// issue slots taken).  Four, four and three CTAs an SM: 78.0 us a call at 128 x 128 x 80 (19 + 23 + 43
+// with a cold cache), 222 at 256 x 256 x 80, 115 at 201 x 173 x 61 (three CTAs for all 83 / 235 / 113);
+// the passes above, run for float, took 154.8, 521.5 and 229.4 us.  Zero numerators that reached the
+// division's slow path (numerator(), div_zero()) were 12 us of it at 128 x 128 x 80.
+
+// a / b, with the IEEE quotient's bits, for numerators that are often exactly zero (a gradient where no
+// flux enters): the division's fast path does not take a zero, and a warp of 32 cells nearly always
+// has one.
+__device__ __forceinline__ float div_zero(float a, float b) {
+  const bool zero = a == 0.f && fabsf(b) > 0.f && fabsf(b) < __int_as_float(0x7f800000);
+  const float q = numerator(!zero, a) / b;
+  return zero ? a * b : q;
+}
+
+// One face of a transposed sweep: t = tb, z = the product with c of B0 (-(|c| tb) on either side),
+// each on the side that takes it (U: the cell below, where c > 0; L: the cell above), and the flux
+// adjoint f likewise.
+struct FaceT {
+  float tU, tL, zU, zL, fU, fL;
+};
+__device__ __forceinline__ FaceT ppm_face_t(float f, float c, bool limited) {
+  const bool pos = c > 0.f;
+  const float n = neg_abs(c);
+  const float t = (limited && f != 0.f) ? f * (1.f + n) : 0.f;
+  const float z = n * t;
+  return FaceT{pos ? t : 0.f, pos ? 0.f : t, pos ? z : 0.f, pos ? 0.f : z, pos ? f : 0.f, pos ? 0.f : f};
+}
+
+// The transposed x sweep of one row: gs the state value at the lane, f and c the flux adjoint and the
+// Courant number of its low face.  Valid from lane 5 to lane 26.
+__device__ __forceinline__ float ppm_row_t(float p1, float p2, float gs, float f, float c) {
+  constexpr float big = 1.2676506002282294e30f;  // 2^100 (ppm_cell)
+  const float als = ppm_al(p1, p2, lane_below<2>(gs), lane_below<1>(gs), gs, lane_above<1>(gs));
+  const bool smt = ((als - gs) * big) * ((lane_above<1>(als) - gs) * big) < 0.f;
+  const FaceT w = ppm_face_t(f, c, here_or_below(smt));
+  const float b0 = lane_above<1>(w.zU) + w.zL;
+  const float alm = w.tL + b0, br = lane_above<1>(w.tU) + b0;
+  const float al = alm + lane_below<1>(br);
+  const float g =
+      fmaf(p1, lane_above<1>(al) + al, fmaf(p2, lane_above<2>(al) + lane_below<1>(al), -alm)) - br;
+  return (g + lane_above<1>(w.fU)) + w.fL;
+}
+
+// The transposed y sweep: step() takes the state value at row r and the face r - 2, and gives the
+// sweep's value at row r - 5.
+struct PpmColumnT {
+  float g1 = 0.f, g2 = 0.f, g3 = 0.f;     // the state at r-1, r-2, r-3
+  float als = 0.f;                        // its edge value at r-2
+  bool smt = false;                       // its flag at r-3
+  float tL = 0.f, zL = 0.f;               // of face r-3
+  float alm1 = 0.f, alm2 = 0.f;           // alm at r-4, r-5
+  float br1 = 0.f, br2 = 0.f;             // br at r-4, r-5
+  float al1 = 0.f, al2 = 0.f, al3 = 0.f;  // al at r-4, r-5, r-6
+  float fU1 = 0.f, fU2 = 0.f;             // fU of faces r-3, r-4
+  float fL1 = 0.f, fL2 = 0.f, fL3 = 0.f;  // fL of faces r-3, r-4, r-5
+  __device__ __forceinline__ float step(float p1, float p2, float g0, float f, float c) {
+    constexpr float big = 1.2676506002282294e30f;
+    const float alsn = ppm_al(p1, p2, g3, g2, g1, g0);  // at r-1
+    const bool smtn = ((als - g2) * big) * ((alsn - g2) * big) < 0.f;
+    const FaceT w = ppm_face_t(f, c, smt || smtn);
+    const float b0 = w.zU + zL;  // of cell r-3
+    const float alm = tL + b0, br = w.tU + b0;
+    const float al = alm + br1;
+    const float g = fmaf(p1, al1 + al2, fmaf(p2, al + al3, -alm2)) - br2;
+    const float out = (g + fU2) + fL3;
+    g3 = g2, g2 = g1, g1 = g0, als = alsn, smt = smtn;
+    tL = w.tL, zL = w.zL;
+    alm2 = alm1, alm1 = alm, br2 = br1, br1 = br, al3 = al2, al2 = al1, al1 = al;
+    fU2 = fU1, fU1 = w.fU, fL3 = fL2, fL2 = fL1, fL1 = w.fL;
+    return out;
+  }
+};
+
+// A: q_ib over i in [-3, nx+2), j in [0, ny): 22 columns a strip.
+struct fvtp2d_adj_qi_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpFvAdjQij);  // the step kernel's id
+  static constexpr int kCols = 22, kApron = 4, kMinCtas = 4;
+  struct Row {
+    float q, cry, yfx, area, ray, crx, xfx, fb;  // q on row s + 3, cry and yfx on s + 1, the rest on s
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ qib, const float* __restrict__ q,
+                                             const float* __restrict__ crx, const float* __restrict__ cry,
+                                             const float* __restrict__ xfx, const float* __restrict__ yfx,
+                                             const float* __restrict__ ra_y, const float* __restrict__ area,
+                                             const float* __restrict__ fx1b, float p1, float p2, Dims d, int rows,
+                                             int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int a0 = -3 + pos.strip * kCols, ja = pos.chunk * rows, jb = min(ja + rows, ny);
+    if (a0 >= nx + 2 || ja >= ny) return;
+    const int lane = (int)threadIdx.x, i = a0 - 5 + lane;
+    const bool in_y = i >= -3 && i < nx + 2, in_x = i >= 0 && i < nx;
+    const bool st = in_y && lane >= 5 && lane < 5 + kCols;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)(ja - 3) * d.sj + i) * 4;  // (i, s)
+    Row n{0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f};
+    auto fetch = [&](auto all, int s, int64_t c) {  // all: every row of them is this chunk's
+      constexpr bool ALL = decltype(all)::value;
+      if (in_y && (ALL || s + 3 <= jb + 2)) n.q = get(q, c + 3 * sjb);
+      if (in_y && (ALL || (s + 1 >= ja && s < jb))) n.cry = get(cry, c + sjb), n.yfx = get(yfx, c + sjb);
+      if (ALL || (s >= ja && s < jb)) {
+        if (in_y) n.area = get(area, c), n.ray = get(ra_y, c);
+        if (in_x) n.crx = get(crx, c), n.xfx = get(xfx, c), n.fb = get(fx1b, c);
+      }
+    };
+    float q0 = 0.f, q1 = 0.f, q2 = 0.f;  // q on rows s, s+1, s+2
+    if (in_y) q0 = get(q, o), q1 = get(q, o + sjb), q2 = get(q, o + 2 * sjb);
+    float al_lo = 0.f, fyy0 = 0.f;
+    PpmCell yc = ppm_cell(0.f, 0.f, 0.f);
+    auto step_row = [&](auto all, int s) {
+      constexpr bool ALL = decltype(all)::value;
+      const Row w = n;
+      fetch(all, s + 1, o + sjb);
+      const float al_hi = ppm_al(p1, p2, q0, q1, q2, w.q);
+      const PpmCell yn = ppm_cell(al_lo, al_hi, q1);
+      const float fyy1 = w.yfx * ppm_face(w.cry, q0, yc.r, yc.b0, q1, yn.m, yn.b0, yc.smt || yn.smt);
+      if (ALL || s >= ja) {
+        const float num = ((q0 * w.area) + fyy0) - fyy1;
+        const float qi = numerator(in_y, num) / w.ray;
+        const float g = ppm_row_t(p1, p2, in_y ? qi : 0.f, in_x ? (0.5f * w.xfx) * w.fb : 0.f, w.crx);
+        if (st) put(qib, o, g);
+      }
+      q0 = q1, q1 = q2, q2 = w.q;
+      al_lo = al_hi, yc = yn, fyy0 = fyy1;
+      o += sjb;
+    };
+    fetch(std::false_type{}, ja - 3, o);
+    int s = ja - 3;
+#pragma unroll 1
+    for (; s < ja; ++s) step_row(std::false_type{}, s);
+#pragma unroll 1
+    for (; s < jb - 1; ++s) step_row(std::true_type{}, s);
+#pragma unroll 1
+    for (; s < jb; ++s) step_row(std::false_type{}, s);
+  }
+};
+
+// B: q_jb over i in [0, nx), j in [-3, ny+2): 26 columns a strip.
+struct fvtp2d_adj_qj_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpFvAdjF2);  // the step kernel's id
+  static constexpr int kCols = 26, kApron = 10, kMinCtas = 4;
+  struct Row {
+    float q, crx, xfx, area, rax;  // on row r
+    float cry, yfx, fb;            // on row r - 2
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ qjb, const float* __restrict__ q,
+                                             const float* __restrict__ crx, const float* __restrict__ cry,
+                                             const float* __restrict__ xfx, const float* __restrict__ yfx,
+                                             const float* __restrict__ ra_x, const float* __restrict__ area,
+                                             const float* __restrict__ fy1b, float p1, float p2, Dims d, int rows,
+                                             int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = pos.strip * kCols, oa = -3 + pos.chunk * rows, ob = min(oa + rows, ny + 2);
+    if (i0 >= nx || oa >= ny + 2) return;
+    const int lane = (int)threadIdx.x, i = i0 - 3 + lane;
+    const bool in_q = i < nx + 3, in_x = i >= 0 && i < nx + 1, in_r = i >= 0 && i < nx;
+    const bool st = in_r && lane >= 3 && lane < 3 + kCols;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)(oa - 5) * d.sj + i) * 4;  // (i, r)
+    Row n{0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f};
+    auto fetch = [&](auto all, int r, int64_t c) {  // all: rows r and r - 2 lie in the interior
+      constexpr bool ALL = decltype(all)::value;
+      if (ALL || (r >= -3 && r < ny + 2)) {
+        if (in_q) n.q = get(q, c);
+        if (in_x) n.crx = get(crx, c), n.xfx = get(xfx, c);
+        if (in_r) n.area = get(area, c), n.rax = get(ra_x, c);
+      }
+      if (in_r && (ALL || (r - 2 >= 0 && r - 2 < ny)))
+        n.cry = get(cry, c - 2 * sjb), n.yfx = get(yfx, c - 2 * sjb), n.fb = get(fy1b, c - 2 * sjb);
+    };
+    PpmColumnT col;
+    auto step_row = [&](auto all, int r) {
+      constexpr bool ALL = decltype(all)::value;
+      const Row w = n;
+      if (ALL || r + 1 < ob + 5) fetch(all, r + 1, o + sjb);
+      float qj = 0.f;
+      if (ALL || (r >= -3 && r < ny + 2)) {
+        const float fxx = w.xfx * ppm_row(p1, p2, w.q, w.crx);
+        const float num = ((w.q * w.area) + fxx) - lane_above<1>(fxx);
+        qj = numerator(in_r, num) / w.rax;
+      }
+      const float f = ALL || (r - 2 >= 0 && r - 2 < ny) ? (0.5f * w.yfx) * w.fb : 0.f;
+      const float g = col.step(p1, p2, qj, f, w.cry);
+      if (st && (ALL || r - 5 >= oa)) put(qjb, o - 5 * sjb, g);
+      o += sjb;
+    };
+    fetch(std::false_type{}, oa - 5, o);
+    int r = oa - 5;
+    const int ra = min(max(oa + 5, 2), ob + 5), rb = max(ra, min(ob + 4, ny - 1));
+#pragma unroll 1
+    for (; r < ra; ++r) step_row(std::false_type{}, r);
+#pragma unroll 1
+    for (; r < rb; ++r) step_row(std::true_type{}, r);
+#pragma unroll 1
+    for (; r < ob + 5; ++r) step_row(std::false_type{}, r);
+  }
+};
+
+// C: qb on [-3, n+3)^2: 22 columns a strip.
+struct fvtp2d_adj_q_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpFvAdjQ);  // the step kernel's id
+  static constexpr int kCols = 22, kApron = 10, kMinCtas = 3;
+  struct Row {
+    float q;                                             // on row r
+    float cry, yfx, ray, qi, fy;                         // on row r - 2
+    float x, crx, xfx, rax, qj, fx, area, ray5, qi5;     // on row w = r - 5 (x: q)
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ qb, const float* __restrict__ q,
+                                             const float* __restrict__ crx, const float* __restrict__ cry,
+                                             const float* __restrict__ xfx, const float* __restrict__ yfx,
+                                             const float* __restrict__ ra_x, const float* __restrict__ ra_y,
+                                             const float* __restrict__ area, const float* __restrict__ fx1b,
+                                             const float* __restrict__ fy1b, const float* __restrict__ qib,
+                                             const float* __restrict__ qjb, float p1, float p2, Dims d, int rows,
+                                             int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int a0 = -3 + pos.strip * kCols, oa = -3 + pos.chunk * rows, ob = min(oa + rows, ny + 3);
+    if (a0 >= nx + 3 || oa >= ny + 3) return;
+    const int lane = (int)threadIdx.x, i = a0 - 5 + lane;
+    const bool in_q = i >= -3 && i < nx + 3, in_y = i >= -3 && i < nx + 2, in_x = i >= 0 && i < nx + 1,
+               in_r = i >= 0 && i < nx;
+    const bool st = in_q && lane >= 5 && lane < 5 + kCols;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)(oa - 5) * d.sj + i) * 4;  // (i, r)
+    Row n{};
+    n.ray = n.rax = n.ray5 = n.area = n.qi = n.qj = 1.f;  // quotients of lanes off the fields are 1 / 1
+    auto fetch = [&](auto all, int r, int64_t c) {  // all: rows r, r - 2 and r - 5 lie in the interior
+      constexpr bool ALL = decltype(all)::value;
+      if (in_q && (ALL || (r >= -3 && r < ny + 3))) n.q = get(q, c);
+      const int p = r - 2, w = r - 5;
+      const int64_t cp = c - 2 * sjb, cw = c - 5 * sjb;
+      if (in_y && (ALL || (p >= 0 && p < ny + 1))) {
+        n.cry = get(cry, cp), n.yfx = get(yfx, cp);
+        if (ALL || p < ny) {
+          n.ray = get(ra_y, cp), n.qi = get(qib, cp);
+          if (in_r) n.fy = get(fy1b, cp);
+        }
+      }
+      if (ALL || w >= oa) {
+        if (in_q) n.x = get(q, cw);
+        if (ALL || w < ny + 2) {
+          if (in_x) n.crx = get(crx, cw), n.xfx = get(xfx, cw);
+          if (in_y) n.area = get(area, cw);
+          if (in_r) n.rax = get(ra_x, cw), n.qj = get(qjb, cw);
+        }
+        if (ALL || (w >= 0 && w < ny)) {
+          if (in_r) n.fx = get(fx1b, cw);
+          if (in_y) n.ray5 = get(ra_y, cw), n.qi5 = get(qib, cw);
+        }
+      }
+    };
+    PpmColumnT col;
+    float ry = 0.f;  // q_ib / ra_y on row r - 3
+    auto step_row = [&](auto all, int r) {
+      constexpr bool ALL = decltype(all)::value;
+      const Row c = n;
+      if (ALL || r + 1 < ob + 5) fetch(all, r + 1, o + sjb);
+      const int p = r - 2, w = r - 5;
+      // the y sweep: face p
+      float f = 0.f, ryn = 0.f;
+      if (ALL || (p >= 0 && p < ny + 1)) {
+        if (ALL || p < ny) ryn = div_zero(c.qi, c.ray);
+        const float g = ((ALL || p < ny) && in_r) ? (0.5f * c.yfx) * c.fy : 0.f;
+        f = in_y ? g + c.yfx * (ryn - ry) : 0.f;
+      }
+      ry = ryn;
+      const float gy = col.step(p1, p2, (ALL || (r >= -3 && r < ny + 3)) ? c.q : 0.f, f, c.cry);
+      if (ALL || w >= oa) {
+        // the x sweep of row w
+        float fx = 0.f;
+        if (ALL || w < ny + 2) {
+          const float rxq = div_zero(c.qj, c.rax);
+          const float rx = in_r ? rxq : 0.f, rm = lane_below<1>(rx);
+          const float g = (in_r && (ALL || (w >= 0 && w < ny))) ? (0.5f * c.xfx) * c.fx : 0.f;
+          fx = in_x ? g + c.xfx * (rx - rm) : 0.f;
+        }
+        float acc = ppm_row_t(p1, p2, c.x, fx, c.crx);
+        const float ax = c.area / c.rax;
+        if (ALL || (w >= 0 && w < ny)) {
+          const float ay = c.area / c.ray5;
+          acc = in_y ? acc + ay * c.qi5 : acc;
+        }
+        if (ALL || w < ny + 2) acc = in_r ? acc + ax * c.qj : acc;
+        if (st) put(qb, o - 5 * sjb, acc + gy);
+      }
+      o += sjb;
+    };
+    fetch(std::false_type{}, oa - 5, o);
+    int r = oa - 5;
+    const int ra = min(max(oa + 5, 5), ob + 5), rb = max(ra, min(ob + 4, ny - 1));
+#pragma unroll 1
+    for (; r < ra; ++r) step_row(std::false_type{}, r);
+#pragma unroll 1
+    for (; r < rb; ++r) step_row(std::true_type{}, r);
+#pragma unroll 1
+    for (; r < ob + 5; ++r) step_row(std::false_type{}, r);
+  }
+};
+
 template <class T, class M3>
 oeb_status fvtp2d_adj_entry(const M3* qb, const M3* q, const M3* crx, const M3* cry, const M3* ra_x, const M3* ra_y,
                             const M3* xfx, const M3* yfx, const M3* area, const M3* fx1b, const M3* fy1b, T p1, T p2,
@@ -923,44 +1238,65 @@ oeb_status fvtp2d_adj_entry(const M3* qb, const M3* q, const M3* crx, const M3* 
                                             gg1.lo, gg1.hi}));
   OEB_RETURN_IF_VALIDATING();
   cudaStream_t st = (cudaStream_t)stream;
-  // scratch in q's layout: q_i, q_j, fx2, fy2 (forward recompute), q_ib, q_jb, fx2b, fy2b
+  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gq.sj, gq.sk};
+  // scratch in q's layout: FP32 q_ib, q_jb; FP64 q_i, q_j, fx2, fy2 (forward recompute), q_ib, q_jb, fx2b, fy2b
   const T* start = (q->allocated && q->allocated <= q->aligned) ? q->allocated : q->aligned;
   const int64_t last = (q->sizes[0] - 1) * q->strides[0] + (q->sizes[1] - 1) * q->strides[1] +
                        (q->sizes[2] - 1) * q->strides[2];
   const int64_t n = (int64_t)(q->aligned - start) + last + 1;
   const int64_t org = (int64_t)(q->aligned - start) + q->offset;
   void* buf = nullptr;
-  OEB_TRY(scratch_alloc(&buf, (size_t)n * 8 * sizeof(T), st));
-  T* base = static_cast<T*>(buf);
-  T *sqi = base + org, *sqj = base + n + org, *sfx2 = base + 2 * n + org, *sfy2 = base + 3 * n + org,
-    *qib = base + 4 * n + org, *qjb = base + 5 * n + org, *fx2b = base + 6 * n + org, *fy2b = base + 7 * n + org;
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gq.sj, gq.sk};
-  const int kb = tuned_kb(kKB);
-  constexpr int LN = adj_lines<T>();
-  const size_t ps = sizeof(PpmAdjSmem<T, LN>);
-  oeb_status stt = launch<fvtp2d_q_kernel<T>>(q_grid(d, kb), sizeof(FvQSmem<T>), st,
-                                              sqi, sqj, sfx2, sfy2, gq.origin, gcx.origin, gcy.origin, grx.origin,
-                                              gry.origin, gxf.origin, gyf.origin, gar.origin, p1, p2, d, kb);
-  // the x and y sweeps of the two PPM adjoints (axis flag 0 / 1)
-  for (int axis = 0; axis < 2 && stt == OEB_OK; ++axis) {
-    const int a = axis ? d.ny : d.nx, l = axis ? d.nx : d.ny;
-    stt = launch<fvtp2d_adj_qij_kernel<T>>(dim3((a + 5 + 31) / 32, (l + LN - 1) / LN, d.nz), ps, st, qib, qjb, sqi, sqj,
-                                           gcx.origin, gcy.origin, gxf.origin, gyf.origin, gf1.origin, gg1.origin, p1,
-                                           p2, d, axis);
+  if constexpr (std::is_same<T, float>::value) {
+    OEB_TRY(scratch_alloc(&buf, (size_t)n * 2 * sizeof(T), st));
+    float *qib = static_cast<float*>(buf) + org, *qjb = qib + n;
+    using A = fvtp2d_adj_qi_f32;
+    using B = fvtp2d_adj_qj_f32;
+    using C = fvtp2d_adj_q_f32;
+    const MarchShape ma = march_shape(d.nx + 5, d.ny, d.nz, 1, A::kCols, A::kApron, A::kMinCtas);
+    oeb_status stt = launch<A>(ma.grid, 0, st, qib, gq.origin, gcx.origin, gcy.origin, gxf.origin, gyf.origin, gry.origin,
+                               gar.origin, gf1.origin, p1, p2, d, ma.rows, ma.wx_log);
+    const MarchShape mb = march_shape(d.nx, d.ny + 5, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    if (stt == OEB_OK)
+      stt = launch<B>(mb.grid, 0, st, qjb, gq.origin, gcx.origin, gcy.origin, gxf.origin, gyf.origin, grx.origin, gar.origin,
+                      gg1.origin, p1, p2, d, mb.rows, mb.wx_log);
+    const MarchShape mc = march_shape(d.nx + 6, d.ny + 6, d.nz, 1, C::kCols, C::kApron, C::kMinCtas);
+    if (stt == OEB_OK)
+      stt = launch<C>(mc.grid, 0, st, gqb.origin, gq.origin, gcx.origin, gcy.origin, gxf.origin, gyf.origin, grx.origin,
+                      gry.origin, gar.origin, gf1.origin, gg1.origin, qib, qjb, p1, p2, d, mc.rows, mc.wx_log);
+    scratch_free(buf, st);
+    return stt;
+  } else {
+    OEB_TRY(scratch_alloc(&buf, (size_t)n * 8 * sizeof(T), st));
+    T* base = static_cast<T*>(buf);
+    T *sqi = base + org, *sqj = base + n + org, *sfx2 = base + 2 * n + org, *sfy2 = base + 3 * n + org,
+      *qib = base + 4 * n + org, *qjb = base + 5 * n + org, *fx2b = base + 6 * n + org, *fy2b = base + 7 * n + org;
+    const int kb = tuned_kb(kKB);
+    constexpr int LN = adj_lines<T>();
+    const size_t ps = sizeof(PpmAdjSmem<T, LN>);
+    oeb_status stt = launch<fvtp2d_q_kernel<T>>(q_grid(d, kb), sizeof(FvQSmem<T>), st,
+                                                sqi, sqj, sfx2, sfy2, gq.origin, gcx.origin, gcy.origin, grx.origin,
+                                                gry.origin, gxf.origin, gyf.origin, gar.origin, p1, p2, d, kb);
+    // the x and y sweeps of the two PPM adjoints (axis flag 0 / 1)
+    for (int axis = 0; axis < 2 && stt == OEB_OK; ++axis) {
+      const int a = axis ? d.ny : d.nx, l = axis ? d.nx : d.ny;
+      stt = launch<fvtp2d_adj_qij_kernel<T>>(dim3((a + 5 + 31) / 32, (l + LN - 1) / LN, d.nz), ps, st, qib, qjb, sqi, sqj,
+                                             gcx.origin, gcy.origin, gxf.origin, gyf.origin, gf1.origin, gg1.origin, p1,
+                                             p2, d, axis);
+    }
+    if (stt == OEB_OK)
+      stt = launch<fvtp2d_adj_f2_kernel<T>>(tile_grid(d.nx + 5, d.ny + 5, d.nz, kT, kT, kb), sizeof(AdjF2Smem<T>), st,
+                                            fx2b, fy2b, qib,
+                                            qjb, gxf.origin, gyf.origin, grx.origin, gry.origin, gf1.origin, gg1.origin, d,
+                                            kb);
+    for (int axis = 0; axis < 2 && stt == OEB_OK; ++axis) {
+      const int a = axis ? d.ny : d.nx, l = axis ? d.nx : d.ny;
+      stt = launch<fvtp2d_adj_q_kernel<T>>(dim3((a + 6 + 31) / 32, (l + 6 + LN - 1) / LN, d.nz), ps, st, gqb.origin,
+                                           gq.origin, gcx.origin, gcy.origin, gar.origin, grx.origin, gry.origin, qib, qjb,
+                                           fx2b, fy2b, p1, p2, d, axis);
+    }
+    scratch_free(buf, st);
+    return stt;
   }
-  if (stt == OEB_OK)
-    stt = launch<fvtp2d_adj_f2_kernel<T>>(tile_grid(d.nx + 5, d.ny + 5, d.nz, kT, kT, kb), sizeof(AdjF2Smem<T>), st,
-                                          fx2b, fy2b, qib,
-                                          qjb, gxf.origin, gyf.origin, grx.origin, gry.origin, gf1.origin, gg1.origin, d,
-                                          kb);
-  for (int axis = 0; axis < 2 && stt == OEB_OK; ++axis) {
-    const int a = axis ? d.ny : d.nx, l = axis ? d.nx : d.ny;
-    stt = launch<fvtp2d_adj_q_kernel<T>>(dim3((a + 6 + 31) / 32, (l + 6 + LN - 1) / LN, d.nz), ps, st, gqb.origin,
-                                         gq.origin, gcx.origin, gcy.origin, gar.origin, grx.origin, gry.origin, qib, qjb,
-                                         fx2b, fy2b, p1, p2, d, axis);
-  }
-  scratch_free(buf, st);
-  return stt;
 }
 
 }  // namespace

@@ -126,9 +126,9 @@ enum StepOpBase : int {
   kOpFvQ,
   kOpFvFlux,
   kOpFvMarch,       // fvtp2d_march_f32: the FP32 fvtp2d in one launch
-  kOpFvAdjQij,
-  kOpFvAdjF2,
-  kOpFvAdjQ,
+  kOpFvAdjQij,  // FP32: fvtp2d_adj_qi_f32
+  kOpFvAdjF2,   // FP32: fvtp2d_adj_qj_f32
+  kOpFvAdjQ,    // FP32: fvtp2d_adj_q_f32
   kOpHadv5AdjTiled,  // hadv_adj_f32<5>: the FP32 advection adjoint in one tiled launch
   kStepOpBases
 };

@@ -48,6 +48,15 @@ __device__ __forceinline__ void put(float* p, int64_t o, float v) {
   *reinterpret_cast<float*>(reinterpret_cast<char*>(p) + o) = v;
 }
 
+// x where `used`, else 1: the numerator of a quotient that other lanes discard.  (The division's fast
+// path does not take a zero, and one lane sends its whole warp through the slow path; the compiler
+// would drop a plain select whose other side is never used.)
+__device__ __forceinline__ float numerator(bool used, float x) {
+  float r = used ? x : 1.f;
+  asm("" : "+f"(r));
+  return r;
+}
+
 // Strip and chunk of a marching warp: a CTA's 8 warps are 2^wx_log strips x the rest in chunks of rows.
 struct MarchPos {
   int strip, chunk;

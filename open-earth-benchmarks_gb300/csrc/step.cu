@@ -79,11 +79,11 @@ using StepBodies = OpList<
     step_hd::hdiffsmag_adj_terms_kernel<float>, step_hd::hdiffsmag_adj_ts_kernel<float>,
     step_hd::hdiffsmag_adj_gather_kernel<float>, step_pw::hadv_adj_f32<5>,
     step_fws::fastwavesuv_adj_terms_kernel<float>, step_fws::fastwavesuv_adj_kernel<float, 0>,
-    step_fv::fvtp2d_q_kernel<F64i>, step_fv::fvtp2d_q_kernel<float>, step_fv::fvtp2d_flux_kernel<F64i>,
+    step_fv::fvtp2d_q_kernel<F64i>, step_fv::fvtp2d_flux_kernel<F64i>,
     step_fv::fvtp2d_march_f32, step_fv::fvtp2d_adj_qij_kernel<F64i>,
-    step_fv::fvtp2d_adj_qij_kernel<float>, step_fv::fvtp2d_adj_f2_kernel<F64i>,
-    step_fv::fvtp2d_adj_f2_kernel<float>, step_fv::fvtp2d_adj_q_kernel<F64i>,
-    step_fv::fvtp2d_adj_q_kernel<float>>;
+    step_fv::fvtp2d_adj_qi_f32, step_fv::fvtp2d_adj_f2_kernel<F64i>,
+    step_fv::fvtp2d_adj_qj_f32, step_fv::fvtp2d_adj_q_kernel<F64i>,
+    step_fv::fvtp2d_adj_q_f32>;
 
 template <class... B>
 constexpr bool ids_valid(OpList<B...>) {

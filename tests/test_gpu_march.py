@@ -67,3 +67,41 @@ def test_row_kernels_match_the_plain_kernels(pkg, fields, cuda, name, size):
     for a in spec.by_role("out3"):
         np.testing.assert_array_equal(dev[a.name].numpy().view(np.uint32), host[a.name].numpy().view(np.uint32),
                                       err_msg="%s.%s %s vs the plain kernel" % (name, a.name, size))
+
+
+def _state(pkg, fields, cuda, name, nx, ny, nz, h, dtype):
+    import torch
+    inputs = fields.make_inputs(name, nx, ny, nz, seed=31, workload="physical", halo=h)
+    dev = lambda v: pkg.Storage(torch.from_numpy(v.astype(np.float32).astype(dtype)).to(cuda), h,  # noqa: E731
+                                nx=nx if v.ndim == 3 else None)
+    rng = np.random.default_rng(37)
+    shape = (nz + 2 * h, ny + 2 * h, nx + 2 * h)
+    ybar = {n: dev(rng.normal(size=shape)) for n in pkg.KERNELS[name].semantic_outputs}
+    xbar = {n: dev(np.full(shape, fields.SENTINEL)) for n in pkg.ACTIVE[name]}
+    sc = {k: float(np.float32(v)) for k, v in fields.make_scalars(name, seed=31).items()}
+    pkg.adjoint(name, {k: dev(v) for k, v in inputs.items()}, ybar, xbar, sc, domain=(nx, ny, nz))
+    torch.cuda.synchronize()
+    return {n: s.numpy().astype(np.float64) for n, s in xbar.items()}
+
+
+@pytest.mark.parametrize("size", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
+@pytest.mark.parametrize("name", ("fvtp2d",))
+def test_marching_adjoint_matches_fp64(pkg, fields, cuda, name, size):
+    """The FP32 adjoint against the FP64 one on the same (FP32) inputs and seeds.  About forty roundings
+    of 6e-8 enter a gradient cell, on terms no larger than a few times the largest gradient: 1e-5
+    of it bounds their sum.  A monotonicity flag decided within a rounding of zero may differ: with
+    |m|, |r| of order 0.05 and values of order 1 that is about 1e-5 of the flags, six cells each."""
+    nx, ny, nz, h, _ = size
+    got = _state(pkg, fields, cuda, name, nx, ny, nz, h, np.float32)
+    want = _state(pkg, fields, cuda, name, nx, ny, nz, h, np.float64)
+    reach = {a.name: a.reach for a in pkg.KERNELS[name].args}
+    for n in want:
+        ilo, ihi, jlo, jhi, klo, khi = reach[n]
+        box = (slice(h - klo, h + nz + khi), slice(h - jlo, h + ny + jhi), slice(h - ilo, h + nx + ihi))
+        off = np.ones(want[n].shape, dtype=bool)
+        off[box] = False
+        assert (got[n][off] == fields.SENTINEL).all(), "%s: %sb written outside its box" % (name, n)
+        err = np.abs(got[n][box] - want[n][box])
+        assert np.isfinite(got[n][box]).all()
+        bad = np.count_nonzero(err > 1e-5 * np.abs(want[n][box]).max())
+        assert bad <= 8 + 1e-3 * err.size, "%s: %d of %d cells of %sb differ" % (name, bad, err.size, n)
