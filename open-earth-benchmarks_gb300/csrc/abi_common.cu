@@ -166,6 +166,23 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
   return k.shape;
 }
 
+int march_levels(int ctas, int nz, int ctas_per_sm) {
+  const double slots = (double)device_sms() * ctas_per_sm;
+  int best = 1;
+  double least = 0.0;
+  for (int chunks = 1; chunks <= nz; ++chunks) {
+    const int kb = (nz + chunks - 1) / chunks;
+    const double waves = (double)ctas * ((nz + kb - 1) / kb) / slots;
+    const double full = (double)(int64_t)waves, rest = waves - full;
+    const double cost = (full < 1.0 ? 1.0 : full + (rest == 0.0 || rest > 0.5 ? rest : 0.5)) * (kb + 4);
+    if (chunks == 1 || cost < least) {
+      least = cost;
+      best = kb;
+    }
+  }
+  return best;
+}
+
 Recorder* recorder() { return t_recorder; }
 void set_recorder(Recorder* r) { t_recorder = r; }
 

@@ -211,9 +211,6 @@ template <class T>
 constexpr int adj_kb() {
   return sizeof(T) == 4 ? 2 : 3;
 }
-// the same for the FP32 march that forms its coefficients itself (each level's are formed
-// (kb + 2) / kb times)
-constexpr int kAdjFusedKB = 4;
 
 template <class T, class M3, class M1>
 oeb_status fastwavesuv_entry(const M3* uout, const M3* vout, const M3* uin, const M3* vin, const M3* utens,
@@ -310,8 +307,7 @@ struct FastwavesAdjTerms {
   T *au, *ax, *av, *ay;  // in the layout of the state fields, 0 outside the interior unread
 };
 
-// What the terms are formed from, for a march that forms them itself (FP32: see
-// fastwavesuv_adj_kernel).
+// What the terms are formed from.
 template <class T>
 struct FastwavesAdjState {
   const T *hhl, *rho, *fx;
@@ -360,17 +356,13 @@ struct FastwavesAdjSmem {
   T av[kR][kT];
 };
 
-// FUSED (1): the march forms au, au gx, av, av gy itself at each level it reads (the FP32 form:
-// its divisions are cheap, and the 16 bytes a point the terms pass writes and the march reads
-// back cost more), from `st`, with the terms pass's expressions; else it reads them from tm.
-template <class T, int FUSED = 0>
+template <class T>
 struct fastwavesuv_adj_kernel {
-  static constexpr int kStepOp = step_op<T>(FUSED ? kOpFwsAdjFused : kOpFwsAdj);  // the step kernel's id
+  static constexpr int kStepOp = step_op<T>(kOpFwsAdj);  // the step kernel's id
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uinb, T* __restrict__ vinb,
                                              T* __restrict__ utensb, T* __restrict__ vtensb, T* __restrict__ ppuvb,
                                              const T* __restrict__ wgtfac, FastwavesAdjTerms<T> tm,
-                                             FastwavesAdjState<T> st, const T* __restrict__ uoutb,
-                                             const T* __restrict__ voutb, T dt, Dims d, int kb) {
+                                             const T* __restrict__ uoutb, const T* __restrict__ voutb, T dt, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FastwavesAdjSmem<T>& s = *reinterpret_cast<FastwavesAdjSmem<T>*>(smem_raw);
     const int i0 = blk.x * kT, j0 = blk.y * kT;
@@ -394,7 +386,6 @@ struct fastwavesuv_adj_kernel {
         return T(0);
       }
       const int64_t o = (int64_t)k * sk + i + j * sj;
-      if constexpr (FUSED) return fastwaves_adj_coef<T, true>(st, uoutb, o, j, sj, sk, dt, ag);
       *ag = ld(tm.ax + o);
       return ld(tm.au + o);
     };
@@ -404,7 +395,6 @@ struct fastwavesuv_adj_kernel {
         return T(0);
       }
       const int64_t o = (int64_t)k * sk + i + j * sj;
-      if constexpr (FUSED) return fastwaves_adj_coef<T, false>(st, voutb, o, j, sj, sk, dt, ag);
       *ag = ld(tm.ay + o);
       return ld(tm.av + o);
     };
@@ -454,6 +444,137 @@ struct fastwavesuv_adj_kernel {
   }
 };
 
+// FP32, marching levels: a warp owns 30 columns (lane = i0 - 1 + lane) and R rows of the box
+// [0, nx] x [0, ny], and marches up a chunk of levels.  At level L every lane forms au, au gx of its R
+// rows and av, av gy of those and the row below; the lane below hands over au(i-1), and the
+// three-level window of cb stays in registers, as do hhl and wgtfac of the level before.  Nothing
+// waits on a barrier.  fastwavesuv_adj_kernel's operations on the same operands in the same order: the
+// same bits.
+//
+// What bounds it: DRAM at large domains (0.47 of the HBM copy rate over the ten fields it must move at
+// 256 x 256 x 80) and issue, its divisions first.  One row a warp, four CTAs an SM: 22.5 us at
+// 128 x 128 x 80, 66.2 at 256 x 256 x 80, 31.6 at 201 x 173 x 61 (two rows and three CTAs 27.0 / 83.3 /
+// 39.9, three rows and two CTAs 24.4 / 64.8 / 33.2: fewer coefficients twice, but fewer warps); the
+// shared-memory march of fastwavesuv_adj_kernel that formed its coefficients itself took 73.0, 161.6
+// and 76.3 us.
+struct fastwavesuv_adj_march_f32 {
+  static constexpr int kStepOp = step_op<float>(kOpFwsAdjFused);  // the step kernel's id
+  static constexpr int R = 1, kCols = 30, kMinCtas = 4;
+  // level L: hhl at L + 1 and rho on rows ja - 1 .. ja + R, voutb on ja - 1 .. ja + R - 1, uoutb and
+  // wgtfac on ja .. ja + R - 1
+  struct Level {
+    float h[R + 2], r[R + 2], yv[R + 1], yu[R], w[R];
+  };
+  static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uinb, float* __restrict__ vinb,
+                                             float* __restrict__ utensb, float* __restrict__ vtensb,
+                                             float* __restrict__ ppuvb, const float* __restrict__ wgtfac,
+                                             FastwavesAdjState<float> st, const float* __restrict__ uoutb,
+                                             const float* __restrict__ voutb, float dt, Dims d, int kb) {
+    const int nx = d.nx, ny = d.ny, nz = d.nz;
+    const int i0 = (int)blk.x * kCols, ja = ((int)blk.y * kTY + (int)threadIdx.y) * R;
+    if (ja > ny) return;
+    const int lane = (int)threadIdx.x, i = i0 - 1 + lane, ic = max(0, min(i, nx));
+    const bool own = lane >= 1 && lane <= kCols && i <= nx, in_i = i >= 0 && i < nx;
+    const int Ks = -1 + (int)blk.z * kb, Ke = min(Ks + kb, nz + 1);
+    const int64_t sjb = d.sj * 4, skb = d.sk * 4;
+    // offsets of rows ja - 1 .. ja + R (clamped to the fields) at level 0
+    int64_t row[R + 2];
+    float fx2[R];
+#pragma unroll
+    for (int b = 0; b < R + 2; ++b) row[b] = ((int64_t)max(0, min(ja - 1 + b, ny)) * d.sj + ic) * 4;
+#pragma unroll
+    for (int b = 0; b < R; ++b) fx2[b] = 2.f * ld(st.fx + (int64_t)min(ja + b, ny - 1) * st.s1d);
+    auto in_j = [&](int j) { return j >= 0 && j < ny; };
+    // hhl at the chunk's first level, wgtfac one level below
+    float h0[R + 2], w0[R];
+#pragma unroll
+    for (int b = 0; b < R + 2; ++b) h0[b] = get(st.hhl, row[b] + (int64_t)max(0, Ks - 1) * skb);
+#pragma unroll
+    for (int b = 0; b < R; ++b) w0[b] = 0.f;
+    Level n;
+    auto fetch = [&](int L) {
+      const int64_t k = (int64_t)L * skb;
+      if (L >= 0 && L < nz) {
+#pragma unroll
+        for (int b = 0; b < R + 2; ++b) n.h[b] = get(st.hhl, row[b] + k + skb), n.r[b] = get(st.rho, row[b] + k);
+#pragma unroll
+        for (int b = 0; b < R + 1; ++b) n.yv[b] = (in_i && in_j(ja - 1 + b)) ? get(voutb, row[b] + k) : 0.f;
+#pragma unroll
+        for (int b = 0; b < R; ++b) n.yu[b] = (in_i && in_j(ja + b)) ? get(uoutb, row[b + 1] + k) : 0.f;
+      }
+      if (L >= 0 && L <= nz) {
+#pragma unroll
+        for (int b = 0; b < R; ++b) n.w[b] = get(wgtfac, row[b + 1] + k);
+      }
+    };
+    n = Level{};
+    fetch(Ks - 1);
+    float cm2[R], cm1[R], dir[R], yu0[R], yv0[R];
+#pragma unroll
+    for (int b = 0; b < R; ++b) cm2[b] = cm1[b] = dir[b] = yu0[b] = yv0[b] = 0.f;
+#pragma unroll 1
+    for (int L = Ks - 1; L <= Ke; ++L) {
+      const Level c = n;
+      if (L < Ke) fetch(L + 1);
+      const bool in_l = L >= 0 && L < nz;
+      float au[R], ax[R], av[R + 1], ay[R + 1], aum[R], axm[R];
+#pragma unroll
+      for (int b = 0; b < R + 1; ++b) {
+        av[b] = ay[b] = 0.f;
+        if (b < R) au[b] = ax[b] = aum[b] = axm[b] = 0.f;
+      }
+      if (in_l) {
+        // the hhl sums and differences and rho of the rows, and of the lane above for the R rows
+        float hs[R + 2], hd[R + 2];
+#pragma unroll
+        for (int b = 0; b < R + 2; ++b) hs[b] = c.h[b] + h0[b], hd[b] = c.h[b] - h0[b], h0[b] = c.h[b];
+#pragma unroll
+        for (int b = 0; b < R + 1; ++b) {
+          const bool ok = in_i && in_j(ja - 1 + b);
+          const float q = st.ed2 / (c.r[b + 1] + c.r[b]);
+          const float a = -(dt * q) * c.yv[b];
+          const float g = numerator(ok, 0.5f * (hs[b] - hs[b + 1])) / (hd[b] + hd[b + 1]);
+          av[b] = ok ? a : 0.f;
+          ay[b] = ok && a != 0.f ? a * g : 0.f;
+        }
+#pragma unroll
+        for (int b = 0; b < R; ++b) {
+          const bool ok = in_i && in_j(ja + b);
+          const float hsn = lane_above<1>(hs[b + 1]), hdn = lane_above<1>(hd[b + 1]), rn = lane_above<1>(c.r[b + 1]);
+          const float q = fx2[b] / (rn + c.r[b + 1]);
+          const float a = -(dt * q) * c.yu[b];
+          const float g = numerator(ok, 0.5f * (hs[b + 1] - hsn)) / (hd[b + 1] + hdn);
+          au[b] = ok ? a : 0.f;
+          ax[b] = ok && a != 0.f ? a * g : 0.f;
+          aum[b] = lane_below<1>(au[b]), axm[b] = lane_below<1>(ax[b]);
+        }
+      }
+      const int K = L - 1;
+#pragma unroll
+      for (int b = 0; b < R; ++b) {
+        const float cl = in_l ? ((ax[b] + axm[b]) + (ay[b + 1] + ay[b])) : 0.f;
+        if (K >= Ks && own && ja + b <= ny) {
+          const int64_t o = row[b + 1] + (int64_t)K * skb;
+          const float kbK = cm2[b] - cm1[b], kbK1 = cm1[b] - cl;
+          float acc = dir[b];
+          if (K >= 0) acc = acc + w0[b] * kbK;
+          if (K + 1 <= nz) acc = acc + (1.f - c.w[b]) * kbK1;
+          put(ppuvb, o, acc);
+          if (K >= 0 && K < nz && in_i && ja + b < ny) {
+            put(uinb, o, yu0[b]);
+            put(vinb, o, yv0[b]);
+            put(utensb, o, dt * yu0[b]);
+            put(vtensb, o, dt * yv0[b]);
+          }
+        }
+        dir[b] = (aum[b] - au[b]) + (av[b] - av[b + 1]);
+        cm2[b] = cm1[b], cm1[b] = cl;
+        yu0[b] = c.yu[b], yv0[b] = c.yv[b + 1], w0[b] = c.w[b];
+      }
+    }
+  }
+};
+
 template <class T, class M3, class M1>
 oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utensb, const M3* vtensb,
                                  const M3* ppuvb, const M3* uin, const M3* vin, const M3* utens, const M3* vtens,
@@ -490,11 +611,11 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
   const FastwavesAdjState<T> state{gh.origin, gr.origin, lfx.origin, lfx.s, ed2};
   if constexpr (std::is_same<T, float>::value) if (adjoint_tiles()) {
     // one launch: the march forms the coefficients at the kb + 2 levels of its k-block
-    const int kb = tuned_kb(kAdjFusedKB);
-    return launch<fastwavesuv_adj_kernel<T, 1>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 2, kT, kT, kb),
-                                                   sizeof(FastwavesAdjSmem<T>), st, gub.origin, gvb.origin,
-                                                   gutb.origin, gvtb.origin, gpb.origin, gw.origin,
-                                                   FastwavesAdjTerms<T>{}, state, guo.origin, gvo.origin, dt, d, kb);
+    using B = fastwavesuv_adj_march_f32;
+    const int gx = (d.nx + B::kCols) / B::kCols, gy = (d.ny + kTY * B::R) / (kTY * B::R);
+    const int kb = tuned_kb(march_levels(gx * gy, d.nz + 2, B::kMinCtas));
+    return launch<B>(dim3((unsigned)gx, (unsigned)gy, (unsigned)((d.nz + 1 + kb) / kb)), 0, st, gub.origin, gvb.origin,
+                     gutb.origin, gvtb.origin, gpb.origin, gw.origin, state, guo.origin, gvo.origin, dt, d, kb);
   }
   // scratch for the four coefficient fields, in uoutb's layout
   const T* start = (uoutb->allocated && uoutb->allocated <= uoutb->aligned) ? uoutb->allocated : uoutb->aligned;
@@ -514,7 +635,7 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
   if (stt == OEB_OK)
     stt = launch<fastwavesuv_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 2, kT, kT, kb),
                                             sizeof(FastwavesAdjSmem<T>), st, gub.origin, gvb.origin, gutb.origin,
-                                            gvtb.origin, gpb.origin, gw.origin, tm, state, guo.origin, gvo.origin, dt,
+                                            gvtb.origin, gpb.origin, gw.origin, tm, guo.origin, gvo.origin, dt,
                                             d, kb);
   scratch_free(buf, st);
   return stt;

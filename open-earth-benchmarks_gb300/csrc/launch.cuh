@@ -113,8 +113,8 @@ enum StepOpBase : int {
   kOpCombine,
   kOpFwsFwd,
   kOpFwsAdjTerms,
-  kOpFwsAdj,       // fastwavesuv_adj_kernel<T, 0>: the march over the terms pass's coefficients
-  kOpFwsAdjFused,  // fastwavesuv_adj_kernel<T, 1>: the march that forms them itself
+  kOpFwsAdj,       // fastwavesuv_adj_kernel: the march over the terms pass's coefficients
+  kOpFwsAdjFused,  // fastwavesuv_adj_march_f32: the FP32 march that forms them itself
   kOpHadv5Fwd,     // + tile shape (3 shapes)
   kOpHadv5AdjTerms = kOpHadv5Fwd + 3,  // + tile shape
   kOpHadv5AdjGather = kOpHadv5AdjTerms + 3,

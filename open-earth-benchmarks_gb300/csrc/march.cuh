@@ -76,5 +76,8 @@ struct MarchShape {
 // cols: columns a strip writes; apron: rows a chunk marches beyond its own; ctas_per_sm: CTAs the
 // kernel's registers allow.
 MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm);
+// Levels a chunk for a kernel that marches nz levels with `ctas` CTAs a chunk and forms two levels
+// beyond its own.
+int march_levels(int ctas, int nz, int ctas_per_sm);
 
 }  // namespace oeb

@@ -65,8 +65,8 @@ struct OpList {};
 using StepBodies = OpList<
     step_ch::combine_kernel<F64i>, step_ch::combine_kernel<float>,
     step_fws::fastwavesuv_kernel<F64i>, step_fws::fastwavesuv_march_f32,
-    step_fws::fastwavesuv_adj_terms_kernel<F64i>, step_fws::fastwavesuv_adj_kernel<F64i, 0>,
-    step_fws::fastwavesuv_adj_kernel<float, 1>,
+    step_fws::fastwavesuv_adj_terms_kernel<F64i>, step_fws::fastwavesuv_adj_kernel<F64i>,
+    step_fws::fastwavesuv_adj_march_f32,
     step_pw::hadv_kernel<F64i, 5, 0>, step_pw::hadv_kernel<F64i, 5, 1>, step_pw::hadv_kernel<F64i, 5, 2>,
     step_pw::hadv_march_f32<5>,
     step_pw::hadv_adj_terms_kernel<F64i, 5, 0>, step_pw::hadv_adj_terms_kernel<F64i, 5, 1>,
@@ -78,7 +78,7 @@ using StepBodies = OpList<
     step_hd::hdiffsmag_adj_gather_kernel<F64i>, step_hd::hdiffsmag_adj_f32,
     step_hd::hdiffsmag_adj_terms_kernel<float>, step_hd::hdiffsmag_adj_ts_kernel<float>,
     step_hd::hdiffsmag_adj_gather_kernel<float>, step_pw::hadv_adj_f32<5>,
-    step_fws::fastwavesuv_adj_terms_kernel<float>, step_fws::fastwavesuv_adj_kernel<float, 0>,
+    step_fws::fastwavesuv_adj_terms_kernel<float>, step_fws::fastwavesuv_adj_kernel<float>,
     step_fv::fvtp2d_q_kernel<F64i>, step_fv::fvtp2d_flux_kernel<F64i>,
     step_fv::fvtp2d_march_f32, step_fv::fvtp2d_adj_qij_kernel<F64i>,
     step_fv::fvtp2d_adj_qi_f32, step_fv::fvtp2d_adj_f2_kernel<F64i>,
