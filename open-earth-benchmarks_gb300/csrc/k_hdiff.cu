@@ -838,37 +838,24 @@ struct hdiffsmag_adj_gather_kernel {
   }
 };
 
-// FP32 adjoint in one launch.  The three passes above write six term fields to scratch and
-// read them back (about 48 bytes a point of FP32 traffic beyond the adjoint's own fields, and
-// three launches).  In FP32 the terms are cheap to recompute, so here a CTA forms, for a
-// 32 x 32 tile of (ubar, vbar), everything its outputs gather in shared memory:
-//   u, v   : 36 x 36 from (i0-2, j0-2)     (the fields, 0 outside their reach [-1, N+1)^2)
-//   t      : 35 x 35 from (i0-1, j0-1)     T on [0, N]^2, else 0
-//   s      : 35 x 35 from (i0-2, j0-2)     S on [-1, N)^2, else 0
-//   lu, lv, xu, xv : 34 x 34 from (i0-1, j0-1), at interior points, else 0
-//   tb     : 33 x 33 from (i0, j0)         TB on [0, N]^2, else 0   } over u, v
-//   sb     : 33 x 33 from (i0-1, j0-1)     SB on [-1, N)^2, else 0  } (dead by then)
-// with the output tile at (i0, j0) = (-1 + 32 bx, -1 + 32 by).  Every value is the same
-// expression on the same operands as in the three passes (T and S from the same
-// differences, the terms, TB and SB with the same guarded sums, the gather in the same
-// order), so the results are theirs, bit for bit; the recomputed apron costs about 20 % more
-// arithmetic than the passes.
-struct SmagAdjF32Smem {
-  union {
-    struct {
-      float u[36][36], v[36][36];
-    } f;
-    struct {
-      float tb[33][33], sb[33][33];
-    } g;
-  } x;
-  float t[35][35], s[35][35];
-  float lu[34][34], lv[34][34], xu[34][34], xv[34][34];
-  float acr[36], cto[36], ctu[36], cvo[36], cvu[36];  // rows j0-2+r
-};
-
+// FP32 adjoint in one launch, marching rows (march.cuh): lane = column i0 - 2 + lane, 28 columns of
+// the box [-1, n+1)^2 a strip.  When row r of u and v arrives, a lane forms T at r and S at r - 1; the
+// terms lu, lv, xu, xv of point p = r - 1; TB at p and SB at r - 2; and gathers (ubar, vbar) of row
+// j = r - 2.  Neighbouring columns come from the lanes beside it, earlier rows from registers, each
+// value formed once a warp.  Every value is the same expression on the same operands as in the three
+// passes above (a term that is zero is added where they skip it), so the results are theirs, bit for
+// bit, without their 48 bytes a point of term scratch.
+//
+// What bounds it: instruction issue (about 320 instructions a row, two square roots and two divisions
+// among them).  79 registers, three CTAs an SM: 25.7 us at 128 x 128 x 80, 82.0 at 256 x 256 x 80, 35.4 at
+// 201 x 173 x 61 (four, which spills, 34.9 / 88.8 / 42.8); the 32 x 32 shared-memory tile it replaces took
+// 43.6, 125.7 and 56.3 us.
 struct hdiffsmag_adj_f32 {
   static constexpr int kStepOp = step_op<float>(kOpSmagAdjFused);  // the step kernel's id
+  static constexpr int kCols = 28, kApron = 4, kMinCtas = 3;
+  struct Row {
+    float u, v, m, yu, yv;  // u and v on row r; mask, uoutb, voutb on row r - 1
+  };
   static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uinb, float* __restrict__ vinb,
                                              const float* __restrict__ uin, const float* __restrict__ vin,
                                              const float* __restrict__ mask, const float* __restrict__ crlavo,
@@ -876,150 +863,104 @@ struct hdiffsmag_adj_f32 {
                                              const float* __restrict__ crlatu, const float* __restrict__ acrlat0,
                                              int64_t s1d, const float* __restrict__ uoutb,
                                              const float* __restrict__ voutb, float eddlat, float eddlon,
-                                             float tau_smag, float weight_smag, Dims d, int kb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SmagAdjF32Smem& s = *reinterpret_cast<SmagAdjF32Smem*>(smem_raw);
+                                             float tau_smag, float weight_smag, Dims d, int rows, int wx_log) {
+    const MarchPos pos = march_pos(blk, wx_log);
+    const int nx = d.nx, ny = d.ny;
+    const int i0 = -1 + pos.strip * kCols, oa = -1 + pos.chunk * rows, ob = min(oa + rows, ny + 1);
+    if (i0 >= nx + 1 || oa >= ny + 1) return;
     constexpr float rr = earth_radius_recip<float>();
     const float c1 = eddlat * rr;
-    const int nx = d.nx, ny = d.ny;
-    const int64_t sj = d.sj;
-    const int i0 = -1 + (int)blk.x * kT, j0 = -1 + (int)blk.y * kT;
-    auto in = [&](int i, int j) { return i >= 0 && i < nx && j >= 0 && j < ny; };
-    auto inT = [&](int i, int j) { return i >= 0 && i <= nx && j >= 0 && j <= ny; };
-    auto inS = [&](int i, int j) { return i >= -1 && i < nx && j >= -1 && j < ny; };
-    const int tid = threadIdx.y * kTX + threadIdx.x;
-    if (tid < 36) {
-      const int j = j0 - 2 + tid;
-      const int64_t jo = (int64_t)j * s1d;
-      const bool in1 = j >= -1 && j < ny + 1, in0 = j >= 0 && j < ny;
-      s.acr[tid] = in1 ? ld(acrlat0 + jo) : 0.f;
-      s.cto[tid] = in0 ? ld(crlato + jo) : 0.f;
-      s.ctu[tid] = in0 ? ld(crlatu + jo) : 0.f;
-      s.cvo[tid] = in0 ? ld(crlavo + jo) : 0.f;
-      s.cvu[tid] = in0 ? ld(crlavu + jo) : 0.f;
-    }
-    const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
-  #pragma unroll 1
-    for (int k = k0; k < k1; ++k) {
-      const int64_t kofs = (int64_t)k * d.sk;
-      for_region<36, 36>([&](int a, int b) {
-        const int i = i0 - 2 + a, j = j0 - 2 + b;
-        const bool ok = i >= -1 && i < nx + 1 && j >= -1 && j < ny + 1;
-        const int64_t o = kofs + i + j * sj;
-        s.x.f.u[b][a] = ok ? ld(uin + o) : 0.f;
-        s.x.f.v[b][a] = ok ? ld(vin + o) : 0.f;
-      });
-      __syncthreads();
-      // T = c1 (v(j-1) - v) - c2 (u(i-1) - u),  S = c1 (u(j+1) - u) + c2 (v(i+1) - v)  (smag_T, smag_S)
-      for_region<35, 35>([&](int a, int b) {
-        const int i = i0 - 1 + a, j = j0 - 1 + b;
-        float t = 0.f;
-        if (inT(i, j)) {
-          const float c2 = s.acr[b + 1] * eddlon;
-          t = c1 * (s.x.f.v[b][a + 1] - s.x.f.v[b + 1][a + 1]) - c2 * (s.x.f.u[b + 1][a] - s.x.f.u[b + 1][a + 1]);
-        }
-        s.t[b][a] = t;
-      });
-      for_region<35, 35>([&](int a, int b) {
-        const int i = i0 - 2 + a, j = j0 - 2 + b;
-        float v = 0.f;
-        if (inS(i, j)) {
-          const float c2 = s.acr[b] * eddlon;
-          v = c1 * (s.x.f.u[b + 1][a] - s.x.f.u[b][a]) + c2 * (s.x.f.v[b][a + 1] - s.x.f.v[b][a]);
-        }
-        s.s[b][a] = v;
-      });
-      __syncthreads();
-      // the terms at interior points (hdiffsmag_adj_terms_kernel)
-      for_region<34, 34>([&](int a, int b) {
-        const int i = i0 - 1 + a, j = j0 - 1 + b;
-        float lu = 0.f, lv = 0.f, xu = 0.f, xv = 0.f;
-        if (in(i, j)) {
-          const int64_t o = kofs + i + j * sj;
-          const float ti = s.t[b][a], tip = s.t[b][a + 1], tjp = s.t[b + 1][a];
-          const float si = s.s[b + 1][a + 1], sjm = s.s[b][a + 1], sim = s.s[b + 1][a];
-          const float xuu = 0.5f * (tip * tip + ti * ti) + 0.5f * (sjm * sjm + si * si);
-          const float xvv = 0.5f * (tjp * tjp + ti * ti) + 0.5f * (sim * sim + si * si);
-          const float hdw = weight_smag * ld(mask + o);
-          const float ru = Prec<float>::sqrt_(xuu), rv = Prec<float>::sqrt_(xvv);
-          const float smu = tau_smag * ru - hdw, smv = tau_smag * rv - hdw;
-          const float su = clamp_smag(smu), sv = clamp_smag(smv);
-          const float u0 = s.x.f.u[b + 1][a + 1], v0 = s.x.f.v[b + 1][a + 1];
-          const float lapu = (s.x.f.u[b + 1][a + 2] + s.x.f.u[b + 1][a] - 2.f * u0) +
-                             s.cto[b + 1] * (s.x.f.u[b + 2][a + 1] - u0) + s.ctu[b + 1] * (s.x.f.u[b][a + 1] - u0);
-          const float lapv = (s.x.f.v[b + 1][a + 2] + s.x.f.v[b + 1][a] - 2.f * v0) +
-                             s.cvo[b + 1] * (s.x.f.v[b + 2][a + 1] - v0) + s.cvu[b + 1] * (s.x.f.v[b][a + 1] - v0);
-          const float yu = ld(uoutb + o), yv = ld(voutb + o);
-          lu = su * yu;
-          lv = sv * yv;
-          xu = (smu > 0.f && smu < 0.5f) ? (lapu * yu) * (tau_smag / (2.f * ru)) : 0.f;
-          xv = (smv > 0.f && smv < 0.5f) ? (lapv * yv) * (tau_smag / (2.f * rv)) : 0.f;
-        }
-        s.lu[b][a] = lu;
-        s.lv[b][a] = lv;
-        s.xu[b][a] = xu;
-        s.xv[b][a] = xv;
-      });
-      __syncthreads();
-      // the T and S adjoints (hdiffsmag_adj_ts_kernel), over the dead u, v
-      for_region<33, 33>([&](int a, int b) {
-        const int i = i0 + a, j = j0 + b;
-        float tb = 0.f;
-        if (inT(i, j)) {
-          float w = 0.f;
-          if (in(i - 1, j)) w = w + s.xu[b + 1][a];
-          if (in(i, j)) w = w + s.xu[b + 1][a + 1] + s.xv[b + 1][a + 1];
-          if (in(i, j - 1)) w = w + s.xv[b][a + 1];
-          tb = (w == 0.f) ? 0.f : s.t[b + 1][a + 1] * w;
-        }
-        s.x.g.tb[b][a] = tb;
-      });
-      for_region<33, 33>([&](int a, int b) {
-        const int i = i0 - 1 + a, j = j0 - 1 + b;
-        float sb = 0.f;
-        if (inS(i, j)) {
-          float w = 0.f;
-          if (in(i, j + 1)) w = w + s.xu[b + 1][a];
-          if (in(i, j)) w = w + s.xu[b][a] + s.xv[b][a];
-          if (in(i + 1, j)) w = w + s.xv[b][a + 1];
-          sb = (w == 0.f) ? 0.f : s.s[b + 1][a + 1] * w;
-        }
-        s.x.g.sb[b][a] = sb;
-      });
-      __syncthreads();
-      // the gather (hdiffsmag_adj_gather_kernel) on [-1, N+1)^2
-      for_region<32, 32>([&](int a, int b) {
-        const int i = i0 + a, j = j0 + b;
-        if (i >= nx + 1 || j >= ny + 1) return;
-        const int64_t o = kofs + i + j * sj;
-        const float c2 = s.acr[b + 2] * eddlon;
-        float ub = 0.f, vb = 0.f;
-        if (in(i, j)) {
-          ub = ld(uoutb + o) - (2.f + s.cto[b + 2] + s.ctu[b + 2]) * s.lu[b + 1][a + 1];
-          vb = ld(voutb + o) - (2.f + s.cvo[b + 2] + s.cvu[b + 2]) * s.lv[b + 1][a + 1];
-        }
-        if (in(i - 1, j)) ub = ub + s.lu[b + 1][a], vb = vb + s.lv[b + 1][a];
-        if (in(i + 1, j)) ub = ub + s.lu[b + 1][a + 2], vb = vb + s.lv[b + 1][a + 2];
-        if (in(i, j - 1)) {
-          ub = fmaf(s.cto[b + 1], s.lu[b][a + 1], ub);
-          vb = fmaf(s.cvo[b + 1], s.lv[b][a + 1], vb);
-        }
-        if (in(i, j + 1)) {
-          ub = fmaf(s.ctu[b + 3], s.lu[b + 2][a + 1], ub);
-          vb = fmaf(s.cvu[b + 3], s.lv[b + 2][a + 1], vb);
-        }
-        const float tb0 = inT(i, j) ? s.x.g.tb[b][a] : 0.f;
-        const float sb0 = inS(i, j) ? s.x.g.sb[b + 1][a + 1] : 0.f;
-        if (inT(i + 1, j)) ub = fmaf(-c2, s.x.g.tb[b][a + 1], ub);
-        ub = fmaf(-c1, sb0, fmaf(c2, tb0, ub));
-        if (inS(i, j - 1)) ub = fmaf(c1, s.x.g.sb[b][a + 1], ub);
-        if (inT(i, j + 1)) vb = fmaf(c1, s.x.g.tb[b + 1][a], vb);
-        vb = fmaf(-c2, sb0, fmaf(-c1, tb0, vb));
-        if (inS(i - 1, j)) vb = fmaf(c2, s.x.g.sb[b + 1][a], vb);
-        uinb[o] = ub;
-        vinb[o] = vb;
-      });
-      __syncthreads();
+    const int lane = (int)threadIdx.x, i = i0 - 2 + lane;
+    const bool ok_i = i >= -1 && i < nx + 1, in_i = i >= 0 && i < nx, t_i = i >= 0 && i <= nx, s_i = i >= -1 && i < nx;
+    const bool st = ok_i && lane >= 2 && lane < 2 + kCols;
+    const int64_t sjb = d.sj * 4;
+    int64_t o = ((int64_t)blk.z * d.sk + (int64_t)(oa - 2) * d.sj + i) * 4;  // (i, r)
+    // the metric terms of 32 rows, one a lane, handed round by shuffles
+    float la, lto, ltu, lvo, lvu;
+    auto metric = [&](int j) {
+      const int64_t ja = (int64_t)max(-1, min(j + lane, ny)) * s1d, jo = (int64_t)max(0, min(j + lane, ny - 1)) * s1d;
+      la = ld(acrlat0 + ja) * eddlon;
+      lto = ld(crlato + jo), ltu = ld(crlatu + jo), lvo = ld(crlavo + jo), lvu = ld(crlavu + jo);
+    };
+    metric(oa - 2);
+    Row n{0.f, 0.f, 0.f, 0.f, 0.f};
+    auto fetch = [&](int r, int64_t q) {
+      const bool ok = ok_i && r >= -1 && r <= ny, in = in_i && r >= 1 && r <= ny;
+      n.u = ok ? get(uin, q) : 0.f, n.v = ok ? get(vin, q) : 0.f;
+      n.m = in ? get(mask, q - sjb) : 0.f;
+      n.yu = in ? get(uoutb, q - sjb) : 0.f, n.yv = in ? get(voutb, q - sjb) : 0.f;
+    };
+    fetch(oa - 2, o);
+    float u1 = 0.f, u2 = 0.f, v1 = 0.f, v2 = 0.f;      // u, v on rows r-1, r-2
+    float um1 = 0.f;                                   // u(i-1) on row r-1
+    float t1 = 0.f, s2 = 0.f;                          // T at r-1, S at r-2
+    float xu2 = 0.f, xv2 = 0.f;                        // at r-2
+    float lu2 = 0.f, lu3 = 0.f, lv2 = 0.f, lv3 = 0.f;  // at r-2, r-3
+    float tb2 = 0.f, sb3 = 0.f, yu2 = 0.f, yv2 = 0.f;  // TB at r-2, SB at r-3, the seeds at r-2
+    float c21 = 0.f, c22 = 0.f;                        // acrlat0 eddlon on rows r-1, r-2
+    // of rows r-2 and r-3
+    float to2 = 0.f, to3 = 0.f, tu2 = 0.f, vo2 = 0.f, vo3 = 0.f, vu2 = 0.f;
+#pragma unroll 1
+    for (int r = oa - 2; r < ob + 2; ++r) {
+      const Row c = n;
+      if (r + 1 < ob + 2) fetch(r + 1, o + sjb);
+      const int src = (r + 2 - oa) & 31, srp = (r + 1 - oa) & 31;
+      // the terms of row p = r - 1 are handed round before the lanes move on to the next 32 rows
+      const float to = __shfl_sync(kWarpMask, lto, srp), tu = __shfl_sync(kWarpMask, ltu, srp),
+                  vo = __shfl_sync(kWarpMask, lvo, srp), vu = __shfl_sync(kWarpMask, lvu, srp);
+      if (src == 0 && r > oa - 2) metric(r);
+      const float c2 = __shfl_sync(kWarpMask, la, src);
+      const int p = r - 1, j = r - 2;
+      const bool in_p = in_i && p >= 0 && p < ny;
+      // T at r and S at p (smag_T, smag_S)
+      const float um = lane_below<1>(c.u);
+      const float tv = c1 * (v1 - c.v) - c2 * (um - c.u);
+      const float t0 = t_i && r >= 0 && r <= ny ? tv : 0.f;
+      const float sv = c1 * (c.u - u1) + c21 * (lane_above<1>(v1) - v1);
+      const float s1 = s_i && p >= -1 && p < ny ? sv : 0.f;
+      // the terms at p (hdiffsmag_adj_terms_kernel)
+      const float tip = lane_above<1>(t1), sim = lane_below<1>(s1);
+      const float xuu = 0.5f * (tip * tip + t1 * t1) + 0.5f * (s2 * s2 + s1 * s1);
+      const float xvv = 0.5f * (t0 * t0 + t1 * t1) + 0.5f * (sim * sim + s1 * s1);
+      const float hdw = weight_smag * c.m;
+      const float ru = sqrtf(numerator(in_p, xuu)), rv = sqrtf(numerator(in_p, xvv));
+      const float smu = tau_smag * ru - hdw, smv = tau_smag * rv - hdw;
+      const float lapu = (lane_above<1>(u1) + um1 - 2.f * u1) + to * (c.u - u1) + tu * (u2 - u1);
+      const float lapv = (lane_above<1>(v1) + lane_below<1>(v1) - 2.f * v1) + vo * (c.v - v1) + vu * (v2 - v1);
+      const bool open_u = in_p && smu > 0.f && smu < 0.5f, open_v = in_p && smv > 0.f && smv < 0.5f;
+      const float xuv = (lapu * c.yu) * (tau_smag / (2.f * numerator(open_u, ru)));
+      const float xvw = (lapv * c.yv) * (tau_smag / (2.f * numerator(open_v, rv)));
+      const float lu1 = in_p ? clamp_smag(smu) * c.yu : 0.f, lv1 = in_p ? clamp_smag(smv) * c.yv : 0.f;
+      const float xu1 = open_u ? xuv : 0.f, xv1 = open_v ? xvw : 0.f;
+      // TB at p and SB at j (hdiffsmag_adj_ts_kernel)
+      const float wt = (((0.f + lane_below<1>(xu1)) + xu1) + xv1) + xv2;
+      const float tb1 = (wt == 0.f || !(t_i && p >= 0 && p <= ny)) ? 0.f : t1 * wt;
+      const float ws = (((0.f + xu1) + xu2) + xv2) + lane_above<1>(xv2);
+      const float sb2 = (ws == 0.f || !(s_i && j >= -1 && j < ny)) ? 0.f : s2 * ws;
+      // the gather at row j (hdiffsmag_adj_gather_kernel)
+      float ub = 0.f, vb = 0.f;
+      if (in_i && j >= 0 && j < ny) {
+        ub = yu2 - (2.f + to2 + tu2) * lu2;
+        vb = yv2 - (2.f + vo2 + vu2) * lv2;
+      }
+      ub = ub + lane_below<1>(lu2), vb = vb + lane_below<1>(lv2);
+      ub = ub + lane_above<1>(lu2), vb = vb + lane_above<1>(lv2);
+      ub = fmaf(to3, lu3, ub), vb = fmaf(vo3, lv3, vb);
+      ub = fmaf(tu, lu1, ub), vb = fmaf(vu, lv1, vb);
+      ub = fmaf(-c22, lane_above<1>(tb2), ub);
+      ub = fmaf(-c1, sb2, fmaf(c22, tb2, ub));
+      ub = fmaf(c1, sb3, ub);
+      vb = fmaf(c1, tb1, vb);
+      vb = fmaf(-c22, sb2, fmaf(-c1, tb2, vb));
+      vb = fmaf(c22, lane_below<1>(sb2), vb);
+      if (st && j >= oa) put(uinb, o - 2 * sjb, ub), put(vinb, o - 2 * sjb, vb);
+      u2 = u1, u1 = c.u, v2 = v1, v1 = c.v, um1 = um;
+      t1 = t0, s2 = s1, xu2 = xu1, xv2 = xv1;
+      lu3 = lu2, lu2 = lu1, lv3 = lv2, lv2 = lv1;
+      tb2 = tb1, sb3 = sb2, yu2 = c.yu, yv2 = c.yv;
+      c22 = c21, c21 = c2;
+      to3 = to2, to2 = to, tu2 = tu, vo3 = vo2, vo2 = vo, vu2 = vu;
+      o += sjb;
     }
   }
 };
@@ -1045,14 +986,13 @@ oeb_status hdiffsmag_adj_entry(const M3* uinb, const M3* vinb, const M3* uin, co
   cudaStream_t st = (cudaStream_t)stream;
   if constexpr (std::is_same<T, float>::value) if (adjoint_tiles()) {
     const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gui.sj, gui.sk};
-    const int kb = tuned_kb(kKB);
-    auto org1 = [](const M1* m) { return (const float*)m->aligned + m->offset; };
-    return launch<hdiffsmag_adj_f32>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, kT, kb), sizeof(SmagAdjF32Smem), st,
-                                     gub.origin, gvb.origin, gui.origin, (const float*)vin->aligned + vin->offset,
-                                     (const float*)mask->aligned + mask->offset, org1(crlavo), org1(crlavu),
-                                     org1(crlato), org1(crlatu), org1(acrlat0), acrlat0->strides[0], guo.origin,
-                                     (const float*)voutb->aligned + voutb->offset, eddlat, eddlon, tau_smag,
-                                     weight_smag, d, kb);
+    using B = hdiffsmag_adj_f32;
+    const MarchShape m = march_shape(d.nx + 2, d.ny + 2, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+    auto org1 = [](const M1* m1) { return (const float*)m1->aligned + m1->offset; };
+    return launch<B>(m.grid, 0, st, gub.origin, gvb.origin, gui.origin, (const float*)vin->aligned + vin->offset,
+                     (const float*)mask->aligned + mask->offset, org1(crlavo), org1(crlavu), org1(crlato), org1(crlatu),
+                     org1(acrlat0), acrlat0->strides[0], guo.origin, (const float*)voutb->aligned + voutb->offset,
+                     eddlat, eddlon, tau_smag, weight_smag, d, m.rows, m.wx_log);
   }
   const T* start = (uin->allocated && uin->allocated <= uin->aligned) ? uin->allocated : uin->aligned;
   const int64_t last = (uin->sizes[0] - 1) * uin->strides[0] + (uin->sizes[1] - 1) * uin->strides[1] +

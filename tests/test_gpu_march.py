@@ -85,7 +85,7 @@ def _state(pkg, fields, cuda, name, nx, ny, nz, h, dtype):
 
 
 @pytest.mark.parametrize("size", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
-@pytest.mark.parametrize("name", ("fvtp2d", "fastwavesuv"))
+@pytest.mark.parametrize("name", ("fvtp2d", "fastwavesuv", "hdiffsmag"))
 def test_marching_adjoint_matches_fp64(pkg, fields, cuda, name, size):
     """The FP32 adjoint against the FP64 one on the same (FP32) inputs and seeds.  About forty roundings
     of 6e-8 enter a gradient cell, on terms no larger than a few times the largest gradient: 1e-5
