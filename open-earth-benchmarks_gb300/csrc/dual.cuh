@@ -34,6 +34,10 @@ __host__ __device__ constexpr Dual<T> operator*(Dual<T> a, Dual<T> b) {
   return Dual<T>(a.v * b.v, a.v * b.d + a.d * b.v);
 }
 template <class T>
+__device__ __forceinline__ Dual<T> mul_zero(Dual<T> a, Dual<T> b) {
+  return Dual<T>(mul_zero(a.v, b.v), mul_zero(a.v, b.d) + mul_zero(a.d, b.v));
+}
+template <class T>
 __host__ __device__ constexpr Dual<T> operator/(Dual<T> a, Dual<T> b) {
   return Dual<T>(a.v / b.v, (a.d * b.v - a.v * b.d) / (b.v * b.v));
 }

@@ -645,7 +645,8 @@ struct PpmAdjSmem {
 // One transposed PPM sweep along AXIS (0: i, 1: j) for outputs A..A+nout-1 on lines
 // L0..L0+nl-1 (nout <= 32, nl <= LN: a tile at the edge of its output box works on its own part of
 // the window and lines only; every phase's window shrinks by the 32 - nout missing outputs).
-// gst(p, l): state value at axis position p of line l (0 where the field is not defined);
+// gst(p, l): state value at axis position p of line l (any finite value where the field is not
+// defined; its nearest defined one, since a zero takes F64i's slow path);
 // cv(p, l): Courant number at flux point p (any value elsewhere);
 // fb(p, l): flux adjoint at p (0 off the flux points);  put(a, l, v): receives gbar(a).
 template <class T, int AXIS, int LN, class GS, class CV, class FB, class PUT>
@@ -700,7 +701,7 @@ __device__ __forceinline__ void ppm_sweep_adjoint(PpmAdjSmem<T, LN>& s, int A, i
     T t = T(0);
     if (f != T(0) && (s.smt[l][w - 1] | s.smt[l][w])) {
       const T c = cv(p, L0 + l);
-      t = f * ((c > T(0)) ? (T(1) - c) : (T(1) + c));
+      t = f * (T(1) + neg_abs(c));
     }
     s.u1.tb[l][w] = t;
   });
@@ -761,7 +762,7 @@ struct fvtp2d_adj_qij_kernel {
       const int A = -3 + (int)blk.x * 32, L0 = (int)blk.y * LN;
       ppm_sweep_adjoint<T, 0, LN>(
           s, A, L0, max(0, min(32, nx + 2 - A)), max(0, min(LN, ny - L0)), p1, p2,
-          [&](int p, int l) { return (p >= -3 && p < nx + 2 && l < ny) ? ld(q_i + kofs + p + l * sj) : T(0); },
+          [&](int p, int l) { return ld(q_i + kofs + max(-3, min(p, nx + 1)) + l * sj); },
           [&](int p, int l) { return ld(crx + kofs + p + l * sj); },
           [&](int p, int l) {
             return (p >= 0 && p < nx && l < ny) ? (T(0.5) * ld(xfx + kofs + p + l * sj)) * ld(fx1b + kofs + p + l * sj)
@@ -775,7 +776,7 @@ struct fvtp2d_adj_qij_kernel {
       const int A = -3 + (int)blk.x * 32, L0 = (int)blk.y * LN;
       ppm_sweep_adjoint<T, 1, LN>(
           s, A, L0, max(0, min(32, ny + 2 - A)), max(0, min(LN, nx - L0)), p1, p2,
-          [&](int p, int l) { return (p >= -3 && p < ny + 2 && l < nx) ? ld(q_j + kofs + l + p * sj) : T(0); },
+          [&](int p, int l) { return ld(q_j + kofs + l + max(-3, min(p, ny + 1)) * sj); },
           [&](int p, int l) { return ld(cry + kofs + l + p * sj); },
           [&](int p, int l) {
             return (p >= 0 && p < ny && l < nx) ? (T(0.5) * ld(yfx + kofs + l + p * sj)) * ld(fy1b + kofs + l + p * sj)
@@ -822,12 +823,12 @@ struct fvtp2d_adj_f2_kernel {
       for_region_lim<32, 33>(vx, vy + 1, [&](int a, int b) {
         const int i = i0 + a, r = j0 - 1 + b;
         const int64_t o = kofs + i + r * sj;
-        s.ry[b][a] = (r >= 0 && r < ny && i < nx + 2) ? qib[o] / ld(ra_y + o) : T(0);
+        s.ry[b][a] = (r >= 0 && r < ny && i < nx + 2) ? div_zero(qib[o], ld(ra_y + o)) : T(0);
       });
       for_region_lim<33, 32>(vx + 1, vy, [&](int a, int b) {
         const int c = i0 - 1 + a, j = j0 + b;
         const int64_t o = kofs + c + j * sj;
-        s.rx[b][a] = (c >= 0 && c < nx && j < ny + 2) ? qjb[o] / ld(ra_x + o) : T(0);
+        s.rx[b][a] = (c >= 0 && c < nx && j < ny + 2) ? div_zero(qjb[o], ld(ra_x + o)) : T(0);
       });
       __syncthreads();
       for_region_lim<32, 32>(vx, vy, [&](int a, int b) {
@@ -836,11 +837,11 @@ struct fvtp2d_adj_f2_kernel {
         const bool interior = i >= 0 && i < nx && j >= 0 && j < ny;
         if (j >= 0 && j < ny + 1) {
           T g = interior ? (T(0.5) * ld(yfx + o)) * ld(fy1b + o) : T(0);
-          fy2b[o] = g + ld(yfx + o) * (s.ry[b + 1][a] - s.ry[b][a]);
+          fy2b[o] = g + mul_zero(s.ry[b + 1][a] - s.ry[b][a], ld(yfx + o));
         }
         if (i >= 0 && i < nx + 1) {
           T g = interior ? (T(0.5) * ld(xfx + o)) * ld(fx1b + o) : T(0);
-          fx2b[o] = g + ld(xfx + o) * (s.rx[b][a + 1] - s.rx[b][a]);
+          fx2b[o] = g + mul_zero(s.rx[b][a + 1] - s.rx[b][a], ld(xfx + o));
         }
       });
       __syncthreads();
@@ -865,7 +866,7 @@ struct fvtp2d_adj_q_kernel {
     const int nx = d.nx, ny = d.ny, sj = (int)d.sj;
     const int64_t kofs = (int64_t)blk.z * d.sk;
     auto qval = [&](int i, int j) {
-      return (i >= -3 && i < nx + 3 && j >= -3 && j < ny + 3) ? ld(q + kofs + i + j * sj) : T(0);
+      return ld(q + kofs + max(-3, min(i, nx + 2)) + max(-3, min(j, ny + 2)) * sj);
     };
     const int A = -3 + (int)blk.x * 32, L0 = -3 + (int)blk.y * LN;
     if (!AXIS_Y) {
@@ -881,8 +882,8 @@ struct fvtp2d_adj_q_kernel {
             if (a >= -3 && a < nx + 3 && l >= -3 && l < ny + 3) {
               const int64_t o = kofs + a + l * sj;
               T acc = v;
-              if (a >= -3 && a < nx + 2 && l >= 0 && l < ny) acc = acc + (ld(area + o) / ld(ra_y + o)) * qib[o];
-              if (a >= 0 && a < nx && l >= -3 && l < ny + 2) acc = acc + (ld(area + o) / ld(ra_x + o)) * qjb[o];
+              if (a >= -3 && a < nx + 2 && l >= 0 && l < ny) acc = acc + mul_zero(qib[o], ld(area + o) / ld(ra_y + o));
+              if (a >= 0 && a < nx && l >= -3 && l < ny + 2) acc = acc + mul_zero(qjb[o], ld(area + o) / ld(ra_x + o));
               qb[o] = acc;
             }
           });
@@ -918,15 +919,6 @@ struct fvtp2d_adj_q_kernel {
 // with a cold cache), 222 at 256 x 256 x 80, 115 at 201 x 173 x 61 (three CTAs for all 83 / 235 / 113);
 // the passes above, run for float, took 154.8, 521.5 and 229.4 us.  Zero numerators that reached the
 // division's slow path (numerator(), div_zero()) were 12 us of it at 128 x 128 x 80.
-
-// a / b, with the IEEE quotient's bits, for numerators that are often exactly zero (a gradient where no
-// flux enters): the division's fast path does not take a zero, and a warp of 32 cells nearly always
-// has one.
-__device__ __forceinline__ float div_zero(float a, float b) {
-  const bool zero = a == 0.f && fabsf(b) > 0.f && fabsf(b) < __int_as_float(0x7f800000);
-  const float q = numerator(!zero, a) / b;
-  return zero ? a * b : q;
-}
 
 // One face of a transposed sweep: t = tb, z = the product with c of B0 (-(|c| tb) on either side),
 // each on the side that takes it (U: the cell below, where c > 0; L: the cell above), and the flux

@@ -290,7 +290,7 @@ struct hdiffsmag_kernel {
           lu.add(-scale2<1>(uc));
           lu.add_prod(s.crlato[b], s.dyu[b + 1][a + 1]);
           lu.add_prod(s.crlatu[b], -s.dyu[b][a + 1]);
-          uout[o] = uc + smag_u * lu.get();
+          uout[o] = uc + mul_zero(smag_u, lu.get());  // the clamp gives many zeros
           // hdiffsmag.h:248-259
           T smag_v = tau_smag * Prec<T>::sqrt_(scale2<-1>(iadd(s.tsq[b + 1][a], s.tsq[b][a])) +
                                                scale2<-1>(s.ssq[b + 1][a] + s.ssq[b + 1][a + 1])) -
@@ -302,7 +302,7 @@ struct hdiffsmag_kernel {
           lv.add(-scale2<1>(vc));
           lv.add_prod(s.crlavo[b], s.dyv[b + 1][a]);
           lv.add_prod(s.crlavu[b], -s.dyv[b][a]);
-          vout[o] = vc + smag_v * lv.get();
+          vout[o] = vc + mul_zero(smag_v, lv.get());
         }
       });
       __syncthreads();
@@ -749,8 +749,8 @@ struct hdiffsmag_adj_terms_kernel {
         const T lapv = (ld(vin + o + 1) + ld(vin + o - 1) - T(2) * v0) + ld(crlavo + jo) * (ld(vin + o + sj) - v0) +
                        ld(crlavu + jo) * (ld(vin + o - sj) - v0);
         const T yu = ld(uoutb + o), yv = ld(voutb + o);
-        tm.lu[o] = su * yu;
-        tm.lv[o] = sv * yv;
+        tm.lu[o] = mul_zero(su, yu);
+        tm.lv[o] = mul_zero(sv, yv);
         tm.xu[o] = (smu > T(0) && smu < T(0.5)) ? (lapu * yu) * (tau_smag / (T(2) * ru)) : T(0);
         tm.xv[o] = (smv > T(0) && smv < T(0.5)) ? (lapv * yv) * (tau_smag / (T(2) * rv)) : T(0);
       });
@@ -773,14 +773,14 @@ struct hdiffsmag_adj_ts_kernel {
       const T c2 = ld(acrlat0 + (int64_t)j * s1d) * eddlon;
       if (i >= 0 && i <= d.nx && j >= 0 && j <= d.ny) {
         T w = T(0);
-        if (in(i - 1, j)) w = w + tm.xu[o - 1];
+        if (in(i - 1, j)) w = tm.xu[o - 1];
         if (in(i, j)) w = w + tm.xu[o] + tm.xv[o];
         if (in(i, j - 1)) w = w + tm.xv[o - sj];
         tm.tb[o] = (w == T(0)) ? T(0) : smag_T(uin, vin, o, sj, c1, c2) * w;
       }
       if (i >= -1 && i < d.nx && j >= -1 && j < d.ny) {
         T w = T(0);
-        if (in(i, j + 1)) w = w + tm.xu[o + sj];
+        if (in(i, j + 1)) w = tm.xu[o + sj];
         if (in(i, j)) w = w + tm.xu[o] + tm.xv[o];
         if (in(i + 1, j)) w = w + tm.xv[o + 1];
         tm.sb[o] = (w == T(0)) ? T(0) : smag_S(uin, vin, o, sj, c1, c2) * w;
@@ -809,8 +809,8 @@ struct hdiffsmag_adj_gather_kernel {
       T ub = T(0), vb = T(0);
       if (in(a, b)) {
         const int64_t bo = (int64_t)b * s1d;
-        ub = ld(uoutb + o) - (T(2) + ld(crlato + bo) + ld(crlatu + bo)) * tm.lu[o];
-        vb = ld(voutb + o) - (T(2) + ld(crlavo + bo) + ld(crlavu + bo)) * tm.lv[o];
+        ub = ld(uoutb + o) - mul_zero(tm.lu[o], T(2) + ld(crlato + bo) + ld(crlatu + bo));
+        vb = ld(voutb + o) - mul_zero(tm.lv[o], T(2) + ld(crlavo + bo) + ld(crlavu + bo));
       }
       if (in(a - 1, b)) ub = ub + tm.lu[o - 1], vb = vb + tm.lv[o - 1];
       if (in(a + 1, b)) ub = ub + tm.lu[o + 1], vb = vb + tm.lv[o + 1];

@@ -16,6 +16,7 @@
 
 #include <cuda_runtime.h>
 
+#include "precision.cuh"
 #include "stencil_util.cuh"
 
 namespace oeb {
@@ -37,24 +38,12 @@ __device__ __forceinline__ bool here_or_below(bool c) {
   return ((m | (m << 1)) >> threadIdx.x) & 1u;
 }
 
-// -|a|
-__device__ __forceinline__ float neg_abs(float a) { return __int_as_float(__float_as_int(a) | (int)0x80000000); }
-
 // The field p at byte offset o.
 __device__ __forceinline__ float get(const float* p, int64_t o) {
   return ld(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + o));
 }
 __device__ __forceinline__ void put(float* p, int64_t o, float v) {
   *reinterpret_cast<float*>(reinterpret_cast<char*>(p) + o) = v;
-}
-
-// x where `used`, else 1: the numerator of a quotient that other lanes discard.  (The division's fast
-// path does not take a zero, and one lane sends its whole warp through the slow path; the compiler
-// would drop a plain select whose other side is never used.)
-__device__ __forceinline__ float numerator(bool used, float x) {
-  float r = used ? x : 1.f;
-  asm("" : "+f"(r));
-  return r;
 }
 
 // Strip and chunk of a marching warp: a CTA's 8 warps are 2^wx_log strips x the rest in chunks of rows.
