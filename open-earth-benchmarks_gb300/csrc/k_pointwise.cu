@@ -42,25 +42,35 @@ struct TileOf {
   static constexpr int J = S == 0 ? 32 : S == 1 ? 8 : 16;
 };
 
-// Visits the points of this thread in a TI x TJ tile: TI / 32 columns 32 apart, TJ / 8 rows 8
-// apart (U of them unrolled); f(o, j) with o the in-plane offset of (i, j) plus the plane
+// Visits the points of this thread in a TI x TJ tile: in each 32 columns TJ / 8 rows 8 apart (U
+// of them unrolled; the cells dealt by TileCells where U is 1); f(o, j) with o the in-plane offset of (i, j) plus the plane
 // offset of k.
 template <int TI, int TJ, int U, class F>
 __device__ __forceinline__ void for_points_tile(const uint3& blk, const Dims& d, int kb, F&& f) {
   const int k0 = blk.z * kb;
   const int k1 = min(k0 + kb, d.nz);
-  const int sj = (int)d.sj;
+  const int sj = (int)d.sj, j0 = (int)blk.y * TJ;
 #pragma unroll 1
   for (int k = k0; k < k1; ++k) {
     const int64_t kofs = (int64_t)k * d.sk;
 #pragma unroll 1
     for (int c = 0; c < TI / 32; ++c) {
-      const int i = blk.x * TI + 32 * c + threadIdx.x;
-      if (i < d.nx) {
+      const int i0 = (int)blk.x * TI + 32 * c;
+      if constexpr (U == 1) {
+        const TileCells t(d.nx - i0, min(d.ny - j0, TJ));
+#pragma unroll 1
+        for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
+          const int b = t.row(e), i = i0 + (e - b * t.w), j = j0 + b;
+          f(kofs + i + j * sj, j);
+        }
+      } else {
+        const int i = i0 + (int)threadIdx.x;
+        if (i < d.nx) {
 #pragma unroll U
-        for (int r = 0; r < TJ / kTY; ++r) {
-          const int j = blk.y * TJ + threadIdx.y + kTY * r;
-          if (j < d.ny) f(kofs + i + j * sj, j);
+          for (int r = 0; r < TJ / kTY; ++r) {
+            const int j = j0 + (int)threadIdx.y + kTY * r;
+            if (j < d.ny) f(kofs + i + j * sj, j);
+          }
         }
       }
     }
@@ -71,20 +81,7 @@ __device__ __forceinline__ void for_points_tile(const uint3& blk, const Dims& d,
 // plane offset of k.
 template <int U = kRows, class F>
 __device__ __forceinline__ void for_points(const uint3& blk, const Dims& d, int kb, F&& f) {
-  const int i = blk.x * kTI + threadIdx.x;
-  if (i >= d.nx) return;
-  const int k0 = blk.z * kb;
-  const int k1 = min(k0 + kb, d.nz);
-  const int sj = (int)d.sj;
-#pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    const int64_t kofs = (int64_t)k * d.sk;
-#pragma unroll U
-    for (int r = 0; r < kRows; ++r) {
-      const int j = blk.y * kTJ + threadIdx.y + kTY * r;
-      if (j < d.ny) f(kofs + i + j * sj, j);
-    }
-  }
+  for_points_tile<kTI, kTJ, U>(blk, d, kb, f);
 }
 
 // The FP32 nh_p_grad waits on its global loads (ncu: long-scoreboard stalls, DRAM under 30 %
@@ -1022,24 +1019,6 @@ struct hadv_adj_terms_kernel {
   }
 };
 
-// Visits every cell of the box [-h, nx+h) x [-h, ny+h) x [0, nz) owned by this thread.
-template <class F>
-__device__ __forceinline__ void for_box_points(const uint3& blk, const Dims& d, int h, int kb, F&& f) {
-  const int i = -h + (int)(blk.x * kTI + threadIdx.x);
-  if (i >= d.nx + h) return;
-  const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
-  const int sj = (int)d.sj;
-#pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    const int64_t kofs = (int64_t)k * d.sk;
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      const int j = -h + (int)(blk.y * kTJ + threadIdx.y) + kTY * r;
-      if (j < d.ny + h) f(kofs + i + j * sj, i, j);
-    }
-  }
-}
-
 // update != 0 fuses the transpose of the chained step's update: the outputs are alpha * (the
 // gathered gradient), plus the seeds (yu, yv) inside the interior -- the same two roundings as
 // the gradient stored and then combined by a separate kernel.
@@ -1049,9 +1028,9 @@ struct hadv_adj_gather_kernel {
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uinb, T* __restrict__ vinb,
                                              HadvTerms<T> tm, Dims d, int kb, const T* __restrict__ yu,
                                              const T* __restrict__ yv, T alpha, int update) {
-    constexpr int h = ORDER == 3 ? 2 : 3;
+    constexpr int h = ORDER == 3 ? 2 : 3, GU = RowUnroll<T>::value;
     const int64_t sj = d.sj;
-    for_box_points(blk, d, h, kb, [&](int64_t o, int a, int b) {
+    for_box<GU>(blk, d, -h, -h, d.nx + 2 * h, d.ny + 2 * h, kb, [&](int64_t o, int a, int b) {
       auto in = [&](int i, int j) { return i >= 0 && i < d.nx && j >= 0 && j < d.ny; };
       T ub = T(0), vb = T(0);
       // upwind stencils: point (a - m, b) reads (a, b) with offset m, and likewise in j

@@ -137,25 +137,55 @@ struct HeavyRowUnroll<F64i> {
   static constexpr int value = 1;
 };
 
+// The cells of a tile's part of a box, w <= 32 columns of up to 32 rows, dealt to the CTA's threads in
+// row order: cell e is row(e), column e - row(e) w.  A full tile gives a warp a row.  A tile at the
+// box's far edge, 6 columns wide say, gives a warp several short rows: the boxes of the adjoint kernels
+// are the interior widened by 1 to 6, so that a lane a column left a fifth of the warps of a
+// 128-column interior nearly empty.  The FP64 loops (U == 1 below) visit cells this way: adjoint
+// of hdiffsmag 255 -> 227 us, of hadvuv5th 268 -> 253 at 128 x 128 x 80, hadvuv 142 -> 132 at
+// 201 x 173 x 61.  The FP32 ones keep a lane a column, whose rows lie at compile-time distances:
+// dealt cells made the laplacian's FP32 adjoint 34.4 us instead of 20.5 at 256 x 256 x 80.
+struct TileCells {
+  int w, n;
+  unsigned m;  // row(e) = e / w for e < 1024: the error e (1 / w - m / 2^16) is less than 1 / w
+  __device__ __forceinline__ TileCells(int cols, int rows)
+      : w(min(cols, 32)), n(w > 0 ? w * max(0, rows) : 0), m(65536u / (unsigned)max(w, 1) + 1u) {}
+  __device__ __forceinline__ int row(int e) const { return (int)(((unsigned)e * m) >> 16); }
+};
+
 // Visits, for this thread, the cells (i, j, k) of the box [ilo, ilo+ni) x [jlo, jlo+nj) x
-// [k0, k0+kb) of its CTA: blk.x/y pick a 32 x 32 tile, each thread takes 4 rows (U of them
-// unrolled).  f(o, i, j) gets the plane-plus-in-plane offset o of (i, j, k) from the
+// [k0, k0+kb) of its CTA: blk.x/y pick a 32 x 32 tile, each thread takes up to 4 cells of a level (U
+// of them unrolled).  f(o, i, j) gets the plane-plus-in-plane offset o of (i, j, k) from the
 // interior origin.
 template <int U = 32 / kTY, class F>
 __device__ __forceinline__ void for_box(const uint3& blk, const Dims& d, int ilo, int jlo, int ni, int nj, int kb,
                                         F&& f) {
-  const int a = (int)(blk.x * 32 + threadIdx.x);
-  if (a >= ni) return;
-  const int i = ilo + a;
   const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
   const int sj = (int)d.sj;
+  if constexpr (U == 1) {
+    const int a0 = (int)blk.x * 32, b0 = (int)blk.y * 32;
+    const TileCells t(ni - a0, min(nj - b0, 32));
 #pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    const int64_t kofs = (int64_t)k * d.sk;
+    for (int k = k0; k < k1; ++k) {
+      const int64_t kofs = (int64_t)k * d.sk;
+#pragma unroll 1
+      for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
+        const int r = t.row(e), i = ilo + a0 + (e - r * t.w), b = b0 + r;
+        f(kofs + i + (jlo + b) * sj, i, jlo + b);
+      }
+    }
+  } else {
+    const int a = (int)(blk.x * 32 + threadIdx.x);
+    if (a >= ni) return;
+    const int i = ilo + a;
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      const int64_t kofs = (int64_t)k * d.sk;
 #pragma unroll U
-    for (int r = 0; r < 32 / kTY; ++r) {
-      const int b = (int)(blk.y * 32 + threadIdx.y) + kTY * r;
-      if (b < nj) f(kofs + i + (jlo + b) * sj, i, jlo + b);
+      for (int r = 0; r < 32 / kTY; ++r) {
+        const int b = (int)(blk.y * 32 + threadIdx.y) + kTY * r;
+        if (b < nj) f(kofs + i + (jlo + b) * sj, i, jlo + b);
+      }
     }
   }
 }
@@ -165,17 +195,31 @@ __device__ __forceinline__ void for_box(const uint3& blk, const Dims& d, int ilo
 template <int U = 32 / kTY, class F>
 __device__ __forceinline__ void for_box_k(const uint3& blk, int64_t sj, int64_t sk, int ilo, int jlo, int ni, int nj,
                                           int nk, int kb, F&& f) {
-  const int a = (int)(blk.x * 32 + threadIdx.x);
-  if (a >= ni) return;
-  const int i = ilo + a;
   const int k0 = blk.z * kb, k1 = min(k0 + kb, nk);
+  if constexpr (U == 1) {
+    const int a0 = (int)blk.x * 32, b0 = (int)blk.y * 32;
+    const TileCells t(ni - a0, min(nj - b0, 32));
 #pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    const int64_t kofs = (int64_t)k * sk;
+    for (int k = k0; k < k1; ++k) {
+      const int64_t kofs = (int64_t)k * sk;
+#pragma unroll 1
+      for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
+        const int r = t.row(e), i = ilo + a0 + (e - r * t.w), b = b0 + r;
+        f(kofs + i + (int64_t)(jlo + b) * sj, i, jlo + b, k);
+      }
+    }
+  } else {
+    const int a = (int)(blk.x * 32 + threadIdx.x);
+    if (a >= ni) return;
+    const int i = ilo + a;
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      const int64_t kofs = (int64_t)k * sk;
 #pragma unroll U
-    for (int r = 0; r < 32 / kTY; ++r) {
-      const int b = (int)(blk.y * 32 + threadIdx.y) + kTY * r;
-      if (b < nj) f(kofs + i + (int64_t)(jlo + b) * sj, i, jlo + b, k);
+      for (int r = 0; r < 32 / kTY; ++r) {
+        const int b = (int)(blk.y * 32 + threadIdx.y) + kTY * r;
+        if (b < nj) f(kofs + i + (int64_t)(jlo + b) * sj, i, jlo + b, k);
+      }
     }
   }
 }
