@@ -204,14 +204,7 @@ struct fastwavesuv_march_f32 {
   }
 };
 
-constexpr int kKB = 1;     // k-levels per CTA by default (the most CTAs hide latency best)
-// the adjoint march's k-levels per CTA (measured at 128 x 128 x 80: FP64 best at 3, FP32 at
-// 2; a block of kb levels reads the coefficients of kb + 2)
-template <class T>
-constexpr int adj_kb() {
-  return sizeof(T) == 4 ? 2 : 3;
-}
-
+constexpr int kKB = 1;  // k-levels per CTA by default (the most CTAs hide latency best)
 template <class T, class M3, class M1>
 oeb_status fastwavesuv_entry(const M3* uout, const M3* vout, const M3* uin, const M3* vin, const M3* utens,
                              const M3* vtens, const M3* wgtfac, const M3* ppuv, const M3* hhl, const M3* rho,
@@ -348,14 +341,16 @@ struct fastwavesuv_adj_terms_kernel {
   }
 };
 
-template <class T>
-struct FastwavesAdjSmem {
-  T ax[kT][kR];  // au(i0-1+a, j0+b) gx, then au itself in the second half
-  T au[kT][kR];
-  T ay[kR][kT];  // av(i0+a, j0-1+b) gy
-  T av[kR][kT];
-};
+constexpr int kAdjJ = 8;  // rows of the transpose's tile: one cell a thread
 
+// The transpose from the terms, a thread a cell of the box [0, nx] x [0, ny] and kb output levels: at level L a cell reads the eight terms that reach it, its own and those of the cells before it
+// in i and j (L1 serves the neighbours), and keeps the two levels of cb behind it in registers.
+//
+// What bounds it: the FP64 pipe (13 additions an output level, the cb of the chunk's two outer levels
+// among them) and the latency of the terms' loads.  FP64 adjoint at 128 x 128 x 80: 102 us (tiles of 16
+// rows 109, of 32 rows, fewer blocks and so shorter ones, 121; the shared-memory tile of the terms it
+// replaces, which added half as many cells again at the box's far edges, 144); at 64 x 64 x 60 36 us,
+// was 72.
 template <class T>
 struct fastwavesuv_adj_kernel {
   static constexpr int kStepOp = step_op<T>(kOpFwsAdj);  // the step kernel's id
@@ -363,83 +358,50 @@ struct fastwavesuv_adj_kernel {
                                              T* __restrict__ utensb, T* __restrict__ vtensb, T* __restrict__ ppuvb,
                                              const T* __restrict__ wgtfac, FastwavesAdjTerms<T> tm,
                                              const T* __restrict__ uoutb, const T* __restrict__ voutb, T dt, Dims d, int kb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    FastwavesAdjSmem<T>& s = *reinterpret_cast<FastwavesAdjSmem<T>*>(smem_raw);
-    const int i0 = blk.x * kT, j0 = blk.y * kT;
-    const int sj = (int)d.sj;
+    const int i0 = (int)blk.x * kT, j0 = (int)blk.y * kAdjJ, sj = (int)d.sj;
     const int64_t sk = d.sk;
     // output levels K in [Ks, Ke) of the extended range [-1, nz+1)
     const int Ks = -1 + (int)blk.z * kb, Ke = min(Ks + kb, d.nz + 1);
-    constexpr int kPts = kT * kT / kThreads;
-    T cm2[kPts], cm1[kPts], dir[kPts];  // cb(L-2), cb(L-1), direct terms of level L-1
-    // outputs of this tile in the box [0, nx] x [0, ny]: a tile at its far edge holds one
-    // column or row of them, and computes au / av only where those outputs read them (the
-    // march below reads no other cell for an output it writes)
-    const int vx = min(kT, d.nx + 1 - i0), vy = min(kT, d.ny + 1 - j0);
-  #pragma unroll
-    for (int t = 0; t < kPts; ++t) cm2[t] = cm1[t] = dir[t] = T(0);
-    const int tid = threadIdx.y * kTX + threadIdx.x;
-    // adjoint of ppgu (au) and of ppgv (av) at an interior point, and the same times g (pass 1)
-    auto au_at = [&](int i, int j, int k, T* ag) -> T {
-      if (i < 0 || i >= d.nx || j < 0 || j >= d.ny || k < 0 || k >= d.nz) {
-        *ag = T(0);
-        return T(0);
-      }
-      const int64_t o = (int64_t)k * sk + i + j * sj;
-      *ag = ld(tm.ax + o);
-      return ld(tm.au + o);
-    };
-    auto av_at = [&](int i, int j, int k, T* ag) -> T {
-      if (i < 0 || i >= d.nx || j < 0 || j >= d.ny || k < 0 || k >= d.nz) {
-        *ag = T(0);
-        return T(0);
-      }
-      const int64_t o = (int64_t)k * sk + i + j * sj;
-      *ag = ld(tm.ay + o);
-      return ld(tm.av + o);
-    };
-  #pragma unroll 1
-    for (int L = Ks - 1; L <= Ke; ++L) {
-      // au, av and their g-weighted versions at level L over the tile plus the low apron
-      for_region_lim<kR, kT>(vx + 1, vy, [&](int a, int b) {
-        const int i = i0 - 1 + a, j = j0 + b;
-        s.au[b][a] = au_at(i, j, L, &s.ax[b][a]);
-      });
-      for_region_lim<kT, kR>(vx, vy + 1, [&](int a, int b) {
-        const int i = i0 + a, j = j0 - 1 + b;
-        s.av[b][a] = av_at(i, j, L, &s.ay[b][a]);
-      });
-      __syncthreads();
-  #pragma unroll
-      for (int t = 0; t < kPts; ++t) {
-        const int e = tid + t * kThreads;
-        const int b = e / kT, a = e - b * kT;
-        const int i = i0 + a, j = j0 + b;
+    const TileCells t(d.nx + 1 - i0, min(d.ny + 1 - j0, kAdjJ));
+#pragma unroll 1
+    for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
+      const int b = t.row(e), i = i0 + (e - b * t.w), j = j0 + b;
+      const bool own = i < d.nx && j < d.ny, west = i > 0 && j < d.ny, south = j > 0 && i < d.nx;
+      int64_t o = (int64_t)(Ks - 1) * sk + i + j * sj;
+      T cm1 = T(0), kbK = T(0), dir = T(0);  // cb(L-1), kb(L-1) = cb(L-2) - cb(L-1), direct terms of level L-1
+#pragma unroll 1
+      for (int L = Ks - 1; L <= Ke; ++L, o += sk) {
+        const bool in_k = L >= 0 && L < d.nz;
+        const bool p = in_k && own, w = in_k && west, q = in_k && south;
         // cb(L) at (i, j): ppgc(i) feeds ppgu(i), ppgu(i-1), ppgv(j), ppgv(j-1)
-        const T cl = (L >= 0 && L < d.nz) ? ((s.ax[b][a + 1] + s.ax[b][a]) + (s.ay[b + 1][a] + s.ay[b][a])) : T(0);
-        const int K = L - 1;  // output level
-        if (K >= Ks && K < Ke && i <= d.nx && j <= d.ny) {
-          const int64_t o = (int64_t)K * sk + i + j * sj;
-          const T kbK = cm2[t] - cm1[t];  // kb(K)   = cb(K-1) - cb(K)
-          const T kbK1 = cm1[t] - cl;     // kb(K+1) = cb(K)   - cb(K+1)
-          T acc = dir[t];
-          if (K >= 0) acc = acc + ld(wgtfac + o) * kbK;
-          if (K + 1 <= d.nz) acc = acc + (T(1.0) - ld(wgtfac + o + sk)) * kbK1;
-          ppuvb[o] = acc;
-          if (K >= 0 && K < d.nz && i < d.nx && j < d.ny) {
-            const T ub = ld(uoutb + o), vb = ld(voutb + o);
-            uinb[o] = ub;
-            vinb[o] = vb;
-            utensb[o] = dt * ub;
-            vtensb[o] = dt * vb;
+        const T x0 = p ? ld(tm.ax + o) : T(0), x1 = w ? ld(tm.ax + o - 1) : T(0);
+        const T y0 = p ? ld(tm.ay + o) : T(0), y1 = q ? ld(tm.ay + o - sj) : T(0);
+        const T cl = (x0 + x1) + (y0 + y1);
+        const T kbL = cm1 - cl;
+        if (L > Ks) {
+          const int K = L - 1;  // output level
+          const int64_t oK = o - sk;
+          T acc = dir;
+          if (K >= 0) acc = acc + ld(wgtfac + oK) * kbK;
+          if (K + 1 <= d.nz) acc = acc + (T(1.0) - ld(wgtfac + o)) * kbL;
+          ppuvb[oK] = acc;
+          if (K >= 0 && K < d.nz && own) {
+            const T ub = ld(uoutb + oK), vb = ld(voutb + oK);
+            uinb[oK] = ub;
+            vinb[oK] = vb;
+            utensb[oK] = dt * ub;
+            vtensb[oK] = dt * vb;
           }
         }
-        // direct terms of level L: au(i-1) - au(i) + av(j-1) - av(j)
-        dir[t] = (s.au[b][a] - s.au[b][a + 1]) + (s.av[b][a] - s.av[b + 1][a]);
-        cm2[t] = cm1[t];
-        cm1[t] = cl;
+        if (L >= Ks && L < Ke) {
+          // direct terms of level L: au(i-1) - au(i) + av(j-1) - av(j)
+          const T u0 = p ? ld(tm.au + o) : T(0), u1 = w ? ld(tm.au + o - 1) : T(0);
+          const T v0 = p ? ld(tm.av + o) : T(0), v1 = q ? ld(tm.av + o - sj) : T(0);
+          dir = (u1 - u0) + (v1 - v0);
+        }
+        cm1 = cl;
+        kbK = kbL;
       }
-      __syncthreads();
     }
   }
 };
@@ -629,12 +591,13 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
   const FastwavesAdjTerms<T> tm{base + org, base + n + org, base + 2 * n + org, base + 3 * n + org};
   oeb_status stt = launch<fastwavesuv_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, 1), 0, st, tm, state,
                                                            guo.origin, gvo.origin, dt, d, 1);
-  // the march carries a three-level window of ppgc terms up the column; a k-block of kb
-  // levels reads the coefficients at kb + 2
-  const int kb = tuned_kb(adj_kb<T>());
+  // a block of kb levels reads the terms of kb + 2: about one wave of blocks, five CTAs an SM (three
+  // 114 us at 128 x 128 x 80 and 322 at 256 x 256 x 80, eight 104 and 329, five 102 and 329)
+  const dim3 cells = tile_grid(d.nx + 1, d.ny + 1, 1, kT, kAdjJ, 1);
+  const int kb = tuned_kb(march_levels((int)(cells.x * cells.y), d.nz + 2, 5));
   if (stt == OEB_OK)
-    stt = launch<fastwavesuv_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 2, kT, kT, kb),
-                                            sizeof(FastwavesAdjSmem<T>), st, gub.origin, gvb.origin, gutb.origin,
+    stt = launch<fastwavesuv_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 2, kT, kAdjJ, kb),
+                                            0, st, gub.origin, gvb.origin, gutb.origin,
                                             gvtb.origin, gpb.origin, gw.origin, tm, guo.origin, gvo.origin, dt,
                                             d, kb);
   scratch_free(buf, st);
