@@ -166,6 +166,10 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
   return k.shape;
 }
 
+bool under_a_wave(dim3 grid, int ctas_per_sm) {
+  return (int64_t)grid.x * grid.y * grid.z < (int64_t)device_sms() * ctas_per_sm;
+}
+
 int march_levels(int ctas, int nz, int ctas_per_sm) {
   const double slots = (double)device_sms() * ctas_per_sm;
   int best = 1;

@@ -12,8 +12,8 @@
 // operands.  Differences are stored once and their negations used where the reference
 // subtracts in the other order (x - y == -(y - x) exactly in IEEE round-to-nearest).
 //
-// Compiled with --fmad=false (see k_pointwise.cu).  One CTA of 32 x 8 threads per
-// 32 x 32 tile and kb k-levels.
+// Compiled with --fmad=false (see k_pointwise.cu).  One CTA of 32 x 8 threads per tile
+// and kb k-levels.
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -33,35 +33,46 @@ namespace OEB_BODIES_NS {
 
 constexpr int kT = 32;  // tile edge
 
+// Rows of a tile of hdiffsa_kernel and hdiffsmag_kernel.  16 let the registers, six CTAs of eight warps
+// an SM, bound the warps in flight, where 32 rows' shared memory (46 and 53 KB in FP64) held them to
+// four: FP64 hdiffsa 44.5 -> 38.9 us and hdiffsmag 98.3 -> 86.4 at 128 x 128 x 80, 145 -> 137 and
+// 341 -> 324 at 256 x 256 x 80 (24 rows 41.6, 94.9, 133, 325), the tangent-linear hdiffsmag 305 -> 265.
+// A grid of less than a wave of those takes 8 rows, whose CTAs are shorter: 13.0 -> 11.0 and
+// 27.1 -> 21.3 us at 64 x 64 x 60 (16 rows 11.8 and 23.5), 8.1 -> 4.3 and 15.1 -> 6.9 at
+// 33 x 20 x 10; at 128 x 128 x 80 8 rows are slower (44.1 and 89.4).  Recorded launches keep 16 rows,
+// the step kernel's form.
+constexpr int kJ = 16, kJShort = 8;
+inline bool short_tiles(const Dims& d, int kb) {
+  return !recorder() && under_a_wave(tile_grid(d.nx, d.ny, d.nz, kT, kJ, kb), 6);
+}
+
 // ============================== hdiffsa ===========================================
-// Shared layout (per k-level), tile origin (i0, j0):
-//   in  : 36 x 36, (i0-2+a, j0-2+b)
-//   dy  : 34 x 35, (i0-1+a, j0-2+b)   dy(i,j)  = in(i,j+1) - in(i,j)
-//   lap : 34 x 34, (i0-1+a, j0-1+b)
-//   flx : 33 x 32, (i0-1+a, j0+b)
-//   fly : 32 x 33, (i0+a,   j0-1+b)
-template <class T>
+// Shared layout (per k-level), tile origin (i0, j0), J rows:
+//   in  : 36 x J+4, (i0-2+a, j0-2+b)
+//   dy  : 34 x J+3, (i0-1+a, j0-2+b)   dy(i,j)  = in(i,j+1) - in(i,j);  fly(i,j) then takes its place
+//   lap : 34 x J+2, (i0-1+a, j0-1+b)
+//   flx : 33 x J,   (i0-1+a, j0+b)
+template <class T, int J>
 struct HdiffsaSmem {
-  T in[36][36];
-  T dy[35][34];
-  T lap[34][34];
-  T flx[32][33];
-  T fly[33][32];
-  T crlato[34];  // j0-1+b
-  T crlatu[34];
+  T in[J + 4][36];
+  T dy[J + 3][34];
+  T lap[J + 2][34];
+  T flx[J][33];
+  T crlato[J + 2];  // j0-1+b
+  T crlatu[J + 2];
 };
 
-template <class T>
+template <class T, int J>
 struct hdiffsa_kernel {
   static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> out, InPtr<T> in,
                                              InPtr<T> mask, InPtr<T> crlato,
                                              InPtr<T> crlatu, int64_t s1d, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HdiffsaSmem<T>& s = *reinterpret_cast<HdiffsaSmem<T>*>(smem_raw);
-    const int i0 = blk.x * kT, j0 = blk.y * kT;
+    HdiffsaSmem<T, J>& s = *reinterpret_cast<HdiffsaSmem<T, J>*>(smem_raw);
+    const int i0 = blk.x * kT, j0 = blk.y * J;
     const int sj = (int)d.sj;
     const int tid = threadIdx.y * kTX + threadIdx.x;
-    if (tid < 34) {
+    if (tid < J + 2) {
       const int j = j0 - 1 + tid;
       const bool ok = j >= -1 && j < d.ny + 1;
       s.crlato[tid] = ok ? ld(crlato + (int64_t)j * s1d) : T(0);
@@ -69,45 +80,44 @@ struct hdiffsa_kernel {
     }
     const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
     // outputs of this tile (fewer at the domain's far edge) and what each phase needs for them
-    const int vx = max(0, min(kT, d.nx - i0)), vy = max(0, min(kT, d.ny - j0));
+    const int vx = max(0, min(kT, d.nx - i0)), vy = max(0, min(J, d.ny - j0));
   #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * d.sk;
       const InPtr<T> pin = in + kofs;
-      for_region_lim<36, 36>(vx + 4, vy + 4, [&](int a, int b) {
+      for_region_lim<36, J + 4>(vx + 4, vy + 4, [&](int a, int b) {
         const int i = i0 - 2 + a, j = j0 - 2 + b;
         const bool ok = i >= -2 && i < d.nx + 2 && j >= -2 && j < d.ny + 2;
         s.in[b][a] = ok ? ld(pin + i + j * sj) : T(0);
       });
       __syncthreads();
-      for_region_lim<34, 35>(vx + 2, vy + 3, [&](int a, int b) { s.dy[b][a] = isub(s.in[b + 1][a + 1], s.in[b][a + 1]); });
+      for_region_lim<34, J + 3>(vx + 2, vy + 3, [&](int a, int b) { s.dy[b][a] = isub(s.in[b + 1][a + 1], s.in[b][a + 1]); });
       __syncthreads();
       // hdiffsa.h:101: in(i-1)+in(i+1) - 2 in + crlato (in(j+1)-in) + crlatu (in(j-1)-in)
-      for_region_lim<34, 34>(vx + 2, vy + 2, [&](int a, int b) {
+      for_region_lim<34, J + 2>(vx + 2, vy + 2, [&](int a, int b) {
         const T c = s.in[b + 1][a + 1];
         s.lap[b][a] = ((iadd(s.in[b + 1][a], s.in[b + 1][a + 2]) - scale2<1>(c)) + s.crlato[b] * s.dy[b + 1][a]) +
                       s.crlatu[b] * (-s.dy[b][a]);
       });
       __syncthreads();
       // hdiffsa.h:106-113: limited fluxes
-      for_region_lim<33, 32>(vx + 1, vy, [&](int a, int b) {
+      for_region_lim<33, J>(vx + 1, vy, [&](int a, int b) {
         T f = s.lap[b + 1][a + 1] - s.lap[b + 1][a];
         if (Prec<T>::prod_gt0(f, s.in[b + 2][a + 2] - s.in[b + 2][a + 1])) f = T(0);
         s.flx[b][a] = f;
       });
-      for_region_lim<32, 33>(vx, vy + 1, [&](int a, int b) {
+      for_region_lim<32, J + 1>(vx, vy + 1, [&](int a, int b) {  // fly(i0+a, j0-1+b)
         T f = s.crlato[b] * (s.lap[b + 1][a + 1] - s.lap[b][a + 1]);
-        if (Prec<T>::prod_gt0(f, s.dy[b + 1][a + 1])) f = T(0);
-        s.fly[b][a] = f;
+        T& g = s.dy[b + 1][a + 1];  // read by this cell alone
+        if (Prec<T>::prod_gt0(f, g)) f = T(0);
+        g = f;
       });
       __syncthreads();
       // hdiffsa.h:118-119
-      for_region<32, 32>([&](int a, int b) {
-        const int i = i0 + a, j = j0 + b;
-        if (i < d.nx && j < d.ny) {
-          const int64_t o = kofs + i + j * sj;
-          out[o] = s.in[b + 2][a + 2] + (((s.flx[b][a] - s.flx[b][a + 1]) + s.fly[b][a]) - s.fly[b + 1][a]) * ld(mask + o);
-        }
+      for_region_lim<32, J>(vx, vy, [&](int a, int b) {
+        const int64_t o = kofs + (i0 + a) + (j0 + b) * sj;
+        out[o] = s.in[b + 2][a + 2] +
+                 (((s.flx[b][a] - s.flx[b][a + 1]) + s.dy[b + 1][a + 1]) - s.dy[b + 2][a + 1]) * ld(mask + o);
       });
       __syncthreads();
     }
@@ -192,30 +202,30 @@ struct hdiffsa_march_f32 {
 };
 
 // ============================== hdiffsmag =========================================
-// Shared layout (per k-level), tile origin (i0, j0):
-//   u, v : 34 x 34, (i0-1+a, j0-1+b)
-//   dyv  : 33 x 33, (i0+a,   j0-1+b)   v(i,j+1) - v(i,j)
-//   dyu  : 33 x 33, (i0-1+a, j0-1+b)   u(i,j+1) - u(i,j)
+// Shared layout (per k-level), tile origin (i0, j0), J rows:
+//   u, v : 34 x J+2, (i0-1+a, j0-1+b)
+//   dyv  : 33 x J+1, (i0+a,   j0-1+b)   v(i,j+1) - v(i,j)
+//   dyu  : 33 x J+1, (i0-1+a, j0-1+b)   u(i,j+1) - u(i,j)
 // (the x differences dxu = u(i+1,j) - u(i,j) at (i0-1+a, j0+b) and dxv = v(i+1,j) - v(i,j)
 // at (i0-1+a, j0-1+b) are each read once, by the deformations of the same cell: they live in
-// registers, which keeps the tile at 53 KB, four CTAs per SM)
-//   tsq  : 33 x 33, (i0+a,   j0+b)     T_s^2
-//   ssq  : 33 x 33, (i0-1+a, j0-1+b)   S_uv^2
-template <class T>
+// registers, which keeps a tile of 16 rows at 28 KB)
+//   tsq  : 33 x J+1, (i0+a,   j0+b)     T_s^2
+//   ssq  : 33 x J+1, (i0-1+a, j0-1+b)   S_uv^2
+template <class T, int J>
 struct HdiffsmagSmem {
-  T u[34][34];
-  T v[34][34];
-  T dyv[33][33];
-  T dyu[33][33];
-  T tsq[33][33];
-  T ssq[33][33];
-  T acrlat0[34];  // j0-1+b
-  T crlato[32], crlatu[32], crlavo[32], crlavu[32];
+  T u[J + 2][34];
+  T v[J + 2][34];
+  T dyv[J + 1][33];
+  T dyu[J + 1][33];
+  T tsq[J + 1][33];
+  T ssq[J + 1][33];
+  T acrlat0[J + 2];  // j0-1+b
+  T crlato[J], crlatu[J], crlavo[J], crlavu[J];
 };
 
-template <class T>
+template <class T, int J>
 struct hdiffsmag_kernel {
-  static constexpr int kStepOp = step_op<T>(kOpSmagFwd);  // the step kernel's id
+  static constexpr int kStepOp = step_op<T>(J == kJ ? kOpSmagFwd : -1);  // the step kernel's id
   static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
                                              InPtr<T> uin, InPtr<T> vin,
                                              InPtr<T> mask, InPtr<T> crlavo,
@@ -223,15 +233,15 @@ struct hdiffsmag_kernel {
                                              InPtr<T> crlatu, InPtr<T> acrlat0, int64_t s1d,
                                              T eddlat, T eddlon, T tau_smag, T weight_smag, Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HdiffsmagSmem<T>& s = *reinterpret_cast<HdiffsmagSmem<T>*>(smem_raw);
-    const int i0 = blk.x * kT, j0 = blk.y * kT;
+    HdiffsmagSmem<T, J>& s = *reinterpret_cast<HdiffsmagSmem<T, J>*>(smem_raw);
+    const int i0 = blk.x * kT, j0 = blk.y * J;
     const int sj = (int)d.sj;
     const int tid = threadIdx.y * kTX + threadIdx.x;
     constexpr T rr = earth_radius_recip<T>();
-    if (tid < 34) {
+    if (tid < J + 2) {
       const int j = j0 - 1 + tid;
       s.acrlat0[tid] = (j >= -1 && j < d.ny + 1) ? ld(acrlat0 + (int64_t)j * s1d) : T(0);
-    } else if (tid >= 64 && tid < 96) {
+    } else if (tid >= 64 && tid < 64 + J) {
       const int b = tid - 64, j = j0 + b;
       const bool ok = j < d.ny;
       const int64_t jo = (int64_t)j * s1d;
@@ -242,11 +252,11 @@ struct hdiffsmag_kernel {
     }
     const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
     // outputs of this tile (fewer at the domain's far edge) and what each phase needs for them
-    const int vx = max(0, min(kT, d.nx - i0)), vy = max(0, min(kT, d.ny - j0));
+    const int vx = max(0, min(kT, d.nx - i0)), vy = max(0, min(J, d.ny - j0));
   #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * d.sk;
-      for_region_lim<34, 34>(vx + 2, vy + 2, [&](int a, int b) {
+      for_region_lim<34, J + 2>(vx + 2, vy + 2, [&](int a, int b) {
         const int i = i0 - 1 + a, j = j0 - 1 + b;
         const bool ok = i >= -1 && i < d.nx + 1 && j >= -1 && j < d.ny + 1;
         const int64_t o = kofs + i + j * sj;
@@ -256,7 +266,7 @@ struct hdiffsmag_kernel {
       __syncthreads();
       // hdiffsmag.h:213 T_s = (v(j-1)-v) eddlat R^-1 - (u(i-1)-u) acrlat0(j) eddlon
       //              :221 S_uv = (u(j+1)-u) eddlat R^-1 + (v(i+1)-v) acrlat0(j) eddlon
-      for_region_lim<33, 33>(vx + 1, vy + 1, [&](int a, int b) {
+      for_region_lim<33, J + 1>(vx + 1, vy + 1, [&](int a, int b) {
         const T dxu = s.u[b + 1][a + 1] - s.u[b + 1][a];
         const T dyv = s.v[b + 1][a + 1] - s.v[b][a + 1];
         const T dyu = s.u[b + 1][a] - s.u[b][a];
@@ -269,41 +279,39 @@ struct hdiffsmag_kernel {
         s.ssq[b][a] = su * su;
       });
       __syncthreads();
-      for_region<32, 32>([&](int a, int b) {
+      for_region_lim<32, J>(vx, vy, [&](int a, int b) {
         const int i = i0 + a, j = j0 + b;
-        if (i < d.nx && j < d.ny) {
-          const int64_t o = kofs + i + j * sj;
-          const T hdweight = weight_smag * ld(mask + o);
-          // hdiffsmag.h:233-244 (the T^2 pair sums as integer-pipe additions: the FP64 pipe is the
-          // busier one here; two per point measured best, four 6 % slower)
-          T smag_u = tau_smag * Prec<T>::sqrt_(scale2<-1>(iadd(s.tsq[b][a + 1], s.tsq[b][a])) +
-                                               scale2<-1>(s.ssq[b][a + 1] + s.ssq[b + 1][a + 1])) -
-                     hdweight;
-          smag_u = clamp_smag(smag_u);
-          const T uc = s.u[b + 1][a + 1];
-          // u(i+1) + u(i-1) - 2u + crlato (u(j+1) - u) + crlatu (u(j-1) - u), the reference's
-          // sum in every precision: FP32 is then bit-identical to the reference compiled for
-          // float.  A compensated FP32 sum (TwoSum / TwoProduct) measured the same largest error
-          // against the FP64 oracle (5.5e-8) at about five times the sum's operations.
-          Acc<T> lu(s.u[b + 1][a + 2]);
-          lu.add(s.u[b + 1][a]);
-          lu.add(-scale2<1>(uc));
-          lu.add_prod(s.crlato[b], s.dyu[b + 1][a + 1]);
-          lu.add_prod(s.crlatu[b], -s.dyu[b][a + 1]);
-          uout[o] = uc + mul_zero(smag_u, lu.get());  // the clamp gives many zeros
-          // hdiffsmag.h:248-259
-          T smag_v = tau_smag * Prec<T>::sqrt_(scale2<-1>(iadd(s.tsq[b + 1][a], s.tsq[b][a])) +
-                                               scale2<-1>(s.ssq[b + 1][a] + s.ssq[b + 1][a + 1])) -
-                     hdweight;
-          smag_v = clamp_smag(smag_v);
-          const T vc = s.v[b + 1][a + 1];
-          Acc<T> lv(s.v[b + 1][a + 2]);
-          lv.add(s.v[b + 1][a]);
-          lv.add(-scale2<1>(vc));
-          lv.add_prod(s.crlavo[b], s.dyv[b + 1][a]);
-          lv.add_prod(s.crlavu[b], -s.dyv[b][a]);
-          vout[o] = vc + mul_zero(smag_v, lv.get());
-        }
+        const int64_t o = kofs + i + j * sj;
+        const T hdweight = weight_smag * ld(mask + o);
+        // hdiffsmag.h:233-244 (the T^2 pair sums as integer-pipe additions: the FP64 pipe is the
+        // busier one here; two per point measured best, four 6 % slower)
+        T smag_u = tau_smag * Prec<T>::sqrt_(scale2<-1>(iadd(s.tsq[b][a + 1], s.tsq[b][a])) +
+                                             scale2<-1>(s.ssq[b][a + 1] + s.ssq[b + 1][a + 1])) -
+                   hdweight;
+        smag_u = clamp_smag(smag_u);
+        const T uc = s.u[b + 1][a + 1];
+        // u(i+1) + u(i-1) - 2u + crlato (u(j+1) - u) + crlatu (u(j-1) - u), the reference's
+        // sum in every precision: FP32 is then bit-identical to the reference compiled for
+        // float.  A compensated FP32 sum (TwoSum / TwoProduct) measured the same largest error
+        // against the FP64 oracle (5.5e-8) at about five times the sum's operations.
+        Acc<T> lu(s.u[b + 1][a + 2]);
+        lu.add(s.u[b + 1][a]);
+        lu.add(-scale2<1>(uc));
+        lu.add_prod(s.crlato[b], s.dyu[b + 1][a + 1]);
+        lu.add_prod(s.crlatu[b], -s.dyu[b][a + 1]);
+        uout[o] = uc + mul_zero(smag_u, lu.get());  // the clamp gives many zeros
+        // hdiffsmag.h:248-259
+        T smag_v = tau_smag * Prec<T>::sqrt_(scale2<-1>(iadd(s.tsq[b + 1][a], s.tsq[b][a])) +
+                                             scale2<-1>(s.ssq[b + 1][a] + s.ssq[b + 1][a + 1])) -
+                   hdweight;
+        smag_v = clamp_smag(smag_v);
+        const T vc = s.v[b + 1][a + 1];
+        Acc<T> lv(s.v[b + 1][a + 2]);
+        lv.add(s.v[b + 1][a]);
+        lv.add(-scale2<1>(vc));
+        lv.add_prod(s.crlavo[b], s.dyv[b + 1][a]);
+        lv.add_prod(s.crlavu[b], -s.dyv[b][a]);
+        vout[o] = vc + mul_zero(smag_v, lv.get());
       });
       __syncthreads();
     }
@@ -426,8 +434,13 @@ oeb_status hdiffsa_entry(const M3* out, const M3* in, const M3* mask, const M1* 
                      d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
-  return launch<hdiffsa_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsaSmem<T>), (cudaStream_t)stream,
-                                   gout.origin, gin.origin, gmask.origin, lo.origin, lu.origin, lo.s, d, kb);
+  auto run = [&](auto rows) {
+    constexpr int J = decltype(rows)::value;
+    return launch<hdiffsa_kernel<T, J>>(tile_grid(d.nx, d.ny, d.nz, kT, J, kb), sizeof(HdiffsaSmem<T, J>),
+                                        (cudaStream_t)stream, gout.origin, gin.origin, gmask.origin, lo.origin,
+                                        lu.origin, lo.s, d, kb);
+  };
+  return short_tiles(d, kb) ? run(std::integral_constant<int, kJShort>()) : run(std::integral_constant<int, kJ>());
 }
 
 template <class T, class M3, class M1>
@@ -462,10 +475,14 @@ oeb_status hdiffsmag_entry(const M3* uout, const M3* vout, const M3* uin, const 
                      m.rows, m.wx_log);
   } else {
     const int kb = tuned_kb(kKB);
-    return launch<hdiffsmag_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsmagSmem<T>),
-                                     (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, gm.origin,
-                                     lvo.origin, lvu.origin, lto.origin, ltu.origin, la0.origin, lvo.s, eddlat, eddlon,
-                                     tau_smag, weight_smag, d, kb);
+    auto run = [&](auto tile_rows) {
+      constexpr int J = decltype(tile_rows)::value;
+      return launch<hdiffsmag_kernel<T, J>>(
+          tile_grid(d.nx, d.ny, d.nz, kT, J, kb), sizeof(HdiffsmagSmem<T, J>), (cudaStream_t)stream, gu.origin, gv.origin,
+          gui.origin, gvi.origin, gm.origin, lvo.origin, lvu.origin, lto.origin, ltu.origin, la0.origin, lvo.s, eddlat,
+          eddlon, tau_smag, weight_smag, d, kb);
+    };
+    return short_tiles(d, kb) ? run(std::integral_constant<int, kJShort>()) : run(std::integral_constant<int, kJ>());
   }
 }
 
@@ -492,7 +509,7 @@ oeb_status hdiffsmag_tl_entry(const M3* duout, const M3* dvout, const M3* uin, c
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  return launch<hdiffsmag_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsmagSmem<D>),
+  return launch<hdiffsmag_kernel<D, kJ>>(tile_grid(d.nx, d.ny, d.nz, kT, kJ, kb), sizeof(HdiffsmagSmem<D, kJ>),
                                       (cudaStream_t)stream, ou, ov, u, v, m, l0, l1, l2, l3, l4, crlavo->strides[0],
                                       D(eddlat), D(eddlon), D(tau_smag), D(weight_smag), d, kb);
 }
@@ -631,8 +648,8 @@ oeb_status hdiffsa_tl_entry(const M3* dout, const M3* in, const M3* mask, const 
   const DualOut<T> y = dual_out<T>(dout);
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]};
   const int kb = tuned_kb(kKB);
-  return launch<hdiffsa_kernel<D>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(HdiffsaSmem<D>),
-                                    (cudaStream_t)stream, y, x, m, lo, lu, crlato->strides[0], d, kb);
+  return launch<hdiffsa_kernel<D, kJ>>(tile_grid(d.nx, d.ny, d.nz, kT, kJ, kb), sizeof(HdiffsaSmem<D, kJ>),
+                                      (cudaStream_t)stream, y, x, m, lo, lu, crlato->strides[0], d, kb);
 }
 
 template <class T, class M3, class M1>

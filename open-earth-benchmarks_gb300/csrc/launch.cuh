@@ -231,7 +231,7 @@ Recorder* recorder();             // the calling thread's recorder, or nullptr
 void set_recorder(Recorder* r);  // installs (or with nullptr removes) it
 // k-levels per CTA set by oeb_set_kblock (0: none).
 int kb_override();
-// Whether the FP32 adjoints that have a tiled one-launch form use it (oeb_set_adjoint_tiles;
+// Whether the FP32 adjoints that have a one-launch form use it (oeb_set_adjoint_tiles;
 // default 1).
 int adjoint_tiles();
 // k-levels per CTA: the recorder's choice while recording, else oeb_set_kblock's, else `def`.
@@ -331,6 +331,11 @@ struct Dual;
 template <template <class> class K>
 struct Rebind<K<Dual<double>>> {
   using type = K<Dual<F64i>>;
+  static constexpr bool on = true;
+};
+template <template <class, int> class K, int N>
+struct Rebind<K<Dual<double>, N>> {
+  using type = K<Dual<F64i>, N>;
   static constexpr bool on = true;
 };
 template <template <class, int, int> class K, int N, int M>

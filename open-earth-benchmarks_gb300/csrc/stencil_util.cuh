@@ -10,7 +10,7 @@
 
 namespace oeb {
 
-// Threads per CTA of every tiled kernel: 32 lanes along i times 8 rows along j.
+// Threads per CTA of every kernel: 32 lanes along i times 8 rows (tiles) or warps (march.cuh).
 constexpr int kTX = 32;
 constexpr int kTY = 8;
 constexpr int kThreads = kTX * kTY;

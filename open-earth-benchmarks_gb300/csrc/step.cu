@@ -73,7 +73,7 @@ using StepBodies = OpList<
     step_pw::hadv_adj_terms_kernel<F64i, 5, 2>, step_pw::hadv_adj_terms_kernel<float, 5, 0>,
     step_pw::hadv_adj_terms_kernel<float, 5, 1>, step_pw::hadv_adj_terms_kernel<float, 5, 2>,
     step_pw::hadv_adj_gather_kernel<F64i, 5>, step_pw::hadv_adj_gather_kernel<float, 5>,
-    step_hd::hdiffsmag_kernel<F64i>, step_hd::hdiffsmag_march_f32,
+    step_hd::hdiffsmag_kernel<F64i, 16>, step_hd::hdiffsmag_march_f32,
     step_hd::hdiffsmag_adj_terms_kernel<F64i>, step_hd::hdiffsmag_adj_ts_kernel<F64i>,
     step_hd::hdiffsmag_adj_gather_kernel<F64i>, step_hd::hdiffsmag_adj_f32,
     step_hd::hdiffsmag_adj_terms_kernel<float>, step_hd::hdiffsmag_adj_ts_kernel<float>,

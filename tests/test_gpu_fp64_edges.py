@@ -76,3 +76,26 @@ def test_zero_seeds(pkg, fields, cuda, name):
         w, a, b = (case.sem_box(n, v[n]) for v in (g, gl, gh))
         assert np.abs(w - (a + b)).max() <= 1e-11 * np.abs(w).max()
         assert (a[..., 52:] == 0.0).all() and (b[..., :25] == 0.0).all()
+
+
+# both tile heights of hdiffsa and hdiffsmag: 8 rows where the grid is small, 16 where it fills the GPU
+TILES = [(32, 7, 2), (33, 8, 2), (31, 9, 1), (1, 16, 3), (64, 17, 2), (40, 15, 500), (33, 16, 500), (20, 17, 520),
+         (65, 33, 140)]
+
+
+@pytest.mark.parametrize("size", TILES, ids=["x".join(map(str, s)) for s in TILES])
+@pytest.mark.parametrize("name", ("hdiffsa", "hdiffsmag"))
+def test_tile_heights_are_the_oracle(pkg, fields, orc, cuda, name, size):
+    import torch
+    nx, ny, nz = size
+    spec = pkg.KERNELS[name]
+    want = {**fields.make_inputs(name, nx, ny, nz, seed=61, workload="fronts", halo=H),
+            **fields.make_outputs(name, nx, ny, nz, halo=H)}
+    sc = fields.make_scalars(name, seed=61)
+    dev = {k: pkg.Storage(torch.from_numpy(v.copy()).to(cuda), H, nx=nx if v.ndim == 3 else None)
+           for k, v in want.items()}
+    orc.run_oracle(spec, want, sc, nx, ny, nz, H)
+    pkg.call(name, dev, sc, domain=(nx, ny, nz))
+    torch.cuda.synchronize()
+    for a in spec.by_role("out3"):
+        np.testing.assert_array_equal(dev[a.name].numpy().view(np.uint64), want[a.name].view(np.uint64), err_msg=a.name)
