@@ -1077,11 +1077,16 @@ struct hadv_adj_gather_kernel {
 // ---- FP32 hadvuv / hadvuv5th adjoint in one tiled launch ----------------------------
 // A CTA owns a 32 x 32 tile of the gradient box [-h, n+h)^2 and a chunk of k-levels.  At each
 // level it forms, in shared memory, the terms and flags of every interior point its cells
-// gather from -- the tile widened by h on each side -- with the terms pass's expressions
-// (hadv_adj_terms_kernel), then each cell gathers them as hadv_adj_gather_kernel does: the
-// same operations on the same operands in the same order, so the same bits.  The apron
-// recomputes (32 + 2h)^2 / 32^2 - 1 = 41 % more terms (h = 3), and the 37 bytes a point of
-// term scratch are neither written nor read back.
+// gather from with the terms pass's expressions (hadv_adj_terms_kernel) -- all nine over the tile and the
+// ring around it, beyond that only those the upwind taps read -- then each cell gathers them as
+// hadv_adj_gather_kernel does: the same operations on the same operands in the same order (a term that
+// is zero is added where the pass skips it), so the same bits.  The 37 bytes a point of term scratch
+// are neither written nor read back.
+//
+// What bounds it: the warps in flight (two phases of loads, each behind a barrier).  64 registers, four
+// CTAs an SM: hadvuv5th 48.3 us at 128 x 128 x 80 and 151.7 at 256 x 256 x 80, hadvuv 36.4 at
+// 128 x 128 x 80 (three CTAs 51.7, 162.4 and 41.1, two 63.4, 204 and 54.9; all nine terms over the whole
+// tile widened by h, a row a thread at a time, with three 51.4, 162.4 and 43.3).
 template <int ORDER>
 struct HadvAdjF32Smem {
   static constexpr int kH = ORDER == 3 ? 2 : 3;
@@ -1093,7 +1098,7 @@ struct HadvAdjF32Smem {
 template <int ORDER>
 struct hadv_adj_f32 {
   static constexpr int kStepOp = step_op<float>(ORDER == 5 ? kOpHadv5AdjTiled : -1);  // the step kernel's id
-  static constexpr int kMinCtas = 3;
+  static constexpr int kMinCtas = 4;
   using Smem = HadvAdjF32Smem<ORDER>;
   static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uinb, float* __restrict__ vinb,
                                              const float* __restrict__ uin, const float* __restrict__ vin,
@@ -1118,68 +1123,109 @@ struct hadv_adj_f32 {
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * d.sk;
-      // the terms (hadv_adj_terms_kernel) of the interior points of the region
-      for (int e = tid; e < W * W; e += kThreads) {
-        const int li = e % W, lj = e / W;
+      // the terms (hadv_adj_terms_kernel), zero off the interior: all of them at the tile's cells and the
+      // ring around those, the ones the upwind taps read beyond it
+      for (int e = tid; e < 34 * 34; e += kThreads) {
+        const int lj = e / 34 + h - 1, li = e % 34 + h - 1;
         const int i = pi0 + li, j = pj0 + lj;
-        if (!in(i, j)) continue;
-        const int64_t o = kofs + i + (int64_t)j * sj;
-        const int64_t jo = (int64_t)j * s1d;
-        const T u0 = ld(uin + o), v0 = ld(vin + o);
-        const T um = ld(uin + o - 1) + u0;
-        const T ua = third * (um + ld(uin + o + 1));
-        const T va = T(0.25) * (((ld(vin + o + 1) + ld(vin + o + 1 - sj)) + v0) + ld(vin + o - sj));
-        const T ub = T(0.25) * ((um + ld(uin + o + sj)) + ld(uin + o - 1 + sj));
-        const T vb = third * ((ld(vin + o - sj) + v0) + ld(vin + o + sj));
-        const T a0 = ld(acrlat0 + jo), a1 = ld(acrlat1 + jo), t0 = ld(tgrlatda0 + jo), t1 = ld(tgrlatda1 + jo);
-        const T Ax = a0 * ua, Ay = rr * va, Bx = a1 * ub, By = rr * vb;
-        const bool px = Ax > 0, py = Ay > 0, qx = Bx > 0, qy = By > 0;
-        const T Px = adv_sum<T, ORDER>(uin, o, 1, px), Py = adv_sum<T, ORDER>(uin, o, sj, py);
-        const T Qx = adv_sum<T, ORDER>(vin, o, 1, qx), Qy = adv_sum<T, ORDER>(vin, o, sj, qy);
-        const T yu = ld(uoutb + o), yv = ld(voutb + o);
-        s.t[AX][lj][li] = (eddlat * Ax) * yu;
-        s.t[AY][lj][li] = (eddlon * Ay) * yu;
-        s.t[BX][lj][li] = ((eddlat * Px) * a0) * (third * yu);
-        s.t[BY][lj][li] = ((eddlon * Py) * rr + t0 * u0) * (T(0.25) * yu);
-        s.t[DD][lj][li] = (t0 * va) * yu;
-        s.t[GX][lj][li] = (eddlat * Bx) * yv;
-        s.t[GY][lj][li] = (eddlon * By) * yv;
-        s.t[EX][lj][li] = ((eddlat * Qx) * a1 - (T(2) * t1) * ub) * (T(0.25) * yv);
-        s.t[EY][lj][li] = ((eddlon * Qy) * rr) * (third * yv);
-        s.fl[lj][li] = (unsigned char)((px ? 1 : 0) | (py ? 2 : 0) | (qx ? 4 : 0) | (qy ? 8 : 0));
+        T t[9] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
+        unsigned char f = 0;
+        if (in(i, j)) {
+          const int64_t o = kofs + i + (int64_t)j * sj;
+          const int64_t jo = (int64_t)j * s1d;
+          const T u0 = ld(uin + o), v0 = ld(vin + o);
+          const T um = ld(uin + o - 1) + u0;
+          const T ua = third * (um + ld(uin + o + 1));
+          const T va = T(0.25) * (((ld(vin + o + 1) + ld(vin + o + 1 - sj)) + v0) + ld(vin + o - sj));
+          const T ub = T(0.25) * ((um + ld(uin + o + sj)) + ld(uin + o - 1 + sj));
+          const T vb = third * ((ld(vin + o - sj) + v0) + ld(vin + o + sj));
+          const T a0 = ld(acrlat0 + jo), a1 = ld(acrlat1 + jo), t0 = ld(tgrlatda0 + jo), t1 = ld(tgrlatda1 + jo);
+          const T Ax = a0 * ua, Ay = rr * va, Bx = a1 * ub, By = rr * vb;
+          const bool px = Ax > 0, py = Ay > 0, qx = Bx > 0, qy = By > 0;
+          const T Px = adv_sum<T, ORDER>(uin, o, 1, px), Py = adv_sum<T, ORDER>(uin, o, sj, py);
+          const T Qx = adv_sum<T, ORDER>(vin, o, 1, qx), Qy = adv_sum<T, ORDER>(vin, o, sj, qy);
+          const T yu = ld(uoutb + o), yv = ld(voutb + o);
+          t[AX] = (eddlat * Ax) * yu;
+          t[AY] = (eddlon * Ay) * yu;
+          t[BX] = ((eddlat * Px) * a0) * (third * yu);
+          t[BY] = ((eddlon * Py) * rr + t0 * u0) * (T(0.25) * yu);
+          t[DD] = (t0 * va) * yu;
+          t[GX] = (eddlat * Bx) * yv;
+          t[GY] = (eddlon * By) * yv;
+          t[EX] = ((eddlat * Qx) * a1 - (T(2) * t1) * ub) * (T(0.25) * yv);
+          t[EY] = ((eddlon * Qy) * rr) * (third * yv);
+          f = (unsigned char)((px ? 1 : 0) | (py ? 2 : 0) | (qx ? 4 : 0) | (qy ? 8 : 0));
+        }
+#pragma unroll
+        for (int q = 0; q < 9; ++q) s.t[q][lj][li] = t[q];
+        s.fl[lj][li] = f;
+      }
+      for (int e = tid; e < 2 * (h - 1) * 32; e += kThreads) {
+        const int q = e / 32, far = q < h - 1 ? q : q + 34, near = e % 32 + h;
+        {  // rows below and above
+          const int i = pi0 + near, j = pj0 + far;
+          T ay = T(0), gy = T(0);
+          unsigned char f = 0;
+          if (in(i, j)) {
+            const int64_t o = kofs + i + (int64_t)j * sj;
+            const T v0 = ld(vin + o);
+            const T va = T(0.25) * (((ld(vin + o + 1) + ld(vin + o + 1 - sj)) + v0) + ld(vin + o - sj));
+            const T vb = third * ((ld(vin + o - sj) + v0) + ld(vin + o + sj));
+            const T Ay = rr * va, By = rr * vb;
+            ay = (eddlon * Ay) * ld(uoutb + o), gy = (eddlon * By) * ld(voutb + o);
+            f = (unsigned char)((Ay > 0 ? 2 : 0) | (By > 0 ? 8 : 0));
+          }
+          s.t[AY][far][near] = ay, s.t[GY][far][near] = gy, s.fl[far][near] = f;
+        }
+        {  // columns to either side
+          const int i = pi0 + far, j = pj0 + near;
+          T ax = T(0), gx = T(0);
+          unsigned char f = 0;
+          if (in(i, j)) {
+            const int64_t o = kofs + i + (int64_t)j * sj;
+            const T um = ld(uin + o - 1) + ld(uin + o);
+            const T ua = third * (um + ld(uin + o + 1));
+            const T ub = T(0.25) * ((um + ld(uin + o + sj)) + ld(uin + o - 1 + sj));
+            const T Ax = ld(acrlat0 + (int64_t)j * s1d) * ua, Bx = ld(acrlat1 + (int64_t)j * s1d) * ub;
+            ax = (eddlat * Ax) * ld(uoutb + o), gx = (eddlat * Bx) * ld(voutb + o);
+            f = (unsigned char)((Ax > 0 ? 1 : 0) | (Bx > 0 ? 4 : 0));
+          }
+          s.t[AX][near][far] = ax, s.t[GX][near][far] = gx, s.fl[near][far] = f;
+        }
       }
       __syncthreads();
-      // the gather (hadv_adj_gather_kernel) of the tile's cells, four rows a thread
-#pragma unroll 1
+      // the gather (hadv_adj_gather_kernel) of the tile's cells, four rows in a row a thread, which share
+      // the y taps (a term that is zero is added where the passes skip it)
+      const int a = ci0 + (int)threadIdx.x, li = (int)threadIdx.x + h, l0 = 4 * (int)threadIdx.y + h;
+      T wy[4 + 2 * h], wg[4 + 2 * h];
+      unsigned char wf[4 + 2 * h];
+#pragma unroll
+      for (int t = 0; t < 4 + 2 * h; ++t)
+        wy[t] = s.t[AY][l0 - h + t][li], wg[t] = s.t[GY][l0 - h + t][li], wf[t] = s.fl[l0 - h + t][li];
+#pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const int a = ci0 + (int)threadIdx.x, b = cj0 + (int)threadIdx.y + 8 * r;
+        const int lj = l0 + r, b = cj0 + lj - h;
         if (a >= d.nx + h || b >= d.ny + h) continue;
-        const int li = a - pi0, lj = b - pj0;
         auto tm = [&](int q, int di, int dj) { return s.t[q][lj + dj][li + di]; };
         T ub = T(0), vb = T(0);
 #pragma unroll
         for (int m = -h; m <= h; ++m) {
-          if (in(a - m, b)) {
-            const unsigned char f = s.fl[lj][li - m];
-            ub = fma(upwind_weight<T, ORDER>(f & 1, m), tm(AX, -m, 0), ub);
-            vb = fma(upwind_weight<T, ORDER>(f & 4, m), tm(GX, -m, 0), vb);
-          }
-          if (in(a, b - m)) {
-            const unsigned char f = s.fl[lj - m][li];
-            ub = fma(upwind_weight<T, ORDER>(f & 2, m), tm(AY, 0, -m), ub);
-            vb = fma(upwind_weight<T, ORDER>(f & 8, m), tm(GY, 0, -m), vb);
-          }
+          const unsigned char f = s.fl[lj][li - m], g = wf[r - m + h];
+          ub = fma(upwind_weight<T, ORDER>(f & 1, m), tm(AX, -m, 0), ub);
+          vb = fma(upwind_weight<T, ORDER>(f & 4, m), tm(GX, -m, 0), vb);
+          ub = fma(upwind_weight<T, ORDER>(g & 2, m), wy[r - m + h], ub);
+          vb = fma(upwind_weight<T, ORDER>(g & 8, m), wg[r - m + h], vb);
         }
-        if (in(a - 1, b)) ub = ub + tm(BX, -1, 0);
-        if (in(a, b)) ub = (ub + tm(BX, 0, 0)) + (tm(DD, 0, 0) + tm(EX, 0, 0));
-        if (in(a + 1, b)) ub = (ub + tm(BX, 1, 0)) + tm(EX, 1, 0);
-        if (in(a, b - 1)) ub = ub + tm(EX, 0, -1);
-        if (in(a + 1, b - 1)) ub = ub + tm(EX, 1, -1);
-        if (in(a - 1, b)) vb = vb + tm(BY, -1, 0);
-        if (in(a - 1, b + 1)) vb = vb + tm(BY, -1, 1);
-        if (in(a, b)) vb = (vb + tm(BY, 0, 0)) + tm(EY, 0, 0);
-        if (in(a, b + 1)) vb = (vb + tm(BY, 0, 1)) + tm(EY, 0, 1);
-        if (in(a, b - 1)) vb = vb + tm(EY, 0, -1);
+        ub = ub + tm(BX, -1, 0);
+        ub = (ub + tm(BX, 0, 0)) + (tm(DD, 0, 0) + tm(EX, 0, 0));
+        ub = (ub + tm(BX, 1, 0)) + tm(EX, 1, 0);
+        ub = ub + tm(EX, 0, -1);
+        ub = ub + tm(EX, 1, -1);
+        vb = vb + tm(BY, -1, 0);
+        vb = vb + tm(BY, -1, 1);
+        vb = (vb + tm(BY, 0, 0)) + tm(EY, 0, 0);
+        vb = (vb + tm(BY, 0, 1)) + tm(EY, 0, 1);
+        vb = vb + tm(EY, 0, -1);
         const int64_t o = kofs + a + (int64_t)b * sj;
         if (update) {
           const T au = alpha * ub, av = alpha * vb;
