@@ -115,10 +115,10 @@ OEB_API int oeb_is_device_pointer(const void* p);
 /* Blocks until all work on `stream` has finished (NULL = legacy default stream). */
 OEB_API oeb_status oeb_stream_synchronize(void* stream);
 /* k-levels each CTA of the tiled stencils covers (1..1024), for every later call on every
- * thread; 0 (the default) restores each kernel's own choice.  A tuning knob: results do not
- * depend on it.  Batch plans record and tune their own. */
+ * thread; 0 (the default) restores each kernel's own choice; the marching FP32 kernels take none.  A
+ * tuning knob: results do not depend on it.  Batch plans record and tune their own. */
 OEB_API oeb_status oeb_set_kblock(int kb);
-/* Tile shape of the pointwise advection kernels (hadvuv, hadvuv5th and their adjoint terms),
+/* Tile shape of the pointwise advection kernels (FP64 hadvuv, hadvuv5th and the adjoint terms),
  * for every later call on every thread: 0 (the default) 32 x 32 cells a CTA, 1 = 32 x 8,
  * 2 = 64 x 16.  OEB_ERR_ARGUMENT for any other value.  A tuning knob: results do not depend
  * on it.  Batch plans choose their own shapes (oeb_batch_autotune). */
@@ -132,7 +132,7 @@ OEB_API oeb_status oeb_set_tile_shape(int shape);
  * depend on it.  Batch plans choose their own grouping (created with 0; oeb_batch_autotune,
  * oeb_batch_set_fusion). */
 /* 1 (the default): the FP32 adjoints of hdiffsmag, hadvuv, hadvuv5th, fastwavesuv, p_grad_c
- * and nh_p_grad run as one tiled launch that forms its terms (coefficients) in shared memory;
+ * and nh_p_grad run as one launch that forms its terms (coefficients) in registers or shared memory;
  * 0: as their multi-pass form, the terms in scratch.  No counterpart in the reference.  Results do not
  * depend on it (the same operations on the same operands); OEB_ERR_ARGUMENT for other
  * values. */
@@ -541,7 +541,8 @@ OEB_API oeb_status oeb_fvtp2d_f32_host(const oeb_memref3d_f32* q_i, const oeb_me
 /* at the state x (every upwind/limiter/PPM/clamp branch frozen at x) applied */
 /* to a perturbation dx of the active inputs.  Device pointers, asynchronous; */
 /* each dx field must have the layout of its state field.  dy is written over */
-/* the forward output's written box.  Device scratch from the library pool.   */
+/* the forward output's written box.  fvtp2d takes device scratch (four       */
+/* fields) from the library pool, the others none.                            */
 /*   hdiffsmag, hadvuv, hadvuv5th : active (uin, vin)                          */
 /*   fastwavesuv                  : active (uin, vin, utens, vtens, ppuv)      */
 /*   fvtp2d                       : active q; dy = all six outputs            */

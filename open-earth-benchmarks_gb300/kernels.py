@@ -85,7 +85,7 @@ def _signature(kernel: str) -> _Signature:
 
 
 def set_adjoint_tiles(on: bool) -> None:
-    """FP32 adjoints of hdiffsmag, hadvuv, hadvuv5th, fastwavesuv, p_grad_c and nh_p_grad as one tiled launch
+    """FP32 adjoints of hdiffsmag, hadvuv, hadvuv5th, fastwavesuv, p_grad_c and nh_p_grad as one launch each
     (True, the default) or in their multi-pass forms (oeb_set_adjoint_tiles); the same bits
     either way."""
     lib = load_library()
