@@ -529,57 +529,59 @@ oeb_status hdiffsmag_tl_entry(const M3* duout, const M3* dvout, const M3* uin, c
 // One kernel: a CTA stages its tile's in and G in shared memory, recomputes lap and the limiter
 // flags exactly as the forward kernel does (the same operations on the same operands), then
 // forms Fx, Fy, lapb and inb in shared memory.  Shared layout (per k-level), inb tile origin
-// (i0, j0):
-//   in   : 38 x 38, (i0-3+a, j0-3+b)
-//   lap  : 36 x 36, (i0-2+a, j0-2+b)
-//   gl   : 36 x 36, G at (i0-2+a, j0-2+b); then lapb, 34 x 34 at (i0-1+a, j0-1+b)
-//   fx   : 35 x 34, (i0-2+a, j0-1+b);   fy : 34 x 35, (i0-1+a, j0-2+b)
-template <class T>
+// (i0, j0), J rows:
+//   in   : 38 x J+6, (i0-3+a, j0-3+b)
+//   lap  : 36 x J+4, (i0-2+a, j0-2+b)
+//   gl   : 36 x J+4, G at (i0-2+a, j0-2+b); then lapb, 34 x J+2 at (i0-1+a, j0-1+b)
+//   fx   : 35 x J+2, (i0-2+a, j0-1+b);   fy : 34 x J+3, (i0-1+a, j0-2+b)
+// A tile at the box's far edge forms only what its own columns and rows need.
+template <class T, int J>
 struct HdiffsaAdjSmem {
-  T in[38][38];
-  T lap[36][36];
-  T gl[36][36];
-  T fx[34][35];
-  T fy[35][34];
-  T crlato[38], crlatu[38];  // j0-3+b
+  T in[J + 6][38];
+  T lap[J + 4][36];
+  T gl[J + 4][36];
+  T fx[J + 2][35];
+  T fy[J + 3][34];
+  T crlato[J + 6], crlatu[J + 6];  // j0-3+b
 };
 
-template <class T>
+template <class T, int J>
 struct hdiffsa_adj_kernel {
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ inb, const T* __restrict__ in,
                                              const T* __restrict__ mask, const T* __restrict__ crlato,
                                              const T* __restrict__ crlatu, int64_t s1d, const T* __restrict__ outb,
                                              Dims d, int kb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HdiffsaAdjSmem<T>& s = *reinterpret_cast<HdiffsaAdjSmem<T>*>(smem_raw);
+    HdiffsaAdjSmem<T, J>& s = *reinterpret_cast<HdiffsaAdjSmem<T, J>*>(smem_raw);
     T(*lapb)[34] = reinterpret_cast<T(*)[34]>(&s.gl[0][0]);
-    const int i0 = -2 + (int)blk.x * kT, j0 = -2 + (int)blk.y * kT;
+    const int i0 = -2 + (int)blk.x * kT, j0 = -2 + (int)blk.y * J;
     const int64_t sj = d.sj;
     const int tid = threadIdx.y * kTX + threadIdx.x;
-    if (tid < 38) {
+    if (tid < J + 6) {
       const int j = j0 - 3 + tid;
       const bool ok = j >= -1 && j < d.ny + 1;
       s.crlato[tid] = ok ? ld(crlato + (int64_t)j * s1d) : T(0);
       s.crlatu[tid] = ok ? ld(crlatu + (int64_t)j * s1d) : T(0);
     }
     auto interior = [&](int i, int j) { return i >= 0 && i < d.nx && j >= 0 && j < d.ny; };
+    const int vx = min(kT, d.nx + 2 - i0), vy = min(J, d.ny + 2 - j0);
     const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
   #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * d.sk;
-      for_region<38, 38>([&](int a, int b) {
+      for_region_lim<38, J + 6>(vx + 6, vy + 6, [&](int a, int b) {
         const int i = i0 - 3 + a, j = j0 - 3 + b;
         const bool ok = i >= -2 && i < d.nx + 2 && j >= -2 && j < d.ny + 2;
         s.in[b][a] = ok ? ld(in + kofs + i + j * sj) : T(0);
       });
-      for_region<36, 36>([&](int a, int b) {
+      for_region_lim<36, J + 4>(vx + 4, vy + 4, [&](int a, int b) {
         const int i = i0 - 2 + a, j = j0 - 2 + b;
         const int64_t o = kofs + i + j * sj;
         s.gl[b][a] = interior(i, j) ? ld(outb + o) * ld(mask + o) : T(0);
       });
       __syncthreads();
       // hdiffsa.h:101 where the forward forms lap (i, j in [-1, N+1)), its operations in its order
-      for_region<36, 36>([&](int a, int b) {
+      for_region_lim<36, J + 4>(vx + 4, vy + 4, [&](int a, int b) {
         const int i = i0 - 2 + a, j = j0 - 2 + b;
         T v = T(0);
         if (i >= -1 && i < d.nx + 1 && j >= -1 && j < d.ny + 1) {
@@ -591,7 +593,7 @@ struct hdiffsa_adj_kernel {
       });
       __syncthreads();
       // hdiffsa.h:106-109: Fx at (i, j), kept where the forward keeps flx
-      for_region<35, 34>([&](int a, int b) {
+      for_region_lim<35, J + 2>(vx + 3, vy + 2, [&](int a, int b) {
         const int i = i0 - 2 + a, j = j0 - 1 + b;
         T v = T(0);
         if (i >= -1 && i < d.nx && j >= 0 && j < d.ny) {
@@ -601,7 +603,7 @@ struct hdiffsa_adj_kernel {
         s.fx[b][a] = v;
       });
       // hdiffsa.h:110-113: Fy at (i, j), crlato(j) folded in
-      for_region<34, 35>([&](int a, int b) {
+      for_region_lim<34, J + 3>(vx + 2, vy + 3, [&](int a, int b) {
         const int i = i0 - 1 + a, j = j0 - 2 + b;
         T v = T(0);
         if (i >= 0 && i < d.nx && j >= -1 && j < d.ny) {
@@ -613,19 +615,17 @@ struct hdiffsa_adj_kernel {
       });
       __syncthreads();
       // lapb over the dead G
-      for_region<34, 34>([&](int a, int b) { lapb[b][a] = (s.fx[b][a] - s.fx[b][a + 1]) + (s.fy[b][a] - s.fy[b + 1][a]); });
+      for_region_lim<34, J + 2>(vx + 2, vy + 2, [&](int a, int b) { lapb[b][a] = (s.fx[b][a] - s.fx[b][a + 1]) + (s.fy[b][a] - s.fy[b + 1][a]); });
       __syncthreads();
-      for_region<32, 32>([&](int a, int b) {
+      for_region_lim<32, J>(vx, vy, [&](int a, int b) {
         const int i = i0 + a, j = j0 + b;
-        if (i < d.nx + 2 && j < d.ny + 2) {
-          const int64_t o = kofs + i + j * sj;
-          const T c = lapb[b + 1][a + 1];
-          T v = (lapb[b + 1][a] + lapb[b + 1][a + 2]) - ((T(2) + s.crlato[b + 3]) + s.crlatu[b + 3]) * c;
-          v = fma(s.crlato[b + 2], lapb[b][a + 1], v);
-          v = fma(s.crlatu[b + 4], lapb[b + 2][a + 1], v);
-          if (interior(i, j)) v = v + ld(outb + o);
-          inb[o] = v;
-        }
+        const int64_t o = kofs + i + j * sj;
+        const T c = lapb[b + 1][a + 1];
+        T v = (lapb[b + 1][a] + lapb[b + 1][a + 2]) - mul_zero(c, (T(2) + s.crlato[b + 3]) + s.crlatu[b + 3]);
+        v = fma(s.crlato[b + 2], lapb[b][a + 1], v);
+        v = fma(s.crlatu[b + 4], lapb[b + 2][a + 1], v);
+        if (interior(i, j)) v = v + ld(outb + o);
+        inb[o] = v;
       });
       __syncthreads();
     }
@@ -673,9 +673,19 @@ oeb_status hdiffsa_adj_entry(const M3* inb, const M3* in, const M3* mask, const 
   OEB_RETURN_IF_VALIDATING();
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gin.sj, gin.sk};
   const int kb = tuned_kb(kKB);
-  return launch<hdiffsa_adj_kernel<T>>(tile_grid(d.nx + 4, d.ny + 4, d.nz, kT, kT, kb), sizeof(HdiffsaAdjSmem<T>),
-                                       (cudaStream_t)stream, gib.origin, gin.origin, gm.origin, lo.origin, lu.origin,
-                                       lo.s, gob.origin, d, kb);
+  auto run = [&](auto rows) {
+    constexpr int J = decltype(rows)::value;
+    return launch<hdiffsa_adj_kernel<T, J>>(tile_grid(d.nx + 4, d.ny + 4, d.nz, kT, J, kb),
+                                            sizeof(HdiffsaAdjSmem<T, J>), (cudaStream_t)stream, gib.origin, gin.origin,
+                                            gm.origin, lo.origin, lu.origin, lo.s, gob.origin, d, kb);
+  };
+  // 16 rows keep more FP64 CTAs an SM (128 x 128 x 80 84.8 us, 32 rows 90.5; whole edge tiles of 32
+  // rows 103.9).  FP32 pays for the larger apron (256 x 256 x 80 77.4 us, 32 rows 68.2, were 73.0) unless
+  // the 32-row grid is under a wave (33 x 20 x 10 4.5 us, 32 rows 6.1).
+  if constexpr (std::is_same<T, float>::value) {
+    if (!under_a_wave(tile_grid(d.nx + 4, d.ny + 4, d.nz, kT, kT, kb), 8)) return run(std::integral_constant<int, kT>());
+  }
+  return run(std::integral_constant<int, kJ>());
 }
 
 // ============================== hdiffsmag adjoint ================================

@@ -51,8 +51,8 @@ EDGES = [(1, 1, 1), (26, 27, 2), (27, 58, 2), (29, 31, 3), (31, 26, 1), (32, 32,
 
 
 @pytest.mark.parametrize("size", EDGES, ids=["x".join(map(str, s)) for s in EDGES])
-@pytest.mark.parametrize("name", ("laplace", "hadvuv", "hadvuv5th", "hdiffsmag", "fastwavesuv", "uvbke", "nh_p_grad",
-                                  "p_grad_c", "fvtp2d"))
+@pytest.mark.parametrize("name", ("laplace", "hdiffsa", "hadvuv", "hadvuv5th", "hdiffsmag", "fastwavesuv", "uvbke",
+                                  "nh_p_grad", "p_grad_c", "fvtp2d"))
 def test_fp64_edge_tiles(pkg, fields, cuda, name, size):
     """<J dx, y> = <dx, J^T y> with y = J dx.  A cell missed, visited twice or at another's place would
     be an error of the order of one over the number of cells, at least 1e-5; the sums' roundings are
@@ -99,3 +99,12 @@ def test_tile_heights_are_the_oracle(pkg, fields, orc, cuda, name, size):
     torch.cuda.synchronize()
     for a in spec.by_role("out3"):
         np.testing.assert_array_equal(dev[a.name].numpy().view(np.uint64), want[a.name].view(np.uint64), err_msg=a.name)
+
+
+@pytest.mark.parametrize("size", [(31, 26, 2), (27, 29, 3), (33, 12, 400), (60, 61, 330)],
+                         ids=["31x26x2", "27x29x3", "33x12x400", "60x61x330"])
+def test_hdiffsa_f32_adjoint_tiles(pkg, fields, cuda, size):
+    """The FP32 hdiffsa adjoint in tiles of 16 rows (small grids) and of 32: <J dx, y> = <dx, J^T y> with
+    y = J dx, to 1e-5, which a cell missed or visited twice would exceed at the small sizes and the
+    existing FP32 bound holds for roundings."""
+    _dot_test(Case(pkg, fields, cuda, "hdiffsa", *size, seed=67, dtype=np.float32), 1e-5)
