@@ -927,6 +927,7 @@ struct hdiffsmag_adj_f32 {
     float c21 = 0.f, c22 = 0.f;                        // acrlat0 eddlon on rows r-1, r-2
     // of rows r-2 and r-3
     float to2 = 0.f, to3 = 0.f, tu2 = 0.f, vo2 = 0.f, vo3 = 0.f, vu2 = 0.f;
+    bool in2 = false, in3 = false;  // whether those rows' points are interior
 #pragma unroll 1
     for (int r = oa - 2; r < ob + 2; ++r) {
       const Row c = n;
@@ -972,8 +973,9 @@ struct hdiffsmag_adj_f32 {
       }
       ub = ub + lane_below<1>(lu2), vb = vb + lane_below<1>(lv2);
       ub = ub + lane_above<1>(lu2), vb = vb + lane_above<1>(lv2);
-      ub = fmaf(to3, lu3, ub), vb = fmaf(vo3, lv3, vb);
-      ub = fmaf(tu, lu1, ub), vb = fmaf(vu, lv1, vb);
+      // (guarded: a metric term need not be finite, and off the interior lu and lv are only stand-ins)
+      if (in3) ub = fmaf(to3, lu3, ub), vb = fmaf(vo3, lv3, vb);
+      if (in_p) ub = fmaf(tu, lu1, ub), vb = fmaf(vu, lv1, vb);
       ub = fmaf(-c22, lane_above<1>(tb2), ub);
       ub = fmaf(-c1, sb2, fmaf(c22, tb2, ub));
       ub = fmaf(c1, sb3, ub);
@@ -987,6 +989,7 @@ struct hdiffsmag_adj_f32 {
       tb2 = tb1, sb3 = sb2, yu2 = c.yu, yv2 = c.yv;
       c22 = c21, c21 = c2;
       to3 = to2, to2 = to, tu2 = tu, vo3 = vo2, vo2 = vo, vu2 = vu;
+      in3 = in2, in2 = in_p;
       o += sjb;
     }
   }
