@@ -929,8 +929,9 @@ struct FaceT {
 __device__ __forceinline__ FaceT ppm_face_t(float f, float c, bool limited) {
   const bool pos = c > 0.f;
   const float n = neg_abs(c);
-  const float t = (limited && f != 0.f) ? f * (1.f + n) : 0.f;
-  const float z = t != 0.f ? n * t : 0.f;  // no infinite or NaN c where nothing passes the face
+  const bool open = limited && f != 0.f;
+  const float t = open ? f * (1.f + n) : 0.f;
+  const float z = open ? n * t : 0.f;  // an infinite or NaN c counts only where something passes the face
   return FaceT{pos ? t : 0.f, pos ? 0.f : t, pos ? z : 0.f, pos ? 0.f : z, pos ? f : 0.f, pos ? 0.f : f};
 }
 
