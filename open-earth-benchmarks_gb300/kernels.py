@@ -164,6 +164,8 @@ def call_profiled(kernel: str, fields: Dict[str, Storage], bases, scalars: Optio
 
 
 def _scalar_args(sig, scalars, precision):
+    if scalars is not None and not isinstance(scalars, dict):
+        scalars = dict(scalars)  # any mapping, or pairs
     out = []
     for name, ctype in sig.scalars[precision]:
         if scalars is not None and name in scalars:

@@ -1,0 +1,42 @@
+"""What a call hands to the library, with the library replaced by a recorder: scalars in every form
+that ``dict.update`` takes."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+H = 3
+
+
+@pytest.fixture
+def calls(pkg, monkeypatch):
+    import importlib
+    kernels = importlib.import_module("oeb_gb300.kernels")
+    seen = []
+    monkeypatch.setattr(kernels, "entry", lambda name: lambda *args: seen.append((name, args)) or 0)
+    monkeypatch.setattr(kernels, "_device_fields", lambda kernel, flat: "f64")
+    monkeypatch.setattr(kernels, "_current_stream", lambda: 0)
+    return seen
+
+
+def _fields(pkg, kernel, names, cls=None):
+    one = {a.name for a in pkg.KERNELS[kernel].args if a.role == "in1"}
+    cls = cls or pkg.Storage
+    return {n: cls(np.zeros((11,) if n in one else (11, 11, 11)), H) for n in names}
+
+
+def _scalars(args):
+    return [a.value for a in args if isinstance(a, (ctypes.c_double, ctypes.c_float))]
+
+
+@pytest.mark.parametrize("form", ["dict", "pairs", "mapping", "none"])
+def test_scalars_in_every_form(pkg, calls, form):
+    from types import MappingProxyType
+    mine = {"p1": 0.25}
+    scalars = {"dict": mine, "pairs": list(mine.items()), "mapping": MappingProxyType(mine), "none": None}[form]
+    names = [a.name for a in pkg.KERNELS["fvtp2d"].abi_args]
+    pkg.call("fvtp2d", _fields(pkg, "fvtp2d", names), scalars, domain=(5, 5, 5))
+    defaults = pkg.DRIVER_SCALARS["fvtp2d"]
+    assert _scalars(calls[0][1]) == [defaults["p1"] if form == "none" else 0.25, defaults["p2"]]
