@@ -66,11 +66,9 @@ class _Signature:
         self.names = tuple(a.name for a in spec.abi_args)
         self.outs = tuple(a.name for a in spec.by_role("out3"))
         self.ins = tuple(a.name for a in spec.args if a.role in ("in3", "in1"))
-        self.active = tuple(ACTIVE[spec.name])
         self.seeds = tuple(spec.semantic_outputs)
         self.scalars = {p: tuple((s.name, ctypes.c_double if (p == "f64" or s.always_double) else ctypes.c_float)
                                  for s in spec.scalars) for p in ("f64", "f32")}
-        self.defaults = dict(DRIVER_SCALARS.get(spec.name, {}))
 
 
 _signatures: Dict[str, _Signature] = {}
@@ -166,12 +164,13 @@ def call_profiled(kernel: str, fields: Dict[str, Storage], bases, scalars: Optio
 def _scalar_args(sig, scalars, precision):
     if scalars is not None and not isinstance(scalars, dict):
         scalars = dict(scalars)  # any mapping, or pairs
+    defaults = DRIVER_SCALARS.get(sig.spec.name, ())
     out = []
     for name, ctype in sig.scalars[precision]:
         if scalars is not None and name in scalars:
             out.append(ctype(scalars[name]))
-        elif name in sig.defaults:
-            out.append(ctype(sig.defaults[name]))
+        elif name in defaults:
+            out.append(ctype(defaults[name]))
         else:
             raise ValueError("%s: missing scalar %r" % (sig.spec.name, name))
     return out
@@ -206,7 +205,7 @@ def tangent_linear(kernel: str, state: Dict[str, Storage], dx: Dict[str, Storage
     dx holds a perturbation of each active input (ACTIVE[kernel]); dy receives the
     perturbation of every output, over the output's written box."""
     sig = _signature(kernel)
-    _device_call("tl", kernel, [dy[n] for n in sig.outs] + [state[n] for n in sig.ins] + [dx[n] for n in sig.active],
+    _device_call("tl", kernel, [dy[n] for n in sig.outs] + [state[n] for n in sig.ins] + [dx[n] for n in ACTIVE[kernel]],
                  scalars, domain, stream)
 
 
@@ -214,7 +213,7 @@ def adjoint(kernel: str, state: Dict[str, Storage], ybar: Dict[str, Storage], xb
             scalars: Optional[Dict[str, float]] = None, domain=None, stream=None) -> None:
     """xbar = J(state)^T ybar for the active inputs; ybar seeds the semantic outputs."""
     sig = _signature(kernel)
-    _device_call("adj", kernel, [xbar[n] for n in sig.active] + [state[n] for n in sig.ins] + [ybar[n] for n in sig.seeds],
+    _device_call("adj", kernel, [xbar[n] for n in ACTIVE[kernel]] + [state[n] for n in sig.ins] + [ybar[n] for n in sig.seeds],
                  scalars, domain, stream)
 
 

@@ -1,5 +1,5 @@
 """What a call hands to the library, with the library replaced by a recorder: scalars in every form
-that ``dict.update`` takes."""
+that ``dict.update`` takes, the tables of defaults and active inputs as they are at the call."""
 from __future__ import annotations
 
 import ctypes
@@ -40,3 +40,21 @@ def test_scalars_in_every_form(pkg, calls, form):
     pkg.call("fvtp2d", _fields(pkg, "fvtp2d", names), scalars, domain=(5, 5, 5))
     defaults = pkg.DRIVER_SCALARS["fvtp2d"]
     assert _scalars(calls[0][1]) == [defaults["p1"] if form == "none" else 0.25, defaults["p2"]]
+
+
+def test_defaults_are_read_at_the_call(pkg, calls, monkeypatch):
+    names = [a.name for a in pkg.KERNELS["fvtp2d"].abi_args]
+    f = _fields(pkg, "fvtp2d", names)
+    pkg.call("fvtp2d", f, domain=(5, 5, 5))
+    monkeypatch.setitem(pkg.DRIVER_SCALARS, "fvtp2d", {"p1": 0.5, "p2": 0.125})
+    pkg.call("fvtp2d", f, domain=(5, 5, 5))
+    assert _scalars(calls[1][1]) == [0.5, 0.125]
+
+
+def test_active_inputs_are_read_at_the_call(pkg, calls, monkeypatch):
+    names = [a.name for a in pkg.KERNELS["laplace"].args]
+    f = _fields(pkg, "laplace", names)
+    pkg.adjoint("laplace", f, f, f, domain=(5, 5, 5))
+    monkeypatch.setitem(pkg.ACTIVE, "laplace", ("out",))
+    with pytest.raises(KeyError):
+        pkg.adjoint("laplace", f, f, {"in": f["in"]}, domain=(5, 5, 5))
