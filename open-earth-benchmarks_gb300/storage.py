@@ -47,6 +47,14 @@ def _is_torch(x) -> bool:
 class Storage:
     """One field: a buffer plus the reference descriptor of it."""
 
+    _packed = (None, None, None)  # what packed() keeps
+
+    def __init_subclass__(cls, **kwargs):
+        super().__init_subclass__(**kwargs)
+        # a subclass that describes itself in its own way is asked each time
+        if "packed" not in cls.__dict__ and (cls.memref is not Storage.memref or cls.data_ptr is not Storage.data_ptr):
+            cls.packed = Storage._packed_anew
+
     def __init__(self, data, halo: int, nx: Optional[int] = None):
         if _is_torch(data):
             if not data.is_contiguous():
@@ -73,7 +81,6 @@ class Storage:
             self.szi = data.shape[0]
             self.pitch = data.shape[0]
         self._memref = None
-        self._packed = (None, None, None)
 
     # -- construction ------------------------------------------------------------------
     @classmethod
@@ -132,6 +139,10 @@ class Storage:
             m = self._describe(ptr)
             self._packed = kept = (key, m, ctypes.byref(m))
         return kept[1], kept[2]
+
+    def _packed_anew(self):
+        m = self.memref()
+        return m, ctypes.byref(m)
 
     # -- views ---------------------------------------------------------------------------
     def box(self, reach=(0, 0, 0, 0, 0, 0), nx=None, ny=None, nz=None):

@@ -1,5 +1,6 @@
 """What a call hands to the library, with the library replaced by a recorder: scalars in every form
-that ``dict.update`` takes, the tables of defaults and active inputs as they are at the call."""
+that ``dict.update`` takes, the tables of defaults and active inputs as they are at the call, and the
+descriptors of a Storage subclass."""
 from __future__ import annotations
 
 import ctypes
@@ -58,3 +59,30 @@ def test_active_inputs_are_read_at_the_call(pkg, calls, monkeypatch):
     monkeypatch.setitem(pkg.ACTIVE, "laplace", ("out",))
     with pytest.raises(KeyError):
         pkg.adjoint("laplace", f, f, {"in": f["in"]}, domain=(5, 5, 5))
+
+
+def test_a_subclass_describes_itself(pkg, calls):
+    class Shifted(pkg.Storage):
+        def memref(self):
+            m = super().memref()
+            m.offset += 1
+            return m
+
+    class Late(pkg.Storage):  # a constructor of its own, and an address of its own
+        def __init__(self, data, halo):
+            self.data, self.halo, self.rank = data, halo, data.ndim
+            self.dtype, self.szi, self.pitch = data.dtype, data.shape[-1], data.shape[-1]
+
+        def data_ptr(self):
+            return super().data_ptr() + 8
+
+    names = [a.name for a in pkg.KERNELS["laplace"].abi_args]
+    plain = _fields(pkg, "laplace", names)
+    for cls in (Shifted, Late):
+        f = {n: cls(s.data, H) for n, s in plain.items()}
+        for _ in range(2):
+            pkg.call("laplace", f, domain=(5, 5, 5))
+            for n, arg in zip(names, calls[-1][1]):
+                m, p = arg._obj, plain[n].memref()
+                assert m.offset == p.offset + (cls is Shifted)
+                assert m.aligned == p.aligned + 8 * (cls is Late)
