@@ -139,6 +139,7 @@ struct fastwavesuv_kernel {
 // 320 x 304 x 137 (five CTAs 48.3 / 17.3 / 114.0, slower on small domains; six, which spills, 75.2);
 // fastwavesuv_kernel<float>'s shared-memory tile took 95.7, 33.5 and 228.8 us.
 struct fastwavesuv_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<float>(kOpFwsFwd);  // the step kernel's id
   static constexpr int kCols = 31, kApron = 1, kMinCtas = 4;
   struct Row {
@@ -353,6 +354,7 @@ constexpr int kAdjJ = 8;  // rows of the transpose's tile: one cell a thread
 // was 72.
 template <class T>
 struct fastwavesuv_adj_kernel {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<T>(kOpFwsAdj);  // the step kernel's id
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ uinb, T* __restrict__ vinb,
                                              T* __restrict__ utensb, T* __restrict__ vtensb, T* __restrict__ ppuvb,
@@ -420,6 +422,7 @@ struct fastwavesuv_adj_kernel {
 // shared-memory march of fastwavesuv_adj_kernel that formed its coefficients itself took 73.0, 161.6
 // and 76.3 us.
 struct fastwavesuv_adj_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<float>(kOpFwsAdjFused);  // the step kernel's id
   static constexpr int R = 1, kCols = 30, kMinCtas = 4;
   // level L: hhl at L + 1 and rho on rows ja - 1 .. ja + R, voutb on ja - 1 .. ja + R - 1, uoutb and

@@ -396,6 +396,7 @@ __device__ __forceinline__ float ppm_row(float p1, float p2, float f, float c) {
 }
 
 struct fvtp2d_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<float>(kOpFvMarch);  // the step kernel's id
   static constexpr int kCols = 26, kApron = 5, kMinCtas = 3;
   // The inputs of iteration s: q on row s + 3, cry and yfx on row s + 1, the rest on s.

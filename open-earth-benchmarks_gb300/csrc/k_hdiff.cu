@@ -64,6 +64,7 @@ struct HdiffsaSmem {
 
 template <class T, int J>
 struct hdiffsa_kernel {
+  static constexpr bool kAnyGrid = true;
   static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> out, InPtr<T> in,
                                              InPtr<T> mask, InPtr<T> crlato,
                                              InPtr<T> crlatu, int64_t s1d, Dims d, int kb) {
@@ -137,6 +138,7 @@ struct hdiffsa_kernel {
 // one row unrolled 26.5 / 58.9; two rows of loads in flight instead of one 26.4 / 59.0); the form
 // before it, a 32 x 32 shared-memory tile marched over the levels, took 37.4 and 94.7 us.
 struct hdiffsa_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kCols = 30, kApron = 3, kMinCtas = 5;
   static __device__ __forceinline__ float limited(float f, float d) {
     constexpr float s = 1.2676506002282294e30f;
@@ -225,6 +227,7 @@ struct HdiffsmagSmem {
 
 template <class T, int J>
 struct hdiffsmag_kernel {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<T>(J == kJ ? kOpSmagFwd : -1);  // the step kernel's id
   static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
                                              InPtr<T> uin, InPtr<T> vin,
@@ -328,6 +331,7 @@ struct hdiffsmag_kernel {
 // and 19.7 at 201 x 173 x 61 (four CTAs 47.6 / 107 / 23.3, six, which spills, 43.7 / 102 / 19.5);
 // hdiffsmag_kernel<float>'s shared-memory tile took 44.2, 103.8 and 24.2 us.
 struct hdiffsmag_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<float>(kOpSmagFwd);  // the step kernel's id
   static constexpr int kCols = 30, kApron = 2, kMinCtas = 5;
   static __device__ __forceinline__ void run(const uint3& blk, float* __restrict__ uout, float* __restrict__ vout,
@@ -547,6 +551,7 @@ struct HdiffsaAdjSmem {
 
 template <class T, int J>
 struct hdiffsa_adj_kernel {
+  static constexpr bool kAnyGrid = true;
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ inb, const T* __restrict__ in,
                                              const T* __restrict__ mask, const T* __restrict__ crlato,
                                              const T* __restrict__ crlatu, int64_t s1d, const T* __restrict__ outb,
@@ -878,6 +883,7 @@ struct hdiffsmag_adj_gather_kernel {
 // 201 x 173 x 61 (four, which spills, 34.9 / 88.8 / 42.8); the 32 x 32 shared-memory tile it replaces took
 // 43.6, 125.7 and 56.3 us.
 struct hdiffsmag_adj_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<float>(kOpSmagAdjFused);  // the step kernel's id
   static constexpr int kCols = 28, kApron = 4, kMinCtas = 3;
   struct Row {

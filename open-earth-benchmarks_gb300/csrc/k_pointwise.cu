@@ -339,6 +339,7 @@ struct hadv_kernel {
 // the selects, measured slower (43.4 us; the arithmetic of a row is then cut into blocks).
 template <int ORDER>
 struct hadv_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kStepOp = step_op<float>(ORDER == 5 ? kOpHadv5Fwd : -1);  // the step kernel's id
   static constexpr int H = ORDER == 5 ? 3 : 2, W = 2 * H + 1;
   static constexpr int kCols = 32, kApron = W - 1, kMinCtas = 4;
@@ -445,6 +446,7 @@ constexpr int kKB = 1;  // k-levels per CTA (one: the most CTAs, which hides FP6
 // 3.1 at 128 x 128 x 80 (eight rows 10.9 / 23.1 / 3.2, marching 13.5 / 32.1 / 3.7; boxes staged by
 // cp.async, the form before, 12.3 / 30.2 / 4.4).
 struct laplace_rows_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kRowsPer = 4;
   static __device__ __forceinline__ void run(const uint3& blk, const float* __restrict__ in, float* __restrict__ out,
                                              Dims d) {
@@ -472,6 +474,7 @@ struct laplace_rows_f32 {
 // an SM (four 45.6 / 104.8 / 15.8, six, which spills, 39.9 / 92.7 / 14.1); p_grad_c_kernel<float>, a
 // point at a time, took 44.5, 106.5 and 15.2 us.
 struct p_grad_c_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kCols = 31, kApron = 1, kMinCtas = 5;
   struct Row {
     float g0, g1, p0, p1, w, u, v, rx, ry;
@@ -522,6 +525,7 @@ struct p_grad_c_march_f32 {
 // takes twenty more register moves a row, 55.8 / 125 / 19.7); the form before it, boxes staged by
 // cp.async and marched over the levels, took 69.7, 194.4 and 21.0 us.
 struct nh_p_grad_march_f32 {
+  static constexpr bool kAnyGrid = true;
   static constexpr int kCols = 31, kApron = 1, kMinCtas = 4;
   struct Row {
     float g0, g1, p0, p1, q0, q1, w;  // row j: gz, pk3, pp at k and k + 1, wk1

@@ -95,6 +95,28 @@ struct ShapeOf<Body, std::void_t<decltype(Body::kShape)>> {
   static constexpr int value = Body::kShape;
 };
 
+// A body that declares kAnyGrid may be launched over more tiles along y or levels along z than the
+// 65535 a grid takes there (its tiles are lower, or its levels fewer, than those of a form whose
+// grids fitted): the CTAs then step through them.
+template <class Body, class = void>
+struct AnyGrid {
+  static constexpr bool value = false;
+};
+template <class Body>
+struct AnyGrid<Body, std::void_t<decltype(Body::kAnyGrid)>> {
+  static constexpr bool value = Body::kAnyGrid;
+};
+constexpr unsigned kMaxGridYZ = 65535;
+
+template <class Body, class... A>
+__global__ void __launch_bounds__(kLaunchTX* kLaunchTY) grid_steps_kernel(dim3 grid, A... a) {
+  for (unsigned z = blockIdx.z; z < grid.z; z += gridDim.z)
+    for (unsigned y = blockIdx.y; y < grid.y; y += gridDim.y) {
+      Body::run(make_uint3(blockIdx.x, y, z), a...);
+      __syncthreads();  // the next tile reuses the shared memory
+    }
+}
+
 // The grid kernel of Body over arguments A...
 template <class Body, class... A>
 constexpr auto grid_entry() {
@@ -407,6 +429,14 @@ oeb_status launch_as(dim3 grid, size_t smem, cudaStream_t st, A... a) {
     }
     r->records.push_back(std::move(rec));
     return OEB_OK;
+  }
+  if constexpr (AnyGrid<Body>::value) {
+    if (grid.y > kMaxGridYZ || grid.z > kMaxGridYZ) {
+      if (smem > 48 * 1024) OEB_TRY(ensure_dyn_smem((const void*)grid_steps_kernel<Body, A...>, (int)smem));
+      const dim3 ctas(grid.x, grid.y < kMaxGridYZ ? grid.y : kMaxGridYZ, grid.z < kMaxGridYZ ? grid.z : kMaxGridYZ);
+      grid_steps_kernel<Body, A...><<<ctas, dim3(kLaunchTX, kLaunchTY), smem, st>>>(grid, a...);
+      return after_launch();
+    }
   }
   if (smem > 48 * 1024) OEB_TRY(ensure_dyn_smem((const void*)grid_entry<Body, A...>(), (int)smem));
   grid_entry<Body, A...>()<<<grid, dim3(kLaunchTX, kLaunchTY), smem, st>>>(a...);
