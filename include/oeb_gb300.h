@@ -170,6 +170,10 @@ OEB_API oeb_status oeb_set_host_async(int enable);
  * integer-pipe result.  Synchronous. */
 OEB_API oeb_status oeb_selftest_fp64(int op, int64_t pairs, uint64_t seed, int mode, uint64_t* mismatches,
                                      uint64_t* first);
+/* A test's hook, for later calls on the calling thread: the rows a warp of the marching FP32 kernels
+ * takes (1..64) and the strips of columns a CTA holds, as a power of two (0..3), instead of the split
+ * they choose from the domain; rows = 0 restores that.  Results do not depend on it. */
+OEB_API oeb_status oeb_selftest_march_shape(int rows, int wx_log);
 /* No counterpart in the reference (a measurement of the GPU the FP64 stencils run on): the FP64
  * pipe's issue rate, as FP64 additions a second over every SM -- eight independent chains of
  * __dadd_rn a thread, eight CTAs of 256 threads an SM, the fastest of three timed launches

@@ -146,9 +146,18 @@ MarchShape find_march_shape(int nx, int ny, int nz, int kb, int cols, int apron,
 }
 }  // namespace
 
+namespace {
+thread_local int t_march_rows = 0, t_march_wx_log = 0;  // oeb_selftest_march_shape
+}
+
 // The search is a function of these sizes alone; a thread keeps the last few it made (a few hundred
 // candidates each, about a microsecond, as long as the launch itself).
 MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm) {
+  if (const int rows = t_march_rows) {
+    const int wl = t_march_wx_log, strips = (nx + cols - 1) / cols, chunks = (ny + rows - 1) / rows;
+    return MarchShape{rows, wl, dim3((unsigned)((strips + (1 << wl) - 1) >> wl),
+                                     (unsigned)((chunks + (kTY >> wl) - 1) / (kTY >> wl)), (unsigned)((nz + kb - 1) / kb))};
+  }
   struct Kept {
     int key[8];
     MarchShape shape;
@@ -525,6 +534,13 @@ extern "C" oeb_status oeb_set_adjoint_tiles(int on) {
 extern "C" oeb_status oeb_set_fusion(int mask) {
   if (mask & ~OEB_FUSE_ALL) return OEB_ERR_ARGUMENT;
   oeb::g_fusion_override.store(mask, std::memory_order_relaxed);
+  return OEB_OK;
+}
+
+extern "C" oeb_status oeb_selftest_march_shape(int rows, int wx_log) {
+  if (rows < 0 || rows > 64 || wx_log < 0 || wx_log > 3) return OEB_ERR_ARGUMENT;
+  oeb::t_march_rows = rows;
+  oeb::t_march_wx_log = wx_log;
   return OEB_OK;
 }
 
