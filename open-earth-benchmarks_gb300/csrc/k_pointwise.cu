@@ -84,24 +84,6 @@ __device__ __forceinline__ void for_points(const uint3& blk, const Dims& d, int 
   for_points_tile<kTI, kTJ, U>(blk, d, kb, f);
 }
 
-// The FP32 nh_p_grad waits on its global loads (ncu: long-scoreboard stalls, DRAM under 30 %
-// busy): the CTA first asks L2 for its tile of every field it reads, at each of its k-levels
-// (`now`) and the level above (`up`, the fields read at k+1) -- 7 % faster at 256 x 256 x 80
-// (the same made p_grad_c 7 % slower; it is not used there).  The FP64 kernels are bound by
-// arithmetic and skip it.
-template <class T, class P, int N, int M>
-__device__ __forceinline__ void prefetch_points(const uint3& blk, const Dims& d, int kb, const P (&now)[N],
-                                                const P (&up)[M]) {
-  if constexpr (std::is_same<T, float>::value) {
-    const int i0 = blk.x * kTI, j0 = blk.y * kTJ, sj = (int)d.sj;
-    const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
-    for (int k = k0; k < k1; ++k) {
-      prefetch_tile<T>(now, (int64_t)k * d.sk, i0, j0, d.nx, d.ny, sj);
-      prefetch_tile<T>(up, (int64_t)(k + 1) * d.sk, i0, j0, d.nx, d.ny, sj);
-    }
-  }
-}
-
 // ---- laplace: kernels/laplace.h:34-43 ----------------------------------------------
 template <class T>
 struct laplace_kernel {
@@ -189,9 +171,6 @@ struct nh_p_grad_kernel {
                                              InPtr<T> pk3, InPtr<T> wk1, T dt, Dims d,
                                              int kb) {
     const int64_t sj = d.sj, sk = d.sk;
-    const InPtr<T> now[8] = {pk3, gz, pp, wk1, uin, vin, rdx, rdy};
-    const InPtr<T> up[3] = {pk3, gz, pp};
-    prefetch_points<T>(blk, d, kb, now, up);
     for_points<HeavyRowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) {
       const T pk0 = ld(pk3 + o), pk1 = ld(pk3 + o + sk);
       const T gz0 = ld(gz + o), gz1 = ld(gz + o + sk);
