@@ -120,14 +120,19 @@ int device_sms() {
 // the first at least half of one.  The split with the least product of the two wins.  Measured for
 // fvtp2d (apron 5, three CTAs an SM): best with 32 rows at 256 x 256 x 80 (89.7 us; 16 rows 93.9,
 // 12 rows 101.7, 8 rows 102.7, 64 rows 113) and with 16 at 128 x 128 x 80 (28.1 us; 8 rows 32.5,
-// 22 rows 31.1, 32 rows 36.6), as the product says.
+// 22 rows 31.1, 32 rows 36.6), as the product says.  Where the fields lie in host memory a CTA holds at
+// least four strips (least_wl 2), whose shared edges its L1 then reads over the link once instead of
+// twice: in place, hdiffsa 41.8 us at 64 x 64 x 60 and 360 at 256 x 256 x 80 (a 16-row tile 43.5 and 395, a
+// 32-row tile 41.2 and 400), hdiffsmag 63.3 and 602 (one strip, or what the product says, 67.6 and 645),
+// fastwavesuv 110 and 1596 (127 and 1849), fvtp2d 141 and 1705 (152 and 1896).
 namespace {
-MarchShape find_march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm, int sms) {
+MarchShape find_march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int ctas_per_sm, int sms,
+                            int least_wl) {
   const double slots = (double)sms * ctas_per_sm;
   const int strips = (nx + cols - 1) / cols, levels = (nz + kb - 1) / kb;
   MarchShape best{};
   double least = 0.0;
-  for (int wl = 0; wl <= 3; ++wl) {
+  for (int wl = least_wl; wl <= 3; ++wl) {
     const int wx = 1 << wl, wy = kTY >> wl;
     for (int rows = 4; rows <= 64; ++rows) {
       const int chunks = (ny + rows - 1) / rows;
@@ -159,19 +164,19 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
                                      (unsigned)((chunks + (kTY >> wl) - 1) / (kTY >> wl)), (unsigned)((nz + kb - 1) / kb))};
   }
   struct Kept {
-    int key[8];
+    int key[9];
     MarchShape shape;
   };
   constexpr int kKept = 16;
   static thread_local Kept kept[kKept] = {};
   static thread_local int next = 0;
-  const int key[8] = {nx, ny, nz, kb, cols, apron, ctas_per_sm, device_sms()};
+  const int key[9] = {nx, ny, nz, kb, cols, apron, ctas_per_sm, device_sms(), fields_in_host_memory() ? 2 : 0};
   for (const Kept& k : kept)
     if (memcmp(k.key, key, sizeof(key)) == 0) return k.shape;
   Kept& k = kept[next];
   next = (next + 1) % kKept;
   memcpy(k.key, key, sizeof(key));
-  k.shape = find_march_shape(nx, ny, nz, kb, cols, apron, ctas_per_sm, key[7]);
+  k.shape = find_march_shape(nx, ny, nz, kb, cols, apron, ctas_per_sm, key[7], key[8]);
   return k.shape;
 }
 

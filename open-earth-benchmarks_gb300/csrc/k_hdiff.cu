@@ -40,9 +40,12 @@ constexpr int kT = 32;  // tile edge
 // A grid of less than a wave of those takes 8 rows, whose CTAs are shorter: 13.0 -> 11.0 and
 // 27.1 -> 21.3 us at 64 x 64 x 60 (16 rows 11.8 and 23.5), 8.1 -> 4.3 and 15.1 -> 6.9 at
 // 33 x 20 x 10; at 128 x 128 x 80 8 rows are slower (44.1 and 89.4).  Recorded launches keep 16 rows,
-// the step kernel's form.
+// the step kernel's form.  Over the host link a tile's apron rows are read again by the next one: there
+// hdiffsa keeps 32 rows (in place at 256 x 256 x 80 625 us, 16 rows 655; 64 x 64 x 60 56.5, 8 rows 58.9), and
+// both take 8 only with fewer 32-row tiles than SMs (hdiffsa 32 x 32 x 10 25.1 us, 32 rows 33.4).
 constexpr int kJ = 16, kJShort = 8;
 inline bool short_tiles(const Dims& d, int kb) {
+  if (fields_in_host_memory()) return under_a_wave(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), 1);
   return !recorder() && under_a_wave(tile_grid(d.nx, d.ny, d.nz, kT, kJ, kb), 6);
 }
 
@@ -431,20 +434,23 @@ oeb_status hdiffsa_entry(const M3* out, const M3* in, const M3* mask, const M1* 
   OEB_TRY(check_no_alias({gout.lo, gout.hi}, {gin.lo, gin.hi, gmask.lo, gmask.hi, lo.lo, lo.hi, lu.lo, lu.hi}));
   OEB_RETURN_IF_VALIDATING();
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gin.sj, gin.sk};
-  if constexpr (std::is_same<T, float>::value) if (!fields_in_host_memory()) {
+  if constexpr (std::is_same<T, float>::value) {
     using B = hdiffsa_march_f32;
     const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
     return launch<B>(m.grid, 0, (cudaStream_t)stream, gout.origin, gin.origin, gmask.origin, lo.origin, lu.origin, lo.s,
                      d, m.rows, m.wx_log);
+  } else {
+    const int kb = tuned_kb(kKB);
+    auto run = [&](auto rows) {
+      constexpr int J = decltype(rows)::value;
+      return launch<hdiffsa_kernel<T, J>>(tile_grid(d.nx, d.ny, d.nz, kT, J, kb), sizeof(HdiffsaSmem<T, J>),
+                                          (cudaStream_t)stream, gout.origin, gin.origin, gmask.origin, lo.origin,
+                                          lu.origin, lo.s, d, kb);
+    };
+    if (short_tiles(d, kb)) return run(std::integral_constant<int, kJShort>());
+    if (fields_in_host_memory()) return run(std::integral_constant<int, kT>());
+    return run(std::integral_constant<int, kJ>());
   }
-  const int kb = tuned_kb(kKB);
-  auto run = [&](auto rows) {
-    constexpr int J = decltype(rows)::value;
-    return launch<hdiffsa_kernel<T, J>>(tile_grid(d.nx, d.ny, d.nz, kT, J, kb), sizeof(HdiffsaSmem<T, J>),
-                                        (cudaStream_t)stream, gout.origin, gin.origin, gmask.origin, lo.origin,
-                                        lu.origin, lo.s, d, kb);
-  };
-  return short_tiles(d, kb) ? run(std::integral_constant<int, kJShort>()) : run(std::integral_constant<int, kJ>());
 }
 
 template <class T, class M3, class M1>

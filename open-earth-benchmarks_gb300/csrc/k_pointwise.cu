@@ -855,26 +855,29 @@ oeb_status hadv_entry(const M3* uout, const M3* vout, const M3* uin, const M3* v
   OEB_TRY(check_no_alias({gu.lo, gu.hi, gv.lo, gv.hi}, {gui.lo, gui.hi, gvi.lo, gvi.hi, a0.lo, a0.hi, a1.lo, a1.hi,
                                                         t0.lo, t0.hi, t1.lo, t1.hi}));
   OEB_RETURN_IF_VALIDATING();
-  if constexpr (std::is_same<T, float>::value) {
-    using B = hadv_march_f32<ORDER>;
-    const Dims d = make_dims(*dom, gu);
-    const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
-    return launch<B>(m.grid, 0, (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin,
-                     a1.origin, t0.origin, t1.origin, a0.s, eddlat, eddlon, d, m.rows, m.wx_log, alpha, update);
-  } else {
-    const int kb = tuned_kb(kKB);
-    auto go = [&](auto body) {
-      using B = decltype(body);
-      constexpr int S = B::kShape;
-      return launch<B>(tile_grid((int)dom->nx, (int)dom->ny, (int)dom->nz, TileOf<S>::I, TileOf<S>::J, kb), 0,
-                       (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin, a1.origin,
-                       t0.origin, t1.origin, a0.s, eddlat, eddlon, make_dims(*dom, gu), kb, alpha, update);
-    };
-    switch (tuned_shape()) {
-      case 1: return go(hadv_kernel<T, ORDER, 1>{});
-      case 2: return go(hadv_kernel<T, ORDER, 2>{});
-      default: return go(hadv_kernel<T, ORDER, 0>{});
+  // Over the host link the march's apron rows cost more than the neighbours the plain kernel reads twice
+  // through L1 (hadvuv5th in place, 64 x 64 x 60: 58.2 us, plain 53.3; 128 x 128 x 80: 169.5 and 158.1),
+  // unless there are fewer plain tiles than SMs (32 x 32 x 10: 28.2, plain 33.9).
+  if constexpr (std::is_same<T, float>::value)
+    if (!fields_in_host_memory() || under_a_wave(grid_for(*dom, 1), 1)) {
+      using B = hadv_march_f32<ORDER>;
+      const Dims d = make_dims(*dom, gu);
+      const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
+      return launch<B>(m.grid, 0, (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin,
+                       a1.origin, t0.origin, t1.origin, a0.s, eddlat, eddlon, d, m.rows, m.wx_log, alpha, update);
     }
+  const int kb = tuned_kb(kKB);
+  auto go = [&](auto body) {
+    using B = decltype(body);
+    constexpr int S = B::kShape;
+    return launch<B>(tile_grid((int)dom->nx, (int)dom->ny, (int)dom->nz, TileOf<S>::I, TileOf<S>::J, kb), 0,
+                     (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin, a1.origin,
+                     t0.origin, t1.origin, a0.s, eddlat, eddlon, make_dims(*dom, gu), kb, alpha, update);
+  };
+  switch (tuned_shape()) {
+    case 1: return go(hadv_kernel<T, ORDER, 1>{});
+    case 2: return go(hadv_kernel<T, ORDER, 2>{});
+    default: return go(hadv_kernel<T, ORDER, 0>{});
   }
 }
 

@@ -44,9 +44,10 @@ struct ValidateOnly {
   } while (0)
 
 // While a HostInPlace guard is alive on this thread, the fields the entry points receive are
-// host memory the device reads in place (the host entry points' direct mode); the FP32 laplace,
-// hdiffsa, p_grad_c and nh_p_grad then keep their plain kernels, which are what that mode was
-// measured and tested with.
+// host memory the device reads in place (the host entry points' direct mode).  What is read twice
+// then crosses the host link twice: the FP32 laplace, p_grad_c and nh_p_grad keep their plain
+// kernels, hadvuv and hadvuv5th above the smallest domains too, FP64 hdiffsa its 32-row tiles, and
+// the marching kernels put strips side by side (march_shape).
 bool fields_in_host_memory();
 struct HostInPlace {
   HostInPlace();
