@@ -119,8 +119,8 @@ OEB_API oeb_status oeb_stream_synchronize(void* stream);
  * tuning knob: results do not depend on it.  Batch plans record and tune their own. */
 OEB_API oeb_status oeb_set_kblock(int kb);
 /* Tile shape of the pointwise advection kernels (FP64 hadvuv, hadvuv5th and the adjoint terms),
- * for every later call on every thread: 0 (the default) 32 x 32 cells a CTA, 1 = 32 x 8,
- * 2 = 64 x 16.  OEB_ERR_ARGUMENT for any other value.  A tuning knob: results do not depend
+ * for every later call on every thread: 0 (the default) 32 x 32 cells a CTA, or 32 x 8 on
+ * domains of few tiles, 1 = 32 x 8, 2 = 64 x 16.  OEB_ERR_ARGUMENT for any other value.  A tuning knob: results do not depend
  * on it.  Batch plans choose their own shapes (oeb_batch_autotune). */
 OEB_API oeb_status oeb_set_tile_shape(int shape);
 /* Fusion groupings of the chained step (no counterpart in the reference, which has no chained

@@ -330,6 +330,7 @@ __device__ __forceinline__ T fastwaves_adj_coef(const FastwavesAdjState<T>& st, 
 
 template <class T>
 struct fastwavesuv_adj_terms_kernel {
+  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 6 : 0;  // (43 registers, five CTAs, 99.6 us a call at 128 x 128 x 80; six 97.8)
   static constexpr int kStepOp = step_op<T>(kOpFwsAdjTerms);  // the step kernel's id
   static __device__ __forceinline__ void run(const uint3& blk, FastwavesAdjTerms<T> tm, FastwavesAdjState<T> st,
                                              const T* __restrict__ uoutb, const T* __restrict__ voutb, T dt, Dims d,
@@ -365,9 +366,8 @@ struct fastwavesuv_adj_kernel {
     // output levels K in [Ks, Ke) of the extended range [-1, nz+1)
     const int Ks = -1 + (int)blk.z * kb, Ke = min(Ks + kb, d.nz + 1);
     const TileCells t(d.nx + 1 - i0, min(d.ny + 1 - j0, kAdjJ));
-#pragma unroll 1
-    for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
-      const int b = t.row(e), i = i0 + (e - b * t.w), j = j0 + b;
+    if (t.r0 < t.rows) {  // a cell a thread
+      const int i = i0 + t.c, j = j0 + t.r0;
       const bool own = i < d.nx && j < d.ny, west = i > 0 && j < d.ny, south = j > 0 && i < d.nx;
       int64_t o = (int64_t)(Ks - 1) * sk + i + j * sj;
       T cm1 = T(0), kbK = T(0), dir = T(0);  // cb(L-1), kb(L-1) = cb(L-2) - cb(L-1), direct terms of level L-1
@@ -592,8 +592,10 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
   OEB_TRY(scratch_alloc(&buf, (size_t)n * 4 * sizeof(T), st));
   T* base = static_cast<T*>(buf);
   const FastwavesAdjTerms<T> tm{base + org, base + n + org, base + 2 * n + org, base + 3 * n + org};
-  oeb_status stt = launch<fastwavesuv_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, kT, 1), 0, st, tm, state,
-                                                           guo.origin, gvo.origin, dt, d, 1);
+  Dims dp = d;
+  dp.tj = point_rows<T>(tile_grid(d.nx, d.ny, d.nz, kT, kT, 1));
+  oeb_status stt = launch<fastwavesuv_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, dp.tj, 1), 0, st, tm, state,
+                                                           guo.origin, gvo.origin, dt, dp, 1);
   // a block of kb levels reads the terms of kb + 2: about one wave of blocks, five CTAs an SM (three
   // 114 us at 128 x 128 x 80 and 322 at 256 x 256 x 80, eight 104 and 329, five 102 and 329)
   const dim3 cells = tile_grid(d.nx + 1, d.ny + 1, 1, kT, kAdjJ, 1);

@@ -1054,15 +1054,17 @@ oeb_status hdiffsmag_adj_entry(const M3* uinb, const M3* vinb, const M3* uin, co
       tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), sizeof(SmagAdjSmem<T>), st, tm, gui.origin, (const T*)vin->aligned + vin->offset,
       (const T*)mask->aligned + mask->offset, org1(crlavo), org1(crlavu), org1(crlato), org1(crlatu), org1(acrlat0), s1d,
       guo.origin, (const T*)voutb->aligned + voutb->offset, eddlat, eddlon, tau_smag, weight_smag, d, kb);
+  Dims dp = d;
+  dp.tj = point_rows<T>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, kT, kb));
   if (stt == OEB_OK)
-    stt = launch<hdiffsmag_adj_ts_kernel<T>>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, kT, kb), 0, st, tm, gui.origin,
+    stt = launch<hdiffsmag_adj_ts_kernel<T>>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, dp.tj, kb), 0, st, tm, gui.origin,
                                              (const T*)vin->aligned + vin->offset, org1(acrlat0), s1d, eddlat, eddlon,
-                                             d, kb);
+                                             dp, kb);
   if (stt == OEB_OK)
     stt = launch<hdiffsmag_adj_gather_kernel<T>>(
-        tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, kT, kb), 0, st, gub.origin, gvb.origin, tm, guo.origin,
+        tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, dp.tj, kb), 0, st, gub.origin, gvb.origin, tm, guo.origin,
         (const T*)voutb->aligned + voutb->offset, org1(crlavo), org1(crlavu), org1(crlato), org1(crlatu), org1(acrlat0),
-        s1d, eddlat, eddlon, d, kb);
+        s1d, eddlat, eddlon, dp, kb);
   scratch_free(buf, st);
   return stt;
 }

@@ -17,6 +17,7 @@
 //
 // One CTA of 32 x 8 threads covers a 32 x 32 (i, j) tile and kb k-levels; each thread
 // computes 4 rows.  Neighbour reads go through L1.
+#include <algorithm>
 #include <type_traits>
 
 #include "march.cuh"
@@ -43,13 +44,13 @@ struct TileOf {
 };
 
 // Visits the points of this thread in a TI x TJ tile: in each 32 columns TJ / 8 rows 8 apart (U
-// of them unrolled; the cells dealt by TileCells where U is 1); f(o, j) with o the in-plane offset of (i, j) plus the plane
-// offset of k.
+// of them unrolled; where U is 1, at most d.tj rows, dealt by TileCells); f(o, j) with o the
+// in-plane offset of (i, j) plus the plane offset of k.
 template <int TI, int TJ, int U, class F>
 __device__ __forceinline__ void for_points_tile(const uint3& blk, const Dims& d, int kb, F&& f) {
   const int k0 = blk.z * kb;
   const int k1 = min(k0 + kb, d.nz);
-  const int sj = (int)d.sj, j0 = (int)blk.y * TJ;
+  const int sj = (int)d.sj, tj = U == 1 ? min(TJ, d.tj) : TJ, j0 = (int)blk.y * tj;
 #pragma unroll 1
   for (int k = k0; k < k1; ++k) {
     const int64_t kofs = (int64_t)k * d.sk;
@@ -57,12 +58,11 @@ __device__ __forceinline__ void for_points_tile(const uint3& blk, const Dims& d,
     for (int c = 0; c < TI / 32; ++c) {
       const int i0 = (int)blk.x * TI + 32 * c;
       if constexpr (U == 1) {
-        const TileCells t(d.nx - i0, min(d.ny - j0, TJ));
-#pragma unroll 1
-        for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
-          const int b = t.row(e), i = i0 + (e - b * t.w), j = j0 + b;
+        const TileCells t(d.nx - i0, min(d.ny - j0, tj));
+        t.each([&](int a, int b) {
+          const int i = i0 + a, j = j0 + b;
           f(kofs + i + j * sj, j);
-        }
+        });
       } else {
         const int i = i0 + (int)threadIdx.x;
         if (i < d.nx) {
@@ -568,6 +568,14 @@ Dims make_dims(const oeb_domain& dom, const Grid<T>& g) {
   return Dims{(int)dom.nx, (int)dom.ny, (int)dom.nz, g.sj, g.sk};
 }
 
+// The same with the rows of a tile for a launch over the interior, kb levels a CTA, and its grid.
+template <class T>
+Dims point_dims(Dims d, int kb) {
+  d.tj = point_rows<T>(tile_grid(d.nx, d.ny, d.nz, kTI, kTJ, kb));
+  return d;
+}
+inline dim3 point_grid(const Dims& d, int kb) { return tile_grid(d.nx, d.ny, d.nz, kTI, d.tj, kb); }
+
 dim3 grid_for(const oeb_domain& dom, int kb) { return tile_grid((int)dom.nx, (int)dom.ny, (int)dom.nz, kTI, kTJ, kb); }
 
 // ------------------------------ entry points -----------------------------------------
@@ -588,8 +596,9 @@ oeb_status laplace_entry(const M3* in, const M3* out, const oeb_domain* dom, voi
                      gout.origin, d);
   }
   const int kb = tuned_kb(kKB);
-  return launch<laplace_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, gin.origin, gout.origin,
-                                   make_dims(*dom, gin), kb);
+  const Dims dp = point_dims<T>(make_dims(*dom, gin), kb);
+  return launch<laplace_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, gin.origin, gout.origin,
+                                   dp, kb);
 }
 
 template <class T, class M3>
@@ -609,8 +618,9 @@ oeb_status uvbke_entry(const M3* ub, const M3* vb, const M3* uc, const M3* vc, c
   OEB_RETURN_IF_VALIDATING();
   const T dt5_hi = T(dt5), dt5_lo = T(dt5 - (double)dt5_hi);  // dt5_lo = 0 for FP64
   const int kb = tuned_kb(kKB);
-  return launch<uvbke_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, gub.origin, gvb.origin, guc.origin,
-                                 gvc.origin, gca.origin, grs.origin, dt5_hi, dt5_lo, make_dims(*dom, gub), kb);
+  const Dims dp = point_dims<T>(make_dims(*dom, gub), kb);
+  return launch<uvbke_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, gub.origin, gvb.origin, guc.origin,
+                                 gvc.origin, gca.origin, grs.origin, dt5_hi, dt5_lo, dp, kb);
 }
 
 // The descriptors' checks of p_grad_c (g: uout, vout, uin, vin, rdxc, rdyc, delpc, gz, pkc).
@@ -644,9 +654,10 @@ oeb_status p_grad_c_entry(const M3* uout, const M3* vout, const M3* uin, const M
                      g[5].origin, g[6].origin, g[7].origin, g[8].origin, dt2, d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
-  return launch<p_grad_c_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
+  const Dims dp = point_dims<T>(make_dims(*dom, g[0]), kb);
+  return launch<p_grad_c_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
                                     g[2].origin, g[3].origin, g[4].origin, g[5].origin, g[6].origin, g[7].origin,
-                                    g[8].origin, dt2, make_dims(*dom, g[0]), kb);
+                                    g[8].origin, dt2, dp, kb);
 }
 
 // The descriptors' checks of nh_p_grad (g: uout, vout, uin, vin, rdx, rdy, gz, pp, pk3, wk1).
@@ -681,9 +692,10 @@ oeb_status nh_p_grad_entry(const M3* uout, const M3* vout, const M3* uin, const 
                      g[5].origin, g[6].origin, g[7].origin, g[8].origin, g[9].origin, dt, d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
-  return launch<nh_p_grad_kernel<T>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
+  const Dims dp = point_dims<T>(make_dims(*dom, g[0]), kb);
+  return launch<nh_p_grad_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
                                      g[2].origin, g[3].origin, g[4].origin, g[5].origin, g[6].origin, g[7].origin,
-                                     g[8].origin, g[9].origin, dt, make_dims(*dom, g[0]), kb);
+                                     g[8].origin, g[9].origin, dt, dp, kb);
 }
 
 // ---- FP32 pressure gradients on profile-relative fields ---------------------------------
@@ -870,9 +882,10 @@ oeb_status hadv_entry(const M3* uout, const M3* vout, const M3* uin, const M3* v
   auto go = [&](auto body) {
     using B = decltype(body);
     constexpr int S = B::kShape;
-    return launch<B>(tile_grid((int)dom->nx, (int)dom->ny, (int)dom->nz, TileOf<S>::I, TileOf<S>::J, kb), 0,
+    const Dims dp = S ? make_dims(*dom, gu) : point_dims<T>(make_dims(*dom, gu), kb);
+    return launch<B>(tile_grid(dp.nx, dp.ny, dp.nz, TileOf<S>::I, std::min(TileOf<S>::J, dp.tj), kb), 0,
                      (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin, a1.origin,
-                     t0.origin, t1.origin, a0.s, eddlat, eddlon, make_dims(*dom, gu), kb, alpha, update);
+                     t0.origin, t1.origin, a0.s, eddlat, eddlon, dp, kb, alpha, update);
   };
   switch (tuned_shape()) {
     case 1: return go(hadv_kernel<T, ORDER, 1>{});
@@ -901,9 +914,9 @@ oeb_status hadv_tl_entry(const M3* duout, const M3* dvout, const M3* uin, const 
   const DualIn<T> a0 = dual_param<T>(acrlat0), a1 = dual_param<T>(acrlat1), t0 = dual_param<T>(tgrlatda0),
                   t1 = dual_param<T>(tgrlatda1);
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  return launch<hadv_kernel<D, ORDER>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, a0, a1, t0, t1,
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb);
+  return launch<hadv_kernel<D, ORDER>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, a0, a1, t0, t1,
                                          acrlat0->strides[0], D(eddlat), D(eddlon), d, kb, D(0), 0);
 }
 
@@ -1276,12 +1289,14 @@ oeb_status hadv_adj_entry(const M3* uinb, const M3* vinb, const M3* uin, const M
   T** fields[9] = {&tm.ax, &tm.ay, &tm.bx, &tm.by, &tm.dd, &tm.gx, &tm.gy, &tm.ex, &tm.ey};
   for (int q = 0; q < 9; ++q) *fields[q] = base + q * n + org;
   tm.fl = reinterpret_cast<unsigned char*>(base + 9 * n) + org;
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gui.sj, gui.sk};
+  Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gui.sj, gui.sk};
   const int kb = tuned_kb(kKB);
+  if (!tuned_shape()) d.tj = point_rows<T>(tile_grid(d.nx + 2 * h, d.ny + 2 * h, d.nz, kTI, kTJ, kb));
   auto terms = [&](auto body) {
     using B = decltype(body);
     constexpr int S = B::kShape;
-    return launch<B>(tile_grid(d.nx, d.ny, d.nz, TileOf<S>::I, TileOf<S>::J, kb), 0, st, tm, gui.origin, gvi.origin,
+    return launch<B>(tile_grid(d.nx, d.ny, d.nz, TileOf<S>::I, std::min(TileOf<S>::J, d.tj), kb), 0, st, tm, gui.origin,
+                     gvi.origin,
                      (const T*)acrlat0->aligned + acrlat0->offset, (const T*)acrlat1->aligned + acrlat1->offset,
                      (const T*)tgrlatda0->aligned + tgrlatda0->offset, (const T*)tgrlatda1->aligned + tgrlatda1->offset,
                      acrlat0->strides[0], guo.origin, gvo.origin, eddlat, eddlon, d, kb);
@@ -1293,7 +1308,7 @@ oeb_status hadv_adj_entry(const M3* uinb, const M3* vinb, const M3* uin, const M
     default: stt = terms(hadv_adj_terms_kernel<T, ORDER, 0>{}); break;
   }
   if (stt == OEB_OK)
-    stt = launch<hadv_adj_gather_kernel<T, ORDER>>(tile_grid(d.nx + 2 * h, d.ny + 2 * h, d.nz, kTI, kTJ, kb), 0, st,
+    stt = launch<hadv_adj_gather_kernel<T, ORDER>>(tile_grid(d.nx + 2 * h, d.ny + 2 * h, d.nz, kTI, d.tj, kb), 0, st,
                                                    gub.origin, gvb.origin, tm, d, kb, update ? guo.origin : nullptr,
                                                    update ? gvo.origin : nullptr, alpha, update);
   scratch_free(buf, st);
@@ -1328,7 +1343,7 @@ struct laplace_adj_kernel {
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ inb, const T* __restrict__ outb,
                                              Dims d, int kb) {
     const int64_t sj = d.sj;
-    for_box_k<RowUnroll<T>::value>(blk, d.sj, d.sk, -1, -1, d.nx + 2, d.ny + 2, d.nz, kb,
+    for_box_k<RowUnroll<T>::value>(blk, d, -1, -1, d.nx + 2, d.ny + 2, d.nz, kb,
                                    [&](int64_t o, int i, int j, int k) {
       T v = inside(d, i, j, k) ? T(-4.0) * ld(outb + o) : T(0);
       if (inside(d, i - 1, j, k)) v = v + ld(outb + o - 1);
@@ -1352,9 +1367,9 @@ oeb_status laplace_tl_entry(const M3* dout, const M3* in, const M3* din, const o
   DualIn<T> x;
   OEB_TRY((dual_in<T>(in, din, &x)));
   const DualOut<T> y = dual_out<T>(dout);
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]};
   const int kb = tuned_kb(kKB);
-  return launch<laplace_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, x, y, d, kb);
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]}, kb);
+  return launch<laplace_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, x, y, d, kb);
 }
 
 template <class T, class M3>
@@ -1370,9 +1385,10 @@ oeb_status laplace_adj_entry(const M3* inb, const M3* in, const M3* outb, const 
   OEB_TRY(check_same_strides<T>({&gib, &gin, &gob}));
   OEB_TRY(check_no_alias({gib.lo, gib.hi}, {gin.lo, gin.hi, gob.lo, gob.hi}));
   OEB_RETURN_IF_VALIDATING();
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gob.sj, gob.sk};
+  Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gob.sj, gob.sk};
   const int kb = tuned_kb(kKB);
-  return launch<laplace_adj_kernel<T>>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kTI, kTJ, kb), 0, (cudaStream_t)stream,
+  d.tj = point_rows<T>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kTI, kTJ, kb));
+  return launch<laplace_adj_kernel<T>>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kTI, d.tj, kb), 0, (cudaStream_t)stream,
                                        gib.origin, gob.origin, d, kb);
 }
 
@@ -1399,7 +1415,7 @@ struct uvbke_adj_kernel {
                                              const T* __restrict__ ubb, const T* __restrict__ vbb, T dt5, Dims d,
                                              int kb) {
     const int64_t sj = d.sj;
-    for_box_k<RowUnroll<T>::value>(blk, d.sj, d.sk, -1, -1, d.nx + 1, d.ny + 1, d.nz, kb,
+    for_box_k<RowUnroll<T>::value>(blk, d, -1, -1, d.nx + 1, d.ny + 1, d.nz, kb,
                                    [&](int64_t o, int i, int j, int k) {
       const bool here = inside(d, i, j, k);
       const T su = here ? uvbke_sub(ubb, vbb, cosa, rsina, o, dt5) : T(0);
@@ -1425,10 +1441,10 @@ oeb_status uvbke_tl_entry(const M3* dub, const M3* dvb, const M3* uc, const M3* 
   OEB_TRY((dual_in<T>(vc, dvc, &v)));
   const DualIn<T> ca = dual_param<T>(cosa), rs = dual_param<T>(rsina);
   const DualOut<T> ou = dual_out<T>(dub), ov = dual_out<T>(dvb);
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uc->strides[1], uc->strides[0]};
-  const T dt5_hi = T(dt5), dt5_lo = T(dt5 - (double)dt5_hi);
   const int kb = tuned_kb(kKB);
-  return launch<uvbke_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, ca, rs, D(dt5_hi),
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uc->strides[1], uc->strides[0]}, kb);
+  const T dt5_hi = T(dt5), dt5_lo = T(dt5 - (double)dt5_hi);
+  return launch<uvbke_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, ca, rs, D(dt5_hi),
                                   D(dt5_lo), d, kb);
 }
 
@@ -1450,9 +1466,10 @@ oeb_status uvbke_adj_entry(const M3* ucb, const M3* vcb, const M3* uc, const M3*
   OEB_TRY(check_no_alias({gucb.lo, gucb.hi, gvcb.lo, gvcb.hi},
                          {gca.lo, gca.hi, grs.lo, grs.hi, gub.lo, gub.hi, gvb.lo, gvb.hi}));
   OEB_RETURN_IF_VALIDATING();
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gub.sj, gub.sk};
+  Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gub.sj, gub.sk};
   const int kb = tuned_kb(kKB);
-  return launch<uvbke_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz, kTI, kTJ, kb), 0, (cudaStream_t)stream,
+  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz, kTI, kTJ, kb));
+  return launch<uvbke_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz, kTI, d.tj, kb), 0, (cudaStream_t)stream,
                                      gucb.origin, gvcb.origin, gca.origin, grs.origin, gub.origin, gvb.origin, T(dt5),
                                      d, kb);
 }
@@ -1504,6 +1521,7 @@ __device__ __forceinline__ void pgc_adj_axis(T* const* t, const T* __restrict__ 
 
 template <class T>
 struct p_grad_c_adj_terms_kernel {
+  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 4 : 0;  // (256 x 256 x 80 275 us; as it likes, three, 280)
   static __device__ __forceinline__ void run(const uint3& blk, PgcTerms<T> tm, T* __restrict__ uinb,
                                              T* __restrict__ vinb, const T* __restrict__ rdxc,
                                              const T* __restrict__ rdyc, const T* __restrict__ delpc,
@@ -1530,7 +1548,7 @@ struct p_grad_c_adj_gather_kernel {
   static __device__ __forceinline__ void run(const uint3& blk, T* __restrict__ delpcb, T* __restrict__ gzb,
                                              T* __restrict__ pkcb, PgcTerms<T> tm, Dims d, int kb) {
     const int64_t sj = d.sj, sk = d.sk;
-    for_box_k<RowUnroll<T>::value>(blk, sj, sk, -1, -1, d.nx + 1, d.ny + 1, d.nz + 1, kb,
+    for_box_k<RowUnroll<T>::value>(blk, d, -1, -1, d.nx + 1, d.ny + 1, d.nz + 1, kb,
                                    [&](int64_t o, int i, int j, int k) {
       T db = T(0), gb = T(0), pb = T(0);
   #pragma unroll
@@ -1693,9 +1711,9 @@ oeb_status p_grad_c_tl_entry(const M3* duout, const M3* dvout, const M3* uin, co
   OEB_TRY((dual_in<T>(pkc, dpkc, &pk)));
   const DualIn<T> rx = dual_param<T>(rdxc), ry = dual_param<T>(rdyc);
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  return launch<p_grad_c_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, dp, g, pk,
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb);
+  return launch<p_grad_c_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, dp, g, pk,
                                      D(dt2), d, kb);
 }
 
@@ -1745,13 +1763,14 @@ oeb_status p_grad_c_adj_entry(const M3* uinb, const M3* vinb, const M3* delpcb, 
   OEB_TRY(scratch_alloc(&buf, (size_t)lay.n * 10 * sizeof(T), st));
   PgcTerms<T> tm;
   for (int q = 0; q < 10; ++q) tm.t[q] = static_cast<T*>(buf) + q * lay.n + lay.org;
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, guo.sj, guo.sk};
+  Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, guo.sj, guo.sk};
   const int kb = tuned_kb(kKB);
-  oeb_status stt = launch<p_grad_c_adj_terms_kernel<T>>(grid_for(*dom, kb), 0, st, tm, gub.origin, gvb.origin,
+  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb));
+  oeb_status stt = launch<p_grad_c_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kTI, d.tj, kb), 0, st, tm, gub.origin, gvb.origin,
                                                         grx.origin, gry.origin, gdp.origin, ggz.origin, gpk.origin,
                                                         guo.origin, gvo.origin, dt2, d, kb);
   if (stt == OEB_OK)
-    stt = launch<p_grad_c_adj_gather_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb), 0, st,
+    stt = launch<p_grad_c_adj_gather_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, d.tj, kb), 0, st,
                                                 gdb.origin, ggb.origin, gpb.origin, tm, d, kb);
   scratch_free(buf, st);
   return stt;
@@ -1844,7 +1863,7 @@ struct nh_p_grad_adj_gather_kernel {
                                              T* __restrict__ pk3b, T* __restrict__ wk1b, NhpTerms<T> tm, Dims d,
                                              int kb) {
     const int64_t sj = d.sj, sk = d.sk;
-    for_box_k<RowUnroll<T>::value>(blk, sj, sk, 0, 0, d.nx + 1, d.ny + 1, d.nz + 1, kb,
+    for_box_k<RowUnroll<T>::value>(blk, d, 0, 0, d.nx + 1, d.ny + 1, d.nz + 1, kb,
                                    [&](int64_t o, int i, int j, int k) {
       T gb = T(0), pb = T(0), kb3 = T(0), wb = T(0);
   #pragma unroll
@@ -2013,9 +2032,9 @@ oeb_status nh_p_grad_tl_entry(const M3* duout, const M3* dvout, const M3* uin, c
   OEB_TRY((dual_in<T>(wk1, dwk1, &w)));
   const DualIn<T> rx = dual_param<T>(rdx), ry = dual_param<T>(rdy);
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]};
   const int kb = tuned_kb(kKB);
-  return launch<nh_p_grad_kernel<D>>(grid_for(*dom, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, g, p, pk, w,
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb);
+  return launch<nh_p_grad_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, g, p, pk, w,
                                       D(dt), d, kb);
 }
 
@@ -2069,13 +2088,14 @@ oeb_status nh_p_grad_adj_entry(const M3* uinb, const M3* vinb, const M3* gzb, co
   OEB_TRY(scratch_alloc(&buf, (size_t)lay.n * 14 * sizeof(T), st));
   NhpTerms<T> tm;
   for (int q = 0; q < 14; ++q) tm.t[q] = static_cast<T*>(buf) + q * lay.n + lay.org;
-  const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, guo.sj, guo.sk};
+  Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, guo.sj, guo.sk};
   const int kb = tuned_kb(kKB);
-  oeb_status stt = launch<nh_p_grad_adj_terms_kernel<T>>(grid_for(*dom, kb), 0, st, tm, gub.origin, gvb.origin,
+  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb));
+  oeb_status stt = launch<nh_p_grad_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kTI, d.tj, kb), 0, st, tm, gub.origin, gvb.origin,
                                                          grx.origin, gry.origin, ggz.origin, gpp.origin, gpk.origin,
                                                          gw1.origin, guo.origin, gvo.origin, dt, d, kb);
   if (stt == OEB_OK)
-    stt = launch<nh_p_grad_adj_gather_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb), 0, st,
+    stt = launch<nh_p_grad_adj_gather_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, d.tj, kb), 0, st,
                                                  ggb.origin, gpb.origin, gkb.origin, gwb.origin, tm, d, kb);
   scratch_free(buf, st);
   return stt;

@@ -68,7 +68,5 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
 // Levels a chunk for a kernel that marches nz levels with `ctas` CTAs a chunk and forms two levels
 // beyond its own.
 int march_levels(int ctas, int nz, int ctas_per_sm);
-// Whether the grid's CTAs, ctas_per_sm at a time on every SM, are fewer than one wave.
-bool under_a_wave(dim3 grid, int ctas_per_sm);
 
 }  // namespace oeb

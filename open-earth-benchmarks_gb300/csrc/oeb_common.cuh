@@ -135,10 +135,12 @@ inline const char* lo_of(const Grid<T>& g) { return g.lo; }
 // Device side
 // ---------------------------------------------------------------------------------------
 
-// Interior extents and the shared strides, passed by value to every kernel.
+// Interior extents and the shared strides, passed by value to every kernel, and the rows of a tile of
+// the FP64 point loops (for_box, for_points).
 struct Dims {
   int nx, ny, nz;
   int64_t sj, sk;
+  int tj = 32;
 };
 
 }  // namespace oeb

@@ -137,42 +137,53 @@ struct HeavyRowUnroll<F64i> {
   static constexpr int value = 1;
 };
 
-// The cells of a tile's part of a box, w <= 32 columns of up to 32 rows, dealt to the CTA's threads in
-// row order: cell e is row(e), column e - row(e) w.  A full tile gives a warp a row.  A tile at the
-// box's far edge, 6 columns wide say, gives a warp several short rows: the boxes of the adjoint kernels
-// are the interior widened by 1 to 6, so that a lane a column left a fifth of the warps of a
-// 128-column interior nearly empty.  The FP64 loops (U == 1 below) visit cells this way: adjoint
-// of hdiffsmag 255 -> 227 us, of hadvuv5th 268 -> 253 at 128 x 128 x 80, hadvuv 142 -> 132 at
-// 201 x 173 x 61.  The FP32 ones keep a lane a column, whose rows lie at compile-time distances:
-// dealt cells made the laplacian's FP32 adjoint 34.4 us instead of 20.5 at 256 x 256 x 80.
+// The cells of a tile's part of a box, up to 32 columns of up to 32 rows, dealt to the CTA's threads: a
+// thread keeps one column and takes every rp-th row of it.  A tile of more than 23 columns gives a warp a
+// row, a narrower one, at the box's far edge, as many short rows as its threads hold (for 24 columns and
+// more that would save no pass over 32 rows).  The boxes of the adjoint kernels are the interior widened
+// by 1 to 6: a lane a column left a fifth of the warps of a 128-column interior nearly empty.  FP64, tiles
+// of 32 rows: adjoint of hadvuv5th 416 -> 390 us at 201 x 173 x 61 and 540 -> 527 at 320 x 320 x 30, hadvuv
+// 143 -> 132 and 176 -> 175, uvbke 34.5 -> 33.0 and 40.7 -> 41.1.  (Cells numbered through a tile and its
+// row found for each by a product took the light kernels 2 to 5 % more than a lane a column where the
+// tiles are full, and 10 % at 120 columns.)  The FP32 loops keep a lane a column, whose rows lie at
+// compile-time distances: dealt cells made the laplacian's FP32 adjoint 34.4 us instead of 20.5 at
+// 256 x 256 x 80.
 struct TileCells {
-  int w, n;
-  unsigned m;  // row(e) = e / w for e < 1024: the error e (1 / w - m / 2^16) is less than 1 / w
-  __device__ __forceinline__ TileCells(int cols, int rows)
-      : w(min(cols, 32)), n(w > 0 ? w * max(0, rows) : 0), m(65536u / (unsigned)max(w, 1) + 1u) {}
-  __device__ __forceinline__ int row(int e) const { return (int)(((unsigned)e * m) >> 16); }
+  int c, r0, rp, rows;  // column, first row, step, end (0 for a thread without cells)
+  __device__ __forceinline__ TileCells(int cols, int nrows) {
+    const int w = cols > 23 ? 32 : max(cols, 1), e = (int)(threadIdx.y * kTX + threadIdx.x);
+    const unsigned m = 65536u / (unsigned)w + 1u;  // e / w = e m >> 16 for e <= 256: e (m / 2^16 - 1 / w) < 1 / w
+    rp = (int)((kThreads * m) >> 16);
+    r0 = (int)(((unsigned)e * m) >> 16);
+    c = e - r0 * w;
+    rows = r0 < rp && c < cols ? nrows : 0;
+  }
+  template <class F>
+  __device__ __forceinline__ void each(F&& f) const {
+#pragma unroll 1
+    for (int r = r0; r < rows; r += rp) f(c, r);
+  }
 };
 
 // Visits, for this thread, the cells (i, j, k) of the box [ilo, ilo+ni) x [jlo, jlo+nj) x
-// [k0, k0+kb) of its CTA: blk.x/y pick a 32 x 32 tile, each thread takes up to 4 cells of a level (U
-// of them unrolled).  f(o, i, j) gets the plane-plus-in-plane offset o of (i, j, k) from the
-// interior origin.
+// [k0, k0+kb) of its CTA: blk.x/y pick a tile of 32 x 32 cells (32 x d.tj where U is 1), of which each
+// thread takes up to 4 a level (U of them unrolled).  f(o, i, j) gets the plane-plus-in-plane offset o
+// of (i, j, k) from the interior origin.
 template <int U = 32 / kTY, class F>
 __device__ __forceinline__ void for_box(const uint3& blk, const Dims& d, int ilo, int jlo, int ni, int nj, int kb,
                                         F&& f) {
   const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
   const int sj = (int)d.sj;
   if constexpr (U == 1) {
-    const int a0 = (int)blk.x * 32, b0 = (int)blk.y * 32;
-    const TileCells t(ni - a0, min(nj - b0, 32));
+    const int a0 = (int)blk.x * 32, b0 = (int)blk.y * d.tj;
+    const TileCells t(ni - a0, min(nj - b0, d.tj));
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
       const int64_t kofs = (int64_t)k * d.sk;
-#pragma unroll 1
-      for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
-        const int r = t.row(e), i = ilo + a0 + (e - r * t.w), b = b0 + r;
-        f(kofs + i + (jlo + b) * sj, i, jlo + b);
-      }
+      t.each([&](int a, int b) {
+        const int i = ilo + a0 + a, j = jlo + b0 + b;
+        f(kofs + i + j * sj, i, j);
+      });
     }
   } else {
     const int a = (int)(blk.x * 32 + threadIdx.x);
@@ -190,23 +201,23 @@ __device__ __forceinline__ void for_box(const uint3& blk, const Dims& d, int ilo
   }
 }
 
-// for_box over the k-levels [k0, k0+kb) of [0, nk) (nk may exceed the interior's nz: the
-// boxes of fields read at k+1), handing f the level as well: f(o, i, j, k).
+// As for_box, over the levels [k0, k0+kb) of [0, nk) (which may extend past the interior's);
+// f(o, i, j, k).
 template <int U = 32 / kTY, class F>
-__device__ __forceinline__ void for_box_k(const uint3& blk, int64_t sj, int64_t sk, int ilo, int jlo, int ni, int nj,
-                                          int nk, int kb, F&& f) {
+__device__ __forceinline__ void for_box_k(const uint3& blk, const Dims& d, int ilo, int jlo, int ni, int nj, int nk,
+                                          int kb, F&& f) {
   const int k0 = blk.z * kb, k1 = min(k0 + kb, nk);
+  const int64_t sj = d.sj;
   if constexpr (U == 1) {
-    const int a0 = (int)blk.x * 32, b0 = (int)blk.y * 32;
-    const TileCells t(ni - a0, min(nj - b0, 32));
+    const int a0 = (int)blk.x * 32, b0 = (int)blk.y * d.tj;
+    const TileCells t(ni - a0, min(nj - b0, d.tj));
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
-      const int64_t kofs = (int64_t)k * sk;
-#pragma unroll 1
-      for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < t.n; e += kThreads) {
-        const int r = t.row(e), i = ilo + a0 + (e - r * t.w), b = b0 + r;
-        f(kofs + i + (int64_t)(jlo + b) * sj, i, jlo + b, k);
-      }
+      const int64_t kofs = (int64_t)k * d.sk;
+      t.each([&](int a, int b) {
+        const int i = ilo + a0 + a, j = jlo + b0 + b;
+        f(kofs + i + j * sj, i, j, k);
+      });
     }
   } else {
     const int a = (int)(blk.x * 32 + threadIdx.x);
@@ -214,7 +225,7 @@ __device__ __forceinline__ void for_box_k(const uint3& blk, int64_t sj, int64_t 
     const int i = ilo + a;
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
-      const int64_t kofs = (int64_t)k * sk;
+      const int64_t kofs = (int64_t)k * d.sk;
 #pragma unroll U
       for (int r = 0; r < 32 / kTY; ++r) {
         const int b = (int)(blk.y * 32 + threadIdx.y) + kTY * r;
@@ -224,8 +235,6 @@ __device__ __forceinline__ void for_box_k(const uint3& blk, int64_t sj, int64_t 
   }
 }
 
-// Grid of a tiled kernel: one CTA per TI x TJ tile of the (i, j) region
-// [ilo, ilo+ni) x [jlo, jlo+nj) and per kb k-levels.
 inline dim3 tile_grid(int ni, int nj, int nz, int ti, int tj, int kb) {
   return dim3((unsigned)((ni + ti - 1) / ti), (unsigned)((nj + tj - 1) / tj), (unsigned)((nz + kb - 1) / kb));
 }
