@@ -14,7 +14,8 @@
 // CTAs walk the items; FP64 members on the caller's stream, FP32 members on a second stream.
 //
 // The autotuner records the step again with other k-blockings (kb: k-levels per tile of the
-// kernels that take one) and times, for every position and precision, each kb in three forms:
+// kernels that take one; 1, 2, 4 and 8, the last also the longer chunks that the fastwavesuv
+// adjoints choose for themselves: tuned_levels) and times, for every position and precision, each kb in three forms:
 // the batched launch as a single persistent wave (occupancy x SMs CTAs), the batched launch
 // with one CTA per tile, and plain per-member launches of the recorded grids (the same tiles,
 // one ordinary launch per member: no item search, arguments in the kernel's parameter space).
@@ -686,6 +687,15 @@ oeb_status create(const oeb_batch_member* in, int count, int modes, oeb_batch_pl
   return OEB_OK;
 }
 
+// Whether two slots of one position launch the same grids over the same arguments (a kernel that takes
+// no kb was recorded alike for each).
+bool same_launches(const Slot& a, const Slot& b) {
+  if (a.fn != b.fn || a.grids.size() != b.grids.size() || a.host_args != b.host_args) return false;
+  for (size_t m = 0; m < a.grids.size(); ++m)
+    if (a.grids[m].x != b.grids[m].x || a.grids[m].y != b.grids[m].y || a.grids[m].z != b.grids[m].z) return false;
+  return true;
+}
+
 oeb_status autotune_slots(oeb_batch_plan* p, cudaStream_t st) {
   const int kbs[] = {1, 2, 4, 8};
   constexpr int kReps = 3;
@@ -717,10 +727,14 @@ oeb_status autotune_slots(oeb_batch_plan* p, cudaStream_t st) {
   oeb_status result = OEB_OK;
   for (size_t i = 0; i < best.size() && result == OEB_OK; ++i) {
     float best_ms = -1.f;
-    for (auto& c : cand) {
-      const Slot& sl = c[i];
-      // a shape other than the default changes nothing for a kernel that takes none
+    for (size_t n = 0; n < cand.size(); ++n) {
+      const Slot& sl = cand[n][i];
+      // a shape other than the default changes nothing for a kernel that takes none, nor does another kb
+      // for one that takes none: each launch is timed once
       if (sl.shape != 0 && sl.shape_tag == 0) continue;
+      bool timed = false;
+      for (size_t q = 0; q < n && !timed; ++q) timed = same_launches(sl, cand[q][i]);
+      if (timed) continue;
       const cudaStream_t s = sl.side ? p->side : st;
       // persistent wave, one CTA per tile (batched launches), then per-member launches
       const int wave = std::min(sl.total, sl.occupancy * p->sms);

@@ -578,7 +578,7 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
     // one launch: the march forms the coefficients at the kb + 2 levels of its k-block
     using B = fastwavesuv_adj_march_f32;
     const int gx = (d.nx + B::kCols) / B::kCols, gy = (d.ny + kTY * B::R) / (kTY * B::R);
-    const int kb = tuned_kb(march_levels(gx * gy, d.nz + 2, B::kMinCtas));
+    const int kb = tuned_levels(march_levels(gx * gy, d.nz + 2, B::kMinCtas));
     return launch<B>(dim3((unsigned)gx, (unsigned)gy, (unsigned)((d.nz + 1 + kb) / kb)), 0, st, gub.origin, gvb.origin,
                      gutb.origin, gvtb.origin, gpb.origin, gw.origin, state, guo.origin, gvo.origin, dt, d, kb);
   }
@@ -599,7 +599,7 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
   // a block of kb levels reads the terms of kb + 2: about one wave of blocks, five CTAs an SM (three
   // 114 us at 128 x 128 x 80 and 322 at 256 x 256 x 80, eight 104 and 329, five 102 and 329)
   const dim3 cells = tile_grid(d.nx + 1, d.ny + 1, 1, kT, kAdjJ, 1);
-  const int kb = tuned_kb(march_levels((int)(cells.x * cells.y), d.nz + 2, 5));
+  const int kb = tuned_levels(march_levels((int)(cells.x * cells.y), d.nz + 2, 5));
   if (stt == OEB_OK)
     stt = launch<fastwavesuv_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 2, kT, kAdjJ, kb),
                                             0, st, gub.origin, gvb.origin, gutb.origin,

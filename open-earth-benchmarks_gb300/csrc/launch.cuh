@@ -264,6 +264,14 @@ inline int tuned_kb(int def) {
   return o > 0 ? o : def;
 }
 
+// The same for a kernel whose own choice may be more levels than the most a batch plan records with:
+// that recording then takes them.
+constexpr int kMostRecordedLevels = 8;
+inline int tuned_levels(int def) {
+  const Recorder* r = recorder();
+  return r && r->kb == kMostRecordedLevels && def > r->kb ? def : tuned_kb(def);
+}
+
 // Tile shapes of the pointwise bodies that take one: 0 = 32 x 32 (the default), 1 = 32 x 8,
 // 2 = 64 x 16 (i x j cells a CTA of 32 x 8 threads covers).
 constexpr int kShapes = 3;
