@@ -353,7 +353,7 @@ inline dim3 flux_grid(const Dims& d, int kb) {
 // instructions a row of 26 columns, 110 of them the arithmetic; DRAM traffic 1.3x the outputs and
 // inputs once).  80 registers, three CTAs an SM: at 256 x 256 x 80 two CTAs (113 registers)
 // measured 106 us, four (64, spilling) 110, three 90; two rows unrolled 91 (83 since the lanes off a
-// field divide 1 by 1, numerator() in march.cuh).  Two levels a warp in
+// field divide 1 by 1, numerator() in precision.cuh).  Two levels a warp in
 // packed FP32 instructions (f32x2) took a quarter fewer instructions but 128 registers: 98 us.
 // The form before it, a 32 x 32 shared-memory tile in nine phases, took 180 us (56 against 25 us
 // at 128 x 128 x 80).
@@ -532,21 +532,21 @@ oeb_status fvtp2d_entry(const M3* q_i, const M3* q_j, const M3* fx1, const M3* f
   OEB_RETURN_IF_VALIDATING();
   const Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gq.sj, gq.sk};
   cudaStream_t st = (cudaStream_t)stream;
-  const int kb = tuned_kb(kKB);
   if constexpr (std::is_same<T, float>::value) {
     using B = fvtp2d_march_f32;
     const MarchShape m = march_shape(d.nx, d.ny, d.nz, 1, B::kCols, B::kApron, B::kMinCtas);
     return launch<B>(m.grid, 0, st, gqi.origin, gqj.origin, gfx1.origin, gfx2.origin, gfy1.origin, gfy2.origin,
                      gq.origin, gcx.origin, gcy.origin, grx.origin, gry.origin, gxf.origin, gyf.origin, gar.origin, p1,
                      p2, d, m.rows, m.wx_log);
+  } else {
+    const int kb = tuned_kb(kKB);
+    OEB_TRY(launch<fvtp2d_q_kernel<T>>(q_grid(d, kb), sizeof(FvQSmem<T>), st, gqi.origin, gqj.origin, gfx2.origin,
+                                       gfy2.origin, gq.origin, gcx.origin, gcy.origin, grx.origin, gry.origin,
+                                       gxf.origin, gyf.origin, gar.origin, p1, p2, d, kb));
+    return launch<fvtp2d_flux_kernel<T>>(flux_grid(d, kb), sizeof(FvFluxSmem<T>), st, gfx1.origin, gfy1.origin,
+                                         gqi.origin, gqj.origin, gfx2.origin, gfy2.origin, gcx.origin, gcy.origin,
+                                         gxf.origin, gyf.origin, p1, p2, d, kb);
   }
-  OEB_TRY(launch<fvtp2d_q_kernel<T>>(q_grid(d, kb), sizeof(FvQSmem<T>), st,
-                                     gqi.origin, gqj.origin, gfx2.origin, gfy2.origin, gq.origin, gcx.origin,
-                                     gcy.origin, grx.origin, gry.origin, gxf.origin, gyf.origin, gar.origin, p1, p2, d,
-                                     kb));
-  return launch<fvtp2d_flux_kernel<T>>(flux_grid(d, kb), sizeof(FvFluxSmem<T>), st,
-                                       gfx1.origin, gfy1.origin, gqi.origin, gqj.origin, gfx2.origin, gfy2.origin,
-                                       gcx.origin, gcy.origin, gxf.origin, gyf.origin, p1, p2, d, kb);
 }
 
 // Tangent-linear fvtp2d with respect to q (the PPM flags frozen at q; the Courant numbers,
@@ -906,7 +906,8 @@ struct fvtp2d_adj_q_kernel {
 
 // ------------------------------ FP32: the adjoint in three marching launches ----------
 // The passes above as warps that march rows (march.cuh), with the same operations on the same
-// operands (a term that is zero is added where the passes skip it):
+// operands (a term that is zero is added where the passes skip it, so that a zero may have the other
+// sign):
 //   A: q_ib.  The y sweep of q gives q_i a row at a time; its row's transposed x sweep follows at
 //      once, the neighbours handed over by the lanes.
 //   B: q_jb.  The x sweep of q gives q_j a row at a time, which feeds the transposed y sweep, its

@@ -43,6 +43,8 @@ constexpr int kT = 32;  // tile edge
 // the step kernel's form.  Over the host link a tile's apron rows are read again by the next one: there
 // hdiffsa keeps 32 rows (in place at 256 x 256 x 80 625 us, 16 rows 655; 64 x 64 x 60 56.5, 8 rows 58.9), and
 // both take 8 only with fewer 32-row tiles than SMs (hdiffsa 32 x 32 x 10 25.1 us, 32 rows 33.4).
+// The tangent-linear forms keep 16: 8 are shorter on the smallest grids (FP64 hdiffsmag 25.9 -> 15.6 us at
+// 32 x 32 x 5) but FP32 is longer from 64 x 64 x 60 on (6.8 -> 7.5 us), and at 100 x 100 x 40 nothing is gained.
 constexpr int kJ = 16, kJShort = 8;
 inline bool short_tiles(const Dims& d, int kb) {
   if (fields_in_host_memory()) return under_a_wave(tile_grid(d.nx, d.ny, d.nz, kT, kT, kb), 1);
@@ -882,7 +884,7 @@ struct hdiffsmag_adj_gather_kernel {
 // j = r - 2.  Neighbouring columns come from the lanes beside it, earlier rows from registers, each
 // value formed once a warp.  Every value is the same expression on the same operands as in the three
 // passes above (a term that is zero is added where they skip it), so the results are theirs, bit for
-// bit, without their 48 bytes a point of term scratch.
+// bit but for the sign of a zero at the box's edge, without their 48 bytes a point of term scratch.
 //
 // What bounds it: instruction issue (about 320 instructions a row, two square roots and two divisions
 // among them).  79 registers, three CTAs an SM: 25.7 us at 128 x 128 x 80, 82.0 at 256 x 256 x 80, 35.4 at

@@ -254,7 +254,8 @@ __device__ __forceinline__ T adv5_axis(P f, int64_t o, int64_t s, T a) {
 // combined by a separate kernel.
 template <class T, int ORDER, int SHAPE = 0>
 struct hadv_kernel {
-  static constexpr int kStepOp = step_op<T>(ORDER == 5 ? kOpHadv5Fwd + SHAPE : -1);  // the step kernel's id
+  // the step kernel's id (FP32: none, hadv_march_f32 has it)
+  static constexpr int kStepOp = step_op<T>(ORDER == 5 && !std::is_same<T, float>::value ? kOpHadv5Fwd + SHAPE : -1);
   static constexpr int kShape = SHAPE;
   static __device__ __forceinline__ void run(const uint3& blk, OutPtr<T> uout, OutPtr<T> vout,
                                              InPtr<T> uin, InPtr<T> vin,
@@ -1079,8 +1080,8 @@ struct hadv_adj_gather_kernel {
 // gather from with the terms pass's expressions (hadv_adj_terms_kernel) -- all nine over the tile and the
 // ring around it, beyond that only those the upwind taps read -- then each cell gathers them as
 // hadv_adj_gather_kernel does: the same operations on the same operands in the same order (a term that
-// is zero is added where the pass skips it), so the same bits.  The 37 bytes a point of term scratch
-// are neither written nor read back.
+// is zero is added where the pass skips it), so the same bits but for the sign of a zero at the box's
+// edge.  The 37 bytes a point of term scratch are neither written nor read back.
 //
 // What bounds it: the warps in flight (two phases of loads, each behind a barrier).  64 registers, four
 // CTAs an SM: hadvuv5th 48.3 us at 128 x 128 x 80 and 151.7 at 256 x 256 x 80, hadvuv 36.4 at

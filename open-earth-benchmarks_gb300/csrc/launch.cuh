@@ -16,7 +16,7 @@
 // double*, and structs or pointers of a template over double) as their F64i twins, which
 // have the same layout.
 //
-// Scratch memory of a call (adjoint terms, dual-number arrays) comes from scratch_alloc: the
+// Scratch memory of a call (adjoint terms, intermediate fields) comes from scratch_alloc: the
 // library's stream-ordered pool normally, the plan's arena while recording (so that it lives
 // as long as the plan).
 #pragma once
@@ -137,7 +137,7 @@ enum StepOpBase : int {
   kOpFwsAdjTerms,
   kOpFwsAdj,       // fastwavesuv_adj_kernel: the march over the terms pass's coefficients
   kOpFwsAdjFused,  // fastwavesuv_adj_march_f32: the FP32 march that forms them itself
-  kOpHadv5Fwd,     // + tile shape (3 shapes)
+  kOpHadv5Fwd,     // + tile shape (3 shapes); FP32: hadv_march_f32 alone, as shape 0
   kOpHadv5AdjTerms = kOpHadv5Fwd + 3,  // + tile shape
   kOpHadv5AdjGather = kOpHadv5AdjTerms + 3,
   kOpSmagFwd,

@@ -113,7 +113,7 @@ __host__ __device__ constexpr T earth_radius_recip() {
   return T(1.0) / T(6371.229e3);
 }
 
-// Rows of a thread's 4 (32 x 32 tile, 8 thread rows) that a kernel unrolls.  The FP64
+// Rows of a thread's 4 (32 x 32 tile, 8 thread rows) that a point loop unrolls.  The FP64
 // kernels' F64i arithmetic is long integer code, and four unrolled copies of a point's work
 // overflow the instruction cache (measured: the advection stencils 16-20 % faster rolled).
 template <class T>
@@ -124,10 +124,9 @@ template <>
 struct RowUnroll<F64i> {
   static constexpr int value = 1;
 };
-// The same for the stencils whose per-point work is longest (advection, pressure gradient):
-// FP32 unrolls two rows (measured at 256 x 256 x 80: hadvuv 89 -> 62 us, hadvuv5th 107 ->
-// 77 us, nh_p_grad 101 -> 94 us against four; the advection times are those of a build with
-// compensated flux sums, since replaced by the plain float sums), FP64 one.
+// The same for the stencils whose per-point work is longest (advection, pressure gradient): two rows
+// in FP32, whose loops run on host memory (on device fields the marching kernels run) and, of dual
+// numbers, as the tangent-linear forms; one in FP64.
 template <class T>
 struct HeavyRowUnroll {
   static constexpr int value = 2;
