@@ -161,7 +161,8 @@ MarchShape march_shape(int nx, int ny, int nz, int kb, int cols, int apron, int 
   if (const int rows = t_march_rows) {
     const int wl = t_march_wx_log, strips = (nx + cols - 1) / cols, chunks = (ny + rows - 1) / rows;
     return MarchShape{rows, wl, dim3((unsigned)((strips + (1 << wl) - 1) >> wl),
-                                     (unsigned)((chunks + (kTY >> wl) - 1) / (kTY >> wl)), (unsigned)((nz + kb - 1) / kb))};
+                                     (unsigned)((chunks + (kTY >> wl) - 1) / (kTY >> wl)),
+                                     (unsigned)((nz + kb - 1) / kb))};
   }
   struct Kept {
     int key[9];

@@ -330,7 +330,8 @@ __device__ __forceinline__ T fastwaves_adj_coef(const FastwavesAdjState<T>& st, 
 
 template <class T>
 struct fastwavesuv_adj_terms_kernel {
-  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 6 : 0;  // (43 registers, five CTAs, 99.6 us a call at 128 x 128 x 80; six 97.8)
+  // six CTAs an SM: 97.8 us a call at 128 x 128 x 80, five (43 registers) 99.6
+  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 6 : 0;
   static constexpr int kStepOp = step_op<T>(kOpFwsAdjTerms);  // the step kernel's id
   static __device__ __forceinline__ void run(const uint3& blk, FastwavesAdjTerms<T> tm, FastwavesAdjState<T> st,
                                              const T* __restrict__ uoutb, const T* __restrict__ voutb, T dt, Dims d,
@@ -593,7 +594,7 @@ oeb_status fastwavesuv_adj_entry(const M3* uinb, const M3* vinb, const M3* utens
   T* base = static_cast<T*>(buf);
   const FastwavesAdjTerms<T> tm{base + org, base + n + org, base + 2 * n + org, base + 3 * n + org};
   Dims dp = d;
-  dp.tj = point_rows<T>(tile_grid(d.nx, d.ny, d.nz, kT, kT, 1));
+  dp.tj = point_rows<T>(tile_grid(d.nx, d.ny, d.nz, kT, kT, 1), kDerivativeTiles);
   oeb_status stt = launch<fastwavesuv_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kT, dp.tj, 1), 0, st, tm, state,
                                                            guo.origin, gvo.origin, dt, dp, 1);
   // a block of kb levels reads the terms of kb + 2: about one wave of blocks, five CTAs an SM (three

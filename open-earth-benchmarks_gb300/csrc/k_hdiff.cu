@@ -1057,7 +1057,7 @@ oeb_status hdiffsmag_adj_entry(const M3* uinb, const M3* vinb, const M3* uin, co
       (const T*)mask->aligned + mask->offset, org1(crlavo), org1(crlavu), org1(crlato), org1(crlatu), org1(acrlat0), s1d,
       guo.origin, (const T*)voutb->aligned + voutb->offset, eddlat, eddlon, tau_smag, weight_smag, d, kb);
   Dims dp = d;
-  dp.tj = point_rows<T>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, kT, kb));
+  dp.tj = point_rows<T>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, kT, kb), kDerivativeTiles);
   if (stt == OEB_OK)
     stt = launch<hdiffsmag_adj_ts_kernel<T>>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kT, dp.tj, kb), 0, st, tm, gui.origin,
                                              (const T*)vin->aligned + vin->offset, org1(acrlat0), s1d, eddlat, eddlon,

@@ -571,8 +571,8 @@ Dims make_dims(const oeb_domain& dom, const Grid<T>& g) {
 
 // The same with the rows of a tile for a launch over the interior, kb levels a CTA, and its grid.
 template <class T>
-Dims point_dims(Dims d, int kb) {
-  d.tj = point_rows<T>(tile_grid(d.nx, d.ny, d.nz, kTI, kTJ, kb));
+Dims point_dims(Dims d, int kb, int tiles) {
+  d.tj = point_rows<T>(tile_grid(d.nx, d.ny, d.nz, kTI, kTJ, kb), tiles);
   return d;
 }
 inline dim3 point_grid(const Dims& d, int kb) { return tile_grid(d.nx, d.ny, d.nz, kTI, d.tj, kb); }
@@ -597,7 +597,7 @@ oeb_status laplace_entry(const M3* in, const M3* out, const oeb_domain* dom, voi
                      gout.origin, d);
   }
   const int kb = tuned_kb(kKB);
-  const Dims dp = point_dims<T>(make_dims(*dom, gin), kb);
+  const Dims dp = point_dims<T>(make_dims(*dom, gin), kb, kForwardTiles);
   return launch<laplace_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, gin.origin, gout.origin,
                                    dp, kb);
 }
@@ -619,7 +619,7 @@ oeb_status uvbke_entry(const M3* ub, const M3* vb, const M3* uc, const M3* vc, c
   OEB_RETURN_IF_VALIDATING();
   const T dt5_hi = T(dt5), dt5_lo = T(dt5 - (double)dt5_hi);  // dt5_lo = 0 for FP64
   const int kb = tuned_kb(kKB);
-  const Dims dp = point_dims<T>(make_dims(*dom, gub), kb);
+  const Dims dp = point_dims<T>(make_dims(*dom, gub), kb, kForwardTiles);
   return launch<uvbke_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, gub.origin, gvb.origin, guc.origin,
                                  gvc.origin, gca.origin, grs.origin, dt5_hi, dt5_lo, dp, kb);
 }
@@ -655,7 +655,7 @@ oeb_status p_grad_c_entry(const M3* uout, const M3* vout, const M3* uin, const M
                      g[5].origin, g[6].origin, g[7].origin, g[8].origin, dt2, d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
-  const Dims dp = point_dims<T>(make_dims(*dom, g[0]), kb);
+  const Dims dp = point_dims<T>(make_dims(*dom, g[0]), kb, kForwardTiles);
   return launch<p_grad_c_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
                                     g[2].origin, g[3].origin, g[4].origin, g[5].origin, g[6].origin, g[7].origin,
                                     g[8].origin, dt2, dp, kb);
@@ -693,7 +693,7 @@ oeb_status nh_p_grad_entry(const M3* uout, const M3* vout, const M3* uin, const 
                      g[5].origin, g[6].origin, g[7].origin, g[8].origin, g[9].origin, dt, d, m.rows, m.wx_log);
   }
   const int kb = tuned_kb(kKB);
-  const Dims dp = point_dims<T>(make_dims(*dom, g[0]), kb);
+  const Dims dp = point_dims<T>(make_dims(*dom, g[0]), kb, kForwardTiles);
   return launch<nh_p_grad_kernel<T>>(point_grid(dp, kb), 0, (cudaStream_t)stream, g[0].origin, g[1].origin,
                                      g[2].origin, g[3].origin, g[4].origin, g[5].origin, g[6].origin, g[7].origin,
                                      g[8].origin, g[9].origin, dt, dp, kb);
@@ -883,7 +883,7 @@ oeb_status hadv_entry(const M3* uout, const M3* vout, const M3* uin, const M3* v
   auto go = [&](auto body) {
     using B = decltype(body);
     constexpr int S = B::kShape;
-    const Dims dp = S ? make_dims(*dom, gu) : point_dims<T>(make_dims(*dom, gu), kb);
+    const Dims dp = S ? make_dims(*dom, gu) : point_dims<T>(make_dims(*dom, gu), kb, kForwardTiles);
     return launch<B>(tile_grid(dp.nx, dp.ny, dp.nz, TileOf<S>::I, std::min(TileOf<S>::J, dp.tj), kb), 0,
                      (cudaStream_t)stream, gu.origin, gv.origin, gui.origin, gvi.origin, a0.origin, a1.origin,
                      t0.origin, t1.origin, a0.s, eddlat, eddlon, dp, kb, alpha, update);
@@ -916,7 +916,8 @@ oeb_status hadv_tl_entry(const M3* duout, const M3* dvout, const M3* uin, const 
                   t1 = dual_param<T>(tgrlatda1);
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const int kb = tuned_kb(kKB);
-  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb);
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb,
+                               kDerivativeTiles);
   return launch<hadv_kernel<D, ORDER>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, a0, a1, t0, t1,
                                          acrlat0->strides[0], D(eddlat), D(eddlon), d, kb, D(0), 0);
 }
@@ -1292,7 +1293,8 @@ oeb_status hadv_adj_entry(const M3* uinb, const M3* vinb, const M3* uin, const M
   tm.fl = reinterpret_cast<unsigned char*>(base + 9 * n) + org;
   Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gui.sj, gui.sk};
   const int kb = tuned_kb(kKB);
-  if (!tuned_shape()) d.tj = point_rows<T>(tile_grid(d.nx + 2 * h, d.ny + 2 * h, d.nz, kTI, kTJ, kb));
+  if (!tuned_shape())
+    d.tj = point_rows<T>(tile_grid(d.nx + 2 * h, d.ny + 2 * h, d.nz, kTI, kTJ, kb), kDerivativeTiles);
   auto terms = [&](auto body) {
     using B = decltype(body);
     constexpr int S = B::kShape;
@@ -1369,7 +1371,7 @@ oeb_status laplace_tl_entry(const M3* dout, const M3* in, const M3* din, const o
   OEB_TRY((dual_in<T>(in, din, &x)));
   const DualOut<T> y = dual_out<T>(dout);
   const int kb = tuned_kb(kKB);
-  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]}, kb);
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, in->strides[1], in->strides[0]}, kb, kDerivativeTiles);
   return launch<laplace_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, x, y, d, kb);
 }
 
@@ -1388,7 +1390,7 @@ oeb_status laplace_adj_entry(const M3* inb, const M3* in, const M3* outb, const 
   OEB_RETURN_IF_VALIDATING();
   Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gob.sj, gob.sk};
   const int kb = tuned_kb(kKB);
-  d.tj = point_rows<T>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kTI, kTJ, kb));
+  d.tj = point_rows<T>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kTI, kTJ, kb), kDerivativeTiles);
   return launch<laplace_adj_kernel<T>>(tile_grid(d.nx + 2, d.ny + 2, d.nz, kTI, d.tj, kb), 0, (cudaStream_t)stream,
                                        gib.origin, gob.origin, d, kb);
 }
@@ -1443,7 +1445,7 @@ oeb_status uvbke_tl_entry(const M3* dub, const M3* dvb, const M3* uc, const M3* 
   const DualIn<T> ca = dual_param<T>(cosa), rs = dual_param<T>(rsina);
   const DualOut<T> ou = dual_out<T>(dub), ov = dual_out<T>(dvb);
   const int kb = tuned_kb(kKB);
-  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uc->strides[1], uc->strides[0]}, kb);
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uc->strides[1], uc->strides[0]}, kb, kDerivativeTiles);
   const T dt5_hi = T(dt5), dt5_lo = T(dt5 - (double)dt5_hi);
   return launch<uvbke_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, ca, rs, D(dt5_hi),
                                   D(dt5_lo), d, kb);
@@ -1469,7 +1471,7 @@ oeb_status uvbke_adj_entry(const M3* ucb, const M3* vcb, const M3* uc, const M3*
   OEB_RETURN_IF_VALIDATING();
   Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, gub.sj, gub.sk};
   const int kb = tuned_kb(kKB);
-  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz, kTI, kTJ, kb));
+  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz, kTI, kTJ, kb), kDerivativeTiles);
   return launch<uvbke_adj_kernel<T>>(tile_grid(d.nx + 1, d.ny + 1, d.nz, kTI, d.tj, kb), 0, (cudaStream_t)stream,
                                      gucb.origin, gvcb.origin, gca.origin, grs.origin, gub.origin, gvb.origin, T(dt5),
                                      d, kb);
@@ -1522,7 +1524,7 @@ __device__ __forceinline__ void pgc_adj_axis(T* const* t, const T* __restrict__ 
 
 template <class T>
 struct p_grad_c_adj_terms_kernel {
-  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 4 : 0;  // (256 x 256 x 80 275 us; as it likes, three, 280)
+  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 4 : 0;  // four CTAs 275 us at 256 x 256 x 80, three 280
   static __device__ __forceinline__ void run(const uint3& blk, PgcTerms<T> tm, T* __restrict__ uinb,
                                              T* __restrict__ vinb, const T* __restrict__ rdxc,
                                              const T* __restrict__ rdyc, const T* __restrict__ delpc,
@@ -1713,7 +1715,8 @@ oeb_status p_grad_c_tl_entry(const M3* duout, const M3* dvout, const M3* uin, co
   const DualIn<T> rx = dual_param<T>(rdxc), ry = dual_param<T>(rdyc);
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const int kb = tuned_kb(kKB);
-  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb);
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb,
+                               kDerivativeTiles);
   return launch<p_grad_c_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, dp, g, pk,
                                      D(dt2), d, kb);
 }
@@ -1766,7 +1769,7 @@ oeb_status p_grad_c_adj_entry(const M3* uinb, const M3* vinb, const M3* delpcb, 
   for (int q = 0; q < 10; ++q) tm.t[q] = static_cast<T*>(buf) + q * lay.n + lay.org;
   Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, guo.sj, guo.sk};
   const int kb = tuned_kb(kKB);
-  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb));
+  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb), kDerivativeTiles);
   oeb_status stt = launch<p_grad_c_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kTI, d.tj, kb), 0, st, tm, gub.origin, gvb.origin,
                                                         grx.origin, gry.origin, gdp.origin, ggz.origin, gpk.origin,
                                                         guo.origin, gvo.origin, dt2, d, kb);
@@ -2034,7 +2037,8 @@ oeb_status nh_p_grad_tl_entry(const M3* duout, const M3* dvout, const M3* uin, c
   const DualIn<T> rx = dual_param<T>(rdx), ry = dual_param<T>(rdy);
   const DualOut<T> ou = dual_out<T>(duout), ov = dual_out<T>(dvout);
   const int kb = tuned_kb(kKB);
-  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb);
+  const Dims d = point_dims<T>(Dims{(int)dom->nx, (int)dom->ny, (int)dom->nz, uin->strides[1], uin->strides[0]}, kb,
+                               kDerivativeTiles);
   return launch<nh_p_grad_kernel<D>>(point_grid(d, kb), 0, (cudaStream_t)stream, ou, ov, u, v, rx, ry, g, p, pk, w,
                                       D(dt), d, kb);
 }
@@ -2091,7 +2095,7 @@ oeb_status nh_p_grad_adj_entry(const M3* uinb, const M3* vinb, const M3* gzb, co
   for (int q = 0; q < 14; ++q) tm.t[q] = static_cast<T*>(buf) + q * lay.n + lay.org;
   Dims d{(int)dom->nx, (int)dom->ny, (int)dom->nz, guo.sj, guo.sk};
   const int kb = tuned_kb(kKB);
-  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb));
+  d.tj = point_rows<T>(tile_grid(d.nx + 1, d.ny + 1, d.nz + 1, kTI, kTJ, kb), kDerivativeTiles);
   oeb_status stt = launch<nh_p_grad_adj_terms_kernel<T>>(tile_grid(d.nx, d.ny, d.nz, kTI, d.tj, kb), 0, st, tm, gub.origin, gvb.origin,
                                                          grx.origin, gry.origin, ggz.origin, gpp.origin, gpk.origin,
                                                          gw1.origin, guo.origin, gvo.origin, dt, d, kb);

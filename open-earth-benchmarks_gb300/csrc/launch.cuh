@@ -296,17 +296,21 @@ inline int tuned_fusion() {
 // Whether the grid's CTAs, ctas_per_sm at a time on every SM, are fewer than one wave.
 bool under_a_wave(dim3 grid, int ctas_per_sm);
 // Rows of a tile of the FP64 point loops (Dims::tj), for a launch whose 32-row tiles would make `grid`: 8, a
-// cell a thread, with fewer than 18 of those an SM.  The arithmetic of a point is one long chain on the
-// FP64 pipe and the integer multiplies, and a launch's end waits for its last CTAs: with four times as
-// many, a quarter as long, small grids fill the SMs and the end is shorter (hadvuv5th 20.4 -> 6.5 us at
-// 32 x 32 x 5, 101 -> 96 at 128 x 128 x 80, its adjoint 36.5 -> 13.1 and 253 -> 239; nh_p_grad's adjoint 37 -> 12
-// and 242 -> 225, 392 -> 371 at 201 x 173 x 61).  From about 20 tiles an SM the ends hardly count and the
-// lighter kernels take longer to start their CTAs (uvbke 41.1 -> 43.3 at 320 x 320 x 30, 66.0 -> 70.8 at
-// 256 x 256 x 80, hadvuv5th 359 -> 371).  Recorded launches keep 32 rows (a batch plan's CTAs search a tile's
-// member), as do fields in host memory, whose neighbouring rows a tile would read over the link again.
+// cell a thread, with fewer than `tiles` of those an SM.  The arithmetic of a point is one long chain on
+// the FP64 pipe and the integer multiplies, and a launch's end waits for its last CTAs: with four times
+// as many, a quarter as long, small grids fill the SMs and the end is shorter (hadvuv5th 20.4 -> 6.5 us at
+// 32 x 32 x 5, 59.4 -> 54.1 at 120 x 90 x 60, its adjoint 36.5 -> 12.3 and, at 128 x 128 x 80, 253 -> 239; there
+// nh_p_grad's adjoint 242 -> 225, 392 -> 371 at 201 x 173 x 61).  From about 20 tiles an SM the ends hardly
+// count and the lighter kernels take longer to start their CTAs (uvbke 41.1 -> 43.3 at 320 x 320 x 30, 66.0
+// -> 70.8 at 256 x 256 x 80, hadvuv5th 359 -> 371).  The forward stencils stop at 8: independent ones run side
+// by side, where another fills a launch's end (ten at once at 128 x 128 x 80: 684 us with 8 rows, 662 with 32;
+// one after another 738 and 765).  Recorded launches keep 32 rows (a batch plan's CTAs search a
+// tile's member), as do fields in host memory, whose neighbouring rows a tile would read over the link
+// again.
+constexpr int kForwardTiles = 8, kDerivativeTiles = 18;
 template <class T>
-int point_rows(dim3 grid) {
-  return std::is_same<T, double>::value && !recorder() && !fields_in_host_memory() && under_a_wave(grid, 18) ? 8 : 32;
+int point_rows(dim3 grid, int tiles) {
+  return std::is_same<T, double>::value && !recorder() && !fields_in_host_memory() && under_a_wave(grid, tiles) ? 8 : 32;
 }
 
 oeb_status scratch_alloc(void** p, size_t bytes, cudaStream_t st);

@@ -162,17 +162,17 @@ def call_profiled(kernel: str, fields: Dict[str, Storage], bases, scalars: Optio
 
 
 def _scalar_args(sig, scalars, precision):
-    if scalars is not None and not isinstance(scalars, dict):
-        scalars = dict(scalars)  # any mapping, or pairs
-    defaults = DRIVER_SCALARS.get(sig.spec.name, ())
+    if scalars.__class__ is not dict:
+        scalars = {} if scalars is None else dict(scalars)  # any mapping, or pairs
     out = []
     for name, ctype in sig.scalars[precision]:
-        if scalars is not None and name in scalars:
+        if name in scalars:
             out.append(ctype(scalars[name]))
-        elif name in defaults:
-            out.append(ctype(defaults[name]))
         else:
-            raise ValueError("%s: missing scalar %r" % (sig.spec.name, name))
+            defaults = DRIVER_SCALARS.get(sig.spec.name, ())
+            if name not in defaults:
+                raise ValueError("%s: missing scalar %r" % (sig.spec.name, name))
+            out.append(ctype(defaults[name]))
     return out
 
 

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 H = 3
 SIZES = [(33, 33), (37, 5), (55, 31), (56, 40), (63, 64)]
 NAMES = ("laplace", "hdiffsmag", "hadvuv", "hadvuv5th", "fastwavesuv", "uvbke", "nh_p_grad", "p_grad_c")
-MANY = 18 * 152  # tiles from which a grid has 32-row ones
+MANY = 18 * 152  # tiles from which every form has 32-row ones (forward from 8 * 152)
 
 
 @pytest.mark.parametrize("size", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
