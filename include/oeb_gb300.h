@@ -120,8 +120,9 @@ OEB_API oeb_status oeb_stream_synchronize(void* stream);
 OEB_API oeb_status oeb_set_kblock(int kb);
 /* Tile shape of the pointwise advection kernels (FP64 hadvuv, hadvuv5th and the adjoint terms),
  * for every later call on every thread: 0 (the default) 32 x 32 cells a CTA, or 32 x 8 on
- * domains of few tiles, 1 = 32 x 8, 2 = 64 x 16.  OEB_ERR_ARGUMENT for any other value.  A tuning knob: results do not depend
- * on it.  Batch plans choose their own shapes (oeb_batch_autotune). */
+ * domains of few tiles, 1 = 32 x 8, 2 = 64 x 16.  OEB_ERR_ARGUMENT for any other value.  A
+ * tuning knob: results do not depend on it.  Batch plans choose their own shapes
+ * (oeb_batch_autotune). */
 OEB_API oeb_status oeb_set_tile_shape(int shape);
 /* Fusion groupings of the chained step (no counterpart in the reference, which has no chained
  * step): a bit mask of stages that run as one kernel in every later oeb_chain_* call.
@@ -853,12 +854,13 @@ OEB_API oeb_status oeb_batch_autotune(oeb_batch_plan* plan, void* stream);
 /* Tuning records (no counterpart in the reference: its drivers take no tuning).  A record
  * keeps the autotuner's choices, so that a later process can apply them to a plan over the
  * same ensemble without timing anything again.  It holds three ints per batched launch, in
- * run order: kb (0 = each kernel's default, or 1, 2, 4, 8), the tile shape (0, 1, 2 as for
+ * run order: kb (0 = each kernel's default, or 1, 2, 4, 8, the last standing for a longer chunk
+ * where a kernel's default is one), the tile shape (0, 1, 2 as for
  * oeb_set_tile_shape; kernels without shapes ignore it) and the launch form (0: one
  * persistent wave, sized on the device it is applied on; 1: one CTA per tile; 2: one
  * ordinary launch per member).
- * oeb_batch_autotune times, for every launch, each kb with each tile shape in each form, and
- *   keeps the fastest.
+ * oeb_batch_autotune times, for every launch, each kb with each tile shape that changes it in
+ *   each form, and keeps the fastest.
  * oeb_batch_tuning_get: *count = the plan's launches; with record != NULL it also writes
  *   3 * count ints there (OEB_ERR_TOO_LARGE if capacity, in launches, is below count).
  * oeb_batch_tuning_apply: OEB_ERR_ARGUMENT if count differs from the plan's launches or a
@@ -868,7 +870,9 @@ OEB_API oeb_status oeb_batch_autotune(oeb_batch_plan* plan, void* stream);
  *   stream capture.
  * oeb_batch_signature: a 64-bit hash of the modes, each member's element size and domain
  *   (in order) and the launch count without fusion.  A record saved with one signature fits
- *   any plan with the same signature, in the same fusion grouping. */
+ *   any plan with the same signature, in the same fusion grouping.  (A library build that
+ *   launches another number of kernels has other signatures; one with as many other kernels
+ *   applies choices timed on the earlier ones.) */
 /* Fusion grouping of a batch plan (OEB_FUSE_* as for oeb_set_fusion): which stages of the
  * chained step each member runs as one kernel.  oeb_batch_autotune tunes the launches of each
  * grouping, times a whole run of each, and keeps the faster grouping with its choices; a

@@ -349,9 +349,9 @@ inline dim3 flux_grid(const Dims& d, int kb) {
 // before the first strip (chunk) and after the last.  The arithmetic is launch 1's and launch
 // 2's on the same operands in the same order: the same bits.
 //
-// What bounds it: instruction issue and the latency of its dependent chains (about 300
-// instructions a row of 26 columns, 110 of them the arithmetic; DRAM traffic 1.3x the outputs and
-// inputs once).  80 registers, three CTAs an SM: at 256 x 256 x 80 two CTAs (113 registers)
+// What bounds it: instruction issue (70 % of the slots taken) and the latency of its dependent chains
+// (about 280 instructions a row of 26 columns, 110 of them the arithmetic; DRAM moves its inputs and
+// outputs once).  80 registers, three CTAs an SM: at 256 x 256 x 80 two CTAs (113 registers)
 // measured 106 us, four (64, spilling) 110, three 90; two rows unrolled 91 (83 since the lanes off a
 // field divide 1 by 1, numerator() in precision.cuh).  Two levels a warp in
 // packed FP32 instructions (f32x2) took a quarter fewer instructions but 128 registers: 98 us.
@@ -916,8 +916,8 @@ struct fvtp2d_adj_q_kernel {
 //      sweep, the transposed y sweep and the area terms meet in one store.
 // q_i, q_j, fx2b, fy2b and the partial qb are never stored: two scratch fields instead of eight.
 //
-// What bounds them: instruction issue (170, 180 and 380 instructions a row for A, B, C; 70 % of the
-// issue slots taken).  Four, four and three CTAs an SM: 78.0 us a call at 128 x 128 x 80 (19 + 23 + 43
+// What bounds them: instruction issue (170, 180 and 380 instructions a row for A, B, C; 63, 67 and 75 % of
+// the issue slots taken at 256 x 256 x 80).  Four, four and three CTAs an SM: 78.0 us a call at 128 x 128 x 80 (19 + 23 + 43
 // with a cold cache), 222 at 256 x 256 x 80, 115 at 201 x 173 x 61 (three CTAs for all 83 / 235 / 113);
 // the passes above, run for float, took 154.8, 521.5 and 229.4 us.  Zero numerators that reached the
 // division's slow path (numerator(), div_zero()) were 12 us of it at 128 x 128 x 80.

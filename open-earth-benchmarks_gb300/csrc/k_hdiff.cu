@@ -137,7 +137,7 @@ struct hdiffsa_kernel {
 // operations on the same operands (the limiter tests on the exact product, its factors scaled by
 // 2^100, so that a nonzero product neither underflows nor loses its sign): the same bits.
 //
-// What bounds it: instruction issue (about 108 instructions a row of 30 columns, 66 % of the issue
+// What bounds it: instruction issue (about 98 instructions a row of 30 columns, 69 % of the issue
 // slots taken) and the ends of a short launch.  48 registers, five CTAs an SM, two rows unrolled:
 // 23.4 us at 256 x 256 x 80 and 50.3 at 320 x 304 x 137 (four CTAs 24.1 / 50.6, six 28.1 / 61.7,
 // one row unrolled 26.5 / 58.9; two rows of loads in flight instead of one 26.4 / 59.0); the form
@@ -331,7 +331,7 @@ struct hdiffsmag_kernel {
 // each row arrives) and forms T^2 at j+1 and S^2 at j, each once; T^2(i+1) and S^2(i-1) come from the
 // lanes beside it.  hdiffsmag_kernel's operations on the same operands in the same order.
 //
-// What bounds it: instruction issue (about 150 instructions a row, two square roots among them) and
+// What bounds it: instruction issue (about 165 instructions a row, two square roots among them; 72 %) and
 // load latency.  48 registers, five CTAs an SM: 39.1 us at 256 x 256 x 80, 89.0 at 320 x 304 x 137
 // and 19.7 at 201 x 173 x 61 (four CTAs 47.6 / 107 / 23.3, six, which spills, 43.7 / 102 / 19.5);
 // hdiffsmag_kernel<float>'s shared-memory tile took 44.2, 103.8 and 24.2 us.
@@ -887,7 +887,7 @@ struct hdiffsmag_adj_gather_kernel {
 // bit but for the sign of a zero at the box's edge, without their 48 bytes a point of term scratch.
 //
 // What bounds it: instruction issue (about 320 instructions a row, two square roots and two divisions
-// among them).  79 registers, three CTAs an SM: 25.7 us at 128 x 128 x 80, 82.0 at 256 x 256 x 80, 35.4 at
+// among them; 86 % of the issue slots taken).  79 registers, three CTAs an SM: 25.7 us at 128 x 128 x 80, 82.0 at 256 x 256 x 80, 35.4 at
 // 201 x 173 x 61 (four, which spills, 34.9 / 88.8 / 42.8); the 32 x 32 shared-memory tile it replaces took
 // 43.6, 125.7 and 56.3 us.
 struct hdiffsmag_adj_f32 {

@@ -310,8 +310,9 @@ struct hadv_kernel {
 // from one address a field, those that the winds wait on a row ahead.  hadv_kernel's operations on
 // the same operands in the same order: the same bits.
 //
-// What bounds it: instruction issue (about 190 instructions a row, 119 of them the arithmetic and
-// its upwind selects; 65-70 % of the issue slots taken) and what its loads leave unhidden.  64
+// What bounds it: instruction issue (about 196 instructions a row, 119 of them the arithmetic and
+// its upwind selects; 72 % of the issue slots taken, 27 % of the load unit's) and what its loads leave
+// unhidden.  64
 // registers, four CTAs an SM, two rows unrolled: hadvuv5th 41.0 us at 256 x 256 x 80 (three CTAs
 // 46.1, one row unrolled 42.7), 98.9 us at 320 x 304 x 137; hadvuv 34.4 us.  hadv_kernel<float>, a
 // point at a time with every neighbour read through L1 (4 of them at selected addresses an axis),
