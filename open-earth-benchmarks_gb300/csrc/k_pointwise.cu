@@ -1523,9 +1523,30 @@ __device__ __forceinline__ void pgc_adj_axis(T* const* t, const T* __restrict__ 
   for (int q = 0; q < 5; ++q) t[q][o] = v[q];
 }
 
+// Visits the points of a 32 x d.tj tile numbered in row order, a thread every 256th; f(o) with o as in
+// for_points_tile.  A thread's next point is then no fixed distance from its last, and the addresses of
+// p_grad_c's twelve outputs and seven reads are formed anew for each instead of carried: the FP64
+// terms pass takes 64 registers instead of 72, 266 us instead of 280 at 256 x 256 x 80 (with its four
+// CTAs forced on the carried form 275).  In the lighter kernels the product a point costs more than that.
+template <class F>
+__device__ __forceinline__ void for_points_numbered(const uint3& blk, const Dims& d, int kb, F&& f) {
+  const int k0 = blk.z * kb, k1 = min(k0 + kb, d.nz);
+  const int sj = (int)d.sj, i0 = (int)blk.x * kTI, j0 = (int)blk.y * d.tj;
+  const int w = min(d.nx - i0, kTI), n = w * min(d.ny - j0, d.tj);
+  const unsigned m = 65536u / (unsigned)w + 1u;  // e / w = e m >> 16 for e < 1024 (TileCells)
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    const int64_t kofs = (int64_t)k * d.sk;
+#pragma unroll 1
+    for (int e = (int)(threadIdx.y * kTX + threadIdx.x); e < n; e += kThreads) {
+      const int b = (int)(((unsigned)e * m) >> 16);
+      f(kofs + (i0 + e - b * w) + (j0 + b) * sj);
+    }
+  }
+}
+
 template <class T>
 struct p_grad_c_adj_terms_kernel {
-  static constexpr int kMinCtas = std::is_same<T, F64i>::value ? 4 : 0;  // four CTAs 275 us at 256 x 256 x 80, three 280
   static __device__ __forceinline__ void run(const uint3& blk, PgcTerms<T> tm, T* __restrict__ uinb,
                                              T* __restrict__ vinb, const T* __restrict__ rdxc,
                                              const T* __restrict__ rdyc, const T* __restrict__ delpc,
@@ -1533,7 +1554,7 @@ struct p_grad_c_adj_terms_kernel {
                                              const T* __restrict__ uoutb, const T* __restrict__ voutb, T dt2, Dims d,
                                              int kb) {
     const int64_t sj = d.sj, sk = d.sk;
-    for_points<RowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) {
+    auto terms = [&](int64_t o) {
       const T gz0 = ld(gz + o), gz1 = ld(gz + o + sk), pk0 = ld(pkc + o), pk1 = ld(pkc + o + sk);
       const T wk = ld(delpc + o);
       const T yu = ld(uoutb + o), yv = ld(voutb + o);
@@ -1541,7 +1562,11 @@ struct p_grad_c_adj_terms_kernel {
       vinb[o] = yv;
       pgc_adj_axis(tm.t, gz, pkc, delpc, o, 1, sk, gz0, gz1, pk0, pk1, wk, dt2 * ld(rdxc + o), yu);
       pgc_adj_axis(tm.t + 5, gz, pkc, delpc, o, sj, sk, gz0, gz1, pk0, pk1, wk, dt2 * ld(rdyc + o), yv);
-    });
+    };
+    if constexpr (std::is_same<T, F64i>::value)
+      for_points_numbered(blk, d, kb, terms);
+    else
+      for_points<RowUnroll<T>::value>(blk, d, kb, [&](int64_t o, int) { terms(o); });
   }
 };
 
